@@ -91,7 +91,7 @@ typedef struct tmps_atoms {
     float* pos32;       /* float[n][4]: offset from cell origin, radius */
     int32_t* cell32;    /* cell coordinate, cx | cy << 10 | cz << 20 */
     float* vel32;       /* float[n][4]: v, mass */
-    float* om32;        /* float[n][4]: omega, v lo x (see the low words below) */
+    float* om32;        /* float[n][4]: omega, omega lo y (see the low words below) */
     float* f32;         /* float[3][n] contact force, mixed form */
     float* torque32;    /* float[3][n] */
     float* o0_32;       /* float[3][n]: offsets at the last build (mixed skin check) */
@@ -99,9 +99,10 @@ typedef struct tmps_atoms {
     /* Low words of the mixed form's double-word state: value = hi + lo with
      * both FP32 (~48-bit significand).  pos32lo = (offset lo, radius lo);
      * the velocity and angular velocity low words are packed so that the
-     * update kernel rewrites no per-build constant beside them: v lo x in
-     * om32's fourth lane, lo32 = (v lo y, v lo z, omega lo x, omega lo y),
-     * wlz32 = omega lo z; inv32 = (1/m, 1/I), read only. */
+     * update kernel finds an unforced atom's velocity in vel32 and lo32 alone
+     * and rewrites no per-build constant: lo32 = (v lo, omega lo x), omega lo
+     * y in om32's fourth lane, wlz32 = omega lo z; inv32 = (1/m, 1/I), read
+     * only. */
     float* pos32lo;
     float* lo32;        /* float[n][4] */
     float* wlz32;       /* float[n] */
@@ -540,6 +541,11 @@ int tmps_batch_c(const tmps_instance* d_inst, const int32_t* d_block_inst, int32
 int tmps_batch_servo(const tmps_instance* d_inst, int32_t ninst, int32_t* d_status, void* stream);
 /* d_state[2 i] = step, d_state[2 i + 1] = aborted of instance i (one copy for the host). */
 int tmps_batch_state(const tmps_instance* d_inst, int32_t ninst, int64_t* d_state, void* stream);
+
+/* Before the first launch A of a run of the FP64 form: A then forms the kinetic
+ * sum of every 32-atom group anew (it keeps the sums of groups whose velocities
+ * its own passes leave unchanged; tmps_fused_bounds drops them too). */
+int tmps_fused_forget_kinetic(int32_t n, void* scratch, void* stream);
 
 /* Applies what the fused step leaves pending -- the second half-kick of the
  * last step and a remap x the servo asked for -- so the state is that of the

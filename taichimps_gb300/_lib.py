@@ -222,6 +222,7 @@ _SIGS = {
     "tmps_selftest_arith": (c_i32, [c_i32, c_vp, c_i32, c_vp, c_vp, c_vp]),
     "tmps_fused_shape": (c_i32, [c_i32, c_i32, c_i32, c_i32, c_i32, ctypes.POINTER(c_i32), ctypes.POINTER(c_i32)]),
     "tmps_fused_scratch_bytes": (ctypes.c_int64, [c_i32, c_i32, c_i32]),
+    "tmps_fused_forget_kinetic": (c_i32, [c_i32, c_vp, c_vp]),
     "tmps_fused_settle": (c_i32, [ctypes.POINTER(Atoms), c_vp, c_vp, c_vp]),
     "tmps_fused_pressure_log": (c_i32, [c_vp, c_vp, c_i32, c_vp]),
     "tmps_batch_blocks": (c_i32, [c_i32, c_i32, c_i32, ctypes.POINTER(c_i32), ctypes.POINTER(c_i32)]),

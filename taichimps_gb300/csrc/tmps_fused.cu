@@ -120,8 +120,9 @@ __device__ __forceinline__ void pdl_enter() {
 
 // Scratch layout of one instance: [flag words, one per 32-atom group + 1]
 // [per-group gaps][per-atom gaps][groups in ascending gap order][their gaps]
-// [sort keys, a power of two of them][virial partials, component-major
-// [6][blocks of A and C]], each region on a 256-byte boundary.
+// [sort keys, a power of two of them][FP64 form: kept kinetic sums, eight
+// doubles per group][virial partials, component-major [6][blocks of A and C]],
+// each region on a 256-byte boundary.
 __host__ __device__ inline size_t lay_round256(size_t b) { return (b + 255) & ~size_t(255); }
 __host__ __device__ inline int lay_groups(int n) { return (n + 31) / 32; }
 __host__ __device__ inline int lay_npad(int n) {
@@ -134,7 +135,8 @@ __host__ __device__ inline size_t lay_agap(int n) { return lay_gap(n) + lay_roun
 __host__ __device__ inline size_t lay_order(int n) { return lay_agap(n) + lay_round256((size_t)n * sizeof(float)); }
 __host__ __device__ inline size_t lay_sgap(int n) { return lay_order(n) + lay_round256((size_t)lay_groups(n) * sizeof(int32_t)); }
 __host__ __device__ inline size_t lay_keys(int n) { return lay_sgap(n) + lay_round256((size_t)lay_groups(n) * sizeof(float)); }
-__host__ __device__ inline size_t lay_part(int n) { return lay_keys(n) + lay_round256((size_t)lay_npad(n) * sizeof(uint64_t)); }
+__host__ __device__ inline size_t lay_kin(int n) { return lay_keys(n) + lay_round256((size_t)lay_npad(n) * sizeof(uint64_t)); }
+__host__ __device__ inline size_t lay_part(int n) { return lay_kin(n) + lay_round256((size_t)lay_groups(n) * 8 * sizeof(double)); }
 
 __device__ __forceinline__ bool rebuild_due(const tmps_engine* __restrict__ e, int64_t s) {
     const int64_t since = s - e->last_build_step;
@@ -160,25 +162,17 @@ __device__ __forceinline__ bool force_live(const uint32_t* __restrict__ flags, i
     return flags == nullptr || ((flags[i >> 5] >> (i & 31)) & 1u);
 }
 
-// A negative zero becomes a positive zero, every other value (NaN included)
-// is kept: the result of adding +0 to it, by integer operations.
-__device__ __forceinline__ double plus_zero(double x) {
-    const long long b = __double_as_longlong(x);
-    return __longlong_as_double(b == (long long)0x8000000000000000ull ? 0ll : b);
-}
-
 // Block sum of the FP64 update's six kinetic components by halving
 // exchanges: the FP64 pipe charges an instruction per warp however few lanes
 // use it, so a shuffle tree per component (30 additions per warp) costs as
 // much as several atoms' updates.  Padded to eight components, each exchange
 // keeps half of what a lane holds (4 + 2 + 1 + 1 + 1 = 9 additions per
 // warp), after which lane l holds component 4 b4 + 2 b3 + b2 (its lane bits
-// 4, 3, 2) of the warp's total.  Lanes 0..5 of warp 0 then add the warp
+// 4, 3, 2: lane >> 2) of the warp's total.  Lanes 0..5 of warp 0 then add the warp
 // totals of their component in warp order and return the block's total; the
 // other threads return 0.  Fixed order: deterministic for a block size.
-__device__ __forceinline__ double block_sum6_halving(const double (&v)[6], double* smem /* [6][kBlockA / 32] */) {
-    constexpr int kW = kBlockA / 32;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+__device__ __forceinline__ double warp_sum6_halving(const double (&v)[6]) {
+    const int lane = threadIdx.x & 31;
     const double a[8] = {v[0], v[1], v[2], v[3], v[4], v[5], 0.0, 0.0};
     const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0, b2 = (lane & 4) != 0;
     double r4[4], r2[2];
@@ -195,8 +189,18 @@ __device__ __forceinline__ double block_sum6_halving(const double (&v)[6], doubl
     double r = (b2 ? r2[1] : r2[0]) + __shfl_xor_sync(0xffffffffu, b2 ? r2[0] : r2[1], 4);
     r += __shfl_xor_sync(0xffffffffu, r, 2);  // both lanes of a pair add the same two values
     r += __shfl_xor_sync(0xffffffffu, r, 1);
-    const int c = (b4 ? 4 : 0) + (b3 ? 2 : 0) + (b2 ? 1 : 0);
-    if ((lane & 3) == 0 && c < 6) smem[c * kW + warp] = r;
+    return r;
+}
+
+// `kept`: lane c < 6 holds a further value of component c; with `any` false
+// (warp-uniform) every v is zero and the exchanges are left out.
+__device__ __forceinline__ double block_sum6_halving(const double (&v)[6], double kept, bool any,
+                                                     double* smem /* [6][kBlockA / 32] */) {
+    constexpr int kW = kBlockA / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double r = 0.0;
+    if (any) r = __shfl_sync(0xffffffffu, warp_sum6_halving(v), (lane << 2) & 31);  // lane c < 6: component c
+    if (lane < 6) smem[lane * kW + warp] = any ? r + kept : kept;
     __syncthreads();
     double t = 0.0;
     if (warp == 0 && lane < 6) {
@@ -216,13 +220,25 @@ __device__ __forceinline__ double block_sum6_halving(const double (&v)[6], doubl
 // An atom whose flag bit is clear holds a force and torque of exact zeros:
 // with 1/m and 1/I positive and finite and dt > 0 (tmps_fused_prepare
 // records any exception in kick_all) its half-kicks v += (dt/2) (f/m) add +0
-// to each component, which changes a negative zero alone, so such an atom
-// takes plus_zero instead of the FP64 kick arithmetic (half of this kernel's
-// FP64 instructions) and its 1/m, 1/I are not read.  The results are the
-// kick's, bit for bit.
+// to each component, which changes a negative zero alone.  Such an atom's
+// velocity and angular velocity are neither kicked nor written, and its
+// angular velocity, force, 1/m and 1/I are not read; a negative zero among
+// them becomes +0 in tmps_fused_settle, whose last half-kick adds the zero
+// kick (until then it enters only products and sums that a zero's sign does
+// not change).  The run's results are the kick's, bit for bit.
+//
+// A group of 32 atoms without a flag also keeps its kinetic sum: while none of
+// its velocities changes, the six numbers of the pass before are read back
+// (kin: eight doubles per group, the seventh 1 when they hold; cleared by
+// tmps_fused_bounds, by a flagged atom and at the start of every run).
+//
+// What bounds it: on a nearly contact-free state the 88 bytes read and 32
+// written per atom (state x, v and the build position; x) and 12 FP64
+// instructions per atom (drift 3, remap 6, displacement 3) -- about even.
 __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __restrict__ b,
                                          tmps_engine* __restrict__ e, const uint32_t* __restrict__ flags,
-                                         double* __restrict__ part, const int bid, const int nblk) {
+                                         double* __restrict__ kin, double* __restrict__ part, const int bid,
+                                         const int nblk) {
     __shared__ double smem[6 * (kBlockA / 32)];
     pdl_enter();
     if (e->aborted || e->step >= e->stop_step) return;
@@ -237,31 +253,65 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
     bool hit = false;
     float dd = 0.0f;
     double K[6] = {0, 0, 0, 0, 0, 0};
+    double kept = 0.0;  // lane c < 6: component c of the kept group sums
+    bool kicked = false;
     const int stride = nblk * blockDim.x;
     for (int b0 = bid * blockDim.x + (threadIdx.x & ~31); b0 < n; b0 += stride) {
         const int i = b0 + lane;
-        if (i >= n) continue;
-        double4 x = ld4(a.xr, i), v = ld4(a.vm, i), w = ld4(a.om, i);
-        // the skin check's reference with the state (not after the stores, which might alias it)
-        const double x0x = __ldcs(a.x0 + i), x0y = __ldcs(a.x0 + n + i), x0z = __ldcs(a.x0 + 2 * n + i);
-        const bool live = force_live(flags, i);
-        if (live || kick_all) {
-            const double im = __ldcs(a.rinv + i), iI = __ldcs(a.rinv + n + i);
-            double f[3] = {0.0, 0.0, 0.0}, t[3] = {0.0, 0.0, 0.0};
-            if (live) {
-                f[0] = __ldcs(a.f + i); f[1] = __ldcs(a.f + n + i); f[2] = __ldcs(a.f + 2 * n + i);
-                t[0] = __ldcs(a.torque + i); t[1] = __ldcs(a.torque + n + i); t[2] = __ldcs(a.torque + 2 * n + i);
-            }
-            if (fin) {  // second half-kick of the previous step
+        const bool mine = i < n;
+        double* const row = kin + 8 * (size_t)(b0 >> 5);
+        const double kr = lane < 8 ? row[lane] : 0.0;
+        double4 x = make_double4(0, 0, 0, 0), v = x;
+        double x0x = 0.0, x0y = 0.0, x0z = 0.0;
+        bool kick = false;
+        if (mine) {
+            x = ld4(a.xr, i);
+            v = ld4(a.vm, i);
+            // the skin check's reference with the state (not after the stores, which might alias it)
+            x0x = __ldcs(a.x0 + i);
+            x0y = __ldcs(a.x0 + n + i);
+            x0z = __ldcs(a.x0 + 2 * n + i);
+            const bool live = force_live(flags, i);
+            kick = live || kick_all;
+            if (kick) {
+                double4 w = ld4(a.om, i);
+                const double im = __ldcs(a.rinv + i), iI = __ldcs(a.rinv + n + i);
+                double f[3] = {0.0, 0.0, 0.0}, t[3] = {0.0, 0.0, 0.0};
+                if (live) {
+                    f[0] = __ldcs(a.f + i); f[1] = __ldcs(a.f + n + i); f[2] = __ldcs(a.f + 2 * n + i);
+                    t[0] = __ldcs(a.torque + i); t[1] = __ldcs(a.torque + n + i); t[2] = __ldcs(a.torque + 2 * n + i);
+                }
+                if (fin) {  // second half-kick of the previous step
+                    v.x += dtf * (f[0] * im); v.y += dtf * (f[1] * im); v.z += dtf * (f[2] * im);
+                    w.x += dtf * (t[0] * iI); w.y += dtf * (t[1] * iI); w.z += dtf * (t[2] * iI);
+                }
                 v.x += dtf * (f[0] * im); v.y += dtf * (f[1] * im); v.z += dtf * (f[2] * im);
                 w.x += dtf * (t[0] * iI); w.y += dtf * (t[1] * iI); w.z += dtf * (t[2] * iI);
+                st4(a.vm, i, v);
+                st4(a.om, i, w);
             }
-            v.x += dtf * (f[0] * im); v.y += dtf * (f[1] * im); v.z += dtf * (f[2] * im);
-            w.x += dtf * (t[0] * iI); w.y += dtf * (t[1] * iI); w.z += dtf * (t[2] * iI);
-        } else {
-            v.x = plus_zero(v.x); v.y = plus_zero(v.y); v.z = plus_zero(v.z);
-            w.x = plus_zero(w.x); w.y = plus_zero(w.y); w.z = plus_zero(w.z);
         }
+        // the kinetic terms: read back where no velocity of the group changed and they are held
+        const bool moved = __any_sync(0xffffffffu, kick);
+        const bool held = !moved && __shfl_sync(0xffffffffu, kr, 6) == 1.0;
+        if (held) {
+            kept += kr;  // (lanes 6 and 7 sum nothing that is used)
+        } else {
+            const double k6[6] = {(v.w * v.x) * v.x, (v.w * v.y) * v.y, (v.w * v.z) * v.z,
+                                  (v.w * v.x) * v.y, (v.w * v.x) * v.z, (v.w * v.y) * v.z};
+            if (moved) {
+                kicked = true;
+#pragma unroll
+                for (int c = 0; c < 6; ++c) K[c] += k6[c];
+                if (lane == 6) row[6] = 0.0;
+            } else {
+                const double t = warp_sum6_halving(k6);
+                const double mine6 = __shfl_sync(0xffffffffu, t, (lane << 2) & 31);
+                if (lane < 7) row[lane] = lane < 6 ? mine6 : 1.0;
+                kept += mine6;
+            }
+        }
+        if (!mine) continue;
         if (remap) {  // remap x of the previous step's servo update
             x.x = b->lo[0] + (x.x - b->old_lo[0]) * e->remap_scale[0];
             x.y = b->lo[1] + (x.y - b->old_lo[1]) * e->remap_scale[1];
@@ -269,8 +319,6 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
         }
         x.x = x.x + dt * v.x; x.y = x.y + dt * v.y; x.z = x.z + dt * v.z;
         st4(a.xr, i, x);
-        st4(a.vm, i, v);
-        st4(a.om, i, w);
         const double d0 = __dsub_rn(x.x, x0x), d1 = __dsub_rn(x.y, x0y), d2 = __dsub_rn(x.z, x0z);
         // |d|^2 first in FP32 from the truncated differences (integer operations;
         // relative error under 1e-5): the exact FP64 test decides only within
@@ -290,21 +338,17 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
         hit = hit || far;
         // the running maximum only has to bound |d|^2 from above (C's cull threshold)
         dd = q32 == q32 ? fmaxf(dd, q32 * 1.00002f + 1e-30f) : __int_as_float(0x7fffffff);
-        const double kin[6] = {(v.w * v.x) * v.x, (v.w * v.y) * v.y, (v.w * v.z) * v.z,
-                               (v.w * v.x) * v.y, (v.w * v.x) * v.z, (v.w * v.y) * v.z};
-#pragma unroll
-        for (int c = 0; c < 6; ++c) K[c] += kin[c];
     }
     if (__any_sync(0xffffffffu, hit) && lane == 0) e->disp_stamp = s;
     note_displacement(e, dd);
-    const double tot = block_sum6_halving(K, smem);
+    const double tot = block_sum6_halving(K, kept, kicked, smem);
     if (threadIdx.x < 6) part[(size_t)threadIdx.x * nb + bid] = tot;
 }
 
 __global__ void __launch_bounds__(kBlockA) k_a64(tmps_atoms a, const tmps_box* __restrict__ b,
                                                   tmps_engine* __restrict__ e, const uint32_t* __restrict__ flags,
-                                                  double* __restrict__ part) {
-    a64_body(a, b, e, flags, part, blockIdx.x, gridDim.x);
+                                                  double* __restrict__ kin, double* __restrict__ part) {
+    a64_body(a, b, e, flags, kin, part, blockIdx.x, gridDim.x);
 }
 
 // ------------------------------------------------------------------ A, mixed
@@ -315,44 +359,25 @@ __device__ __forceinline__ int cell_z(int32_t c) { return (c >> 20) & 1023; }
 
 // The mixed form's velocity and angular velocity words of atom i as four
 // float4: v = (v hi, m), vl = (v lo, 1/m), w = (omega hi, -), wl = (omega lo,
-// 1/I).  In memory the low words are packed so that no per-build constant is
-// rewritten with them: om32 = (omega hi, v lo x), lo32 = (v lo y, v lo z,
-// omega lo x, omega lo y), wlz32 = omega lo z, inv32 = (1/m, 1/I) (read only).
-// CS: the low words with streaming (evict-first) hints; INV: also 1/m and 1/I
-// (else vl.w and wl.w are left 0).
-template <bool CS, bool INV = true>
+// 1/I).  In memory the low words are packed so that what an atom without a
+// force needs -- v hi, v lo -- lies in two records, and no per-build constant
+// is rewritten: vel32 = (v hi, m), lo32 = (v lo, omega lo x), om32 = (omega hi,
+// omega lo y), wlz32 = omega lo z, inv32 = (1/m, 1/I) (read only).
 __device__ __forceinline__ void load_vw(const tmps_atoms& a, int i, float4& v, float4& vl, float4& w, float4& wl) {
     v = ld4f(a.vel32, i);
-    const float4 o = ld4f(a.om32, i);
-    float4 q;
-    float wz;
-    float2 inv = make_float2(0.0f, 0.0f);
-    if constexpr (CS) {
-        q = __ldcs(reinterpret_cast<const float4*>(a.lo32) + i);
-        wz = __ldcs(a.wlz32 + i);
-        if constexpr (INV) inv = __ldcs(reinterpret_cast<const float2*>(a.inv32) + i);
-    } else {
-        q = ld4f(a.lo32, i);
-        wz = a.wlz32[i];
-        if constexpr (INV) inv = reinterpret_cast<const float2*>(a.inv32)[i];
-    }
+    const float4 o = ld4f(a.om32, i), q = ld4f(a.lo32, i);
+    const float wz = a.wlz32[i];
+    const float2 inv = reinterpret_cast<const float2*>(a.inv32)[i];
     w = make_float4(o.x, o.y, o.z, 0.0f);
-    vl = make_float4(o.w, q.x, q.y, inv.x);
-    wl = make_float4(q.z, q.w, wz, inv.y);
+    vl = make_float4(q.x, q.y, q.z, inv.x);
+    wl = make_float4(q.w, o.w, wz, inv.y);
 }
 
-template <bool CS>
 __device__ __forceinline__ void store_vw(const tmps_atoms& a, int i, float4 v, float4 vl, float4 w, float4 wl) {
     st4f(a.vel32, i, v);
-    st4f(a.om32, i, make_float4(w.x, w.y, w.z, vl.x));
-    const float4 q = make_float4(vl.y, vl.z, wl.x, wl.y);
-    if constexpr (CS) {
-        __stcs(reinterpret_cast<float4*>(a.lo32) + i, q);
-        __stcs(a.wlz32 + i, wl.z);
-    } else {
-        reinterpret_cast<float4*>(a.lo32)[i] = q;
-        a.wlz32[i] = wl.z;
-    }
+    st4f(a.om32, i, make_float4(w.x, w.y, w.z, wl.y));
+    st4f(a.lo32, i, make_float4(vl.x, vl.y, vl.z, wl.x));
+    a.wlz32[i] = wl.z;
 }
 
 // Streaming (evict-first) loads and stores for the per-atom words only A
@@ -388,21 +413,28 @@ __device__ __forceinline__ void a32_body(const tmps_atoms& a, const tmps_box* __
         const int i = b0 + lane;
         if (i >= n) continue;
         float4 p = ld4f(a.pos32, i), pl = ld4f_cs(a.pos32lo, i);
-        float4 v, vl, w, wl;
-        load_vw<true, false>(a, i, v, vl, w, wl);
+        float4 v = ld4f(a.vel32, i), q4 = ld4f_cs(a.lo32, i);  // q4 = (v lo, omega lo x)
         // the skin check's words with the state's, in the same round trip (the stores below could
         // alias them as far as the compiler knows, so it would not hoist these loads above them)
         const int32_t c = __ldcs(a.cell32 + i);
         const float o0x = __ldcs(a.o0_32 + i), o0y = __ldcs(a.o0_32 + n + i), o0z = __ldcs(a.o0_32 + 2 * n + i);
-        if (force_live(flags, i)) {  // an unflagged atom's force is an exact zero: nothing to add
+        // an unflagged atom's force is an exact zero: nothing to add, and its velocity and angular
+        // velocity stay in memory as they are (the angular velocity is not even read)
+        if (force_live(flags, i)) {
             const float2 inv = __ldcs(reinterpret_cast<const float2*>(a.inv32) + i);  // 1/m, 1/I
+            float4 w = ld4f(a.om32, i);  // (omega hi, omega lo y)
+            float wz = a.wlz32[i];
             const float km = kick * inv.x, kI = kick * inv.y;
-            dw_add(v.x, vl.x, km * __ldcs(a.f32 + i));
-            dw_add(v.y, vl.y, km * __ldcs(a.f32 + n + i));
-            dw_add(v.z, vl.z, km * __ldcs(a.f32 + 2 * n + i));
-            dw_add(w.x, wl.x, kI * __ldcs(a.torque32 + i));
-            dw_add(w.y, wl.y, kI * __ldcs(a.torque32 + n + i));
-            dw_add(w.z, wl.z, kI * __ldcs(a.torque32 + 2 * n + i));
+            dw_add(v.x, q4.x, km * __ldcs(a.f32 + i));
+            dw_add(v.y, q4.y, km * __ldcs(a.f32 + n + i));
+            dw_add(v.z, q4.z, km * __ldcs(a.f32 + 2 * n + i));
+            dw_add(w.x, q4.w, kI * __ldcs(a.torque32 + i));
+            dw_add(w.y, w.w, kI * __ldcs(a.torque32 + n + i));
+            dw_add(w.z, wz, kI * __ldcs(a.torque32 + 2 * n + i));
+            st4f(a.vel32, i, v);
+            st4f_cs(a.lo32, i, q4);
+            st4f(a.om32, i, w);
+            a.wlz32[i] = wz;
         }
         if (remap) {
             // remap x scales a cell-relative offset with the box: o += o * eps
@@ -411,12 +443,11 @@ __device__ __forceinline__ void a32_body(const tmps_atoms& a, const tmps_box* __
             dw_add(p.z, pl.z, p.z * e->eps_hi[2] + (p.z * e->eps_lo[2] + pl.z * e->eps_hi[2]));
         }
         // drift o += dt * v in double words
-        dw_add_prod(p.x, pl.x, dth, dtl, v.x, vl.x);
-        dw_add_prod(p.y, pl.y, dth, dtl, v.y, vl.y);
-        dw_add_prod(p.z, pl.z, dth, dtl, v.z, vl.z);
+        dw_add_prod(p.x, pl.x, dth, dtl, v.x, q4.x);
+        dw_add_prod(p.y, pl.y, dth, dtl, v.y, q4.y);
+        dw_add_prod(p.z, pl.z, dth, dtl, v.z, q4.z);
         st4f(a.pos32, i, p);
         st4f_cs(a.pos32lo, i, pl);
-        store_vw<true>(a, i, v, vl, w, wl);
         // displacement since the build: offset change + cell origin change
         const float d0 = ((p.x - o0x) + pl.x) + (float)cell_x(c) * e->dh32[0] + e->dlo32[0];
         const float d1 = ((p.y - o0y) + pl.y) + (float)cell_y(c) * e->dh32[1] + e->dlo32[1];
@@ -489,7 +520,7 @@ __device__ __forceinline__ void zero_force(const tmps_atoms& A, int i) {
 // its force may be nonzero.
 __global__ void __launch_bounds__(kBlockA) k_bounds(tmps_atoms A, tmps_nlist L, const tmps_box* __restrict__ B,
                                                      tmps_engine* __restrict__ E, int hist, int cull, uint32_t* flags,
-                                                     float* gap, float* agap) {
+                                                     float* gap, float* agap, double* __restrict__ kin) {
     const int n = A.n;
     const int lane = threadIdx.x & 31;
     const int ngroups = (n + 31) >> 5;
@@ -555,6 +586,7 @@ __global__ void __launch_bounds__(kBlockA) k_bounds(tmps_atoms A, tmps_nlist L, 
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) gmin = fminf(gmin, __shfl_down_sync(0xffffffffu, gmin, o));
         if (lane == 0) {
+            kin[8 * (size_t)g + 6] = 0.0;  // no kept kinetic sum (a64_body)
             gap[g] = gmin;
             // bits of existing atoms only: a set bit makes C clear that atom's force
             const int rem = n - (g << 5);
@@ -2009,7 +2041,8 @@ __global__ void __launch_bounds__(kBlockA) kb_a64(const tmps_instance* __restric
     __shared__ tmps_instance si;
     const tmps_instance& I = stage_instance(si, inst, block_inst[blockIdx.x]);
     char* sc = static_cast<char*>(I.scratch);
-    a64_body(I.a, I.box, I.eng, reinterpret_cast<const uint32_t*>(sc), reinterpret_cast<double*>(sc + lay_part(I.a.n)),
+    a64_body(I.a, I.box, I.eng, reinterpret_cast<const uint32_t*>(sc),
+             reinterpret_cast<double*>(sc + lay_kin(I.a.n)), reinterpret_cast<double*>(sc + lay_part(I.a.n)),
              (int)blockIdx.x - I.a_first, I.a_blocks);
 }
 
@@ -2114,7 +2147,7 @@ __global__ void __launch_bounds__(kBlockA) k_prepare(tmps_atoms a, const tmps_bo
     // the rounded FP64 ones; no FP64 division)
     const float m32 = f32_rn(v.w), I32 = f32_rn(w.w);
     reinterpret_cast<float2*>(a.inv32)[i] = make_float2(__frcp_rn(m32), __frcp_rn(I32));
-    store_vw<false>(a, i, make_float4(vh[0], vh[1], vh[2], m32), make_float4(vlo[0], vlo[1], vlo[2], 0.0f),
+    store_vw(a, i, make_float4(vh[0], vh[1], vh[2], m32), make_float4(vlo[0], vlo[1], vlo[2], 0.0f),
                     make_float4(wh[0], wh[1], wh[2], 0.0f), make_float4(wlo[0], wlo[1], wlo[2], 0.0f));
 }
 
@@ -2151,7 +2184,7 @@ __global__ void __launch_bounds__(kBlockA) k_unpack(tmps_atoms a, const tmps_box
     double4 x = ld4(a.xr, i), v = ld4(a.vm, i), w = ld4(a.om, i);
     const float4 p = ld4f(a.pos32, i), pl = ld4f(a.pos32lo, i);
     float4 vv, vl, ww, wl;
-    load_vw<false>(a, i, vv, vl, ww, wl);
+    load_vw(a, i, vv, vl, ww, wl);
     const int32_t c = a.cell32[i];
     // the FP32 forces with the rest, before any store (see k_prepare)
     float f32[3], t32[3];
@@ -2187,7 +2220,7 @@ __global__ void __launch_bounds__(kBlockA) k_settle(tmps_atoms a, const tmps_box
     if constexpr (MIXED) {
         float4 p = ld4f(a.pos32, i), pl = ld4f(a.pos32lo, i);
         float4 v, vl, w, wl;
-        load_vw<false>(a, i, v, vl, w, wl);
+        load_vw(a, i, v, vl, w, wl);
         if (e->final_pending) {
             const float dtf = 0.5f * e->dt_hi;
             const float km = dtf * vl.w, kI = dtf * wl.w;
@@ -2205,7 +2238,7 @@ __global__ void __launch_bounds__(kBlockA) k_settle(tmps_atoms a, const tmps_box
         }
         st4f(a.pos32, i, p);
         st4f(a.pos32lo, i, pl);
-        store_vw<false>(a, i, v, vl, w, wl);
+        store_vw(a, i, v, vl, w, wl);
         return;
     }
     double4 x = ld4(a.xr, i), v = ld4(a.vm, i), w = ld4(a.om, i);
@@ -2231,6 +2264,11 @@ __global__ void k_set_log(tmps_engine* e, double* log, int32_t len) {
     if (threadIdx.x || blockIdx.x) return;
     e->plog = log;
     e->plog_len = log ? len : 0;
+}
+
+__global__ void __launch_bounds__(256) k_forget_kinetic(double* __restrict__ kin, int ng) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < ng) kin[8 * (size_t)g + 6] = 0.0;
 }
 
 __global__ void k_settle_flags(tmps_box* b, tmps_engine* e) {
@@ -2431,7 +2469,8 @@ int tmps_fused_a(const tmps_atoms* a, tmps_box* d_box, tmps_engine* d_eng, int32
         if (!mixed_ok(a)) return TMPS_ERR_BAD_ARG;
         launch_pdl(k_a32, g, kBlockA, s, *a, (const tmps_box*)d_box, d_eng, flags, part);
     } else {
-        launch_pdl(k_a64, g, kBlockA, s, *a, (const tmps_box*)d_box, d_eng, flags, part);
+        launch_pdl(k_a64, g, kBlockA, s, *a, (const tmps_box*)d_box, d_eng, flags,
+                   (double*)((char*)scratch + lay_kin(n)), part);
     }
     note_launches(1);
     return launch_ok() ? TMPS_OK : TMPS_ERR_CUDA;
@@ -2495,7 +2534,8 @@ int tmps_fused_bounds(const tmps_atoms* a, const tmps_nlist* nl, const tmps_box*
     float* agap = (float*)((char*)scratch + atom_gap_offset(n));
     const int g = n > 0 ? grid_for(n, kBlockA) : 1;
     cudaStream_t st = (cudaStream_t)stream;
-    k_bounds<<<g, kBlockA, 0, st>>>(*a, *nl, d_box, d_eng, has_hist ? 1 : 0, cull ? 1 : 0, flags, gap, agap);
+    k_bounds<<<g, kBlockA, 0, st>>>(*a, *nl, d_box, d_eng, has_hist ? 1 : 0, cull ? 1 : 0, flags, gap, agap,
+                                  (double*)((char*)scratch + lay_kin(n)));
     note_launches(1);
     if (cull && n > 0) {
         // the groups in ascending gap order (C's ordered pass)
@@ -2594,6 +2634,16 @@ int tmps_batch_state(const tmps_instance* d_inst, int32_t ninst, int64_t* d_stat
     if (!d_inst || ninst < 0 || !d_state) return TMPS_ERR_BAD_ARG;
     if (ninst == 0) return TMPS_OK;
     kb_state<<<grid_for(ninst, 128), 128, 0, (cudaStream_t)stream>>>(d_inst, ninst, d_state);
+    note_launches(1);
+    return launch_ok() ? TMPS_OK : TMPS_ERR_CUDA;
+}
+
+int tmps_fused_forget_kinetic(int32_t n, void* scratch, void* stream) {
+    if (n < 0 || !scratch) return TMPS_ERR_BAD_ARG;
+    if (n == 0) return TMPS_OK;
+    const int ng = lay_groups(n);
+    k_forget_kinetic<<<grid_for(ng, 256), 256, 0, (cudaStream_t)stream>>>(
+        reinterpret_cast<double*>(static_cast<char*>(scratch) + lay_kin(n)), ng);
     note_launches(1);
     return launch_ok() ? TMPS_OK : TMPS_ERR_CUDA;
 }

@@ -318,6 +318,9 @@ class FusedEngine:
         sim = self.sim
         L = _device.lib()
         st = _device.stream()
+        if not self.mixed and self._n > 0:
+            # the FP64 update's kept kinetic sums hold while only its own steps change a velocity
+            _lib.check(L.tmps_fused_forget_kinetic(self._n, self.part.data_ptr(), st), "tmps_fused_forget_kinetic")
         start = sim.timestep
         target = start + int(nsteps)
         while True:
