@@ -211,6 +211,27 @@ __device__ __forceinline__ double block_sum6_halving(const double (&v)[6], doubl
     return t;
 }
 
+// x - x0 of two doubles as an FP32 value from their bits: where sign and
+// exponent agree (an atom moves little between builds) the difference of the
+// significands is an integer count of units in the last place, of which the
+// low 21 bits are dropped.  `err` grows by the bound of what that loses, 2^-31
+// of the magnitude; `same` is false (and the result 0) where the bits do not
+// line up or the scale leaves the FP32 range.  Integer operations and one
+// FP32 product: the FP64 pipe is this kernel's bound, and three subtractions
+// per atom are a quarter of its work there.
+__device__ __forceinline__ float bits_diff(double x, double x0, float& err, bool& same) {
+    const long long a = __double_as_longlong(x), b = __double_as_longlong(x0);
+    const int se = (int)(a >> 52), e = se & 0x7ff;  // sign and exponent
+    if (se != (int)(b >> 52) || e < 1023 - 126 + 31 || e > 1023 + 127 + 31 - 1) {
+        same = false;
+        return 0.0f;
+    }
+    const float unit = __uint_as_float((uint32_t)(e - 1023 - 31 + 127) << 23);  // 2^21 units in the last place
+    err += unit;
+    const float d = (float)(int)((a - b) >> 21) * unit;
+    return se < 0 ? -d : d;
+}
+
 // A runs as one resident wave striding over the atoms; besides the update
 // it sums the kinetic part of the virial, sum m v(t+dt/2) v(t+dt/2), over
 // every atom into per-block partials: an atom C finds contact-free ends the
@@ -233,8 +254,8 @@ __device__ __forceinline__ double block_sum6_halving(const double (&v)[6], doubl
 // tmps_fused_bounds, by a flagged atom and at the start of every run).
 //
 // What bounds it: on a nearly contact-free state the 88 bytes read and 32
-// written per atom (state x, v and the build position; x) and 12 FP64
-// instructions per atom (drift 3, remap 6, displacement 3) -- about even.
+// written per atom (state x, v and the build position; x) against 9 FP64
+// instructions per atom (drift 3, remap 6).
 __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __restrict__ b,
                                          tmps_engine* __restrict__ e, const uint32_t* __restrict__ flags,
                                          double* __restrict__ kin, double* __restrict__ part, const int bid,
@@ -249,7 +270,7 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
     const double dt = e->dt, dtf = 0.5 * dt;
     const bool fin = e->final_pending != 0, remap = b->remap_pending != 0;
     const bool kick_all = e->kick_all != 0 || !(dtf > 0.0);
-    const float trig32 = approx_f32(e->trigger_sq);
+    const float trig32 = approx_f32(e->trigger_sq), trigd = sqrtf(trig32);
     bool hit = false;
     float dd = 0.0f;
     double K[6] = {0, 0, 0, 0, 0, 0};
@@ -293,7 +314,7 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
         }
         // the kinetic terms: read back where no velocity of the group changed and they are held
         const bool moved = __any_sync(0xffffffffu, kick);
-        const bool held = !moved && __shfl_sync(0xffffffffu, kr, 6) == 1.0;
+        const bool held = !moved && __shfl_sync(0xffffffffu, __double2hiint(kr), 6) != 0;
         if (held) {
             kept += kr;  // (lanes 6 and 7 sum nothing that is used)
         } else {
@@ -319,25 +340,37 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
         }
         x.x = x.x + dt * v.x; x.y = x.y + dt * v.y; x.z = x.z + dt * v.z;
         st4(a.xr, i, x);
-        const double d0 = __dsub_rn(x.x, x0x), d1 = __dsub_rn(x.y, x0y), d2 = __dsub_rn(x.z, x0z);
-        // |d|^2 first in FP32 from the truncated differences (integer operations;
-        // relative error under 1e-5): the exact FP64 test decides only within
-        // that margin of the trigger, or for a non-finite displacement
-        const float f0 = approx_f32(d0), f1 = approx_f32(d1), f2 = approx_f32(d2);
+        // |d|^2 of the displacement d = x - x0 first in FP32 (bits_diff: |d| is within err of the
+        // FP32 one; where the bits do not line up, from the truncated FP64 differences, relative
+        // error under 1e-5): the exact FP64 test decides only within that margin of the trigger, or
+        // for a non-finite displacement
+        float err = 0.0f;
+        bool same = true;
+        float f0 = bits_diff(x.x, x0x, err, same), f1 = bits_diff(x.y, x0y, err, same),
+              f2 = bits_diff(x.z, x0z, err, same);
+        if (!same) {
+            err = 0.0f;
+            f0 = approx_f32(__dsub_rn(x.x, x0x));
+            f1 = approx_f32(__dsub_rn(x.y, x0y));
+            f2 = approx_f32(__dsub_rn(x.z, x0z));
+        }
         const float q32 = (f0 * f0 + f1 * f1) + f2 * f2;
+        const float slack = err * (2.1f * trigd + err);  // (trigger + err)^2 - trigger^2, rounded up
         bool far;
-        if (q32 < trig32 * 0.99998f) {
+        if (q32 < trig32 * 0.99998f - slack) {
             far = false;
-        } else if (q32 > trig32 * 1.00002f && q32 <= 3e38f) {
+        } else if (q32 > trig32 * 1.00002f + slack && q32 <= 3e38f) {
             far = true;
         } else {
+            const double d0 = __dsub_rn(x.x, x0x), d1 = __dsub_rn(x.y, x0y), d2 = __dsub_rn(x.z, x0z);
             const double q = __dadd_rn(__dadd_rn(__dmul_rn(d0, d0), __dmul_rn(d1, d1)), __dmul_rn(d2, d2));
             // a non-finite displacement forces the rebuild, whose binning reports the position
             far = !(q <= e->trigger_sq);
         }
         hit = hit || far;
         // the running maximum only has to bound |d|^2 from above (C's cull threshold)
-        dd = q32 == q32 ? fmaxf(dd, q32 * 1.00002f + 1e-30f) : __int_as_float(0x7fffffff);
+        const float up = q32 * 1.00002f + (err * (2.1f * l1f(f0, f1, f2) + err) + 1e-30f);
+        dd = q32 == q32 ? fmaxf(dd, up) : __int_as_float(0x7fffffff);
     }
     if (__any_sync(0xffffffffu, hit) && lane == 0) e->disp_stamp = s;
     note_displacement(e, dd);
@@ -345,7 +378,9 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
     if (threadIdx.x < 6) part[(size_t)threadIdx.x * nb + bid] = tot;
 }
 
-__global__ void __launch_bounds__(kBlockA) k_a64(tmps_atoms a, const tmps_box* __restrict__ b,
+// Three resident blocks per SM (80 registers): the contact-dense 110k update
+// runs in 19.7 instead of 22.5 us, the dilute 1M one in 33.4 instead of 34.9.
+__global__ void __launch_bounds__(kBlockA, 3) k_a64(tmps_atoms a, const tmps_box* __restrict__ b,
                                                   tmps_engine* __restrict__ e, const uint32_t* __restrict__ flags,
                                                   double* __restrict__ kin, double* __restrict__ part) {
     a64_body(a, b, e, flags, kin, part, blockIdx.x, gridDim.x);
