@@ -231,6 +231,8 @@ typedef struct tmps_engine {
                               * finite number (or dt <= 0): the FP64 update then kicks every atom;
                               * else it skips the kick of an atom whose force and torque are exact
                               * zeros (its C flag clear), which would leave it unchanged */
+    int64_t pairs;           /* entries of the last tmps_fused_bounds' rows whose partner has the
+                              * higher index: the pairs of tmps_pairs_build */
 } tmps_engine;
 
 /* One instance of a batched run (tmps_batch_*): the device state of one
@@ -464,13 +466,31 @@ int tmps_fused_a(const tmps_atoms* a, tmps_box* d_box, tmps_engine* d_eng, int32
  * caller memory: flag words, per-group and per-atom gaps, then the
  * d_eng->nblocks virial partial sums, A's blocks then C's).  c_blocks: C's
  * grid from tmps_fused_shape, or <= 0 for the default; d_eng->nblocks must be
- * A's blocks + C's blocks of the same shape.  rows != 0 takes the per-atom-row
- * path instead: every atom's row, one thread per atom, no group ruled out --
- * for contact-dense states, where the screen rules out almost nothing.  Both
- * paths sum each atom's contacts in slot order and keep the flag words'
- * meaning, so they may alternate between builds. */
+ * A's blocks + C's blocks of the same shape.  `rows` is taken and ignored: the
+ * path for contact-dense states is tmps_fused_c_pairs, and both sum each atom's
+ * contacts in slot order and keep the flag words' meaning, so they may
+ * alternate between builds. */
 int tmps_fused_c(const tmps_atoms* a, const tmps_nlist* nl, const tmps_box* d_box, tmps_engine* d_eng,
                  const tmps_pair_params* p, int32_t c_blocks, void* scratch, int32_t rows, void* stream);
+
+/* C for contact-dense states: every contact evaluated once, over the half list
+ * of pairs (i < j in internal order) of the rows, then each atom's row summed
+ * in slot order from the pairs' records (two launches).  The pair buffer
+ * (tmps_pairs_bytes; npairs = d_eng->pairs of the last tmps_fused_bounds, read
+ * by the host; 256-byte aligned, caller memory) belongs to one build:
+ * tmps_pairs_build fills it from the rows and takes the histories of the
+ * touching entries in (doubles; mixed != 0 keeps them as FP32 double words),
+ * and tmps_pairs_history writes them and the touch masks back to the rows
+ * (doubles again, both copies) before anything reads them there -- a rebuild's
+ * carry-over, a per-hook kernel, a restart file, the end of a run. */
+int64_t tmps_pairs_bytes(int32_t n, int32_t slots, int32_t npairs, int32_t style, int32_t mixed, int32_t rolling);
+int tmps_pairs_build(const tmps_nlist* nl, const tmps_pair_params* p, int32_t npairs, int32_t mixed, void* pairs,
+                     void* stream);
+int tmps_pairs_history(const tmps_nlist* nl, const tmps_pair_params* p, int32_t npairs, int32_t mixed, void* pairs,
+                       void* stream);
+int tmps_fused_c_pairs(const tmps_atoms* a, const tmps_nlist* nl, const tmps_box* d_box, tmps_engine* d_eng,
+                       const tmps_pair_params* p, int32_t c_blocks, void* scratch, int32_t npairs, void* pairs,
+                       void* stream);
 
 /* Launch S: rebuild decision, virial total (from C's scratch), servo. */
 int tmps_fused_servo(tmps_box* d_box, tmps_servo* d_servo, tmps_engine* d_eng, const void* scratch,

@@ -107,6 +107,7 @@ class Engine(ctypes.Structure):
         ("cull_tol", ctypes.c_float),
         ("plog", ctypes.c_void_p), ("plog_len", c_i32), ("order_ready", c_i32),
         ("stop_step", ctypes.c_int64), ("touching", c_i32), ("kick_all", c_i32),
+        ("pairs", ctypes.c_int64),
     ]
 
 
@@ -216,6 +217,11 @@ _SIGS = {
     "tmps_fused_a": (c_i32, [ctypes.POINTER(Atoms), c_vp, c_vp, c_i32, c_vp, c_vp]),
     "tmps_fused_c": (c_i32, [ctypes.POINTER(Atoms), ctypes.POINTER(NList), c_vp, c_vp,
                              ctypes.POINTER(PairParams), c_i32, c_vp, c_i32, c_vp]),
+    "tmps_pairs_bytes": (ctypes.c_int64, [c_i32, c_i32, c_i32, c_i32, c_i32, c_i32]),
+    "tmps_pairs_build": (c_i32, [ctypes.POINTER(NList), ctypes.POINTER(PairParams), c_i32, c_i32, c_vp, c_vp]),
+    "tmps_pairs_history": (c_i32, [ctypes.POINTER(NList), ctypes.POINTER(PairParams), c_i32, c_i32, c_vp, c_vp]),
+    "tmps_fused_c_pairs": (c_i32, [ctypes.POINTER(Atoms), ctypes.POINTER(NList), c_vp, c_vp,
+                                   ctypes.POINTER(PairParams), c_i32, c_vp, c_i32, c_vp, c_vp]),
     "tmps_fused_servo": (c_i32, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "tmps_fused_blocks": (c_i32, [c_i32, c_i32, c_i32]),
     "tmps_probe_fp64": (c_i32, [c_i32, c_i32, c_i32, c_vp, c_vp]),

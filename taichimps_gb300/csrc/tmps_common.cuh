@@ -21,6 +21,10 @@ namespace tmps {
 // threads); read through tmps_launch_count().
 void note_launches(int k);
 
+// start[0..m] = exclusive scan of count[0..m), start[m] the total; tile_sum:
+// one word per 4,096 of them (two launches, tmps_nlist.cu).
+void exclusive_scan(const int32_t* count, int32_t* start, int32_t* tile_sum, int m, cudaStream_t s);
+
 inline int grid_for(int64_t n, int block) {
     int64_t g = (n + block - 1) / block;
     return (int)(g < 1 ? 1 : g);

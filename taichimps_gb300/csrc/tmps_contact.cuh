@@ -299,7 +299,15 @@ TMPS_DEV void contact_law(const PP& P, T dt, int shearupdate, const PairIn<T>& i
             }
             default: break;
         }
-        T fntot = fne - dpf * vnnr;
+        // the mixed form's multiply-add is written out: which of the two products is fused into the
+        // difference must not depend on the kernel the law is inlined into
+        T fntot;
+        if constexpr (sizeof(T) == sizeof(float)) {
+            const T kna = P.normal_id != 0 ? T(P.kn) * a : T(P.kn);
+            fntot = __fmaf_rn(kna, delta, -__fmul_rn(dpf, vnnr));
+        } else {
+            fntot = fne - dpf * vnnr;
+        }
         if (P.limit_damping == 1 && fntot < T(0)) fntot = T(0);
         const T fscrit = T(P.mu) * fabs(fntot);
         T fs[3] = {T(0), T(0), T(0)};

@@ -29,6 +29,7 @@ namespace {
 
 constexpr int kBlockA = 256;
 constexpr int kBlockC = 128;
+constexpr int kPairMaxBlocks = 8192;  // virial partials of the pair pass: at least any contact grid
 
 // Error-free transformations in FP32 (Knuth's two-sum; FMA for products):
 // s + e == a + b exactly.  Used to form the separation and the overlap of a
@@ -588,12 +589,14 @@ __global__ void __launch_bounds__(kBlockA) k_bounds(tmps_atoms A, tmps_nlist L, 
     for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < ngroups; g += nwarps) {
         const int i = (g << 5) + lane;
         float gmin = 3e38f;
+        unsigned above = 0u;  // row entries with a partner above the atom: the pairs it is the first of
         if (i < n) {
             const double xi[3] = {A.x0[i], A.x0[n + i], A.x0[2 * n + i]};
             const float ri = approx_f32(A.xr[4 * (size_t)i + 3]);
             const int nn = L.nnb[i];
             for (int k = 0; k < nn; ++k) {
                 const int j = L.nbr[(size_t)k * n + i] & kNbrIndexMask;
+                above += j > i;
                 const double dd[3] = {xi[0] - A.x0[j], xi[1] - A.x0[n + j], xi[2] - A.x0[2 * n + j]};
                 float d[3], mag = 0.0f;
 #pragma unroll
@@ -617,6 +620,8 @@ __global__ void __launch_bounds__(kBlockA) k_bounds(tmps_atoms A, tmps_nlist L, 
         {
             const int t = __popc(__ballot_sync(0xffffffffu, i < n && !(gmin > 0.0f)));
             if (lane == 0 && t) atomicAdd(&E->touching, t);
+            above = __reduce_add_sync(0xffffffffu, above);
+            if (lane == 0 && above) atomicAdd(reinterpret_cast<unsigned long long*>(&E->pairs), (unsigned long long)above);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) gmin = fminf(gmin, __shfl_down_sync(0xffffffffu, gmin, o));
@@ -792,69 +797,58 @@ struct CfLoad {
     HT shr[3], rlr[3];
 };
 
-template <int STYLE, bool MIXED, bool DENSE>
-__device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L, const tmps_pair_params& P,
-                                        const tmps_box* __restrict__ B, tmps_engine* __restrict__ E,
-                                        uint32_t* __restrict__ flags, const float* __restrict__ gap,
-                                        const float* __restrict__ agap, const int32_t* __restrict__ order,
-                                        const float* __restrict__ sgap, double* __restrict__ part, const int bid,
-                                        const int nblk) {
+// What a contact needs besides the states of its two atoms: the step's box,
+// its images and the law's switches.  `soff`, `sofl` (mixed form, shared
+// memory): the 27 stencil offsets times the cell edge, high and low words.
+template <int STYLE, bool MIXED>
+struct CfEnv {
     using T = typename std::conditional<MIXED, float, double>::type;
-    // histories: doubles in the FP64 form, FP32 double words in the mixed form
-    using HT = typename std::conditional<MIXED, DW, double>::type;
-    using S4 = typename std::conditional<MIXED, float4, double4>::type;  // a state word
-    __shared__ double smem[6 * (kBlockC / 32)];
-    __shared__ uint32_t cwords[kBlockC / 32][kLive];
-    // the kLive groups of the batch in hand: group, old and near words (warp-uniform)
-    __shared__ int32_t bgrp[kBlockC / 32][kLive];
-    __shared__ uint32_t bold[kBlockC / 32][kLive], bnear[kBlockC / 32][kLive];
-    __shared__ CfWarp<MIXED> cwarp[DENSE ? 1 : kBlockC / 32];
-    pdl_enter();
-    if (E->aborted || E->step >= E->stop_step) return;
-    const int64_t s = E->step + 1;
-    if (rebuild_due(E, s)) return;  // S marks the step aborted; the host rebuilds
-    const int nb = E->nblocks;      // partials are component-major, [6][nb]
-    part += nb - nblk;              // C's blocks follow A's
-    constexpr bool kHist = STYLE == STYLE_HOOKE_HISTORY || STYLE == STYLE_HERTZ_HISTORY || STYLE == STYLE_GRANULAR;
-    const bool hist = kHist && (STYLE != STYLE_GRANULAR || P.tangential_id >= 2 || P.rolling_id != 0);
-    const bool roll = STYLE == STYLE_GRANULAR && P.rolling_id != 0;
-    const int n = A.n;
+    static constexpr bool kHist = STYLE == STYLE_HOOKE_HISTORY || STYLE == STYLE_HERTZ_HISTORY || STYLE == STYLE_GRANULAR;
     T dt;
-    if constexpr (MIXED) dt = E->dt_hi;
-    else dt = E->dt;
-    // per-step constants
-    T hh[3] = {0, 0, 0}, prd[3], iprd[3];
-    float hlo[3] = {0, 0, 0}, prdlo[3] = {0, 0, 0};
+    T hh[3], prd[3], iprd[3];
+    float hlo[3], prdlo[3];
     int per[3], single[3], gdim[3];
-    T hrate[3] = {0, 0, 0}, hshear[3] = {0, 0, 0};
-    const bool vremap = B->vremap != 0;
+    T hrate[3], hshear[3];
+    bool vremap, hist, roll;
+
+    __device__ __forceinline__ void load(const tmps_pair_params& P, const tmps_box* __restrict__ B,
+                                         const tmps_engine* __restrict__ E) {
+        hist = kHist && (STYLE != STYLE_GRANULAR || P.tangential_id >= 2 || P.rolling_id != 0);
+        roll = STYLE == STYLE_GRANULAR && P.rolling_id != 0;
+        if constexpr (MIXED) dt = E->dt_hi;
+        else dt = E->dt;
+        vremap = B->vremap != 0;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        per[c] = B->per[c];
-        gdim[c] = B->g[c];
-        if constexpr (MIXED) {
-            hh[c] = E->h32[c];
-            hlo[c] = E->hlo32[c];
-            prd[c] = E->prd32[c];
-            prdlo[c] = E->prdlo32[c];
-            iprd[c] = E->iprd32[c];
-            single[c] = E->single_bin[c];
-        } else {
-            prd[c] = B->prd[c];
-            iprd[c] = B->inv_prd[c];
-            single[c] = 0;
+        for (int c = 0; c < 3; ++c) {
+            hh[c] = 0;
+            hlo[c] = prdlo[c] = 0.f;
+            hrate[c] = hshear[c] = 0;
+            per[c] = B->per[c];
+            gdim[c] = B->g[c];
+            if constexpr (MIXED) {
+                hh[c] = E->h32[c];
+                hlo[c] = E->hlo32[c];
+                prd[c] = E->prd32[c];
+                prdlo[c] = E->prdlo32[c];
+                iprd[c] = E->iprd32[c];
+                single[c] = E->single_bin[c];
+            } else {
+                prd[c] = B->prd[c];
+                iprd[c] = B->inv_prd[c];
+                single[c] = 0;
+            }
+        }
+        if (vremap) {
+            // n . h_rate for the image count n = (n0, n1, n2) of the partner
+            hrate[0] = (T)B->h_rate[0]; hrate[1] = (T)B->h_rate[1]; hrate[2] = (T)B->h_rate[2];
+            hshear[0] = (T)B->h_rate[3]; hshear[1] = (T)B->h_rate[4]; hshear[2] = (T)B->h_rate[5];
         }
     }
-    if (vremap) {
-        // n . h_rate for the image count n = (n0, n1, n2) of the partner
-        hrate[0] = (T)B->h_rate[0]; hrate[1] = (T)B->h_rate[1]; hrate[2] = (T)B->h_rate[2];
-        hshear[0] = (T)B->h_rate[3]; hshear[1] = (T)B->h_rate[4]; hshear[2] = (T)B->h_rate[5];
-    }
+
     // mixed form: the 27 stencil offsets (ox, oy, oz) in {-1, 0, 1} times the
-    // cell edge, both words (exact products), by the code a list entry carries
-    __shared__ float4 soff[MIXED ? 27 : 1], sofl[MIXED ? 27 : 1];
-    __shared__ PairParams32 sP;  // the mixed law's coefficients, converted once per block
-    if constexpr (MIXED) {
+    // cell edge, both words (exact products), by the code a list entry carries,
+    // and the law's coefficients, converted once per block
+    __device__ __forceinline__ void tables(const tmps_pair_params& P, float4* soff, float4* sofl, PairParams32& sP) const {
         if (threadIdx.x == 32) params32(P, sP);
         if (threadIdx.x < 27) {
             const int code = threadIdx.x;
@@ -864,10 +858,240 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
         }
         __syncthreads();
     }
+};
+
+// One contact: row atom i (its state words Pi, PLi (mixed: low words and radius
+// lo), Vi, Wi and packed cell Ci) with the partner of a row entry of stencil
+// offset `code`, from the partner's loads `cl`; `lo`: the row atom has the
+// lower internal index, so it is `a` of the canonical pair.  Returns whether
+// they touch, and if so the canonical separation (in.d), the law's result and
+// the updated history (canonical sense) in sh, rl.
+template <int STYLE, bool MIXED, typename PP>
+__device__ __forceinline__ bool contact_core(
+    const CfEnv<STYLE, MIXED>& V, const PP& sP, const float4* soff, const float4* sofl, const bool lo, const int code,
+    const typename CfLoad<MIXED>::S4 Pi, const float4 PLi, const typename CfLoad<MIXED>::S4 Vi,
+    const typename CfLoad<MIXED>::S4 Wi, const int32_t Ci, const CfLoad<MIXED>& cl,
+    PairIn<typename CfEnv<STYLE, MIXED>::T>& in, PairOut<typename CfEnv<STYLE, MIXED>::T>& out,
+    typename CfLoad<MIXED>::HT (&sh)[3], typename CfLoad<MIXED>::HT (&rl)[3]) {
+    using T = typename CfEnv<STYLE, MIXED>::T;
+    using HT = typename CfLoad<MIXED>::HT;
+    (void)PLi;
+    (void)Ci;
+    (void)soff;
+    (void)sofl;
+    const bool was = cl.was;
+    T xi[3], xj[3], ri, rj;
+    int32_t ci = 0, cj = 0;
+    float4 il = make_float4(0.f, 0.f, 0.f, 0.f), jl = il;
+    T vi[3], wi[3], mi, vj[3], wj[3], mj;
+    HT shr[3], rlr[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        shr[c] = cl.shr[c];
+        rlr[c] = cl.rlr[c];
+    }
+    if constexpr (MIXED) {
+        const float4 pi = Pi, pj = cl.pj;
+        il = PLi;
+        jl = cl.jl;
+        const float4 v = Vi, w = Wi;
+        const float4 v2 = cl.v2, w2 = cl.w2;
+        if (V.vremap) {
+            ci = Ci;
+            cj = cl.cj;
+        }
+        xi[0] = pi.x; xi[1] = pi.y; xi[2] = pi.z; ri = pi.w;
+        xj[0] = pj.x; xj[1] = pj.y; xj[2] = pj.z; rj = pj.w;
+        vi[0] = v.x; vi[1] = v.y; vi[2] = v.z; mi = v.w;
+        wi[0] = w.x; wi[1] = w.y; wi[2] = w.z;
+        vj[0] = v2.x; vj[1] = v2.y; vj[2] = v2.z; mj = v2.w;
+        wj[0] = w2.x; wj[1] = w2.y; wj[2] = w2.z;
+    } else {
+        const double4 pi = Pi, pj = cl.pj;
+        const double4 v = Vi, w = Wi;
+        const double4 v2 = cl.v2, w2 = cl.w2;
+        xi[0] = pi.x; xi[1] = pi.y; xi[2] = pi.z; ri = pi.w;
+        xj[0] = pj.x; xj[1] = pj.y; xj[2] = pj.z; rj = pj.w;
+        vi[0] = v.x; vi[1] = v.y; vi[2] = v.z; mi = v.w;
+        wi[0] = w.x; wi[1] = w.y; wi[2] = w.z;
+        vj[0] = v2.x; vj[1] = v2.y; vj[2] = v2.z; mj = v2.w;
+        wj[0] = w2.x; wj[1] = w2.y; wj[2] = w2.z;
+    }
+    // separation x_i - x_j
+    T d[3];
+    T nimg[3] = {0, 0, 0};
+    float offh[3] = {0.f, 0.f, 0.f}, offl[3] = {0.f, 0.f, 0.f};
+    if constexpr (MIXED) {
+        const float4 so = soff[code], sl = sofl[code];
+        offh[0] = so.x; offh[1] = so.y; offh[2] = so.z;
+        offl[0] = sl.x; offl[1] = sl.y; offl[2] = sl.z;
+        // offsets are relative to each atom's own cell: j's cell is
+        // the stencil offset (ox, oy, oz) away from i's, so
+        // x_i - x_j = (o_i - o_j) - offset * h
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            d[c] = (xi[c] - xj[c]) - offh[c];
+            if (V.single[c]) {
+                nimg[c] = rintf(d[c] * V.iprd[c]);
+                d[c] -= nimg[c] * V.prd[c];
+            }
+        }
+        if (V.vremap) {  // image count for the partner velocity shift
+            const int off[3] = {code % 3 - 1, (code / 3) % 3 - 1, code / 9 - 1};
+            const int cc[3] = {cell_x(ci) + off[0] - cell_x(cj), cell_y(ci) + off[1] - cell_y(cj),
+                               cell_z(ci) + off[2] - cell_z(cj)};
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                if (!V.single[c] && V.per[c] == 1) nimg[c] = (T)(cc[c] / V.gdim[c]);
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            d[c] = xi[c] - xj[c];
+            if (V.per[c] == 1) {
+                nimg[c] = rint(d[c] * V.iprd[c]);
+                d[c] = image_sub64(d[c], nimg[c], V.prd[c]);
+            }
+        }
+    }
+    const T sg = lo ? T(1) : T(-1);
+    in.ra = lo ? ri : rj;
+    in.rb = lo ? rj : ri;
+    bool near;
+    if constexpr (MIXED) {
+        // separation, |d|^2, |d| and the overlap from the high and
+        // low FP32 words, so the overlap keeps ~2^-48 of |d| (an
+        // FP32 difference of two unit-size numbers keeps 2^-24)
+        const float xil[3] = {il.x, il.y, il.z}, xjl[3] = {jl.x, jl.y, jl.z};
+        float dh[3], dl[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            float s1, e1, s2, e2;
+            two_sum(xi[c], -xj[c], s1, e1);
+            two_sum(s1, -offh[c], s2, e2);
+            const float low = __fadd_rn(__fsub_rn(__fsub_rn(xil[c], xjl[c]), offl[c]), __fadd_rn(e1, e2));
+            two_sum(s2, low, dh[c], dl[c]);
+            if (V.single[c]) {
+                const float ni = rintf(dh[c] * V.iprd[c]);
+                float s3, e3;
+                two_sum(dh[c], -ni * V.prd[c], s3, e3);
+                two_sum(s3, __fadd_rn(__fsub_rn(dl[c], ni * V.prdlo[c]), e3), dh[c], dl[c]);
+            }
+            dh[c] = sg * dh[c];
+            dl[c] = sg * dl[c];
+        }
+        // |d|^2 = sum hi^2 (exact via FMA) + 2 hi lo
+        float pp[3], pe[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            pp[c] = __fmul_rn(dh[c], dh[c]);
+            pe[c] = __fmaf_rn(dh[c], dh[c], -pp[c]);
+        }
+        float t1, te1, rh, re;
+        two_sum(pp[0], pp[1], t1, te1);
+        two_sum(t1, pp[2], rh, re);
+        const float cross = __fmul_rn(2.0f, __fadd_rn(__fadd_rn(__fmul_rn(dh[0], dl[0]),
+                                                                __fmul_rn(dh[1], dl[1])),
+                                                     __fmul_rn(dh[2], dl[2])));
+        const float rl0 = __fadd_rn(__fadd_rn(__fadd_rn(te1, re), __fadd_rn(__fadd_rn(pe[0], pe[1]), pe[2])),
+                                    cross);
+        float rsh, rsl;
+        two_sum(rh, rl0, rsh, rsl);
+        // r_hi need not be the rounded root: the residual rsh - r_hi^2 (one FMA,
+        // within an ulp of exact for an r_hi a few ulp off) corrects it in r_lo
+        const float r_hi = lsqrt(rsh);
+        const float res = __fmaf_rn(-r_hi, r_hi, rsh);
+        const float r_lo = __fdividef(__fadd_rn(res, rsl), __fmul_rn(2.0f, r_hi));
+        // ra + rb, both words
+        const float4 al = lo ? il : jl, bl = lo ? jl : il;
+        float sh_, se_;
+        two_sum(in.ra, in.rb, sh_, se_);
+        const float rad_lo = __fadd_rn(__fadd_rn(al.w, bl.w), se_);
+        const float delta = __fadd_rn(__fsub_rn(sh_, r_hi), __fsub_rn(rad_lo, r_lo));
+        near = delta > 0.0f && rsh > 1e-28f;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) in.d[c] = dh[c];
+        in.rsq = rsh;
+        in.r = r_hi;
+        in.delta = delta;
+    } else {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) in.d[c] = sg * d[c];
+        in.rsq = rsq64(in.d);
+        const T radsum = in.ra + in.rb;
+        near = in.rsq < __dmul_rn(radsum, radsum) && in.rsq > T(1e-28);
+        if (near) {
+            in.r = sqrt(in.rsq);
+            in.delta = radsum - in.r;
+        }
+    }
+    if (near) {
+        T dv[3] = {0, 0, 0};
+        if (V.vremap) {
+            // image count of x_a - x_b, then n . h_rate for partner b
+            T na[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) na[c] = sg * nimg[c];
+            dv[0] = (na[0] * V.hrate[0] + na[1] * V.hshear[2]) + na[2] * V.hshear[1];
+            dv[1] = na[1] * V.hrate[1] + na[2] * V.hshear[0];
+            dv[2] = na[2] * V.hrate[2];
+        }
+        in.ma = lo ? mi : mj;
+        in.mb = lo ? mj : mi;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            in.va[c] = lo ? vi[c] : vj[c];
+            in.vb[c] = (lo ? vj[c] : vi[c]) + dv[c];
+            in.wa[c] = lo ? wi[c] : wj[c];
+            in.wb[c] = lo ? wj[c] : wi[c];
+        }
+        if (V.hist && was) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                sh[c] = hsign(shr[c], lo);
+                rl[c] = hsign(rlr[c], lo);
+            }
+        }
+        contact_law<T, STYLE>(sP, V.dt, 1, in, sh, rl, out);
+    }
+    return near;
+}
+
+template <int STYLE, bool MIXED>
+__device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L, const tmps_pair_params& P,
+                                        const tmps_box* __restrict__ B, tmps_engine* __restrict__ E,
+                                        uint32_t* __restrict__ flags, const float* __restrict__ gap,
+                                        const float* __restrict__ agap, const int32_t* __restrict__ order,
+                                        const float* __restrict__ sgap, double* __restrict__ part, const int bid,
+                                        const int nblk) {
+    using T = typename CfEnv<STYLE, MIXED>::T;
+    // histories: doubles in the FP64 form, FP32 double words in the mixed form
+    using HT = typename CfLoad<MIXED>::HT;
+    using S4 = typename CfLoad<MIXED>::S4;  // a state word
+    __shared__ double smem[6 * (kBlockC / 32)];
+    __shared__ uint32_t cwords[kBlockC / 32][kLive];
+    // the kLive groups of the batch in hand: group, old and near words (warp-uniform)
+    __shared__ int32_t bgrp[kBlockC / 32][kLive];
+    __shared__ uint32_t bold[kBlockC / 32][kLive], bnear[kBlockC / 32][kLive];
+    __shared__ CfWarp<MIXED> cwarp[kBlockC / 32];
+    pdl_enter();
+    if (E->aborted || E->step >= E->stop_step) return;
+    const int64_t s = E->step + 1;
+    if (rebuild_due(E, s)) return;  // S marks the step aborted; the host rebuilds
+    const int nb = E->nblocks;      // partials are component-major, [6][nb]
+    part += nb - nblk;              // C's blocks follow A's
+    const int n = A.n;
+    CfEnv<STYLE, MIXED> V;
+    V.load(P, B, E);
+    const T dt = V.dt;
+    const bool hist = V.hist, roll = V.roll, vremap = V.vremap;
+    __shared__ float4 soff[MIXED ? 27 : 1], sofl[MIXED ? 27 : 1];
+    __shared__ PairParams32 sP;
+    if constexpr (MIXED) V.tables(P, soff, sofl, sP);
     double Vd[6] = {0, 0, 0, 0, 0, 0};
     float Vh[6] = {0, 0, 0, 0, 0, 0}, Vl[6] = {0, 0, 0, 0, 0, 0};  // mixed: per-thread double words
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    CfWarp<MIXED>& W = cwarp[DENSE ? 0 : wib];
+    CfWarp<MIXED>& W = cwarp[wib];
     const int ngroups = (n + 31) >> 5;
     const int nwarps = (nblk * blockDim.x) >> 5;
     const size_t ss = (size_t)L.slots * n;
@@ -881,12 +1105,6 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
         thr = ((2.0f * md) * 1.0001f + E->shift_bound) + E->cull_tol;
     }
 
-    // The contact of row atom ia (its state words Pi, PLi (mixed: low words and
-    // radius lo), Vi, Wi and packed cell Ci) with the partner of row entry e at
-    // slot k (its high position word Pj), `was` its touch bit: whether they
-    // touch, and if so the row atom's force, torque and pair virial terms in
-    // fc, tc, vc; the contact's history is updated in place.  Every other load
-    // of the contact is issued here together (one round trip).
     // The loads of a contact (row atom ia, row entry e at slot k, touch bit
     // `was`, partner high position word Pj), all issued at once: one round trip.
     auto contact_fetch = [&](const int ia, const int e, const int k, const bool was, const S4 Pj) {
@@ -926,198 +1144,24 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
         return cl;
     };
 
-    // The contact of row atom ia (its state words Pi, PLi (mixed: low words and
-    // radius lo), Vi, Wi and packed cell Ci) with the partner of row entry e at
-    // slot k, from its loads `cl`: whether they touch, and if so the row atom's
+    // The contact of row atom ia with the partner of row entry e at slot k, from
+    // its loads `cl` (contact_core): whether they touch, and if so the row atom's
     // force, torque and pair virial terms in fc, tc, vc; the contact's history
     // is updated in place.
     auto contact_eval = [&](const int ia, const int e, const int k, const S4 Pi, const float4 PLi, const S4 Vi,
                             const S4 Wi, const int32_t Ci, const CfLoad<MIXED>& cl, T (&fc)[3], T (&tc)[3],
                             T (&vc)[6]) -> bool {
-        (void)PLi;
-        (void)Ci;
-        const int j = e & kNbrIndexMask;
-        const bool lo = ia < j;
+        const bool lo = ia < (e & kNbrIndexMask);
         const size_t so = (size_t)k * n + ia;
-        const bool was = cl.was;
-        T xi[3], xj[3], ri, rj;
-        int32_t ci = 0, cj = 0;
-        float4 il = make_float4(0.f, 0.f, 0.f, 0.f), jl = il;
-        T vi[3], wi[3], mi, vj[3], wj[3], mj;
-        HT shr[3], rlr[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            shr[c] = cl.shr[c];
-            rlr[c] = cl.rlr[c];
-        }
-        if constexpr (MIXED) {
-            const float4 pi = Pi, pj = cl.pj;
-            il = PLi;
-            jl = cl.jl;
-            const float4 v = Vi, w = Wi;
-            const float4 v2 = cl.v2, w2 = cl.w2;
-            if (vremap) {
-                ci = Ci;
-                cj = cl.cj;
-            }
-            xi[0] = pi.x; xi[1] = pi.y; xi[2] = pi.z; ri = pi.w;
-            xj[0] = pj.x; xj[1] = pj.y; xj[2] = pj.z; rj = pj.w;
-            vi[0] = v.x; vi[1] = v.y; vi[2] = v.z; mi = v.w;
-            wi[0] = w.x; wi[1] = w.y; wi[2] = w.z;
-            vj[0] = v2.x; vj[1] = v2.y; vj[2] = v2.z; mj = v2.w;
-            wj[0] = w2.x; wj[1] = w2.y; wj[2] = w2.z;
-        } else {
-            const double4 pi = Pi, pj = cl.pj;
-            const double4 v = Vi, w = Wi;
-            const double4 v2 = cl.v2, w2 = cl.w2;
-            xi[0] = pi.x; xi[1] = pi.y; xi[2] = pi.z; ri = pi.w;
-            xj[0] = pj.x; xj[1] = pj.y; xj[2] = pj.z; rj = pj.w;
-            vi[0] = v.x; vi[1] = v.y; vi[2] = v.z; mi = v.w;
-            wi[0] = w.x; wi[1] = w.y; wi[2] = w.z;
-            vj[0] = v2.x; vj[1] = v2.y; vj[2] = v2.z; mj = v2.w;
-            wj[0] = w2.x; wj[1] = w2.y; wj[2] = w2.z;
-        }
-        // separation x_i - x_j
-        T d[3];
-        T nimg[3] = {0, 0, 0};
-        const int code = (unsigned)e >> kNbrIndexBits;
-        float offh[3] = {0.f, 0.f, 0.f}, offl[3] = {0.f, 0.f, 0.f};
-        if constexpr (MIXED) {
-            const float4 so = soff[code], sl = sofl[code];
-            offh[0] = so.x; offh[1] = so.y; offh[2] = so.z;
-            offl[0] = sl.x; offl[1] = sl.y; offl[2] = sl.z;
-            // offsets are relative to each atom's own cell: j's cell is
-            // the stencil offset (ox, oy, oz) away from i's, so
-            // x_i - x_j = (o_i - o_j) - offset * h
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                d[c] = (xi[c] - xj[c]) - offh[c];
-                if (single[c]) {
-                    nimg[c] = rintf(d[c] * iprd[c]);
-                    d[c] -= nimg[c] * prd[c];
-                }
-            }
-            if (vremap) {  // image count for the partner velocity shift
-                const int off[3] = {code % 3 - 1, (code / 3) % 3 - 1, code / 9 - 1};
-                const int cc[3] = {cell_x(ci) + off[0] - cell_x(cj), cell_y(ci) + off[1] - cell_y(cj),
-                                   cell_z(ci) + off[2] - cell_z(cj)};
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-                    if (!single[c] && per[c] == 1) nimg[c] = (T)(cc[c] / gdim[c]);
-            }
-        } else {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                d[c] = xi[c] - xj[c];
-                if (per[c] == 1) {
-                    nimg[c] = rint(d[c] * iprd[c]);
-                    d[c] = image_sub64(d[c], nimg[c], prd[c]);
-                }
-            }
-        }
         PairIn<T> in;
-        const T sg = lo ? T(1) : T(-1);
-        in.ra = lo ? ri : rj;
-        in.rb = lo ? rj : ri;
+        PairOut<T> out;
+        HT sh[3] = {}, rl[3] = {};
         bool near;
-        if constexpr (MIXED) {
-            // separation, |d|^2, |d| and the overlap from the high and
-            // low FP32 words, so the overlap keeps ~2^-48 of |d| (an
-            // FP32 difference of two unit-size numbers keeps 2^-24)
-            const float xil[3] = {il.x, il.y, il.z}, xjl[3] = {jl.x, jl.y, jl.z};
-            float dh[3], dl[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                float s1, e1, s2, e2;
-                two_sum(xi[c], -xj[c], s1, e1);
-                two_sum(s1, -offh[c], s2, e2);
-                const float low = __fadd_rn(__fsub_rn(__fsub_rn(xil[c], xjl[c]), offl[c]), __fadd_rn(e1, e2));
-                two_sum(s2, low, dh[c], dl[c]);
-                if (single[c]) {
-                    const float ni = rintf(dh[c] * iprd[c]);
-                    float s3, e3;
-                    two_sum(dh[c], -ni * prd[c], s3, e3);
-                    two_sum(s3, __fadd_rn(__fsub_rn(dl[c], ni * prdlo[c]), e3), dh[c], dl[c]);
-                }
-                dh[c] = sg * dh[c];
-                dl[c] = sg * dl[c];
-            }
-            // |d|^2 = sum hi^2 (exact via FMA) + 2 hi lo
-            float pp[3], pe[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                pp[c] = __fmul_rn(dh[c], dh[c]);
-                pe[c] = __fmaf_rn(dh[c], dh[c], -pp[c]);
-            }
-            float t1, te1, rh, re;
-            two_sum(pp[0], pp[1], t1, te1);
-            two_sum(t1, pp[2], rh, re);
-            const float cross = __fmul_rn(2.0f, __fadd_rn(__fadd_rn(__fmul_rn(dh[0], dl[0]),
-                                                                    __fmul_rn(dh[1], dl[1])),
-                                                         __fmul_rn(dh[2], dl[2])));
-            const float rl0 = __fadd_rn(__fadd_rn(__fadd_rn(te1, re), __fadd_rn(__fadd_rn(pe[0], pe[1]), pe[2])),
-                                        cross);
-            float rsh, rsl;
-            two_sum(rh, rl0, rsh, rsl);
-            // r_hi need not be the rounded root: the residual rsh - r_hi^2 (one FMA,
-            // within an ulp of exact for an r_hi a few ulp off) corrects it in r_lo
-            const float r_hi = lsqrt(rsh);
-            const float res = __fmaf_rn(-r_hi, r_hi, rsh);
-            const float r_lo = __fdividef(__fadd_rn(res, rsl), __fmul_rn(2.0f, r_hi));
-            // ra + rb, both words
-            const float4 al = lo ? il : jl, bl = lo ? jl : il;
-            float sh_, se_;
-            two_sum(in.ra, in.rb, sh_, se_);
-            const float rad_lo = __fadd_rn(__fadd_rn(al.w, bl.w), se_);
-            const float delta = __fadd_rn(__fsub_rn(sh_, r_hi), __fsub_rn(rad_lo, r_lo));
-            near = delta > 0.0f && rsh > 1e-28f;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) in.d[c] = dh[c];
-            in.rsq = rsh;
-            in.r = r_hi;
-            in.delta = delta;
-        } else {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) in.d[c] = sg * d[c];
-            in.rsq = rsq64(in.d);
-            const T radsum = in.ra + in.rb;
-            near = in.rsq < __dmul_rn(radsum, radsum) && in.rsq > T(1e-28);
-            if (near) {
-                in.r = sqrt(in.rsq);
-                in.delta = radsum - in.r;
-            }
-        }
+        const int code = (unsigned)e >> kNbrIndexBits;
+        if constexpr (MIXED) near = contact_core<STYLE, MIXED>(V, sP, soff, sofl, lo, code, Pi, PLi, Vi, Wi, Ci, cl, in, out, sh, rl);
+        else near = contact_core<STYLE, MIXED>(V, P, soff, sofl, lo, code, Pi, PLi, Vi, Wi, Ci, cl, in, out, sh, rl);
         if (near) {
-            T dv[3] = {0, 0, 0};
-            if (vremap) {
-                // image count of x_a - x_b, then n . h_rate for partner b
-                T na[3];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) na[c] = sg * nimg[c];
-                dv[0] = (na[0] * hrate[0] + na[1] * hshear[2]) + na[2] * hshear[1];
-                dv[1] = na[1] * hrate[1] + na[2] * hshear[0];
-                dv[2] = na[2] * hrate[2];
-            }
-            in.ma = lo ? mi : mj;
-            in.mb = lo ? mj : mi;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                in.va[c] = lo ? vi[c] : vj[c];
-                in.vb[c] = (lo ? vj[c] : vi[c]) + dv[c];
-                in.wa[c] = lo ? wi[c] : wj[c];
-                in.wb[c] = lo ? wj[c] : wi[c];
-            }
-            HT sh[3] = {}, rl[3] = {};
-            if (hist && was) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    sh[c] = hsign(shr[c], lo);
-                    rl[c] = hsign(rlr[c], lo);
-                }
-            }
-            PairOut<T> out;
-            if constexpr (MIXED) contact_law<T, STYLE>(sP, dt, 1, in, sh, rl, out);
-            else contact_law<T, STYLE>(P, dt, 1, in, sh, rl, out);
+            const T sg = lo ? T(1) : T(-1);
             if (hist) {
                 HT* hs = reinterpret_cast<HT*>(L.shear);
                 hs[so] = hsign(sh[0], lo);
@@ -1309,7 +1353,7 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
 #pragma unroll
                         for (int c = 0; c < 3; ++c) {
                             d[c] = (xi[c] - xj[c]) - oh[c];
-                            if (single[c]) d[c] -= rintf(d[c] * iprd[c]) * prd[c];
+                            if (V.single[c]) d[c] -= rintf(d[c] * V.iprd[c]) * V.prd[c];
                         }
                         const float rq = (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2];
                         const float rs = (pi.w + pj[u].w) * 1.00001f;
@@ -1338,7 +1382,7 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
                         double d[3] = {pi.x - pj[u].x, pi.y - pj[u].y, pi.z - pj[u].z};
 #pragma unroll
                         for (int c = 0; c < 3; ++c)
-                            if (per[c] == 1) d[c] = image_sub64(d[c], rint(d[c] * iprd[c]), prd[c]);
+                            if (V.per[c] == 1) d[c] = image_sub64(d[c], rint(d[c] * V.iprd[c]), V.prd[c]);
                         // the contact test itself, as the law makes it (|d|^2 of either orientation)
                         const double rsq = rsq64(d);
                         const double radsum = pi.w + pj[u].w;
@@ -1440,165 +1484,6 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
         }
     };
 
-    if constexpr (DENSE) {
-        // Per-atom rows (the contact-dense path): every atom, one lane each,
-        // whole 32-atom groups per warp.  Its row entries are loaded four at a
-        // time (coalesced over the lanes) with their partners' high position
-        // words, and the near test (the screened path's, word for word) marks
-        // the near slots; the contacts of the near slots then run in ascending
-        // slot order, each lane on its own atom, summed into the atom's force,
-        // torque and virial in that order -- the sums the screened path forms
-        // for the same atom.  Nothing is staged in shared memory and no group
-        // is ruled out, which suits a state where nearly every atom touches.
-        for (int base = bid * (int)blockDim.x + (int)(threadIdx.x & ~31u); base < n; base += nblk * (int)blockDim.x) {
-            const int i = base + lane;
-            const bool mine = i < n;
-            S4 Pi{}, Vi{}, Wi{};
-            float4 PLi = make_float4(0.f, 0.f, 0.f, 0.f);
-            int32_t Ci = 0;
-            int nn = 0;
-            uint64_t touch = 0ull;
-            if (mine) {
-                nn = L.nnb[i];
-                if (hist) touch = L.touch[i];
-                if constexpr (MIXED) {
-                    Pi = ld4f(A.pos32, i);
-                    PLi = ld4f(A.pos32lo, i);
-                    Vi = ld4f(A.vel32, i);
-                    Wi = ld4f(A.om32, i);
-                    if (vremap) Ci = A.cell32[i];
-                } else {
-                    Pi = ld4(A.xr, i);
-                    Vi = ld4(A.vm, i);
-                    Wi = ld4(A.om, i);
-                }
-            }
-            const uint32_t old = flags[base >> 5];
-            // near test of the row, four entries at a time
-            uint64_t nmask = 0ull;
-            for (int k0 = 0; k0 < nn; k0 += 4) {
-                int ee[4];
-                S4 pj[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) ee[u] = k0 + u < nn ? L.nbr[(size_t)(k0 + u) * n + i] : 0;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (k0 + u < nn) {
-                        if constexpr (MIXED) pj[u] = ld4f(A.pos32, ee[u] & kNbrIndexMask);
-                        else pj[u] = ld4(A.xr, ee[u] & kNbrIndexMask);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (k0 + u >= nn) continue;
-                    bool nr;
-                    if constexpr (MIXED) {
-                        const float4 so = soff[(unsigned)ee[u] >> kNbrIndexBits];
-                        const float xi[3] = {Pi.x, Pi.y, Pi.z}, xj[3] = {pj[u].x, pj[u].y, pj[u].z};
-                        const float oh[3] = {so.x, so.y, so.z};
-                        float d[3];
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            d[c] = (xi[c] - xj[c]) - oh[c];
-                            if (single[c]) d[c] -= rintf(d[c] * iprd[c]) * prd[c];
-                        }
-                        const float rq = (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2];
-                        const float rs = (Pi.w + pj[u].w) * 1.00001f;
-                        nr = rq < rs * rs;
-                    } else {
-                        double d[3] = {Pi.x - pj[u].x, Pi.y - pj[u].y, Pi.z - pj[u].z};
-#pragma unroll
-                        for (int c = 0; c < 3; ++c)
-                            if (per[c] == 1) d[c] = image_sub64(d[c], rint(d[c] * iprd[c]), prd[c]);
-                        const double rsq = rsq64(d);
-                        const double radsum = Pi.w + pj[u].w;
-                        nr = rsq < __dmul_rn(radsum, radsum) && rsq > 1e-28;
-                    }
-                    if (nr) nmask |= 1ull << (k0 + u);
-                }
-            }
-            // the near slots' contacts in ascending slot order (each contact's
-            // loads issued together, then its evaluation; issuing the next
-            // contact's loads before evaluating the current one was measured
-            // slower: the second set of registers spills)
-            T F[3] = {0, 0, 0}, Tq[3] = {0, 0, 0}, V[6] = {0, 0, 0, 0, 0, 0};
-            uint64_t nt = 0ull;
-            for (uint64_t m = nmask; m; m &= m - 1ull) {
-                const int k = __ffsll((long long)m) - 1;
-                const int e = L.nbr[(size_t)k * n + i];
-                S4 Pj;
-                if constexpr (MIXED) Pj = ld4f(A.pos32, e & kNbrIndexMask);
-                else Pj = ld4(A.xr, e & kNbrIndexMask);
-                const CfLoad<MIXED> cl = contact_fetch(i, e, k, ((touch >> k) & 1ull) != 0, Pj);
-                T fc[3] = {0, 0, 0}, tc[3] = {0, 0, 0}, vc[6] = {0, 0, 0, 0, 0, 0};
-                if (contact_eval(i, e, k, Pi, PLi, Vi, Wi, Ci, cl, fc, tc, vc)) nt |= 1ull << k;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    F[c] += fc[c];
-                    Tq[c] += tc[c];
-                }
-#pragma unroll
-                for (int c = 0; c < 6; ++c) V[c] += vc[c];
-            }
-            // finish the atom (the screened path's step 5)
-            if (mine) {
-                if (hist && nt != touch) L.touch[i] = nt;
-                if (nmask != 0ull) {
-                    const T vi[3] = {Vi.x, Vi.y, Vi.z}, wi[3] = {Wi.x, Wi.y, Wi.z};
-                    const T mi = Vi.w;
-                    if (E->cundall) {  // FixDampingCundall.post_force_kernel
-                        T gl, ga;
-                        if constexpr (MIXED) {
-                            gl = E->gamma_lin32;
-                            ga = E->gamma_ang32;
-                        } else {
-                            gl = E->gamma_lin;
-                            ga = E->gamma_ang;
-                        }
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            const T sf = F[c] * vi[c] >= T(0) ? T(1) : T(-1);
-                            F[c] *= T(1) - gl * sf;
-                            const T st = Tq[c] * wi[c] >= T(0) ? T(1) : T(-1);
-                            Tq[c] *= T(1) - ga * st;
-                        }
-                    }
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        if constexpr (MIXED) {
-                            A.f32[c * n + i] = F[c];
-                            A.torque32[c * n + i] = Tq[c];
-                        } else {
-                            A.f[c * n + i] = F[c];
-                            A.torque[c * n + i] = Tq[c];
-                        }
-                    }
-                    T im;
-                    if constexpr (MIXED) im = __fdividef(1.0f, mi);
-                    else im = A.rinv[i];
-                    const T hdt = T(0.5) * dt;
-                    T vf[3];
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) vf[c] = vi[c] + hdt * (F[c] * im);
-                    const T kin[6] = {(mi * vf[0]) * vf[0], (mi * vf[1]) * vf[1], (mi * vf[2]) * vf[2],
-                                      (mi * vf[0]) * vf[1], (mi * vf[0]) * vf[2], (mi * vf[1]) * vf[2]};
-                    const T kh[6] = {(mi * vi[0]) * vi[0], (mi * vi[1]) * vi[1], (mi * vi[2]) * vi[2],
-                                     (mi * vi[0]) * vi[1], (mi * vi[0]) * vi[2], (mi * vi[1]) * vi[2]};
-                    if constexpr (MIXED) {
-#pragma unroll
-                        for (int c = 0; c < 6; ++c) dw_add(Vh[c], Vl[c], V[c] + (kin[c] - kh[c]));
-                    } else {
-#pragma unroll
-                        for (int c = 0; c < 6; ++c) Vd[c] += (V[c] + kin[c]) - kh[c];
-                    }
-                }
-            }
-            // the group's new flag word; stale forces of atoms no longer flagged
-            const uint32_t w = __ballot_sync(0xffffffffu, mine && nmask != 0ull);
-            if (lane == 0 && w != old) flags[base >> 5] = w;
-            if (mine && ((old >> lane) & 1u) && !((w >> lane) & 1u)) zero_force<MIXED>(A, i);
-        }
-    } else {
     if (lane < kLive) cwords[wib][lane] = 0u;
     __syncwarp();
     // Ordered pass: after the first pass that follows the bounds (which
@@ -1705,7 +1590,6 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
             __syncwarp();
         }
     }
-    }  // screened path
     if constexpr (MIXED) {
         block_sum_dw<6, kBlockC>(Vh, Vl, reinterpret_cast<float2*>(smem));
         if (threadIdx.x == 0) {
@@ -1722,14 +1606,614 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
     if (threadIdx.x == 0 && bid == 0) E->final_pending = 1;
 }
 
-template <int STYLE, bool MIXED, bool DENSE = false>
+template <int STYLE, bool MIXED>
 __global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
     k_cf(tmps_atoms A, tmps_nlist L, tmps_pair_params P, const tmps_box* __restrict__ B,
          tmps_engine* __restrict__ E, uint32_t* __restrict__ flags, const float* __restrict__ gap,
          const float* __restrict__ agap, double* __restrict__ part) {
     const char* sc = reinterpret_cast<const char*>(flags);  // the scratch base
-    cf_body<STYLE, MIXED, DENSE>(A, L, P, B, E, flags, gap, agap, reinterpret_cast<const int32_t*>(sc + lay_order(A.n)),
+    cf_body<STYLE, MIXED>(A, L, P, B, E, flags, gap, agap, reinterpret_cast<const int32_t*>(sc + lay_order(A.n)),
                           reinterpret_cast<const float*>(sc + lay_sgap(A.n)), part, blockIdx.x, gridDim.x);
+}
+
+// ------------------------------------------------- C, contact-dense states
+//
+// Where most atoms touch, the screened path evaluates every contact twice,
+// once for each of its atoms, and that evaluation is what bounds it: ~450 FP32
+// instructions a contact in the mixed form, ~500 on the narrow FP64 pipe in
+// the FP64 form.  This path evaluates each contact once, over the half list
+// of pairs (i < j, in row order) that tmps_pairs_build derives from the rows:
+//
+//   k_pair_contacts  one lane per pair: the near test of 32 pairs at a time,
+//                    the near ones queued, the law run 32 contacts at a time
+//                    with full lanes; force, torque term and (granular)
+//                    rolling torque go to the pair's record, the history to
+//                    the pair's slot;
+//   k_pair_gather    one lane per atom: its row's records summed in slot
+//                    order with the signs of its side -- the sums the
+//                    screened path forms, bit for bit -- then Cundall damping,
+//                    the force and torque, the kinetic correction, the flags.
+//
+// The mixed form sums the virial per atom too, in FP32 from the separation in
+// the record and then, atoms a grid stride apart, into double words: the sums
+// of a one-thread-per-atom pass of 128-thread blocks, bit for bit, since the
+// servo feeds a pressure's last bits back into the FP32 roundings of every
+// contact.  The FP64 form sums it per pair.
+//
+// The records cost 48 to 80 bytes a contact, written once and read twice,
+// against half of the arithmetic.  The histories live per pair while the run
+// lasts (one copy, coalesced; the mixed form's as double words) and return to
+// the rows' both-sided doubles through tmps_pairs_history.
+
+// Words of a pair's record: f.xyz and the torque term; granular adds the
+// rolling torque and the overlap, the mixed form the separation.
+template <int STYLE>
+constexpr int kRecWords = STYLE == STYLE_GRANULAR ? 16 : 12;      // mixed, floats (16-byte multiples)
+template <int STYLE>
+constexpr int kRecDoubles = STYLE == STYLE_GRANULAR ? 10 : 6;     // FP64
+
+constexpr int32_t kPairSecond = (int32_t)0x80000000u;  // row index bit: the row atom is the pair's second
+constexpr int32_t kPairNone = -1;                      // no such pair (a row that does not mirror its partner's)
+
+__host__ __device__ inline size_t pair_rec_bytes(int style, bool mixed) {
+    return mixed ? (style == STYLE_GRANULAR ? 64 : 48) : (style == STYLE_GRANULAR ? 80 : 48);
+}
+
+// A pair buffer's parts (tmps_pairs_bytes), each on a 256-byte boundary.
+struct PairLay {
+    int32_t *begin, *count, *first, *entry, *row;
+    uint32_t* touch;
+    double *shear, *rolling, *part;
+    char* rec;
+    size_t bytes;
+};
+__host__ __device__ inline PairLay pair_lay(void* base, int n, int slots, int np, int style, bool mixed, bool roll) {
+    const size_t P = (size_t)np;
+    char* const b = static_cast<char*>(base);
+    size_t off = 0;
+    PairLay l;
+    auto take = [&](size_t bytes) {
+        char* p = b + off;
+        off += lay_round256(bytes);
+        return p;
+    };
+    l.begin = reinterpret_cast<int32_t*>(take(((size_t)n + 1) * 4));
+    l.count = reinterpret_cast<int32_t*>(take(((size_t)n + n / 4096 + 1) * 4));  // counts, then the scan's tile totals
+    l.first = reinterpret_cast<int32_t*>(take(P * 4));
+    l.entry = reinterpret_cast<int32_t*>(take(P * 4));
+    l.row = reinterpret_cast<int32_t*>(take((size_t)slots * n * 4));
+    l.touch = reinterpret_cast<uint32_t*>(take((P + 31) / 32 * 4));
+    l.shear = reinterpret_cast<double*>(take(3 * P * 8));
+    l.rolling = roll ? reinterpret_cast<double*>(take(3 * P * 8)) : nullptr;
+    l.part = reinterpret_cast<double*>(take((size_t)6 * 8 * kPairMaxBlocks));
+    l.rec = take(P * pair_rec_bytes(style, mixed));
+    l.bytes = off;
+    return l;
+}
+
+__global__ void __launch_bounds__(256) k_pair_count(tmps_nlist L, int32_t* __restrict__ count) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = L.n;
+    if (i >= n) return;
+    const int nn = L.nnb[i];
+    int c = 0;
+    for (int k = 0; k < nn; ++k) c += (L.nbr[(size_t)k * n + i] & kNbrIndexMask) > i;
+    count[i] = c;
+}
+
+// The pairs of each atom as the first (its row entries with a partner above
+// it, in slot order) with their histories as they stand in its row.
+__global__ void __launch_bounds__(256) k_pair_fill(tmps_nlist L, PairLay Q, int np, int hist, int mixed) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = L.n;
+    if (i >= n) return;
+    const int nn = L.nnb[i];
+    const uint64_t touch = hist ? L.touch[i] : 0ull;
+    const size_t ss = (size_t)L.slots * n;
+    int p = Q.begin[i];
+    for (int k = 0; k < nn; ++k) {
+        const size_t so = (size_t)k * n + i;
+        const int e = L.nbr[so];
+        if ((e & kNbrIndexMask) <= i) continue;
+        Q.first[p] = i;
+        Q.entry[p] = e;
+        Q.row[so] = p;
+        if ((touch >> k) & 1ull) {
+            atomicOr(&Q.touch[p >> 5], 1u << (p & 31));
+            for (int arr = 0; arr < 2; ++arr) {
+                const double* h = arr == 0 ? L.shear : L.rolling;
+                double* o = arr == 0 ? Q.shear : Q.rolling;
+                if (!o) continue;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const double v = h[c * ss + so];
+                    double* dst = o + (size_t)c * np + p;
+                    if (mixed) {
+                        const float hi = __double2float_rn(v);
+                        *reinterpret_cast<DW*>(dst) = DW{hi, __double2float_rn(v - (double)hi)};
+                    } else {
+                        *dst = v;
+                    }
+                }
+            }
+        }
+        ++p;
+    }
+}
+
+// The row index of every entry with a partner below the atom: the pair that
+// partner's row holds for it.
+__global__ void __launch_bounds__(256) k_pair_back(tmps_nlist L, PairLay Q) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = L.n;
+    if (i >= n) return;
+    const int nn = L.nnb[i];
+    for (int k = 0; k < nn; ++k) {
+        const int j = L.nbr[(size_t)k * n + i] & kNbrIndexMask;
+        if (j >= i) continue;
+        // row j's pairs are begin[j] .. begin[j + 1] - 1, their partners in `entry`
+        int32_t r = kPairNone;
+        for (int p = Q.begin[j]; p < Q.begin[j + 1]; ++p)
+            if ((Q.entry[p] & kNbrIndexMask) == i) r = p | kPairSecond;
+        Q.row[(size_t)k * n + i] = r;
+    }
+}
+
+// The histories back into the rows: touch masks, and each touching entry's
+// doubles in its row atom's sense (the second atom's are the exact negatives).
+__global__ void __launch_bounds__(256) k_pair_history(tmps_nlist L, PairLay Q, int np, int mixed) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = L.n;
+    if (i >= n) return;
+    const int nn = L.nnb[i];
+    const size_t ss = (size_t)L.slots * n;
+    uint64_t touch = 0ull;
+    for (int k = 0; k < nn; ++k) {
+        const size_t so = (size_t)k * n + i;
+        const int32_t r = Q.row[so];
+        const int p = r & 0x7fffffff;
+        if (r == kPairNone || !((Q.touch[p >> 5] >> (p & 31)) & 1u)) continue;
+        touch |= 1ull << k;
+        for (int arr = 0; arr < 2; ++arr) {
+            const double* h = arr == 0 ? Q.shear : Q.rolling;
+            double* o = arr == 0 ? L.shear : L.rolling;
+            if (!h) continue;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                double v = h[(size_t)c * np + p];
+                if (mixed) {
+                    const DW w = *reinterpret_cast<const DW*>(&h[(size_t)c * np + p]);
+                    v = f64_of(w.hi) + f64_of(w.lo);
+                }
+                o[c * ss + so] = r < 0 ? -v : v;
+            }
+        }
+    }
+    L.touch[i] = touch;
+}
+
+constexpr int kPairRing = 64;  // queued pairs per warp: < 32 waiting + 32 from one near test
+
+template <int STYLE, bool MIXED>
+__global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
+    k_pair_contacts(tmps_atoms A, tmps_pair_params P, const tmps_box* __restrict__ B, const tmps_engine* __restrict__ E,
+                    PairLay Q, int np) {
+    using T = typename CfEnv<STYLE, MIXED>::T;
+    using HT = typename CfLoad<MIXED>::HT;
+    using S4 = typename CfLoad<MIXED>::S4;
+    __shared__ double smem[6 * (kBlockC / 32)];
+    __shared__ uint32_t sring[kBlockC / 32][kPairRing];                          // pair | touch bit << 31
+    __shared__ int32_t sfirst[kBlockC / 32][kPairRing], sentry[kBlockC / 32][kPairRing];  // and its words
+    __shared__ float4 soff[MIXED ? 27 : 1], sofl[MIXED ? 27 : 1];
+    __shared__ PairParams32 sP;
+    pdl_enter();
+    if (E->aborted || E->step >= E->stop_step) return;
+    if (rebuild_due(E, E->step + 1)) return;  // S marks the step aborted; the host rebuilds
+    CfEnv<STYLE, MIXED> V;
+    V.load(P, B, E);
+    if constexpr (MIXED) V.tables(P, soff, sofl, sP);
+    double Vd[6] = {0, 0, 0, 0, 0, 0};
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    uint32_t* const ring = sring[wib];
+
+    auto state = [&](int i) {
+        if constexpr (MIXED) return ld4f(A.pos32, i);
+        else return ld4(A.xr, i);
+    };
+    // the law for `cnt` (<= 32) queued pairs from ring position `head`, one per lane
+    auto law = [&](int cnt, int head) {
+        __syncwarp();
+        if (lane < cnt) {
+            const int slot = (head + lane) & (kPairRing - 1);
+            const uint32_t q = ring[slot];
+            const int p = (int)(q & 0x7fffffffu);
+            const int i = sfirst[wib][slot], e = sentry[wib][slot];
+            const int j = e & kNbrIndexMask;
+            CfLoad<MIXED> cl;
+            cl.was = (q >> 31) != 0;
+            const S4 Pi = state(i);
+            cl.pj = state(j);
+            S4 Vi, Wi;
+            float4 PLi = make_float4(0.f, 0.f, 0.f, 0.f);
+            int32_t Ci = 0;
+            cl.cj = 0;
+            cl.jl = PLi;
+            if constexpr (MIXED) {
+                PLi = ld4f(A.pos32lo, i);
+                cl.jl = ld4f(A.pos32lo, j);
+                Vi = ld4f(A.vel32, i);
+                cl.v2 = ld4f(A.vel32, j);
+                Wi = ld4f(A.om32, i);
+                cl.w2 = ld4f(A.om32, j);
+                if (V.vremap) {
+                    Ci = A.cell32[i];
+                    cl.cj = A.cell32[j];
+                }
+            } else {
+                Vi = ld4(A.vm, i);
+                cl.v2 = ld4(A.vm, j);
+                Wi = ld4(A.om, i);
+                cl.w2 = ld4(A.om, j);
+            }
+            HT* const hs = reinterpret_cast<HT*>(Q.shear) + p;
+            HT* const hr = reinterpret_cast<HT*>(Q.rolling) + p;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                cl.shr[c] = HT{};
+                cl.rlr[c] = HT{};
+            }
+            if (V.hist && cl.was) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    cl.shr[c] = hs[(size_t)c * np];
+                    if (V.roll) cl.rlr[c] = hr[(size_t)c * np];
+                }
+            }
+            PairIn<T> in;
+            PairOut<T> out;
+            HT sh[3] = {}, rl[3] = {};
+            bool on;
+            const int code = (unsigned)e >> kNbrIndexBits;
+            const bool lo = i < j;  // always
+            if constexpr (MIXED) on = contact_core<STYLE, MIXED>(V, sP, soff, sofl, lo, code, Pi, PLi, Vi, Wi, Ci, cl, in, out, sh, rl);
+            else on = contact_core<STYLE, MIXED>(V, P, soff, sofl, lo, code, Pi, PLi, Vi, Wi, Ci, cl, in, out, sh, rl);
+            if (on) {
+                if (V.hist) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        hs[(size_t)c * np] = sh[c];
+                        if (V.roll) hr[(size_t)c * np] = rl[c];
+                    }
+                }
+                if constexpr (MIXED) {
+                    float4* r = reinterpret_cast<float4*>(Q.rec) + (size_t)p * (kRecWords<STYLE> / 4);
+                    r[0] = make_float4(out.f[0], out.f[1], out.f[2], out.tor[0]);
+                    if constexpr (STYLE == STYLE_GRANULAR) {
+                        r[1] = make_float4(out.tor[1], out.tor[2], in.d[0], in.d[1]);
+                        r[2] = make_float4(in.d[2], in.delta, out.troll[0], out.troll[1]);
+                        r[3] = make_float4(out.troll[2], 0.f, 0.f, 0.f);
+                    } else {
+                        r[1] = make_float4(out.tor[1], out.tor[2], in.d[0], in.d[1]);
+                        r[2] = make_float4(in.d[2], 0.f, 0.f, 0.f);
+                    }
+                } else {
+                    double2* r = reinterpret_cast<double2*>(Q.rec) + (size_t)p * (kRecDoubles<STYLE> / 2);
+                    r[0] = make_double2(out.f[0], out.f[1]);
+                    r[1] = make_double2(out.f[2], out.tor[0]);
+                    r[2] = make_double2(out.tor[1], out.tor[2]);
+                    if constexpr (STYLE == STYLE_GRANULAR) {
+                        r[3] = make_double2(out.troll[0], out.troll[1]);
+                        r[4] = make_double2(out.troll[2], in.delta);
+                    }
+                    // the pair's virial: half of it each for its two atoms (thermo.py:62-109)
+                    const double v6[6] = {in.d[0] * out.f[0], in.d[1] * out.f[1], in.d[2] * out.f[2],
+                                          in.d[0] * out.f[1], in.d[0] * out.f[2], in.d[1] * out.f[2]};
+#pragma unroll
+                    for (int c = 0; c < 6; ++c) Vd[c] = add_rn(Vd[c], v6[c]);
+                }
+            } else {
+                // within the near test's margin but not touching (mixed form)
+                atomicAnd(&Q.touch[p >> 5], ~(1u << (p & 31)));
+            }
+        }
+        __syncwarp();
+    };
+
+    // all warps sweep the pairs from the last down, so that the gather, which starts with the first
+    // atoms, finds the records written last in L2 (contiguous runs per warp: 6 us slower per step of
+    // 1M jammed spheres)
+    const int words = (np + 31) >> 5;
+    const int nwarps = (gridDim.x * kBlockC) >> 5, gw = blockIdx.x * (kBlockC / 32) + wib;
+    int head = 0, tail = 0;
+    // the words of the next 32 pairs are on their way while these are tested
+    int i_n = 0, e_n = 0;
+    uint32_t old_n = 0u;
+    auto fetch = [&](int w) {
+        const int p = (w << 5) + lane;
+        if (w >= 0) {
+            old_n = Q.touch[w];
+            if (p < np) {
+                i_n = Q.first[p];
+                e_n = Q.entry[p];
+            }
+        }
+    };
+    fetch(words - 1 - gw);
+    for (int w = words - 1 - gw; w >= 0; w -= nwarps) {
+        const int p = (w << 5) + lane;
+        bool near = false;
+        const uint32_t old = old_n;
+        const int i = i_n, e = e_n;
+        fetch(w - nwarps);
+        if (p < np) {
+            const S4 pi = state(i), pj = state(e & kNbrIndexMask);
+            if constexpr (MIXED) {
+                // a conservative FP32 contact test, as in the screened path
+                const float4 so = soff[(unsigned)e >> kNbrIndexBits];
+                const float xi[3] = {pi.x, pi.y, pi.z}, xj[3] = {pj.x, pj.y, pj.z}, oh[3] = {so.x, so.y, so.z};
+                float d[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    d[c] = (xi[c] - xj[c]) - oh[c];
+                    if (V.single[c]) d[c] -= rintf(d[c] * V.iprd[c]) * V.prd[c];
+                }
+                const float rq = (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2];
+                const float rs = (pi.w + pj.w) * 1.00001f;
+                near = rq < rs * rs;
+            } else {
+                // the contact test itself, as the law makes it
+                double d[3] = {pi.x - pj.x, pi.y - pj.y, pi.z - pj.z};
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    if (V.per[c] == 1) d[c] = image_sub64(d[c], rint(d[c] * V.iprd[c]), V.prd[c]);
+                const double rsq = rsq64(d);
+                const double radsum = pi.w + pj.w;
+                near = rsq < __dmul_rn(radsum, radsum) && rsq > 1e-28;
+            }
+        }
+        const uint32_t bal = __ballot_sync(0xffffffffu, near);
+        if (lane == 0 && bal != old) Q.touch[w] = bal;  // before the law, which clears what only came near
+        const uint32_t was = (old >> lane) & 1u;
+        if (near) {
+            const int slot = (tail + __popc(bal & lanemask_lt())) & (kPairRing - 1);
+            ring[slot] = (uint32_t)p | (was << 31);
+            sfirst[wib][slot] = i;
+            sentry[wib][slot] = e;
+        }
+        tail += __popc(bal);
+        if (tail - head >= 32) {
+            law(32, head);
+            head += 32;
+        }
+    }
+    if (tail > head) law(tail - head, head);
+    if constexpr (!MIXED) {
+        block_sum<6, kBlockC>(Vd, smem);
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int c = 0; c < 6; ++c) Q.part[(size_t)c * gridDim.x + blockIdx.x] = Vd[c];
+        }
+    }
+}
+
+constexpr int kBlockG = 256;
+constexpr int kSubG = kBlockG / kBlockC;  // sub-blocks of kBlockC threads
+constexpr int kCompG = 6 / kSubG;         // virial components a sub-block adds
+
+// One lane per atom, in two passes over its row: the first only finds the
+// touching slots (pair indices, coalesced over the lanes, and the pairs' touch
+// bits), the second runs over those alone, so a warp makes as many rounds as
+// its busiest atom has contacts, not list entries (about 7 of 11 on a jammed
+// packing), the next record on its way while one is summed.
+//
+// One block takes kSubG consecutive strides of kBlockC atoms at once, one per
+// sub-block.  The mixed form's virial terms then go through shared memory:
+// sub-block u adds kCompG of the six components of the kSubG strides' atoms in
+// stride order, so every sum is that of a kBlockC-thread block that takes the
+// strides one after another (those bits are wanted; see above), with more
+// warps and the additions spread over all of them.
+template <int STYLE, bool MIXED>
+__global__ void __launch_bounds__(kBlockG, MIXED ? 4 : 3)
+    k_pair_gather(tmps_atoms A, tmps_nlist L, const tmps_box* __restrict__ B, tmps_engine* __restrict__ E,
+                  uint32_t* __restrict__ flags, double* __restrict__ part, PairLay Q) {
+    using T = typename std::conditional<MIXED, float, double>::type;
+    using W4 = typename std::conditional<MIXED, float4, double2>::type;
+    constexpr int kW = MIXED ? kRecWords<STYLE> / 4 : kRecDoubles<STYLE> / 2;  // 16-byte words of a record
+    __shared__ double smem[6 * (kBlockG / 32)];
+    __shared__ float sV[MIXED ? 6 : 1][kBlockG];
+    pdl_enter();
+    if (E->aborted || E->step >= E->stop_step) return;
+    if (rebuild_due(E, E->step + 1)) return;
+    const int nb = E->nblocks;
+    part += nb - gridDim.x;  // C's blocks follow A's
+    const int n = A.n, lane = threadIdx.x & 31;
+    T dt, gl, ga;
+    if constexpr (MIXED) {
+        dt = E->dt_hi;
+        gl = E->gamma_lin32;
+        ga = E->gamma_ang32;
+    } else {
+        dt = E->dt;
+        gl = E->gamma_lin;
+        ga = E->gamma_ang;
+    }
+    const bool cundall = E->cundall != 0;
+    double Vd[6] = {0, 0, 0, 0, 0, 0};
+    float Vh[kCompG] = {}, Vl[kCompG] = {};  // mixed: components kCompG sub ..
+    const int sub = threadIdx.x / kBlockC, tid = threadIdx.x % kBlockC;
+    const long long stride = (long long)gridDim.x * kBlockC;
+    for (long long first = (long long)blockIdx.x * kBlockC; first < n; first += kSubG * stride) {
+        const long long at = first + sub * stride + (tid & ~31);
+        const bool inside = at < n;  // warp-uniform
+        const int base = inside ? (int)at : 0;
+        const int i = base + lane;
+        const bool mine = inside && i < n;
+        const int nn = mine ? L.nnb[i] : 0;
+        const uint32_t old = inside ? flags[base >> 5] : 0u;
+        T vi[3] = {0, 0, 0}, wi[3] = {0, 0, 0}, mi = 0, ri = 0;
+        if (mine) {
+            if constexpr (MIXED) {
+                const float4 v = ld4f(A.vel32, i), w = ld4f(A.om32, i);
+                vi[0] = v.x; vi[1] = v.y; vi[2] = v.z; mi = v.w;
+                wi[0] = w.x; wi[1] = w.y; wi[2] = w.z;
+                ri = A.pos32[4 * (size_t)i + 3];
+            } else {
+                const double4 v = ld4(A.vm, i), w = ld4(A.om, i);
+                vi[0] = v.x; vi[1] = v.y; vi[2] = v.z; mi = v.w;
+                wi[0] = w.x; wi[1] = w.y; wi[2] = w.z;
+                ri = A.xr[4 * (size_t)i + 3];
+            }
+        }
+        // the touching slots, four entries at a time
+        uint64_t on = 0ull;
+        for (int k0 = 0; k0 < nn; k0 += 4) {
+            int32_t r[4];
+            uint32_t w[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) r[u] = k0 + u < nn ? Q.row[(size_t)(k0 + u) * n + i] : kPairNone;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) w[u] = r[u] != kPairNone ? Q.touch[(r[u] & 0x7fffffff) >> 5] : 0u;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) on |= (uint64_t)((w[u] >> (r[u] & 31)) & 1u) << (k0 + u);
+        }
+        T F[3] = {0, 0, 0}, Tq[3] = {0, 0, 0};
+        float V[6] = {0, 0, 0, 0, 0, 0};  // mixed: the atom's virial terms
+        const bool any = on != 0ull;
+        // their records in slot order
+        int32_t r = 0;
+        W4 q[kW];
+        auto fetch = [&]() {
+            if (on == 0ull) return;
+            r = Q.row[(size_t)(__ffsll((long long)on) - 1) * n + i];
+            const W4* const rec = reinterpret_cast<const W4*>(Q.rec) + (size_t)(r & 0x7fffffff) * kW;
+#pragma unroll
+            for (int w = 0; w < kW; ++w) q[w] = rec[w];
+        };
+        fetch();
+        while (on != 0ull) {
+            const bool second = r < 0;
+            W4 c[kW];
+#pragma unroll
+            for (int w = 0; w < kW; ++w) c[w] = q[w];
+            on &= on - 1ull;
+            fetch();
+            T f[3], tor[3], troll[3] = {0, 0, 0}, arm = -ri;
+            if constexpr (MIXED) {
+                f[0] = c[0].x; f[1] = c[0].y; f[2] = c[0].z;
+                tor[0] = c[0].w; tor[1] = c[1].x; tor[2] = c[1].y;
+                const float d[3] = {c[1].z, c[1].w, c[2].x};
+                V[0] += 0.5f * (d[0] * f[0]);
+                V[1] += 0.5f * (d[1] * f[1]);
+                V[2] += 0.5f * (d[2] * f[2]);
+                V[3] += 0.5f * (d[0] * f[1]);
+                V[4] += 0.5f * (d[0] * f[2]);
+                V[5] += 0.5f * (d[1] * f[2]);
+                if constexpr (STYLE == STYLE_GRANULAR) {
+                    arm = ri - 0.5f * c[2].y;
+                    troll[0] = c[2].z; troll[1] = c[2].w; troll[2] = c[kW - 1].x;
+                }
+            } else {
+                f[0] = c[0].x; f[1] = c[0].y; f[2] = c[1].x;
+                tor[0] = c[1].y; tor[1] = c[2].x; tor[2] = c[2].y;
+                if constexpr (STYLE == STYLE_GRANULAR) {
+                    arm = ri - 0.5 * c[kW - 1].y;
+                    troll[0] = c[kW - 2].x; troll[1] = c[kW - 2].y; troll[2] = c[kW - 1].x;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                F[k] += second ? -f[k] : f[k];
+                const T t = mul_rn(arm, tor[k]);
+                if constexpr (STYLE == STYLE_GRANULAR) Tq[k] += add_rn(t, second ? -troll[k] : troll[k]);
+                else Tq[k] = add_rn(Tq[k], t);
+            }
+        }
+        if (any) {
+            if (cundall) {  // FixDampingCundall.post_force_kernel
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const T sf = F[c] * vi[c] >= T(0) ? T(1) : T(-1);
+                    F[c] *= T(1) - gl * sf;
+                    const T st = Tq[c] * wi[c] >= T(0) ? T(1) : T(-1);
+                    Tq[c] *= T(1) - ga * st;
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if constexpr (MIXED) {
+                    A.f32[c * n + i] = F[c];
+                    A.torque32[c * n + i] = Tq[c];
+                } else {
+                    A.f[c * n + i] = F[c];
+                    A.torque[c * n + i] = Tq[c];
+                }
+            }
+            // the kinetic correction for the end-of-step velocity (the screened path's step 5)
+            T im;
+            if constexpr (MIXED) im = __fdividef(1.0f, mi);
+            else im = A.rinv[i];
+            const T hdt = T(0.5) * dt;
+            T vf[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) vf[c] = vi[c] + hdt * (F[c] * im);
+            const T kin[6] = {(mi * vf[0]) * vf[0], (mi * vf[1]) * vf[1], (mi * vf[2]) * vf[2],
+                              (mi * vf[0]) * vf[1], (mi * vf[0]) * vf[2], (mi * vf[1]) * vf[2]};
+            const T kh[6] = {(mi * vi[0]) * vi[0], (mi * vi[1]) * vi[1], (mi * vi[2]) * vi[2],
+                             (mi * vi[0]) * vi[1], (mi * vi[0]) * vi[2], (mi * vi[1]) * vi[2]};
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                if constexpr (MIXED) V[c] = V[c] + (kin[c] - kh[c]);
+                else Vd[c] += kin[c] - kh[c];
+            }
+        }
+        // the group's new flag word; stale forces of atoms no longer flagged
+        const uint32_t w = __ballot_sync(0xffffffffu, any);
+        if (inside && lane == 0 && w != old) flags[base >> 5] = w;
+        if (mine && ((old >> lane) & 1u) && !any) zero_force<MIXED>(A, i);
+        if constexpr (MIXED) {
+#pragma unroll
+            for (int c = 0; c < 6; ++c) sV[c][threadIdx.x] = V[c];
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < kSubG; ++u)
+#pragma unroll
+                for (int k = 0; k < kCompG; ++k) dw_add(Vh[k], Vl[k], sV[sub * kCompG + k][u * kBlockC + tid]);
+            __syncthreads();
+        }
+    }
+    if constexpr (MIXED) {
+        // block_sum_dw over the kBlockC threads of each component
+        float2* const ws = reinterpret_cast<float2*>(smem);
+#pragma unroll
+        for (int k = 0; k < kCompG; ++k) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const float bh = __shfl_down_sync(0xffffffffu, Vh[k], o), bl = __shfl_down_sync(0xffffffffu, Vl[k], o);
+                dw_add2(Vh[k], Vl[k], bh, bl);
+            }
+            if (lane == 0) ws[(sub * kCompG + k) * (kBlockC / 32) + (tid >> 5)] = make_float2(Vh[k], Vl[k]);
+        }
+        __syncthreads();
+        if (threadIdx.x < 6) {
+            static_assert(kBlockC == 128, "four warps: the tree adds w and w + 2, then the two sums");
+            float2 w[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w[k] = ws[threadIdx.x * 4 + k];
+            dw_add2(w[0].x, w[0].y, w[2].x, w[2].y);
+            dw_add2(w[1].x, w[1].y, w[3].x, w[3].y);
+            dw_add2(w[0].x, w[0].y, w[1].x, w[1].y);
+            reinterpret_cast<float2*>(part)[(size_t)threadIdx.x * nb + blockIdx.x] = w[0];
+        }
+    } else {
+        block_sum<6, kBlockG>(Vd, smem);
+        if (threadIdx.x == 0) {
+            // the pair pass's partial of the same number joins this block's
+#pragma unroll
+            for (int c = 0; c < 6; ++c)
+                part[(size_t)c * nb + blockIdx.x] = Vd[c] + Q.part[(size_t)c * gridDim.x + blockIdx.x];
+        }
+    }
+    if (threadIdx.x == 0 && blockIdx.x == 0) E->final_pending = 1;
 }
 
 // ---------------------------------------------------------------------- S
@@ -2098,7 +2582,7 @@ __global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
     char* sc = static_cast<char*>(I.scratch);
     const int n = I.a.n;
     double* part = reinterpret_cast<double*>(sc + lay_part(n));
-    cf_body<STYLE, MIXED, false>(I.a, I.nl, I.p, I.box, I.eng, reinterpret_cast<uint32_t*>(sc),
+    cf_body<STYLE, MIXED>(I.a, I.nl, I.p, I.box, I.eng, reinterpret_cast<uint32_t*>(sc),
                           reinterpret_cast<const float*>(sc + lay_gap(n)), reinterpret_cast<const float*>(sc + lay_agap(n)),
                           reinterpret_cast<const int32_t*>(sc + lay_order(n)),
                           reinterpret_cast<const float*>(sc + lay_sgap(n)), part, (int)blockIdx.x - I.c_first,
@@ -2191,6 +2675,7 @@ __global__ void k_prepare_engine(const tmps_box* __restrict__ b, tmps_engine* e,
     e->part_off = part_off;
     e->cull = 0;  // until tmps_fused_bounds sets the bounds
     e->touching = 0;
+    e->pairs = 0;
     e->kick_all = 0;  // k_prepare, launched next, sets it for an atom of odd mass or inertia
     e->maxd2_bits = 0u;
     e->shift_bound = 0.0f;
@@ -2444,6 +2929,16 @@ __global__ void __launch_bounds__(256) k_history_form(tmps_nlist L, int to_dw) {
     }
 }
 
+bool has_history(const tmps_pair_params* p) {
+    return p->style == 1 || p->style == 3 || (p->style == 4 && (p->tangential_id >= 2 || p->rolling_id != 0));
+}
+bool pairs_ok(const tmps_nlist* nl, const tmps_pair_params* p, int32_t npairs, const void* pairs) {
+    if (!nl || !p || !pairs || nl->n < 0 || npairs < 0 || p->style < 0 || p->style > 4) return false;
+    if (nl->slots < 1 || nl->slots > kMaxSlots || !nl->nbr || !nl->nnb) return false;
+    if (has_history(p) && (!nl->touch || !nl->shear)) return false;
+    return !(p->style == 4 && p->rolling_id != 0 && !nl->rolling);
+}
+
 }  // namespace
 
 extern "C" {
@@ -2517,6 +3012,7 @@ int tmps_fused_c(const tmps_atoms* a, const tmps_nlist* nl, const tmps_box* d_bo
     if (!a->pos32 && !a->rinv) return TMPS_ERR_BAD_ARG;
     if (p->style < 0 || p->style > 4 || nl->slots < 1 || nl->slots > kMaxSlots) return TMPS_ERR_BAD_ARG;
     if (p->style == 4 && p->rolling_id != 0 && !nl->rolling) return TMPS_ERR_BAD_ARG;
+    (void)rows;  // once chose a path for contact-dense states, which tmps_fused_c_pairs is now
     const int n = a->n;
     const bool mixed = a->pos32 != nullptr;
     const int g2def = contact_blocks(n, p->style, mixed);
@@ -2530,11 +3026,7 @@ int tmps_fused_c(const tmps_atoms* a, const tmps_nlist* nl, const tmps_box* d_bo
     cudaStream_t s = (cudaStream_t)stream;
     if (mixed && !mixed_ok(a)) return TMPS_ERR_BAD_ARG;
 #define TMPS_LAUNCH_C(ST)                                                                                          \
-    if (mixed && rows) launch_pdl(k_cf<ST, true, true>, g2, kBlockC, s, *a, *nl, *p, d_box, d_eng, flags, gap, agap, \
-                                  part2);                                                                        \
-    else if (mixed) launch_pdl(k_cf<ST, true>, g2, kBlockC, s, *a, *nl, *p, d_box, d_eng, flags, gap, agap, part2); \
-    else if (rows) launch_pdl(k_cf<ST, false, true>, g2, kBlockC, s, *a, *nl, *p, d_box, d_eng, flags, gap, agap,   \
-                              part2);                                                                            \
+    if (mixed) launch_pdl(k_cf<ST, true>, g2, kBlockC, s, *a, *nl, *p, d_box, d_eng, flags, gap, agap, part2); \
     else launch_pdl(k_cf<ST, false>, g2, kBlockC, s, *a, *nl, *p, d_box, d_eng, flags, gap, agap, part2);
     switch (p->style) {
         case 0: TMPS_LAUNCH_C(0) break;
@@ -2545,6 +3037,72 @@ int tmps_fused_c(const tmps_atoms* a, const tmps_nlist* nl, const tmps_box* d_bo
     }
 #undef TMPS_LAUNCH_C
     note_launches(1);
+    return launch_ok() ? TMPS_OK : TMPS_ERR_CUDA;
+}
+
+int64_t tmps_pairs_bytes(int32_t n, int32_t slots, int32_t npairs, int32_t style, int32_t mixed, int32_t rolling) {
+    if (n < 0 || slots < 1 || slots > kMaxSlots || npairs < 0 || style < 0 || style > 4) return -1;
+    return (int64_t)pair_lay(nullptr, n, slots, npairs, style, mixed != 0, rolling != 0).bytes;
+}
+
+int tmps_pairs_build(const tmps_nlist* nl, const tmps_pair_params* p, int32_t npairs, int32_t mixed, void* pairs,
+                     void* stream) {
+    if (!pairs_ok(nl, p, npairs, pairs)) return TMPS_ERR_BAD_ARG;
+    if (nl->n == 0) return TMPS_OK;
+    cudaStream_t s = (cudaStream_t)stream;
+    const int n = nl->n, g = grid_for(n, 256);
+    const PairLay Q = pair_lay(pairs, n, nl->slots, npairs, p->style, mixed != 0, p->rolling_id != 0);
+    if (cudaMemsetAsync(Q.touch, 0, ((size_t)npairs + 31) / 32 * 4, s) != cudaSuccess) return TMPS_ERR_CUDA;
+    k_pair_count<<<g, 256, 0, s>>>(*nl, Q.count);
+    exclusive_scan(Q.count, Q.begin, Q.count + n, n, s);
+    k_pair_fill<<<g, 256, 0, s>>>(*nl, Q, npairs, has_history(p) ? 1 : 0, mixed ? 1 : 0);
+    k_pair_back<<<g, 256, 0, s>>>(*nl, Q);
+    note_launches(5);
+    return launch_ok() ? TMPS_OK : TMPS_ERR_CUDA;
+}
+
+int tmps_pairs_history(const tmps_nlist* nl, const tmps_pair_params* p, int32_t npairs, int32_t mixed, void* pairs,
+                       void* stream) {
+    if (!pairs_ok(nl, p, npairs, pairs)) return TMPS_ERR_BAD_ARG;
+    if (nl->n == 0 || !has_history(p)) return TMPS_OK;
+    const PairLay Q = pair_lay(pairs, nl->n, nl->slots, npairs, p->style, mixed != 0, p->rolling_id != 0);
+    k_pair_history<<<grid_for(nl->n, 256), 256, 0, (cudaStream_t)stream>>>(*nl, Q, npairs, mixed ? 1 : 0);
+    note_launches(1);
+    return launch_ok() ? TMPS_OK : TMPS_ERR_CUDA;
+}
+
+int tmps_fused_c_pairs(const tmps_atoms* a, const tmps_nlist* nl, const tmps_box* d_box, tmps_engine* d_eng,
+                       const tmps_pair_params* p, int32_t c_blocks, void* scratch, int32_t npairs, void* pairs,
+                       void* stream) {
+    if (!a || !d_box || !d_eng || !scratch || a->n < 0 || !pairs_ok(nl, p, npairs, pairs) || nl->n != a->n)
+        return TMPS_ERR_BAD_ARG;
+    const int n = a->n;
+    const bool mixed = a->pos32 != nullptr;
+    if (mixed ? !mixed_ok(a) : !a->rinv) return TMPS_ERR_BAD_ARG;
+    const int gdef = contact_blocks(n, p->style, mixed);
+    if (c_blocks > gdef || gdef > kPairMaxBlocks) return TMPS_ERR_BAD_ARG;
+    const int g = c_blocks > 0 ? c_blocks : gdef;
+    const PairLay Q = pair_lay(pairs, n, nl->slots, npairs, p->style, mixed, p->rolling_id != 0);
+    uint32_t* flags = (uint32_t*)scratch;
+    double* part = (double*)((char*)scratch + part_offset(n));
+    cudaStream_t s = (cudaStream_t)stream;
+#define TMPS_LAUNCH_P(ST)                                                                                           \
+    if (mixed) {                                                                                                    \
+        launch_pdl(k_pair_contacts<ST, true>, g, kBlockC, s, *a, *p, d_box, (const tmps_engine*)d_eng, Q, (int)npairs); \
+        launch_pdl(k_pair_gather<ST, true>, g, kBlockG, s, *a, *nl, d_box, d_eng, flags, part, Q);                  \
+    } else {                                                                                                        \
+        launch_pdl(k_pair_contacts<ST, false>, g, kBlockC, s, *a, *p, d_box, (const tmps_engine*)d_eng, Q, (int)npairs); \
+        launch_pdl(k_pair_gather<ST, false>, g, kBlockG, s, *a, *nl, d_box, d_eng, flags, part, Q);                 \
+    }
+    switch (p->style) {
+        case 0: TMPS_LAUNCH_P(0) break;
+        case 1: TMPS_LAUNCH_P(1) break;
+        case 2: TMPS_LAUNCH_P(2) break;
+        case 3: TMPS_LAUNCH_P(3) break;
+        default: TMPS_LAUNCH_P(4) break;
+    }
+#undef TMPS_LAUNCH_P
+    note_launches(2);
     return launch_ok() ? TMPS_OK : TMPS_ERR_CUDA;
 }
 
@@ -2562,14 +3120,12 @@ int tmps_fused_bounds(const tmps_atoms* a, const tmps_nlist* nl, const tmps_box*
         return TMPS_ERR_BAD_ARG;
     if (nl->slots < 1 || nl->slots > kMaxSlots) return TMPS_ERR_BAD_ARG;
     const int n = a->n;
-    const bool has_hist = p->style == 1 || p->style == 3 ||
-                          (p->style == 4 && (p->tangential_id >= 2 || p->rolling_id != 0));
     uint32_t* flags = (uint32_t*)scratch;
     float* gap = (float*)((char*)scratch + gap_offset(n));
     float* agap = (float*)((char*)scratch + atom_gap_offset(n));
     const int g = n > 0 ? grid_for(n, kBlockA) : 1;
     cudaStream_t st = (cudaStream_t)stream;
-    k_bounds<<<g, kBlockA, 0, st>>>(*a, *nl, d_box, d_eng, has_hist ? 1 : 0, cull ? 1 : 0, flags, gap, agap,
+    k_bounds<<<g, kBlockA, 0, st>>>(*a, *nl, d_box, d_eng, has_history(p) ? 1 : 0, cull ? 1 : 0, flags, gap, agap,
                                   (double*)((char*)scratch + lay_kin(n)));
     note_launches(1);
     if (cull && n > 0) {

@@ -419,15 +419,15 @@ bool launch_ok() { return cudaPeekAtLastError() == cudaSuccess; }
 
 size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
+}  // namespace
+
 // start = exclusive scan of count over m cells; tile_sum (at least one word per
 // kScanTile cells, m words always suffice) holds the tile totals in between
-void scan_cells(const int32_t* count, int32_t* start, int32_t* tile_sum, int m, cudaStream_t s) {
+void tmps::exclusive_scan(const int32_t* count, int32_t* start, int32_t* tile_sum, int m, cudaStream_t s) {
     const int tiles = (m + kScanTile - 1) / kScanTile;
     k_scan_tiles<<<tiles, kScanBlock, 0, s>>>(count, m, tile_sum);
     k_scan_apply<<<tiles, kScanBlock, 0, s>>>(count, start, m, tile_sum);
 }
-
-}  // namespace
 
 extern "C" {
 
@@ -466,7 +466,7 @@ int tmps_nlist_build(const tmps_atoms* src, const tmps_atoms* dst, const tmps_bo
     if (cudaMemsetAsync(count, 0, (size_t)m * 4, s) != cudaSuccess) return TMPS_ERR_CUDA;
     const int gb = grid_for(n, kBlock);
     k_bin<<<gb, kBlock, 0, s>>>(*src, d_box, cell_rank, old_cell, count, d_status);
-    scan_cells(count, start, fill, m, s);
+    exclusive_scan(count, start, fill, m, s);
     // `fill` held the scan's tile totals; the scatter counts in it from zero
     if (cudaMemsetAsync(fill, 0, (size_t)m * 4, s) != cudaSuccess) return TMPS_ERR_CUDA;
     k_scatter<<<gb, kBlock, 0, s>>>(n, cell_rank, old_cell, start, fill, order);
@@ -555,7 +555,7 @@ extern "C" int tmps_nlist_build_noalloc(const tmps_atoms* src, const tmps_atoms*
     if (cudaMemsetAsync(count, 0, (size_t)m * 4, s) != cudaSuccess) return TMPS_ERR_CUDA;
     const int gb = grid_for(n, kBlock);
     k_bin<<<gb, kBlock, 0, s>>>(*src, d_box, cell_rank, old_cell, count, d_status);
-    scan_cells(count, start, fill, m, s);
+    exclusive_scan(count, start, fill, m, s);
     // `fill` held the scan's tile totals; the scatter counts in it from zero
     if (cudaMemsetAsync(fill, 0, (size_t)m * 4, s) != cudaSuccess) return TMPS_ERR_CUDA;
     k_scatter<<<gb, kBlock, 0, s>>>(n, cell_rank, old_cell, start, fill, order);

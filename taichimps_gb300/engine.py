@@ -51,8 +51,9 @@ def fusable(sim) -> bool:
 
 
 class FusedEngine:
-    # kernels per step: A, C, S
+    # kernels per step: A, C, S (C is two launches on the rows path)
     LAUNCHES_PER_STEP = 3
+    MAX_PAIRS = 2**31 - 64  # pair indices carry one more bit
 
     def __init__(self, sim, precision: str = "fp64", chunk: int = 64, graphs: bool = True,
                  cull: bool = True, launch_shape: tuple[int, int] | None = None,
@@ -84,12 +85,15 @@ class FusedEngine:
         # C skips 32-atom groups whose gap bound rules out any contact (exact;
         # off screens every group, with bit-identical results)
         self.cull = bool(cull)
-        # C's path (tmps_fused_c): "screened" rules contact-free 32-atom groups out and runs the contacts
-        # of the rest 32 at a time; "rows" runs every atom's row, one thread per atom; "auto" picks rows
-        # for the mixed form at a build where more than half of the atoms touch or overlap at the build
-        # positions (their gap bound is <= 0), screened otherwise (the FP64 form's screened path was
-        # measured faster on contact-dense states too).  Both paths sum each atom's contacts in slot
-        # order with the same per-contact code; only the order of the virial partial sums differs.
+        # C's path: "screened" (tmps_fused_c) rules contact-free 32-atom groups out and runs the contacts
+        # of the rest 32 at a time, each for both of its atoms; "rows" (tmps_fused_c_pairs) runs every
+        # contact once and sums every atom's row from the pairs' records.  "auto" picks rows at a build
+        # where more than half of the atoms touch or overlap at the build positions (their gap bound is
+        # <= 0): there the screen rules out little and half of the contact arithmetic is saved (jammed
+        # packings, C per step: 1M spheres mixed 278 -> 193 us, 109k FP64 363 -> 177 us); on dilute
+        # states the screen reads a few bytes per group where rows would read every list entry.  Both
+        # paths sum each atom's contacts in slot order with the same per-contact code; only the order of
+        # the virial sums differs.
         self.contact_path = contact_path
         self.rows = contact_path == "rows"
         # launch shape (tmps_fused_shape): 32-atom groups per warp of A and of C, 0 = the default grid;
@@ -103,6 +107,11 @@ class FusedEngine:
         self._seen_key = None
         self.capture_first = False
         self._hist_dw = False
+        # the rows path's buffer (tmps_pairs_*): the pairs of the current build and, while `_in_pairs`,
+        # the contact histories
+        self.pairs: torch.Tensor | None = None
+        self.npairs = 0
+        self._in_pairs = False
         self.graph_replays = 0
         self.graph_kernel_launches = 0
         # (engine record, status) as the last run() left them, while nothing has been launched since:
@@ -239,25 +248,54 @@ class FusedEngine:
         rc = L.tmps_fused_bounds(atoms, sim.history.cstruct(nl), sim.domain.dbox, self._eng.data_ptr(),
                                  sim.pair_style.params, 1 if self.cull else 0, self.part.data_ptr(), st)
         _lib.check(rc, "tmps_fused_bounds")
-        # one synchronisation for what the host needs before the steps: the count of touching atoms
-        # (the contact path) and the status of a neighbor build that did not wait for the device
-        auto_rows = self.contact_path == "auto" and self.mixed
+        # one synchronisation for what the host needs before the steps: the counts of touching atoms
+        # and of pairs (the contact path) and the status of a neighbor build that did not wait for the
+        # device
+        counts = self.contact_path != "screened"
         items = []
-        if auto_rows:
+        if counts:
             off = _lib.Engine.touching.offset
-            items.append((self._eng[off:off + 4], None))
+            items.append((self._eng[off:], None))
         if nl.status_pending:
             items.append((nl.status, None))
         got = _device.pull_many(items) if items else []
         if nl.status_pending:
             nl.check_status(int(got[-1].view(np.int32)[0]))
-        if self.contact_path == "auto" and not self.mixed:
-            self.rows = False
-        elif auto_rows:
-            # the bounds kernel counted the atoms whose gap bound is <= 0 into the engine record
-            touching = int(got[0].view(np.int32)[0])
-            self.rows = self._n > 0 and touching * 2 > self._n
-        self._history_form(True)
+        if counts:
+            # the bounds kernel counted the atoms whose gap bound is <= 0, and the pairs, into the
+            # engine record
+            touching = int(got[0][:4].view(np.int32)[0])
+            at = _lib.Engine.pairs.offset - off
+            self.npairs = int(got[0][at:at + 8].view(np.int64)[0])
+            self.rows = self.contact_path == "rows" or touching * 2 > self._n
+            self.rows = self.rows and self._n > 0 and self.npairs <= self.MAX_PAIRS
+        if self.rows:
+            self._build_pairs()
+        else:
+            self._history_form(True)
+
+    def _build_pairs(self) -> None:
+        """The rows path's pair buffer for the current list, with the contact histories."""
+        sim = self.sim
+        nl, par, L = sim.neighbor, sim.pair_style.params, _device.lib()
+        mixed = 1 if self.mixed else 0
+        need = int(L.tmps_pairs_bytes(self._n, nl.slots, self.npairs, int(par.style), mixed, int(par.rolling_id)))
+        if self.pairs is None or self.pairs.numel() < need:
+            self.pairs = None
+            self.pairs = torch.empty(need, dtype=torch.uint8, device=self.dev)
+        _lib.check(L.tmps_pairs_build(sim.history.cstruct(nl), par, self.npairs, mixed, self.pairs.data_ptr(),
+                                      _device.stream()), "tmps_pairs_build")
+        self._in_pairs = True
+
+    def _history_back(self) -> None:
+        """The contact histories back in the list's rows as doubles, both copies of each."""
+        if self._in_pairs:
+            sim = self.sim
+            _lib.check(_device.lib().tmps_pairs_history(sim.history.cstruct(sim.neighbor), sim.pair_style.params,
+                                                        self.npairs, 1 if self.mixed else 0, self.pairs.data_ptr(),
+                                                        _device.stream()), "tmps_pairs_history")
+            self._in_pairs = False
+        self._history_form(False)
 
     def _history_form(self, dw: bool) -> None:
         """The mixed form keeps the contact histories as FP32 double words while it runs, and
@@ -276,12 +314,19 @@ class FusedEngine:
             rc = L.tmps_fused_a(atoms, dbox, eng, self.a_blocks, self.part.data_ptr(), st)
         _lib.check(rc, "tmps_fused_a")
         with _device.timed("fused_c"):
-            rc = L.tmps_fused_c(atoms, nl_struct, dbox, eng, params, self.c_blocks, self.part.data_ptr(),
-                                1 if self.rows else 0, st)
-        _lib.check(rc, "tmps_fused_c")
+            self._launch_c(L, st, atoms, nl_struct, params)
         with _device.timed("fused_s"):
             rc = L.tmps_fused_servo(dbox, self._servo_ptr(), eng, self.part.data_ptr(), self.status.data_ptr(), st)
         _lib.check(rc, "tmps_fused_servo")
+
+    def _launch_c(self, L, st, atoms, nl_struct, params) -> None:
+        dbox, eng, part = self.sim.domain.dbox, self._eng.data_ptr(), self.part.data_ptr()
+        if self.rows:
+            _lib.check(L.tmps_fused_c_pairs(atoms, nl_struct, dbox, eng, params, self.c_blocks, part, self.npairs,
+                                            self.pairs.data_ptr(), st), "tmps_fused_c_pairs")
+        else:
+            _lib.check(L.tmps_fused_c(atoms, nl_struct, dbox, eng, params, self.c_blocks, part, 0, st),
+                       "tmps_fused_c")
 
     def instance(self, a_first: int, a_blocks: int, c_first: int, c_blocks: int) -> _lib.Instance:
         """This system's descriptor for a batched run (tmps_instance)."""
@@ -354,7 +399,7 @@ class FusedEngine:
         self._known = None
         sim = self.sim
         key = (sim.neighbor.build_count, sim.atom.buffers.xr.data_ptr(), sim.history.touch.data_ptr(),
-               sim.neighbor.nbr.data_ptr(), self.rows, self.chunk)
+               sim.neighbor.nbr.data_ptr(), self.rows, self.pairs.data_ptr() if self.rows else 0, self.chunk)
         if self._graph is None or self._graph_key != key:
             self._graph = None
             atoms = self.atoms()
@@ -378,7 +423,7 @@ class FusedEngine:
             self._graph, self._graph_key = _device.capture_graph(chunk), key
         self._graph.replay()
         self.graph_replays += 1
-        self.graph_kernel_launches += self.chunk * self.LAUNCHES_PER_STEP
+        self.graph_kernel_launches += self.chunk * (self.LAUNCHES_PER_STEP + (1 if self.rows else 0))
 
     def cull_stats(self) -> tuple[int, int]:
         """(32-atom groups, groups the contact bound rules out right now), from the
@@ -424,7 +469,7 @@ class FusedEngine:
         nl.current_step = s
         if self.mixed:
             _lib.check(L.tmps_mixed_unpack(self.atoms(), sim.domain.dbox, st), "tmps_mixed_unpack")
-        self._history_form(False)
+        self._history_back()
         sim.domain.mark_device_authoritative()
         sim.domain.pull()
         sim.history.save_state(atom, nl)
@@ -442,8 +487,7 @@ class FusedEngine:
         atoms = self.atoms()
         nl_struct = sim.history.cstruct(nl)
         dbox, eng = sim.domain.dbox, self._eng.data_ptr()
-        _lib.check(L.tmps_fused_c(atoms, nl_struct, dbox, eng, sim.pair_style.params, self.c_blocks,
-                                  self.part.data_ptr(), 1 if self.rows else 0, st), "tmps_fused_c")
+        self._launch_c(L, st, atoms, nl_struct, sim.pair_style.params)
         _lib.check(L.tmps_fused_servo(dbox, self._servo_ptr(), eng, self.part.data_ptr(), self.status.data_ptr(),
                                       st), "tmps_fused_servo")
 
@@ -460,7 +504,7 @@ class FusedEngine:
         _lib.check(L.tmps_fused_settle(atoms, sim.domain.dbox, self._eng.data_ptr(), st), "tmps_fused_settle")
         if self.mixed:
             _lib.check(L.tmps_mixed_unpack(atoms, sim.domain.dbox, st), "tmps_mixed_unpack")
-        self._history_form(False)
+        self._history_back()
         sim.domain.mark_device_authoritative()
         # the engine record, the status word, the box and the servo record: one synchronisation
         items = [(self._eng, _lib.Engine), (self.status, None), (sim.domain.dbox_tensor, _lib.Box)]
