@@ -96,6 +96,65 @@ TMPS_DEV void split_dw(double v, float& hi, float& lo) {
     lo = f32_rn(__dsub_rn(v, f64_of(hi)));
 }
 
+// FP64 reciprocals and square roots.  This part issues an FP64 instruction for
+// a warp every 16 cycles per SM, and the compiler's correctly rounded division
+// and square root are some ten to twenty of them each.  These start from the
+// hardware's 20-bit approximations (rcp.approx, rsqrt.approx: not on the FP64
+// pipe) and take one third-order step -- Halley's iteration, whose error is
+// the cube of the seed's -- in three to five instructions; results are within
+// two units in the last place (sqrt64's root within one).  Arguments outside
+// 2^+-1000, zeros, infinities and NaNs take the correctly rounded operation.
+TMPS_DEV bool plain64(double x) {
+    const int e = (__double2hiint(x) >> 20) & 0x7ff;
+    return e >= 23 && e <= 2023;
+}
+
+// 1 / x
+TMPS_DEV double rcp64(double x) {
+    if (!plain64(x)) return 1.0 / x;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = __fma_rn(-x, y, 1.0);
+    return __fma_rn(y, __fma_rn(e, e, e), y);
+}
+
+// 1 / sqrt(x) for x > 0
+TMPS_DEV double rsqrt64(double x) {
+    if (!plain64(x) || !(__double2hiint(x) > 0)) return 1.0 / sqrt(x);
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = __fma_rn(-__dmul_rn(x, y), y, 1.0);
+    return __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
+}
+
+// root = sqrt(x) and inv = 1 / sqrt(x): the product x * inv corrected by its
+// own residual, which rounds it correctly (Markstein) but for rare last bits.
+TMPS_DEV void sqrt_rsqrt64(double x, double& root, double& inv) {
+    if (!plain64(x) || !(__double2hiint(x) > 0)) {
+        root = sqrt(x);
+        inv = 1.0 / root;
+        return;
+    }
+    inv = rsqrt64(x);
+    const double g = __dmul_rn(x, inv);
+    root = __fma_rn(__fma_rn(-g, g, x), __dmul_rn(0.5, inv), g);
+}
+TMPS_DEV double sqrt64(double x) {
+    double root, inv;
+    sqrt_rsqrt64(x, root, inv);
+    return root;
+}
+
+// a * b >= 0.0, as the FP64 product compares: from the sign bits where the
+// exponents keep the product clear of underflow (and neither is a NaN), the
+// product itself otherwise.
+TMPS_DEV bool prod_nonneg(double a, double b) {
+    const int ha = __double2hiint(a), hb = __double2hiint(b);
+    const int ea = (ha >> 20) & 0x7ff, eb = (hb >> 20) & 0x7ff;
+    if (ea > 0x200 && ea < 0x600 && eb > 0x200 && eb < 0x600) return (ha ^ hb) >= 0;
+    return a * b >= 0.0;
+}
+
 TMPS_DEV double4 ld4(const double* p, int i) { return reinterpret_cast<const double4*>(p)[i]; }
 TMPS_DEV void st4(double* p, int i, double4 v) { reinterpret_cast<double4*>(p)[i] = v; }
 TMPS_DEV float4 ld4f(const float* p, int i) { return reinterpret_cast<const float4*>(p)[i]; }

@@ -24,12 +24,11 @@ __global__ void __launch_bounds__(kBlock)
     if (i >= n) return;
     const bool hist = kHist && (STYLE != STYLE_GRANULAR || P.tangential_id >= 2 || P.rolling_id != 0);
     const bool roll = STYLE == STYLE_GRANULAR && P.rolling_id != 0;
-    double prd[3], iprd[3];
+    Period64 box[3];
     int per[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        prd[k] = B->prd[k];
-        iprd[k] = B->inv_prd[k];
+        box[k].set(B->prd[k], B->inv_prd[k]);
         per[k] = B->per[k];
     }
     const int vremap = B->vremap;
@@ -54,15 +53,15 @@ __global__ void __launch_bounds__(kBlock)
         for (int c = 0; c < 3; ++c) {
             nimg[c] = 0.0;
             if (per[c] == 1) {
-                nimg[c] = rint(in.d[c] * iprd[c]);
-                in.d[c] = image_sub64(in.d[c], nimg[c], prd[c]);
+                nimg[c] = box[c].count(in.d[c]);
+                in.d[c] = box[c].sub(in.d[c]);
             }
         }
         in.rsq = rsq64(in.d);
         in.ra = xa.w;
         in.rb = xb.w;
         const double radsum = in.ra + in.rb;
-        return in.rsq < __dmul_rn(radsum, radsum) && in.rsq > 1e-28;
+        return in.rsq < __dmul_rn(radsum, radsum) && apart64(in.rsq);
     };
     // The contact test of every row entry, four at a time (all loads in
     // flight together), then the law over the slots in contact, in slot order.
@@ -75,8 +74,8 @@ __global__ void __launch_bounds__(kBlock)
     float prd32[3], iprd32[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        prd32[c] = approx_f32(prd[c]);
-        iprd32[c] = approx_f32(iprd[c]);
+        prd32[c] = approx_f32(box[c].prd);
+        iprd32[c] = approx_f32(box[c].iprd);
     }
     const float base32 = l1f(xi32[0], xi32[1], xi32[2]) + l1f(prd32[0], prd32[1], prd32[2]);
     uint64_t cmask = 0ull;
@@ -115,7 +114,7 @@ __global__ void __launch_bounds__(kBlock)
         double nimg[3];
         geom(j, ld4(A.xr, j), in, nimg);
         const double radsum = in.ra + in.rb;
-        in.r = sqrt(in.rsq);
+        sqrt_rsqrt64(in.rsq, in.r, in.rinv);
         in.delta = radsum - in.r;
         const double4 vj = ld4(A.vm, j), wj = ld4(A.om, j);
         const double4 va = lo ? vi : vj, vb = lo ? vj : vi, wa = lo ? wi : wj, wb = lo ? wj : wi;

@@ -27,18 +27,25 @@ struct StyleTraits {
     static constexpr bool legacy_history = STYLE == STYLE_HOOKE_HISTORY || STYLE == STYLE_HERTZ_HISTORY;
 };
 
-// Division and square root of the law.  The FP64 form keeps IEEE-rounded
-// operations (its results follow the reference to 1e-12).  The mixed form's
+// Division and square root of the law.  The FP64 form forms quotients from
+// rcp64 and roots from rsqrt64 (within two units in the last place: the
+// results follow the reference to 1e-12; the contact distance |d|, whose
+// difference from the radii cancels three digits, keeps the rounded root of
+// the caller).  The mixed form's
 // law is FP32 arithmetic whose every operation already rounds at 2^-24, so
 // it uses the hardware's approximate reciprocal and reciprocal square root
 // (errors of a few ulp, the same order): a tenth of the instructions of the
 // IEEE sequences.
 template <typename T>
-TMPS_DEV T ldiv(T a, T b) { return a / b; }
+TMPS_DEV T ldiv(T a, T b);
+template <>
+TMPS_DEV double ldiv<double>(double a, double b) { return a * rcp64(b); }
 template <>
 TMPS_DEV float ldiv<float>(float a, float b) { return __fdividef(a, b); }
 template <typename T>
-TMPS_DEV T lsqrt(T a) { return sqrt(a); }
+TMPS_DEV T lsqrt(T a);
+template <>
+TMPS_DEV double lsqrt<double>(double a) { return sqrt64(a); }
 template <>
 TMPS_DEV float lsqrt<float>(float a) {
     // a * rsqrt(a); IEEE sqrtf for zero and for tiny arguments, whose reciprocal
@@ -52,6 +59,30 @@ TMPS_DEV float lsqrt<float>(float a) {
 // about three digits, so a contracted |d|^2 or image shift would move a force
 // by ~1e-13 relative.
 TMPS_DEV double image_sub64(double d, double nimg, double prd) { return __dsub_rn(d, __dmul_rn(nimg, prd)); }
+// The image of a separation component: d - n prd with n = rint(d / prd), which
+// is 0 (and d unchanged) below 0.49 of the period.
+struct Period64 {
+    double prd, iprd;
+    int near;  // high word of 0.49 prd
+    TMPS_DEV void set(double p, double ip) {
+        prd = p;
+        iprd = ip;
+        near = __double2hiint(0.49 * p);
+    }
+    TMPS_DEV double count(double d) const {
+        if ((__double2hiint(d) & 0x7fffffff) < near) return 0.0;
+        return rint(d * iprd);
+    }
+    TMPS_DEV double sub(double d) const {
+        if ((__double2hiint(d) & 0x7fffffff) < near) return d;
+        return image_sub64(d, rint(d * iprd), prd);
+    }
+};
+// x > 1e-28, by its high word where that settles it
+TMPS_DEV bool apart64(double x) {
+    const int h = __double2hiint(x), t = __double2hiint(1e-28);
+    return h != t ? h > t && x == x : x > 1e-28;
+}
 TMPS_DEV double rsq64(const double* d) {
     return __dadd_rn(__dadd_rn(__dmul_rn(d[0], d[0]), __dmul_rn(d[1], d[1])), __dmul_rn(d[2], d[2]));
 }
@@ -130,6 +161,7 @@ struct PairIn {
     T d[3];      // x_a - x_b, minimum image
     T rsq;
     T r;         // |d|
+    T rinv;      // 1 / |d| (FP64 form only)
     T delta;     // overlap ra + rb - r (the caller may form it more accurately than T allows)
     T ra, rb, ma, mb;
     T va[3], vb[3];  // vb already shifted by the remap-v image velocity
@@ -184,8 +216,14 @@ TMPS_DEV void contact_law(const PP& P, T dt, int shearupdate, const PairIn<T>& i
             polyhertz = lsqrt(reff * delta);
         }
         const T meff = ldiv(in.ma * in.mb, in.ma + in.mb);
-        const T rsqinv = ldiv(T(1), in.rsq);
-        const T rinv = ldiv(T(1), r);
+        T rsqinv, rinv;
+        if constexpr (sizeof(T) == sizeof(double)) {
+            rinv = in.rinv;
+            rsqinv = rinv * rinv;
+        } else {
+            rsqinv = ldiv(T(1), in.rsq);
+            rinv = ldiv(T(1), r);
+        }
         T vrel_t[3], vt[3], wr[3], cr[3], vtr[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) vrel_t[k] = in.va[k] - in.vb[k];
@@ -220,7 +258,9 @@ TMPS_DEV void contact_law(const PP& P, T dt, int shearupdate, const PairIn<T>& i
             }
 #pragma unroll
             for (int k = 0; k < 3; ++k) shf[k] = HS::template get<T>(sh[k]);
-            const T shrmag = norm3(shf);
+            bool moved;  // |shear| != 0
+            if constexpr (sizeof(T) == sizeof(double)) moved = __double_as_longlong(dot3(shf, shf)) != 0;
+            else moved = norm3(shf) != T(0);
             if (shearupdate) {
                 const T rsht = dot3(shf, in.d) * rsqinv;
 #pragma unroll
@@ -235,11 +275,21 @@ TMPS_DEV void contact_law(const PP& P, T dt, int shearupdate, const PairIn<T>& i
                 if constexpr (S::hertz) fs[k] = (-polyhertz) * t;
                 else fs[k] = -t;
             }
-            const T fsmag = norm3(fs);
             const T fn = T(P.xmu) * fabs(ccel * r);
-            if (fsmag > fn) {
-                if (shrmag != T(0)) {
-                    const T ratio = ldiv(fn, fsmag);
+            T fsmag, fs2 = T(0);
+            bool slip;
+            if constexpr (sizeof(T) == sizeof(double)) {  // the squares decide: a root only where it slips
+                fs2 = dot3(fs, fs);
+                slip = fs2 > fn * fn;
+            } else {
+                fsmag = norm3(fs);
+                slip = fsmag > fn;
+            }
+            if (slip) {
+                if (moved) {
+                    T ratio;
+                    if constexpr (sizeof(T) == sizeof(double)) ratio = fn * rsqrt64(fs2);
+                    else ratio = ldiv(fn, fsmag);
 #pragma unroll
                     for (int k = 0; k < 3; ++k) {
                         const T dc = ldiv(geff * vtr[k], T(P.kt));
@@ -261,7 +311,9 @@ TMPS_DEV void contact_law(const PP& P, T dt, int shearupdate, const PairIn<T>& i
         out.arm_b = -in.rb;
     } else {
         const T r = in.r;
-        const T rinv = ldiv(T(1), r);
+        T rinv;
+        if constexpr (sizeof(T) == sizeof(double)) rinv = in.rinv;
+        else rinv = ldiv(T(1), r);
         T nv[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) nv[k] = in.d[k] * rinv;
@@ -280,7 +332,6 @@ TMPS_DEV void contact_law(const PP& P, T dt, int shearupdate, const PairIn<T>& i
         cross3(wr, nv, cr);
 #pragma unroll
         for (int k = 0; k < 3; ++k) vtr[k] = vt[k] - cr[k];
-        const T vrel = norm3(vtr);
         const T fne = P.normal_id != 0 ? (T(P.kn) * a) * delta : T(P.kn) * delta;
         T dpf = T(0);
         switch (P.damping_id) {
@@ -312,6 +363,7 @@ TMPS_DEV void contact_law(const PP& P, T dt, int shearupdate, const PairIn<T>& i
         const T fscrit = T(P.mu) * fabs(fntot);
         T fs[3] = {T(0), T(0), T(0)};
         if (P.tangential_id == 1) {
+            const T vrel = norm3(vtr);
             const T damp_t = T(P.xt) * dpf;
             T ft = T(0);
             if (vrel != T(0)) {

@@ -195,9 +195,10 @@ __device__ __forceinline__ double warp_sum6_halving(const double (&v)[6]) {
 
 // `kept`: lane c < 6 holds a further value of component c; with `any` false
 // (warp-uniform) every v is zero and the exchanges are left out.
+template <int BLOCK>
 __device__ __forceinline__ double block_sum6_halving(const double (&v)[6], double kept, bool any,
-                                                     double* smem /* [6][kBlockA / 32] */) {
-    constexpr int kW = kBlockA / 32;
+                                                     double* smem /* [6][BLOCK / 32] */) {
+    constexpr int kW = BLOCK / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double r = 0.0;
     if (any) r = __shfl_sync(0xffffffffu, warp_sum6_halving(v), (lane << 2) & 31);  // lane c < 6: component c
@@ -375,7 +376,7 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
     }
     if (__any_sync(0xffffffffu, hit) && lane == 0) e->disp_stamp = s;
     note_displacement(e, dd);
-    const double tot = block_sum6_halving(K, kept, kicked, smem);
+    const double tot = block_sum6_halving<kBlockA>(K, kept, kicked, smem);
     if (threadIdx.x < 6) part[(size_t)threadIdx.x * nb + bid] = tot;
 }
 
@@ -808,6 +809,7 @@ struct CfEnv {
     T hh[3], prd[3], iprd[3];
     float hlo[3], prdlo[3];
     int per[3], single[3], gdim[3];
+    Period64 box[MIXED ? 1 : 3];
     T hrate[3], hshear[3];
     bool vremap, hist, roll;
 
@@ -833,8 +835,7 @@ struct CfEnv {
                 iprd[c] = E->iprd32[c];
                 single[c] = E->single_bin[c];
             } else {
-                prd[c] = B->prd[c];
-                iprd[c] = B->inv_prd[c];
+                box[c].set(B->prd[c], B->inv_prd[c]);
                 single[c] = 0;
             }
         }
@@ -949,8 +950,8 @@ __device__ __forceinline__ bool contact_core(
         for (int c = 0; c < 3; ++c) {
             d[c] = xi[c] - xj[c];
             if (V.per[c] == 1) {
-                nimg[c] = rint(d[c] * V.iprd[c]);
-                d[c] = image_sub64(d[c], nimg[c], V.prd[c]);
+                nimg[c] = V.box[c].count(d[c]);
+                d[c] = V.box[c].sub(d[c]);
             }
         }
     }
@@ -1019,9 +1020,9 @@ __device__ __forceinline__ bool contact_core(
         for (int c = 0; c < 3; ++c) in.d[c] = sg * d[c];
         in.rsq = rsq64(in.d);
         const T radsum = in.ra + in.rb;
-        near = in.rsq < __dmul_rn(radsum, radsum) && in.rsq > T(1e-28);
+        near = in.rsq < __dmul_rn(radsum, radsum) && apart64(in.rsq);
         if (near) {
-            in.r = sqrt(in.rsq);
+            sqrt_rsqrt64(in.rsq, in.r, in.rinv);
             in.delta = radsum - in.r;
         }
     }
@@ -1055,6 +1056,66 @@ __device__ __forceinline__ bool contact_core(
         contact_law<T, STYLE>(sP, V.dt, 1, in, sh, rl, out);
     }
     return near;
+}
+
+// FixDampingCundall.post_force_kernel (damping_cundall.py:36-53) on one atom.
+// FP64: the factors 1 -+ gamma (the same two roundings) chosen by the sign of
+// the product, so a component costs one FP64 multiplication.
+template <typename T>
+__device__ __forceinline__ void cundall_damp(T (&F)[3], T (&Tq)[3], const T* vi, const T* wi, T gl, T ga) {
+    if constexpr (sizeof(T) == sizeof(double)) {
+        const T lp = T(1) - gl, lm = T(1) + gl, ap = T(1) - ga, am = T(1) + ga;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            F[c] = mul_rn(F[c], prod_nonneg(F[c], vi[c]) ? lp : lm);
+            Tq[c] = mul_rn(Tq[c], prod_nonneg(Tq[c], wi[c]) ? ap : am);
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const T sf = F[c] * vi[c] >= T(0) ? T(1) : T(-1);
+            F[c] *= T(1) - gl * sf;
+            const T st = Tq[c] * wi[c] >= T(0) ? T(1) : T(-1);
+            Tq[c] *= T(1) - ga * st;
+        }
+    }
+}
+
+// The kinetic part of the virial with the end-of-step velocity
+// vf = v(t+dt/2) + dt/2 f/m (thermo.py:94-101) less the one with v(t+dt/2),
+// which A counted for every atom: m vf vf - m vi vi.
+// Mixed: from the same words and products, so that a zero force gives an exact
+// zero; the difference is exact where the force changed v little (Sterbenz),
+// elsewhere it rounds once, as the larger term did.
+// FP64: with g = dt/2 f the change m vf_a vf_b - m vi_a vi_b is g_a vf_b +
+// vi_a g_b (m times 1/m left out), without the cancellation and a third of
+// the instructions.
+template <typename T>
+__device__ __forceinline__ void kinetic_change(T mi, T im, T hdt, const T (&F)[3], const T* vi, T (&dk)[6]) {
+    T vf[3];
+    if constexpr (sizeof(T) == sizeof(double)) {
+        T g[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            g[c] = hdt * F[c];
+            vf[c] = vi[c] + g[c] * im;
+        }
+        dk[0] = g[0] * (vf[0] + vi[0]);
+        dk[1] = g[1] * (vf[1] + vi[1]);
+        dk[2] = g[2] * (vf[2] + vi[2]);
+        dk[3] = g[0] * vf[1] + vi[0] * g[1];
+        dk[4] = g[0] * vf[2] + vi[0] * g[2];
+        dk[5] = g[1] * vf[2] + vi[1] * g[2];
+    } else {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) vf[c] = vi[c] + hdt * (F[c] * im);
+        const T kin[6] = {(mi * vf[0]) * vf[0], (mi * vf[1]) * vf[1], (mi * vf[2]) * vf[2],
+                          (mi * vf[0]) * vf[1], (mi * vf[0]) * vf[2], (mi * vf[1]) * vf[2]};
+        const T kh[6] = {(mi * vi[0]) * vi[0], (mi * vi[1]) * vi[1], (mi * vi[2]) * vi[2],
+                         (mi * vi[0]) * vi[1], (mi * vi[0]) * vi[2], (mi * vi[1]) * vi[2]};
+#pragma unroll
+        for (int c = 0; c < 6; ++c) dk[c] = kin[c] - kh[c];
+    }
 }
 
 template <int STYLE, bool MIXED>
@@ -1382,11 +1443,11 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
                         double d[3] = {pi.x - pj[u].x, pi.y - pj[u].y, pi.z - pj[u].z};
 #pragma unroll
                         for (int c = 0; c < 3; ++c)
-                            if (V.per[c] == 1) d[c] = image_sub64(d[c], rint(d[c] * V.iprd[c]), V.prd[c]);
+                            if (V.per[c] == 1) d[c] = V.box[c].sub(d[c]);
                         // the contact test itself, as the law makes it (|d|^2 of either orientation)
                         const double rsq = rsq64(d);
                         const double radsum = pi.w + pj[u].w;
-                        nr = rsq < __dmul_rn(radsum, radsum) && rsq > 1e-28;
+                        nr = rsq < __dmul_rn(radsum, radsum) && apart64(rsq);
                     }
                     const uint32_t bal = __ballot_sync(0xffffffffu, nr);
                     if (nr) {
@@ -1434,13 +1495,7 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
                         gl = E->gamma_lin;
                         ga = E->gamma_ang;
                     }
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const T sf = F[c] * vi[c] >= T(0) ? T(1) : T(-1);
-                        F[c] *= T(1) - gl * sf;
-                        const T st = Tq[c] * wi[c] >= T(0) ? T(1) : T(-1);
-                        Tq[c] *= T(1) - ga * st;
-                    }
+                    cundall_damp<T>(F, Tq, vi, wi, gl, ga);
                 }
                 if constexpr (MIXED) {
 #pragma unroll
@@ -1455,30 +1510,15 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
                         A.torque[c * n + i] = Tq[c];
                     }
                 }
-                // kinetic part of the virial with the end-of-step velocity
-                // v(t+dt) = v(t+dt/2) + dt/2 f/m (thermo.py:94-101): A counted
-                // m v(t+dt/2) v(t+dt/2) for every atom; the difference goes here
-                // (the same products from the same words, so a zero force adds an
-                // exact zero)
                 T im;
                 if constexpr (MIXED) im = __fdividef(1.0f, mi);
                 else im = A.rinv[i];
-                const T hdt = T(0.5) * dt;
-                T vf[3];
+                T dk[6];
+                kinetic_change<T>(mi, im, T(0.5) * dt, F, vi, dk);
 #pragma unroll
-                for (int c = 0; c < 3; ++c) vf[c] = vi[c] + hdt * (F[c] * im);
-                const T kin[6] = {(mi * vf[0]) * vf[0], (mi * vf[1]) * vf[1], (mi * vf[2]) * vf[2],
-                                  (mi * vf[0]) * vf[1], (mi * vf[0]) * vf[2], (mi * vf[1]) * vf[2]};
-                const T kh[6] = {(mi * vi[0]) * vi[0], (mi * vi[1]) * vi[1], (mi * vi[2]) * vi[2],
-                                 (mi * vi[0]) * vi[1], (mi * vi[0]) * vi[2], (mi * vi[1]) * vi[2]};
-                if constexpr (MIXED) {
-                    // kin - kh is exact where the force changed v little (Sterbenz); elsewhere
-                    // kh is the smaller term and the difference rounds once, as kin did
-#pragma unroll
-                    for (int c = 0; c < 6; ++c) dw_add(Vh[c], Vl[c], V[c] + (kin[c] - kh[c]));
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 6; ++c) Vd[c] += (V[c] + kin[c]) - kh[c];
+                for (int c = 0; c < 6; ++c) {
+                    if constexpr (MIXED) dw_add(Vh[c], Vl[c], V[c] + dk[c]);
+                    else Vd[c] += V[c] + dk[c];
                 }
             }
         }
@@ -1597,11 +1637,8 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
             for (int c = 0; c < 6; ++c) reinterpret_cast<float2*>(part)[(size_t)c * nb + bid] = make_float2(Vh[c], Vl[c]);
         }
     } else {
-        block_sum<6, kBlockC>(Vd, smem);
-        if (threadIdx.x == 0) {
-#pragma unroll
-            for (int c = 0; c < 6; ++c) part[(size_t)c * nb + bid] = Vd[c];
-        }
+        const double tot = block_sum6_halving<kBlockC>(Vd, 0.0, true, smem);
+        if (threadIdx.x < 6) part[(size_t)threadIdx.x * nb + bid] = tot;
     }
     if (threadIdx.x == 0 && bid == 0) E->final_pending = 1;
 }
@@ -1909,7 +1946,7 @@ __global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
                     const double v6[6] = {in.d[0] * out.f[0], in.d[1] * out.f[1], in.d[2] * out.f[2],
                                           in.d[0] * out.f[1], in.d[0] * out.f[2], in.d[1] * out.f[2]};
 #pragma unroll
-                    for (int c = 0; c < 6; ++c) Vd[c] = add_rn(Vd[c], v6[c]);
+                    for (int c = 0; c < 6; ++c) Vd[c] += v6[c];
                 }
             } else {
                 // within the near test's margin but not touching (mixed form)
@@ -1965,10 +2002,10 @@ __global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
                 double d[3] = {pi.x - pj.x, pi.y - pj.y, pi.z - pj.z};
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
-                    if (V.per[c] == 1) d[c] = image_sub64(d[c], rint(d[c] * V.iprd[c]), V.prd[c]);
+                    if (V.per[c] == 1) d[c] = V.box[c].sub(d[c]);
                 const double rsq = rsq64(d);
                 const double radsum = pi.w + pj.w;
-                near = rsq < __dmul_rn(radsum, radsum) && rsq > 1e-28;
+                near = rsq < __dmul_rn(radsum, radsum) && apart64(rsq);
             }
         }
         const uint32_t bal = __ballot_sync(0xffffffffu, near);
@@ -1988,11 +2025,8 @@ __global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
     }
     if (tail > head) law(tail - head, head);
     if constexpr (!MIXED) {
-        block_sum<6, kBlockC>(Vd, smem);
-        if (threadIdx.x == 0) {
-#pragma unroll
-            for (int c = 0; c < 6; ++c) Q.part[(size_t)c * gridDim.x + blockIdx.x] = Vd[c];
-        }
+        const double tot = block_sum6_halving<kBlockC>(Vd, 0.0, true, smem);
+        if (threadIdx.x < 6) Q.part[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = tot;
     }
 }
 
@@ -2129,15 +2163,7 @@ __global__ void __launch_bounds__(kBlockG, MIXED ? 4 : 3)
             }
         }
         if (any) {
-            if (cundall) {  // FixDampingCundall.post_force_kernel
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const T sf = F[c] * vi[c] >= T(0) ? T(1) : T(-1);
-                    F[c] *= T(1) - gl * sf;
-                    const T st = Tq[c] * wi[c] >= T(0) ? T(1) : T(-1);
-                    Tq[c] *= T(1) - ga * st;
-                }
-            }
+            if (cundall) cundall_damp<T>(F, Tq, vi, wi, gl, ga);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 if constexpr (MIXED) {
@@ -2148,22 +2174,15 @@ __global__ void __launch_bounds__(kBlockG, MIXED ? 4 : 3)
                     A.torque[c * n + i] = Tq[c];
                 }
             }
-            // the kinetic correction for the end-of-step velocity (the screened path's step 5)
             T im;
             if constexpr (MIXED) im = __fdividef(1.0f, mi);
             else im = A.rinv[i];
-            const T hdt = T(0.5) * dt;
-            T vf[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) vf[c] = vi[c] + hdt * (F[c] * im);
-            const T kin[6] = {(mi * vf[0]) * vf[0], (mi * vf[1]) * vf[1], (mi * vf[2]) * vf[2],
-                              (mi * vf[0]) * vf[1], (mi * vf[0]) * vf[2], (mi * vf[1]) * vf[2]};
-            const T kh[6] = {(mi * vi[0]) * vi[0], (mi * vi[1]) * vi[1], (mi * vi[2]) * vi[2],
-                             (mi * vi[0]) * vi[1], (mi * vi[0]) * vi[2], (mi * vi[1]) * vi[2]};
+            T dk[6];
+            kinetic_change<T>(mi, im, T(0.5) * dt, F, vi, dk);
 #pragma unroll
             for (int c = 0; c < 6; ++c) {
-                if constexpr (MIXED) V[c] = V[c] + (kin[c] - kh[c]);
-                else Vd[c] += kin[c] - kh[c];
+                if constexpr (MIXED) V[c] = V[c] + dk[c];
+                else Vd[c] += dk[c];
             }
         }
         // the group's new flag word; stale forces of atoms no longer flagged
@@ -2205,13 +2224,10 @@ __global__ void __launch_bounds__(kBlockG, MIXED ? 4 : 3)
             reinterpret_cast<float2*>(part)[(size_t)threadIdx.x * nb + blockIdx.x] = w[0];
         }
     } else {
-        block_sum<6, kBlockG>(Vd, smem);
-        if (threadIdx.x == 0) {
-            // the pair pass's partial of the same number joins this block's
-#pragma unroll
-            for (int c = 0; c < 6; ++c)
-                part[(size_t)c * nb + blockIdx.x] = Vd[c] + Q.part[(size_t)c * gridDim.x + blockIdx.x];
-        }
+        const double tot = block_sum6_halving<kBlockG>(Vd, 0.0, true, smem);
+        // the pair pass's partial of the same number joins this block's
+        if (threadIdx.x < 6)
+            part[(size_t)threadIdx.x * nb + blockIdx.x] = tot + Q.part[(size_t)threadIdx.x * gridDim.x + blockIdx.x];
     }
     if (threadIdx.x == 0 && blockIdx.x == 0) E->final_pending = 1;
 }

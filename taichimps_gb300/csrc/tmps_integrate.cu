@@ -59,16 +59,6 @@ __global__ void __launch_bounds__(kBlock) k_verlet_final(tmps_atoms a, double dt
     st4(a.om, i, w);
 }
 
-// a * b >= 0.0, as the FP64 product compares: from the sign bits where the
-// exponents keep the product clear of underflow (and neither is a NaN), the
-// product itself otherwise.
-__device__ __forceinline__ bool prod_nonneg(double a, double b) {
-    const int ha = __double2hiint(a), hb = __double2hiint(b);
-    const int ea = (ha >> 20) & 0x7ff, eb = (hb >> 20) & 0x7ff;
-    if (ea > 0x200 && ea < 0x600 && eb > 0x200 && eb < 0x600) return (ha ^ hb) >= 0;
-    return a * b >= 0.0;
-}
-
 // FixDampingCundall.post_force (damping_cundall.py:36-53):
 //   f_d *= 1 - gamma_lin sign(f_d v_d),  torque_d *= 1 - gamma_ang sign(torque_d omega_d)
 // The factors 1 -+ gamma are the same two roundings for every atom (gamma *

@@ -42,6 +42,10 @@ extern "C" int tmps_probe_fp64(int32_t blocks, int32_t threads, int32_t iters, d
 //   which 0: (float)a[i]             f32_rn    vs the hardware conversion (float bits)
 //   which 1: (double)(float)a[i]     f64_of    vs the hardware widening
 //   which 2: hi, lo split of a[i]    split_dw  vs the hardware's (float bits, two outputs per operand)
+// and the reciprocals and roots beside the correctly rounded operations:
+//   which 3: 1 / a[i]                rcp64
+//   which 4: 1 / sqrt(a[i])          rsqrt64   (a[i] >= 0)
+//   which 5: sqrt(a[i])              sqrt64    (a[i] >= 0)
 namespace {
 
 __global__ void k_selftest(int which, const double* __restrict__ a, int n, double* __restrict__ mine,
@@ -60,6 +64,18 @@ __global__ void k_selftest(int which, const double* __restrict__ a, int n, doubl
             hw[i] = (double)f;
             break;
         }
+        case 3:
+            mine[i] = rcp64(x);
+            hw[i] = 1.0 / x;
+            break;
+        case 4:
+            mine[i] = rsqrt64(x);
+            hw[i] = 1.0 / sqrt(x);
+            break;
+        case 5:
+            mine[i] = sqrt64(x);
+            hw[i] = sqrt(x);
+            break;
         default: {
             float h, l;
             split_dw(x, h, l);
@@ -78,7 +94,7 @@ __global__ void k_selftest(int which, const double* __restrict__ a, int n, doubl
 
 extern "C" int tmps_selftest_arith(int32_t which, const double* d_a, int32_t n, double* d_mine, double* d_hw,
                                    void* stream) {
-    if (which < 0 || which > 2 || n < 0 || !d_a || !d_mine || !d_hw) return TMPS_ERR_BAD_ARG;
+    if (which < 0 || which > 5 || n < 0 || !d_a || !d_mine || !d_hw) return TMPS_ERR_BAD_ARG;
     if (n == 0) return TMPS_OK;
     k_selftest<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(which, d_a, n, d_mine, d_hw);
     note_launches(1);

@@ -1,0 +1,44 @@
+"""
+The FP64 form's reciprocals and square roots (rcp64, rsqrt64, sqrt64): against extended precision on
+random operands over the exponents, powers of two and their neighbours, and the operands that must take
+the correctly rounded operation (zeros, infinities, NaNs, the ends of the exponent range).
+"""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(which, a):
+    import torch
+    from taichimps_gb300 import _device, _lib
+    d = torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    mine, hw = torch.empty_like(d), torch.empty_like(d)
+    rc = _device.lib().tmps_selftest_arith(which, d.data_ptr(), len(a), mine.data_ptr(), hw.data_ptr(),
+                                           _device.stream())
+    assert rc == _lib.TMPS_OK
+    return mine.cpu().numpy(), hw.cpu().numpy()
+
+
+# rcp64 and rsqrt64 are stated to two units in the last place, sqrt64 to one
+@pytest.mark.parametrize("which,ulps", [(3, 2.0), (4, 2.0), (5, 1.0)])
+def test_reciprocals_and_roots(gpu, which, ulps):
+    rng = np.random.default_rng(which)
+    wide = np.ldexp(rng.uniform(1.0, 2.0, size=200_000), rng.integers(-995, 995, size=200_000))
+    usual = rng.uniform(1e-4, 1e4, size=200_000)
+    p2 = np.ldexp(1.0, np.arange(-990, 990))
+    a = np.concatenate([wide, usual, p2, np.nextafter(p2, 0.0), np.nextafter(p2, np.inf)])
+    if which == 3:
+        a = a * rng.choice([1.0, -1.0], size=len(a))
+    mine, _ = _run(which, a)
+    x = a.astype(np.longdouble)
+    with np.errstate(over="ignore"):
+        want = 1 / x if which == 3 else (1 / np.sqrt(x) if which == 4 else np.sqrt(x))
+    if np.finfo(np.longdouble).nmant <= 52:  # a host without extended precision: its own rounding beside
+        ulps += 1.0
+    err = np.abs((mine.astype(np.longdouble) - want) / np.spacing(np.abs(want.astype(np.float64))).astype(np.longdouble))
+    assert float(err.max()) <= ulps, (float(err.max()), a[int(err.argmax())])
+    edge = np.array([0.0, np.inf, np.nan, 5e-324, 2.0 ** -1022, 2.0 ** -1005, 2.0 ** 1005, 1.7e308])
+    mine, hw = _run(which, edge)
+    np.testing.assert_array_equal(mine, hw)
