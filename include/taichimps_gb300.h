@@ -728,6 +728,29 @@ int tmps_adj_initial(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps
 int tmps_adj_finish(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_adj_servo* sv,
                     const tmps_adj_tape* tape, tmps_adj_rec* d_rec, int64_t step, void* work, void* stream);
 
+/* Steps first .. last queued at once (tmps_adj_initial and tmps_adj_finish of
+ * each, no host synchronisation in between).  The tape of step first + k lies
+ * k atom_stride doubles (xh, vh, wh, f, t) and k pair_stride pairs (shear: 3
+ * doubles each; mask) past the pointers in `tape`; strides 0 keep the last step's alone.  A step in
+ * which some |xh - d_xbuild|^2 exceeds trigger_sq halts the run after its
+ * first half: d_queue[0] is that step (0: none), d_queue[1] the last step
+ * finished (int64[2], device).  The host then rebuilds the pair list, calls
+ * tmps_adj_finish for it and queues the steps after it. */
+int tmps_adj_forward(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_adj_servo* sv,
+                     const tmps_adj_tape* tape, int64_t atom_stride, int64_t pair_stride, tmps_adj_rec* d_rec,
+                     int64_t first, int64_t last, const double* d_xbuild, double trigger_sq, int64_t* d_queue, void* work,
+                     void* stream);
+
+/* Reverse of steps last .. first (one pair list), tapes laid out as above.
+ * qbar (host) holds dL/dq of steps first - 1 .. last; d_fprev / d_tprev are the
+ * forces step `first` started from.  d_xprev, if not NULL, is the xh of step
+ * first - 1: the call then also reverses that step's remap and servo, and the
+ * call for the steps below it passes linked = 1. */
+int tmps_adj_reverse(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_adj_servo* sv,
+                     const tmps_adj_tape* tape, int64_t atom_stride, int64_t pair_stride, const tmps_adj_rec* d_rec,
+                     int64_t first, int64_t last, const double* d_fprev, const double* d_tprev, const double* d_xprev,
+                     int32_t linked, const double* qbar, const tmps_adj_bar* b, void* work, void* stream);
+
 /* Reverse of step s (from d_rec[s - 1] to d_rec[s]), given the adjoint of
  * the state after it in `b`; leaves the adjoint of the state before it.
  * `qbar` is dL/dq of step s; d_fprev / d_tprev the forces step s started

@@ -13,6 +13,7 @@ from pathlib import Path
 from . import build as _build
 
 c_i32 = ctypes.c_int32
+c_i64 = ctypes.c_int64
 c_f64 = ctypes.c_double
 c_vp = ctypes.c_void_p
 
@@ -248,6 +249,12 @@ _SIGS = {
                                  c_vp, c_vp]),
     "tmps_adj_finish": (c_i32, [ctypes.POINTER(AdjSys), ctypes.POINTER(AdjParams), ctypes.POINTER(AdjServo),
                                 ctypes.POINTER(AdjTape), c_vp, ctypes.c_int64, c_vp, c_vp]),
+    "tmps_adj_forward": (c_i32, [ctypes.POINTER(AdjSys), ctypes.POINTER(AdjParams), ctypes.POINTER(AdjServo),
+                                 ctypes.POINTER(AdjTape), c_i64, c_i64, c_vp, c_i64, c_i64, c_vp, c_f64, c_vp, c_vp,
+                                 c_vp]),
+    "tmps_adj_reverse": (c_i32, [ctypes.POINTER(AdjSys), ctypes.POINTER(AdjParams), ctypes.POINTER(AdjServo),
+                                 ctypes.POINTER(AdjTape), c_i64, c_i64, c_vp, c_i64, c_i64, c_vp, c_vp, c_vp, c_i32,
+                                 c_vp, ctypes.POINTER(AdjBar), c_vp, c_vp]),
     "tmps_adj_step_back": (c_i32, [ctypes.POINTER(AdjSys), ctypes.POINTER(AdjParams), ctypes.POINTER(AdjServo),
                                    ctypes.POINTER(AdjTape), c_vp, ctypes.c_int64, c_vp, c_vp, c_f64,
                                    ctypes.POINTER(AdjBar), c_vp, c_vp]),

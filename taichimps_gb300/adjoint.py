@@ -87,22 +87,27 @@ class _Pairs:
         return _Pairs(n, pi[:npairs], pj[:npairs], ibeg)
 
 
-class _Tape:
-    """One step's record (atom arrays [3][n], pair arrays [3][npairs])."""
+class _Tapes:
+    """The records of `steps` steps over one pair list: atom arrays [steps][5][3][n] (xh, vh, wh, f, t) and
+    pair arrays [steps][3][npairs], [steps][npairs] (history, mask).  Left unset: every launch that reads
+    a step's record follows the launches that write it in full.  `atoms`: share another record's atom
+    arrays (a rebuild changes the pairs alone)."""
 
-    def __init__(self, n: int, npairs: int, dev):
-        f64 = dict(dtype=torch.float64, device=dev)
-        self.xh, self.vh, self.wh = (torch.zeros((3, n), **f64) for _ in range(3))
-        self.f, self.t = torch.zeros((3, n), **f64), torch.zeros((3, n), **f64)
-        self.resize(npairs, dev)
+    def __init__(self, steps: int, n: int, npairs: int, dev, atoms: torch.Tensor | None = None):
+        np_ = max(npairs, 1)
+        self.atoms = torch.empty((steps, 5, 3, n), dtype=torch.float64, device=dev) if atoms is None else atoms
+        self.shear = torch.empty((steps, 3, np_), dtype=torch.float64, device=dev)
+        self.mask = torch.empty((steps, np_), dtype=torch.uint8, device=dev)
+        self.atom_stride, self.pair_stride = 15 * n, np_
 
-    def resize(self, npairs: int, dev) -> None:
-        self.shear = torch.zeros((3, max(npairs, 1)), dtype=torch.float64, device=dev)
-        self.mask = torch.zeros(max(npairs, 1), dtype=torch.uint8, device=dev)
+    def field(self, k: int, name: str) -> torch.Tensor:
+        return self.atoms[k, ("xh", "vh", "wh", "f", "t").index(name)]
 
-    def cstruct(self) -> _lib.AdjTape:
-        return _lib.AdjTape(_p(self.xh), _p(self.vh), _p(self.wh), _p(self.f), _p(self.t), _p(self.shear),
-                            _p(self.mask))
+    def cstruct(self, k: int = 0) -> _lib.AdjTape:
+        a, step = self.atoms.data_ptr() + 8 * self.atom_stride * k, 8 * self.atom_stride // 5
+        return _lib.AdjTape(a, a + step, a + 2 * step, a + 3 * step, a + 4 * step,
+                            self.shear.data_ptr() + 24 * self.pair_stride * k,
+                            self.mask.data_ptr() + self.pair_stride * k)
 
 
 class AdjointRun:
@@ -216,38 +221,47 @@ class AdjointRun:
         self.lists, self.events = [pairs], {}
         li = 0
         shear = torch.zeros((3, max(pairs.npairs, 1)), **f64)
-        tape = _Tape(self.n, pairs.npairs, self.dev)
+        tape = _Tapes(1, self.n, pairs.npairs, self.dev)
         _lib.check(L.tmps_adj_setup(self._sys(st, pairs, shear), self.prm, self._rec_ptr(0), tape.cstruct(),
                                     _p(self._work(pairs.npairs)), sc), "tmps_adj_setup")
         self.ckpt = {}
         xbuild = st["x"].clone()
-        disp = torch.zeros(1, dtype=torch.int64, device=self.dev)
+        queue = torch.zeros(2, dtype=torch.int64, device=self.dev)
         trig = 0.25 * self.skin * self.skin
         self.rebuilds = 0
         digest = torch.zeros((), dtype=torch.int64, device=self.dev)
-        for s in range(1, self.steps + 1):
-            if (s - 1) % self.checkpoint_every == 0:
-                self.ckpt[s - 1] = ({k: a.clone() for k, a in st.items()}, shear.clone(), li)
-            disp.zero_()
-            _lib.check(L.tmps_adj_initial(self._sys(st, pairs, shear), self.prm, tape.cstruct(), _p(xbuild), _p(disp),
-                                          sc), "tmps_adj_initial")
-            if float(disp.view(torch.float64).item()) > trig:
-                new = _Pairs.build(tape.xh, self.r, self._rec_ptr(s - 1), self.skin)
+        s = 0
+        while s < self.steps:
+            if s % self.checkpoint_every == 0 and s not in self.ckpt:
+                self.ckpt[s] = ({k: a.clone() for k, a in st.items()}, shear.clone(), li)
+            # the steps up to the next checkpoint in one call, one synchronisation after them (one at a
+            # time where every step's masks are wanted)
+            last = min((s // self.checkpoint_every + 1) * self.checkpoint_every, self.steps)
+            last = s + 1 if track_masks else last
+            _lib.check(L.tmps_adj_forward(self._sys(st, pairs, shear), self.prm, self.servo, tape.cstruct(), 0, 0,
+                                          self.rec.data_ptr(), s + 1, last, _p(xbuild), trig, _p(queue),
+                                          _p(self._work(pairs.npairs)), sc), "tmps_adj_forward")
+            hit = int(queue[0].item())
+            if hit:
+                # step `hit` has had its first half: a new pair list, then the rest of it
+                new = _Pairs.build(tape.field(0, "xh"), self.r, self._rec_ptr(hit - 1), self.skin)
                 m = torch.zeros(max(pairs.npairs, 1), dtype=torch.int32, device=self.dev)
                 _lib.check(L.tmps_adj_pair_map(pairs.npairs, _p(pairs.pi), _p(pairs.pj), _p(new.ibeg), _p(new.pj),
                                                _p(m), sc), "tmps_adj_pair_map")
                 shear = self._carry(pairs, new, m, shear, False)
                 self.lists.append(new)
                 li = len(self.lists) - 1
-                self.events[s] = (li, m)
+                self.events[hit] = (li, m)
                 pairs = new
-                tape.resize(pairs.npairs, self.dev)
-                xbuild = tape.xh.clone()
+                tape = _Tapes(1, self.n, pairs.npairs, self.dev, atoms=tape.atoms)
+                xbuild = tape.field(0, "xh").clone()
                 self.rebuilds += 1
-            _lib.check(L.tmps_adj_finish(self._sys(st, pairs, shear), self.prm, self.servo, tape.cstruct(),
-                                         self.rec.data_ptr(), s, _p(self._work(pairs.npairs)), sc), "tmps_adj_finish")
+                _lib.check(L.tmps_adj_finish(self._sys(st, pairs, shear), self.prm, self.servo, tape.cstruct(),
+                                             self.rec.data_ptr(), hit, _p(self._work(pairs.npairs)), sc),
+                           "tmps_adj_finish")
+            s = hit if hit else last
             if track_masks:
-                digest = self._digest_step(digest, tape.mask[:pairs.npairs], s if s in self.events else 0)
+                digest = self._digest_step(digest, tape.mask[0, :pairs.npairs], s if s in self.events else 0)
         self.final_state = st
         self.mask_digest = int(digest.item()) if track_masks else None
         self._fwd = True
@@ -297,48 +311,65 @@ class AdjointRun:
             return _lib.AdjBar(_p(bar["x"]), _p(bar["v"]), _p(bar["w"]), _p(bar["f"]), _p(bar["t"]), _p(sh),
                                _p(bar["radius"]), _p(bar["mass"]), _p(bar["params"]), _p(bar["box"]))
 
-        disp = torch.zeros(1, dtype=torch.int64, device=self.dev)
+        queue = torch.zeros(2, dtype=torch.int64, device=self.dev)
+        work = self._work(max(p.npairs for p in self.lists))
         for start in sorted(self.ckpt, reverse=True):
             end = min(start + self.checkpoint_every, self.steps)
             saved, shear, li = self.ckpt[start]
             st = {k: a.clone() for k, a in saved.items()}
             shear = shear.clone()
             pairs = self.lists[li]
-            tapes = {}
-            for s in range(start + 1, end + 1):
-                ev = self.events.get(s)
-                npairs = self.lists[ev[0]].npairs if ev else pairs.npairs
-                tape = _Tape(n, npairs, self.dev)
-                _lib.check(L.tmps_adj_initial(self._sys(st, pairs, shear), self.prm, tape.cstruct(), _p(st["x"]),
-                                              _p(disp), sc), "tmps_adj_initial")
+            # the segment again, its records kept: ranges (first, last, pairs, tapes) of steps on one list
+            ranges, first = [], start + 1
+            atoms = torch.empty((end - start, 5, 3, n), **f64)
+            while first <= end:
+                ev = self.events.get(first)
                 if ev:
+                    # the first half on the old list's step, the history carried over, the rest on the new list
+                    t = _Tapes(1, n, pairs.npairs, self.dev, atoms=atoms[first - start - 1:])
+                    _lib.check(L.tmps_adj_initial(self._sys(st, pairs, shear), self.prm, t.cstruct(), _p(st["x"]),
+                                                  _p(queue), sc), "tmps_adj_initial")
                     new = self.lists[ev[0]]
                     shear = self._carry(pairs, new, ev[1], shear, False)
                     pairs = new
-                _lib.check(L.tmps_adj_finish(self._sys(st, pairs, shear), self.prm, self.servo, tape.cstruct(),
-                                             self.rec.data_ptr(), s, _p(self._work(pairs.npairs)), sc),
-                           "tmps_adj_finish")
-                tapes[s] = (tape, pairs)
-            for s in range(end, start, -1):
-                tape, pairs = tapes[s]
-                prev = tapes[s - 1][0] if s - 1 > start else None
-                fprev = prev.f if prev is not None else saved["f"]
-                tprev = prev.t if prev is not None else saved["t"]
-                _lib.check(L.tmps_adj_step_back(self._sys(st, pairs, tape.shear), self.prm, self.servo,
-                                                tape.cstruct(), self.rec.data_ptr(), s, _p(fprev), _p(tprev),
-                                                float(qb[s]), bar_struct(bar_sh), _p(self._work(pairs.npairs)), sc),
-                           "tmps_adj_step_back")
-                ev = self.events.get(s)
+                last = first
+                while last < end and last + 1 not in self.events:
+                    last += 1
+                t = _Tapes(last - first + 1, n, pairs.npairs, self.dev, atoms=atoms[first - start - 1:])
+                sys = self._sys(st, pairs, shear)
                 if ev:
-                    old = tapes[s - 1][1] if s - 1 > start else self.lists[self.ckpt[start][2]]
+                    _lib.check(L.tmps_adj_finish(sys, self.prm, self.servo, t.cstruct(), self.rec.data_ptr(), first,
+                                                 _p(work), sc), "tmps_adj_finish")
+                at = first + 1 if ev else first
+                if at <= last:
+                    # (no displacement check: the rebuild steps are known)
+                    _lib.check(L.tmps_adj_forward(sys, self.prm, self.servo, t.cstruct(at - first), t.atom_stride,
+                                                  t.pair_stride, self.rec.data_ptr(), at, last, _p(st["x"]), math.inf,
+                                                  _p(queue), _p(work), sc), "tmps_adj_forward")
+                ranges.append((first, last, pairs, t))
+                first = last + 1
+            for k in range(len(ranges) - 1, -1, -1):
+                first, last, pairs, t = ranges[k]
+                inner = first - 1 > start
+                before = atoms[first - start - 2] if inner else None
+                fprev, tprev = (before[3], before[4]) if inner else (saved["f"], saved["t"])
+                q = np.ascontiguousarray(qb[first - 1:last + 1])
+                _lib.check(L.tmps_adj_reverse(self._sys(st, pairs, t.shear[0]), self.prm, self.servo, t.cstruct(),
+                                              t.atom_stride, t.pair_stride, self.rec.data_ptr(), first, last, _p(fprev),
+                                              _p(tprev), _p(before[0]) if inner else None,
+                                              1 if k + 1 < len(ranges) else 0, q.ctypes.data, bar_struct(bar_sh), _p(work),
+                                              sc), "tmps_adj_reverse")
+                ev = self.events.get(first)
+                if ev:
+                    old = ranges[k - 1][2] if k > 0 else self.lists[self.ckpt[start][2]]
                     bar_sh = self._carry(old, pairs, ev[1], bar_sh, True)
-            del tapes
+            del ranges, atoms
         # the setup force evaluation
         saved, _, li = self.ckpt[0]
         pairs = self.lists[li]
         st = {k: a.clone() for k, a in saved.items()}
         shear = torch.zeros((3, max(pairs.npairs, 1)), **f64)
-        tape = _Tape(n, pairs.npairs, self.dev)
+        tape = _Tapes(1, n, pairs.npairs, self.dev)
         _lib.check(L.tmps_adj_setup(self._sys(st, pairs, shear), self.prm, self._rec_ptr(0), tape.cstruct(),
                                     _p(self._work(pairs.npairs)), sc), "tmps_adj_setup")
         st = {k: a.clone() for k, a in saved.items()}

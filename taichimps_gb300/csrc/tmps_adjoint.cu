@@ -7,13 +7,24 @@
 // values.
 //
 // Forward of step s (Simulation._sub_step_inner, simulation.py:205-247):
-//   k_initial   v += dtf f / m; x += dt v; w += dtf t / I     (nve_sphere.py:56-80)
+//   k_initial   (remap of step s - 1;) v += dtf f / m; x += dt v; w += dtf t / I;
+//               displacement check                            (nve_sphere.py:56-80)
 //   k_pairs     contacts on the tape's xh, vh, wh (hertz_history.py:92-157)
 //   k_gather    f, t per atom; v += dtf f / m; w += dtf t / I; kinetic partials
 //   k_servo     virial total, pressure, servo, new box        (deform_pressure.py:598-702)
-//   k_remap     x from the old box into the new one           (deform_pressure.py:493-530)
-// Reverse of step s runs these backwards: k_b_remap, k_b_servo, k_b_final,
-// k_b_pairs, k_b_reduce, k_b_gather, k_b_initial.
+//   k_remap     x from the old box into the new one           (deform_pressure.py:493-530),
+//               once per queued run of steps: between them k_initial does it
+// Reverse of step s: k_b_servo (with k_b_reduce's sums of step s + 1), k_b_final,
+// k_b_pairs, k_b_atoms (gather, first half-kick, remap of step s - 1).
+//
+// What bounds these kernels: the FP64 pipe (one instruction of a warp every 16
+// cycles per SM, 64 cycles to its result) and, below a few ten thousand
+// spheres, the chain of such results.  Hence small blocks (two warps), so that
+// a few thousand atoms already reach every SM; reciprocals by rcp64 instead of
+// divisions; pairs out of contact dropped before the law, so that its warps run
+// full; and few launches, queued by one call for a run of steps with no host
+// synchronisation in between: a step whose displacement check fires marks the
+// run and every later launch of it does nothing.
 #include "tmps_adjoint.cuh"
 #include "tmps_common.cuh"
 
@@ -22,8 +33,10 @@ using namespace tmps_adj;
 
 namespace {
 
-constexpr int kBlk = 256;
-constexpr int kNG = 16;  // doubles per pair in the reverse's per-pair record
+constexpr int kBlk = 64;       // threads of the per-atom and per-pair kernels
+constexpr int kPairTile = 128;  // pairs a block of the contact passes takes
+constexpr int kOne = 512;      // threads of the one-block kernels
+constexpr int kNG = 16;        // doubles per pair in the reverse's per-pair record
 
 inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
@@ -38,7 +51,7 @@ struct Work {
 };
 
 Work carve(void* base, int n, int npairs) {
-    const int nbA = grid_for(n, kBlk), nbP = grid_for(npairs, kBlk);
+    const int nbA = grid_for(n, kBlk), nbP = grid_for(npairs, kPairTile);
     char* p = static_cast<char*>(base);
     Work w;
     w.fp = reinterpret_cast<double*>(p); p += align256(sizeof(double) * 3 * (size_t)npairs);
@@ -52,7 +65,7 @@ Work carve(void* base, int n, int npairs) {
 }
 
 size_t work_bytes(int n, int npairs) {
-    const int nbA = grid_for(n, kBlk), nbP = grid_for(npairs, kBlk);
+    const int nbA = grid_for(n, kBlk), nbP = grid_for(npairs, kPairTile);
     return align256(sizeof(double) * 3 * (size_t)npairs) * 2 + align256(sizeof(double) * kNG * (size_t)npairs) +
            align256(sizeof(double) * 6 * (size_t)nbP) + align256(sizeof(double) * 6 * (size_t)nbA) +
            align256(sizeof(double) * 8 * (size_t)nbP) + align256(sizeof(double) * 8);
@@ -76,25 +89,58 @@ Params to_params(const tmps_adj_params& p) {
 __device__ __forceinline__ void min_image(const double* prd, const double* iprd, double* d, double* nimg) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        nimg[c] = rint(d[c] * iprd[c]);
-        d[c] -= nimg[c] * prd[c];
+        nimg[c] = 0.0;  // below 0.49 of the period without asking
+        if ((__double2hiint(d[c]) & 0x7fffffff) >= __double2hiint(0.49 * prd[c])) {
+            nimg[c] = rint(d[c] * iprd[c]);
+            d[c] -= nimg[c] * prd[c];
+        }
     }
 }
 
 __device__ __forceinline__ double inertia(double m, double r) { return ((0.4 * m) * r) * r; }
 
-// Sum over the blocks' partials [NV][nb] into out[NV]: warp c sums component
-// c with lane-strided partial sums and a shuffle tree (fixed order).
+// Sum over the blocks' partials [NV][nb] into out[NV]: one warp per component
+// (warps first, first + 1, ...), eight loads of a lane in flight at once, four
+// running sums and a shuffle tree (fixed order).
 template <int NV>
-__device__ void sum_partials(const double* part, int nb, double* out) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (warp < NV) {
-        double s = 0.0;
-        for (int k = lane; k < nb; k += 32) s += part[(size_t)warp * nb + k];
+__device__ void sum_partials(const double* part, int nb, double* out, int first) {
+    const int c = (threadIdx.x >> 5) - first, lane = threadIdx.x & 31;
+    if (c < 0 || c >= NV) return;
+    const double* row = part + (size_t)c * nb;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int k0 = lane; k0 < nb; k0 += 256) {
+        double v[8];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        if (lane == 0) out[warp] = s;
+        for (int u = 0; u < 8; ++u) v[u] = k0 + 32 * u < nb ? row[k0 + 32 * u] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s[u & 3] += v[u];
     }
+    double t = (s[0] + s[1]) + (s[2] + s[3]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (lane == 0) out[c] = t;
+}
+
+// Programmatic dependent launch (see tmps_fused.cu): wait for the kernel before
+// to complete, then let the next one be scheduled.
+__device__ __forceinline__ void enter() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// A queued run of steps: `hit` is the step whose displacement check fired (0:
+// none).  That step's later launches and every launch of a later step return.
+struct Queue {
+    int64_t hit, done;
+};
+__device__ __forceinline__ bool halted(const Queue* q) { return q && *(volatile const int64_t*)&q->hit != 0; }
+
+// x / prd with the box's reciprocal at hand: the product corrected by its
+// residual, correctly rounded but for rare last bits (a position must not
+// move by one: the overlaps cancel its leading digits).
+__device__ __forceinline__ double over(double x, double prd, double iprd) {
+    const double q = __dmul_rn(x, iprd);
+    return __fma_rn(__fma_rn(-q, prd, x), iprd, q);
 }
 
 // ------------------------------------------------------------------ pairs
@@ -195,25 +241,47 @@ __global__ void k_carry(int nold, int nnew, const int32_t* __restrict__ map, dou
 
 // ---------------------------------------------------------------- forward
 
-__global__ void __launch_bounds__(kBlk) k_initial(tmps_adj_sys S, double dt, tmps_adj_tape T,
-                                                  const double* __restrict__ xbuild, unsigned long long* disp) {
+// First half of a step from S (remap == 0) or, inside a queued run, from the
+// tape of the step before: its xh remapped from box `before` to `prev`.  The
+// displacement check stamps q->hit (queued runs) or keeps the largest squared
+// displacement (disp).
+__global__ void __launch_bounds__(kBlk) k_initial(tmps_adj_sys S, double dt, tmps_adj_tape T, const double* xlast,
+                                                  const tmps_adj_rec* before, const tmps_adj_rec* prev,
+                                                  const double* __restrict__ xbuild, unsigned long long* disp, Queue* q,
+                                                  int64_t step, double trig) {
+    enter();
+    if (q) {
+        const int64_t h = *(volatile const int64_t*)&q->hit;
+        if (h != 0 && h != step) return;  // (another block of this step may have stamped it)
+    }
     const int n = S.n;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     double dd = 0.0;
     if (i < n) {
         const double dtf = 0.5 * dt;
-        const double m = S.mass[i], r = S.radius[i], I = inertia(m, r);
+        const double m = S.mass[i], r = S.radius[i], im = rcp64(m), iI = rcp64(inertia(m, r));
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const size_t k = (size_t)c * n + i;
-            const double v = S.v[k] + dtf * (S.f[k] / m);
-            const double x = S.x[k] + dt * v;
+            const double v = S.v[k] + dtf * (S.f[k] * im);
+            double x0;
+            if (before) {
+                const double lam = over(xlast[k] - before->lo[c], before->prd[c], rcp64(before->prd[c]));
+                x0 = prev->prd[c] * lam + prev->lo[c];
+            } else {
+                x0 = S.x[k];
+            }
+            const double x = x0 + dt * v;
             T.vh[k] = v;
             T.xh[k] = x;
-            T.wh[k] = S.w[k] + dtf * (S.t[k] / I);
+            T.wh[k] = S.w[k] + dtf * (S.t[k] * iI);
             const double e = x - xbuild[k];
             dd += e * e;
         }
+    }
+    if (q) {
+        if (__any_sync(0xffffffffu, dd > trig) && (threadIdx.x & 31) == 0) *(volatile int64_t*)&q->hit = step;
+        return;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dd = fmax(dd, __shfl_down_sync(0xffffffffu, dd, o));
@@ -241,22 +309,77 @@ __device__ __forceinline__ void load_pair(const tmps_adj_sys& S, const double* x
     (void)p;
 }
 
+// The pairs of a tile whose `in` holds, packed to the front of `list` in pair
+// order (two warps, each two rounds of 32); returns their number.
+__device__ __forceinline__ int pack_tile(const bool (&in)[kPairTile / kBlk], int* list /* [kPairTile] */,
+                                         int* count /* [kPairTile / 32] */) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t b[kPairTile / kBlk];
+#pragma unroll
+    for (int u = 0; u < kPairTile / kBlk; ++u) {
+        b[u] = __ballot_sync(0xffffffffu, in[u]);
+        if (lane == 0) count[u * (kBlk / 32) + warp] = __popc(b[u]);
+    }
+    __syncthreads();
+    int total = 0;
+#pragma unroll
+    for (int w = 0; w < kPairTile / 32; ++w) {
+#pragma unroll
+        for (int u = 0; u < kPairTile / kBlk; ++u)
+            if (w == u * (kBlk / 32) + warp && in[u]) list[total + __popc(b[u] & ((1u << lane) - 1u))] = u * kBlk + threadIdx.x;
+        total += count[w];
+    }
+    __syncthreads();
+    return total;
+}
+
 // Contacts of one pass: pair forces and torque terms into the workspace,
 // history updated in place (the entering history recorded), virial partials.
+// The tile's distances first; pairs out of contact are finished with zeros,
+// the law runs over the rest with full warps.
 __global__ void __launch_bounds__(kBlk) k_pairs(tmps_adj_sys S, Params P, int shearupdate, const double* xs,
                                                 const double* vs, const double* ws, const tmps_adj_rec* __restrict__ box,
-                                                double* __restrict__ sh_rec, uint8_t* __restrict__ mask_rec, Work W) {
+                                                double* __restrict__ sh_rec, uint8_t* __restrict__ mask_rec, Work W,
+                                                const Queue* q) {
     __shared__ double smem[6 * (kBlk / 32)];
-    const int np = S.npairs;
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    double vir[6] = {0, 0, 0, 0, 0, 0};
-    if (p < np) {
-        double prd[3], iprd[3], nimg[3];
+    __shared__ int list[kPairTile], count[kPairTile / 32];
+    enter();
+    if (halted(q)) return;
+    const int n = S.n, np = S.npairs;
+    double prd[3], iprd[3], nimg[3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            prd[c] = box->prd[c];
-            iprd[c] = 1.0 / prd[c];
+    for (int c = 0; c < 3; ++c) {
+        prd[c] = box->prd[c];
+        iprd[c] = rcp64(prd[c]);
+    }
+    double vir[6] = {0, 0, 0, 0, 0, 0};
+    bool in_[kPairTile / kBlk];
+#pragma unroll
+    for (int u = 0; u < kPairTile / kBlk; ++u) {
+        const int p = blockIdx.x * kPairTile + u * kBlk + threadIdx.x;
+        in_[u] = false;
+        if (p < np) {
+            const int i = S.pi[p], j = S.pj[p];
+            double d[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) d[c] = xs[(size_t)c * n + i] - xs[(size_t)c * n + j];
+            min_image(prd, iprd, d, nimg);
+            const double rsq = (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2];
+            const double radsum = S.radius[i] + S.radius[j];
+            in_[u] = rsq < radsum * radsum && rsq > 1e-28;
+            if (!in_[u]) {
+                mask_rec[p] = 0;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    sh_rec[(size_t)c * np + p] = S.shear[(size_t)c * np + p];
+                    S.shear[(size_t)c * np + p] = 0.0;
+                }
+            }
         }
+    }
+    const int total = pack_tile(in_, list, count);
+    for (int k = threadIdx.x; k < total; k += kBlk) {
+        const int p = blockIdx.x * kPairTile + list[k];
         PairIn in;
         load_pair(S, xs, vs, ws, prd, iprd, p, S.pi[p], S.pj[p], in, nimg);
 #pragma unroll
@@ -275,49 +398,51 @@ __global__ void __launch_bounds__(kBlk) k_pairs(tmps_adj_sys S, Params P, int sh
             W.fp[(size_t)c * np + p] = o.F[c];
             W.tp[(size_t)c * np + p] = o.tor[c];
         }
-        vir[0] = in.d[0] * o.F[0];
-        vir[1] = in.d[1] * o.F[1];
-        vir[2] = in.d[2] * o.F[2];
-        vir[3] = in.d[0] * o.F[1];
-        vir[4] = in.d[0] * o.F[2];
-        vir[5] = in.d[1] * o.F[2];
+        vir[0] += in.d[0] * o.F[0];
+        vir[1] += in.d[1] * o.F[1];
+        vir[2] += in.d[2] * o.F[2];
+        vir[3] += in.d[0] * o.F[1];
+        vir[4] += in.d[0] * o.F[2];
+        vir[5] += in.d[1] * o.F[2];
     }
-    block_sum<6, kBlk>(vir, smem);
-    if (threadIdx.x == 0) {
-        const int nb = gridDim.x;
-#pragma unroll
-        for (int c = 0; c < 6; ++c) W.partw[(size_t)c * nb + blockIdx.x] = vir[c];
-    }
+    const double tot = block_sum6_halving<kBlk>(vir, 0.0, true, smem);
+    if (threadIdx.x < 6) W.partw[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = tot;
 }
 
-// Per-atom force and torque from the pairs (as i: +F, then as j: -F; the
-// torque term times -r either way), then the second half-kick (final = 1)
-// and the kinetic partials m v v.
+// Per-atom force and torque from the pairs in contact (as i: +F, then as j:
+// -F; the torque term times -r either way), then the second half-kick (final =
+// 1) and the kinetic partials m v v.
 __global__ void __launch_bounds__(kBlk) k_gather(tmps_adj_sys S, double dt, int final_, const double* __restrict__ vh,
                                                  const double* __restrict__ wh, double* __restrict__ ft,
-                                                 double* __restrict__ tt, Work W) {
+                                                 double* __restrict__ tt, const uint8_t* mask, Work W, const Queue* q) {
     __shared__ double smem[6 * (kBlk / 32)];
+    enter();
+    if (halted(q)) return;
     const int n = S.n, np = S.npairs;
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     double kin[6] = {0, 0, 0, 0, 0, 0};
     if (a < n) {
         double F[3] = {0, 0, 0}, Tq[3] = {0, 0, 0};
         const double ra = S.radius[a];
-        for (int q = S.ibeg[a]; q < S.ibeg[a + 1]; ++q)
+        const int i0 = S.ibeg[a], i1 = S.ibeg[a + 1], j0 = S.jbeg[a], j1 = S.jbeg[a + 1];
+        for (int p = i0; p < i1; ++p) {
+            if (!mask[p]) continue;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                F[c] += W.fp[(size_t)c * np + q];
-                Tq[c] += -ra * W.tp[(size_t)c * np + q];
-            }
-        for (int k = S.jbeg[a]; k < S.jbeg[a + 1]; ++k) {
-            const int q = S.jlist[k];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                F[c] -= W.fp[(size_t)c * np + q];
-                Tq[c] += -ra * W.tp[(size_t)c * np + q];
+                F[c] += W.fp[(size_t)c * np + p];
+                Tq[c] += -ra * W.tp[(size_t)c * np + p];
             }
         }
-        const double m = S.mass[a], I = inertia(m, ra), dtf = 0.5 * dt;
+        for (int k = j0; k < j1; ++k) {
+            const int p = S.jlist[k];
+            if (!mask[p]) continue;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                F[c] -= W.fp[(size_t)c * np + p];
+                Tq[c] += -ra * W.tp[(size_t)c * np + p];
+            }
+        }
+        const double m = S.mass[a], im = rcp64(m), iI = rcp64(inertia(m, ra)), dtf = 0.5 * dt;
         double v[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -329,9 +454,9 @@ __global__ void __launch_bounds__(kBlk) k_gather(tmps_adj_sys S, double dt, int 
                 tt[k] = Tq[c];
             }
             if (final_) {
-                v[c] = vh[k] + dtf * (F[c] / m);
+                v[c] = vh[k] + dtf * (F[c] * im);
                 S.v[k] = v[c];
-                S.w[k] = wh[k] + dtf * (Tq[c] / I);
+                S.w[k] = wh[k] + dtf * (Tq[c] * iI);
             }
         }
         if (final_) {
@@ -344,12 +469,8 @@ __global__ void __launch_bounds__(kBlk) k_gather(tmps_adj_sys S, double dt, int 
         }
     }
     if (!final_) return;
-    block_sum<6, kBlk>(kin, smem);
-    if (threadIdx.x == 0) {
-        const int nb = gridDim.x;
-#pragma unroll
-        for (int c = 0; c < 6; ++c) W.partk[(size_t)c * nb + blockIdx.x] = kin[c];
-    }
+    const double tot = block_sum6_halving<kBlk>(kin, 0.0, true, smem);
+    if (threadIdx.x < 6) W.partk[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = tot;
 }
 
 // The servo rate of a pressure axis: gain, normalize/pressure, max/rate
@@ -395,19 +516,22 @@ __device__ void coupled(int couple, const double* P, double* p) {
 }
 
 // Virial total, pressure tensor, deviatoric stress, the servo's new box.
-__global__ void __launch_bounds__(256) k_servo(tmps_adj_servo sv, double dt, int64_t step, const tmps_adj_rec* prev,
-                                               tmps_adj_rec* next, int nbP, int nbA, Work W) {
+__global__ void __launch_bounds__(kOne) k_servo(tmps_adj_servo sv, double dt, int64_t step, const tmps_adj_rec* prev,
+                                                tmps_adj_rec* next, int nbP, int nbA, Work W, Queue* q) {
     __shared__ double sw[6], sk[6];
-    sum_partials<6>(W.partw, nbP, sw);
-    sum_partials<6>(W.partk, nbA, sk);
+    enter();
+    if (halted(q)) return;
+    sum_partials<6>(W.partw, nbP, sw, 0);
+    sum_partials<6>(W.partk, nbA, sk, 6);
     __syncthreads();
     if (threadIdx.x != 0) return;
+    if (q) q->done = step;
     tmps_adj_rec r = *prev;
-    const double vol = (r.prd[0] * r.prd[1]) * r.prd[2];
+    const double vol = (r.prd[0] * r.prd[1]) * r.prd[2], ivol = rcp64(vol);
     double Pt[6];
     for (int c = 0; c < 6; ++c) {
         r.w[c] = sw[c] + sk[c];
-        Pt[c] = r.w[c] / vol;
+        Pt[c] = over(r.w[c], vol, ivol);
     }
     r.q = Pt[2] - 0.5 * (Pt[0] + Pt[1]);
     r.elapsed = (double)step * dt;
@@ -438,62 +562,48 @@ __global__ void __launch_bounds__(256) k_servo(tmps_adj_servo sv, double dt, int
 }
 
 __global__ void __launch_bounds__(kBlk) k_remap(int n, const double* __restrict__ xh, const tmps_adj_rec* prev,
-                                                const tmps_adj_rec* next, double* __restrict__ x) {
+                                                const tmps_adj_rec* next, double* __restrict__ x, const Queue* q) {
+    enter();
+    if (halted(q)) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const size_t k = (size_t)c * n + i;
-        const double lam = (xh[k] - prev->lo[c]) / prev->prd[c];
+        const double lam = over(xh[k] - prev->lo[c], prev->prd[c], rcp64(prev->prd[c]));
         x[k] = next->prd[c] * lam + next->lo[c];
     }
 }
 
 // ---------------------------------------------------------------- reverse
 
-// x' = prd' (xh - lo) / prd + lo': the adjoint of xh in place, and the
-// partial sums of x'bar and x'bar lam per dimension for the box adjoints.
-__global__ void __launch_bounds__(kBlk) k_b_remap(int n, const double* __restrict__ xh, const tmps_adj_rec* prev,
-                                                  const tmps_adj_rec* next, double* __restrict__ xb, Work W) {
-    __shared__ double smem[6 * (kBlk / 32)];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double s[6] = {0, 0, 0, 0, 0, 0};
-    if (i < n) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const size_t k = (size_t)c * n + i;
-            const double lam = (xh[k] - prev->lo[c]) / prev->prd[c];
-            const double g = xb[k];
-            s[c] = g;
-            s[3 + c] = g * lam;
-            xb[k] = g * (next->prd[c] / prev->prd[c]);
-        }
-    }
-    block_sum<6, kBlk>(s, smem);
-    if (threadIdx.x == 0) {
-        const int nb = gridDim.x;
-#pragma unroll
-        for (int c = 0; c < 6; ++c) W.partk[(size_t)c * nb + blockIdx.x] = s[c];
-    }
-}
-
-// Reverse of the servo and the pressure: box adjoints (slot of record n =
+// The parameter and image partials of step `step` + 1's contact pass (reduce =
+// 1), then the reverse of step `step`'s servo and pressure (servo = 1): box adjoints (slot of record n =
 // step - 1 and of record n + 1 by parity), dL/d(virial total) into W.wbar.
-__global__ void __launch_bounds__(256) k_b_servo(tmps_adj_servo sv, double dt, int64_t step, const tmps_adj_rec* prev,
-                                                 const tmps_adj_rec* next, double qbar, int nbA, double* box_bar, Work W) {
-    __shared__ double s[6];
-    sum_partials<6>(W.partk, nbA, s);
+__global__ void __launch_bounds__(kOne) k_b_servo(tmps_adj_servo sv, double dt, int64_t step, const tmps_adj_rec* prev,
+                                                  const tmps_adj_rec* next, double qbar, int nbA, int nbP, int reduce,
+                                                  int servo, int slot, tmps_adj_bar B, Work W) {
+    __shared__ double s[6], g[8];
+    enter();
+    if (servo) sum_partials<6>(W.partk, nbA, s, 0);
+    if (reduce) sum_partials<8>(W.partg, nbP, g, 6);
     __syncthreads();
     if (threadIdx.x != 0) return;
+    double* const box_bar = B.box;
+    if (reduce) {
+        for (int c = 0; c < 5; ++c) B.params[c] += g[c];
+        for (int c = 0; c < 3; ++c) box_bar[9 * slot + 3 + c] += g[5 + c];
+    }
+    if (!servo) return;
     const int n = (int)(step - 1);
     double* bn = box_bar + 9 * (n & 1);          // record n: lo 0..2, prd 3..5, cum 6..8
     double* bn1 = box_bar + 9 * ((n + 1) & 1);   // record n + 1
     double Pt[6], p[3], pb[3] = {0, 0, 0}, Pb[6] = {0, 0, 0, 0, 0, 0};
-    const double vol = (prev->prd[0] * prev->prd[1]) * prev->prd[2];
-    for (int c = 0; c < 6; ++c) Pt[c] = next->w[c] / vol;
+    const double vol = (prev->prd[0] * prev->prd[1]) * prev->prd[2], ivol = rcp64(vol);
+    for (int c = 0; c < 6; ++c) Pt[c] = over(next->w[c], vol, ivol);
     coupled(sv.couple, Pt, p);
     for (int d = 0; d < 3; ++d) {
-        const double ratio = next->prd[d] / prev->prd[d];
+        const double ratio = next->prd[d] * rcp64(prev->prd[d]);
         // remap
         bn1[d] += s[d];
         bn1[3 + d] += s[3 + d];
@@ -539,8 +649,8 @@ __global__ void __launch_bounds__(256) k_b_servo(tmps_adj_servo sv, double dt, i
     // P = W / vol
     double volb = 0.0;
     for (int c = 0; c < 6; ++c) {
-        W.wbar[c] = Pb[c] / vol;
-        volb -= Pb[c] * Pt[c] / vol;
+        W.wbar[c] = Pb[c] * ivol;
+        volb -= Pb[c] * Pt[c] * ivol;
     }
     bn[3] += volb * prev->prd[1] * prev->prd[2];
     bn[4] += volb * prev->prd[0] * prev->prd[2];
@@ -549,10 +659,11 @@ __global__ void __launch_bounds__(256) k_b_servo(tmps_adj_servo sv, double dt, i
 
 // Reverse of the second half-kick and of the kinetic virial term.
 __global__ void __launch_bounds__(kBlk) k_b_final(tmps_adj_sys S, double dt, tmps_adj_tape T, tmps_adj_bar B, Work W) {
+    enter();
     const int n = S.n;
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= n) return;
-    const double m = S.mass[a], r = S.radius[a], I = inertia(m, r), dtf = 0.5 * dt;
+    const double m = S.mass[a], r = S.radius[a], im = rcp64(m), iI = rcp64(inertia(m, r)), dtf = 0.5 * dt;
     double wb[6];
 #pragma unroll
     for (int c = 0; c < 6; ++c) wb[c] = W.wbar[c];
@@ -561,7 +672,7 @@ __global__ void __launch_bounds__(kBlk) k_b_final(tmps_adj_sys S, double dt, tmp
     for (int c = 0; c < 3; ++c) {
         const size_t k = (size_t)c * n + a;
         f[c] = T.f[k];
-        v[c] = T.vh[k] + dtf * (f[c] / m);
+        v[c] = T.vh[k] + dtf * (f[c] * im);
         vb[c] = B.v[k];
     }
     // kinetic m v_a v_b
@@ -576,36 +687,51 @@ __global__ void __launch_bounds__(kBlk) k_b_final(tmps_adj_sys S, double dt, tmp
         const size_t k = (size_t)c * n + a;
         // v = vh + dtf f / m
         B.v[k] = vb[c];
-        B.f[k] += dtf * vb[c] / m;
-        mb -= dtf * vb[c] * f[c] / (m * m);
+        const double kb = dtf * vb[c] * im;
+        B.f[k] += kb;
+        mb -= kb * f[c] * im;
         // w = wh + dtf t / I
-        const double wbar = B.w[k];
-        B.t[k] += dtf * wbar / I;
-        Ib -= dtf * wbar * T.t[k] / (I * I);
+        const double tb = dtf * B.w[k] * iI;
+        B.t[k] += tb;
+        Ib -= tb * T.t[k] * iI;
     }
     B.mass[a] += mb + Ib * 0.4 * r * r;
     B.radius[a] += Ib * 0.8 * m * r;
 }
 
-// Reverse of the contact pass: per pair, recompute under the recorded mask,
-// then the reverse; per-pair adjoints for the gather, the entering history's
-// adjoint in place, parameter and image partials.
+// Reverse of the contact pass: per pair in contact, recompute under the
+// recorded mask, then the reverse; per-pair adjoints for the gather, the
+// entering history's adjoint in place, parameter and image partials.
 __global__ void __launch_bounds__(kBlk) k_b_pairs(tmps_adj_sys S, Params P, int shearupdate, const double* xs,
                                                   const double* vs, const double* ws, const double* __restrict__ sh_rec,
                                                   const uint8_t* __restrict__ mask_rec,
                                                   const tmps_adj_rec* __restrict__ box, const double* __restrict__ wbar,
                                                   tmps_adj_bar B, Work W) {
     __shared__ double smem[8 * (kBlk / 32)];
+    __shared__ int list[kPairTile], count[kPairTile / 32];
+    enter();
     const int n = S.n, np = S.npairs;
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    double part[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (p < np) {
-        double prd[3], iprd[3], nimg[3];
+    double prd[3], iprd[3], nimg[3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            prd[c] = box->prd[c];
-            iprd[c] = 1.0 / prd[c];
+    for (int c = 0; c < 3; ++c) {
+        prd[c] = box->prd[c];
+        iprd[c] = rcp64(prd[c]);
+    }
+    bool in_[kPairTile / kBlk];
+#pragma unroll
+    for (int u = 0; u < kPairTile / kBlk; ++u) {
+        const int p = blockIdx.x * kPairTile + u * kBlk + threadIdx.x;
+        in_[u] = p < np && mask_rec[p] != 0;
+        // out of contact: no force, and the history that leaves is zero whatever entered
+        if (p < np && !in_[u]) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) B.shear[(size_t)c * np + p] = 0.0;
         }
+    }
+    const int total = pack_tile(in_, list, count);
+    double part[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int k = threadIdx.x; k < total; k += kBlk) {
+        const int p = blockIdx.x * kPairTile + list[k];
         const int i = S.pi[p], j = S.pj[p];
         PairIn in;
         load_pair(S, xs, vs, ws, prd, iprd, p, i, j, in, nimg);
@@ -642,14 +768,14 @@ __global__ void __launch_bounds__(kBlk) k_b_pairs(tmps_adj_sys S, Params P, int 
         G[(size_t)13 * np + p] = g.rb;
         G[(size_t)14 * np + p] = g.ma;
         G[(size_t)15 * np + p] = g.mb;
-        part[0] = g.kn;
-        part[1] = g.kt;
-        part[2] = g.gamman;
-        part[3] = g.gammat;
-        part[4] = g.xmu;
+        part[0] += g.kn;
+        part[1] += g.kt;
+        part[2] += g.gamman;
+        part[3] += g.gammat;
+        part[4] += g.xmu;
         // d = xa - xb - nimg prd
 #pragma unroll
-        for (int c = 0; c < 3; ++c) part[5 + c] = -nimg[c] * g.d[c];
+        for (int c = 0; c < 3; ++c) part[5 + c] -= nimg[c] * g.d[c];
     }
     block_sum<8, kBlk>(part, smem);
     if (threadIdx.x == 0) {
@@ -659,78 +785,94 @@ __global__ void __launch_bounds__(kBlk) k_b_pairs(tmps_adj_sys S, Params P, int 
     }
 }
 
-__global__ void __launch_bounds__(256) k_b_reduce(int nbP, int slot, tmps_adj_bar B, Work W) {
-    __shared__ double s[8];
-    sum_partials<8>(W.partg, nbP, s);
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    for (int c = 0; c < 5; ++c) B.params[c] += s[c];
-    for (int c = 0; c < 3; ++c) B.box[9 * slot + 3 + c] += s[5 + c];
-}
-
-// Per-atom sums of the pairs' adjoints (as i, then as j).
-__global__ void __launch_bounds__(kBlk) k_b_gather(tmps_adj_sys S, tmps_adj_bar B, Work W) {
+// Per atom: the sums of the pairs' adjoints (as i, then as j) and the reverse
+// of the first half-kick and the drift of a step (gather = 1: leaves the
+// adjoint of the state before it, and of the forces it started from; kick = 0:
+// the sums alone), then the reverse of the remap that ended the step before
+// (xh != NULL): x' = prd' (xh - lo) / prd + lo', the adjoint of xh in place and
+// the partial sums of x'bar and x'bar lam per dimension for the box adjoints.
+__global__ void __launch_bounds__(kBlk) k_b_atoms(tmps_adj_sys S, double dt, int gather, int kick,
+                                                  const uint8_t* mask, const double* __restrict__ fprev,
+                                                  const double* __restrict__ tprev, const double* __restrict__ xh,
+                                                  const tmps_adj_rec* prev, const tmps_adj_rec* next, tmps_adj_bar B,
+                                                  Work W) {
+    __shared__ double smem[6 * (kBlk / 32)];
+    enter();
     const int n = S.n, np = S.npairs;
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= n) return;
-    const double* G = W.gp;
-    double xb[3] = {0, 0, 0}, vb[3] = {0, 0, 0}, wb[3] = {0, 0, 0}, rb = 0.0, mb = 0.0;
-    for (int q = S.ibeg[a]; q < S.ibeg[a + 1]; ++q) {
+    double s[6] = {0, 0, 0, 0, 0, 0};
+    if (a < n) {
+        double xb[3] = {0, 0, 0};
+        if (gather) {
+            const double* G = W.gp;
+            double vb[3] = {0, 0, 0}, wb[3] = {0, 0, 0}, rb = 0.0, mb = 0.0;
+            const int i0 = S.ibeg[a], i1 = S.ibeg[a + 1], j0 = S.jbeg[a], j1 = S.jbeg[a + 1];
+            for (int p = i0; p < i1; ++p) {
+                if (!mask[p]) continue;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            xb[c] += G[(size_t)c * np + q];
-            vb[c] += G[(size_t)(3 + c) * np + q];
-            wb[c] += G[(size_t)(6 + c) * np + q];
+                for (int c = 0; c < 3; ++c) {
+                    xb[c] += G[(size_t)c * np + p];
+                    vb[c] += G[(size_t)(3 + c) * np + p];
+                    wb[c] += G[(size_t)(6 + c) * np + p];
+                }
+                rb += G[(size_t)12 * np + p];
+                mb += G[(size_t)14 * np + p];
+            }
+            for (int k = j0; k < j1; ++k) {
+                const int p = S.jlist[k];
+                if (!mask[p]) continue;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    xb[c] -= G[(size_t)c * np + p];
+                    vb[c] -= G[(size_t)(3 + c) * np + p];
+                    wb[c] += G[(size_t)(9 + c) * np + p];
+                }
+                rb += G[(size_t)13 * np + p];
+                mb += G[(size_t)15 * np + p];
+            }
+            const double m = S.mass[a], r = S.radius[a], im = rcp64(m), iI = rcp64(inertia(m, r)), dtf = 0.5 * dt;
+            double Ib = 0.0;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const size_t k = (size_t)c * n + a;
+                xb[c] = B.x[k] + xb[c];
+                const double v1 = B.v[k] + vb[c], w1 = B.w[k] + wb[c];
+                if (kick) {
+                    // x = x0 + dt vh; vh = v0 + dtf f / m; wh = w0 + dtf t / I
+                    const double vhb = v1 + dt * xb[c];
+                    const double fb = dtf * vhb * im, tb = dtf * w1 * iI;
+                    B.v[k] = vhb;
+                    B.f[k] = fb;
+                    mb -= fb * fprev[k] * im;
+                    B.w[k] = w1;
+                    B.t[k] = tb;
+                    Ib -= tb * tprev[k] * iI;
+                } else {
+                    B.v[k] = v1;
+                    B.w[k] = w1;
+                }
+                if (!xh) B.x[k] = xb[c];
+            }
+            B.mass[a] += mb + Ib * 0.4 * r * r;
+            B.radius[a] += rb + Ib * 0.8 * m * r;
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) xb[c] = B.x[(size_t)c * n + a];
         }
-        rb += G[(size_t)12 * np + q];
-        mb += G[(size_t)14 * np + q];
-    }
-    for (int k = S.jbeg[a]; k < S.jbeg[a + 1]; ++k) {
-        const int q = S.jlist[k];
+        if (xh) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            xb[c] -= G[(size_t)c * np + q];
-            vb[c] -= G[(size_t)(3 + c) * np + q];
-            wb[c] += G[(size_t)(9 + c) * np + q];
+            for (int c = 0; c < 3; ++c) {
+                const size_t k = (size_t)c * n + a;
+                const double ip = rcp64(prev->prd[c]);
+                s[c] = xb[c];
+                s[3 + c] = xb[c] * ((xh[k] - prev->lo[c]) * ip);
+                B.x[k] = xb[c] * (next->prd[c] * ip);
+            }
         }
-        rb += G[(size_t)13 * np + q];
-        mb += G[(size_t)15 * np + q];
     }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const size_t k = (size_t)c * n + a;
-        B.x[k] += xb[c];
-        B.v[k] += vb[c];
-        B.w[k] += wb[c];
-    }
-    B.radius[a] += rb;
-    B.mass[a] += mb;
-}
-
-// Reverse of the first half-kick and the drift: leaves the adjoint of the
-// state before the step, and the adjoint of the forces it started from.
-__global__ void __launch_bounds__(kBlk) k_b_initial(tmps_adj_sys S, double dt, const double* __restrict__ fprev,
-                                                    const double* __restrict__ tprev, tmps_adj_bar B) {
-    const int n = S.n;
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= n) return;
-    const double m = S.mass[a], r = S.radius[a], I = inertia(m, r), dtf = 0.5 * dt;
-    double mb = 0.0, Ib = 0.0;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const size_t k = (size_t)c * n + a;
-        // x = x0 + dt vh; vh = v0 + dtf f / m
-        const double vhb = B.v[k] + dt * B.x[k];
-        B.v[k] = vhb;
-        B.f[k] = dtf * vhb / m;
-        mb -= dtf * vhb * fprev[k] / (m * m);
-        // wh = w0 + dtf t / I
-        const double whb = B.w[k];
-        B.t[k] = dtf * whb / I;
-        Ib -= dtf * whb * tprev[k] / (I * I);
-    }
-    B.mass[a] += mb + Ib * 0.4 * r * r;
-    B.radius[a] += Ib * 0.8 * m * r;
+    if (!xh) return;
+    const double tot = block_sum6_halving<kBlk>(s, 0.0, true, smem);
+    if (threadIdx.x < 6) W.partk[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = tot;
 }
 
 bool ok() { return cudaPeekAtLastError() == cudaSuccess; }
@@ -738,6 +880,57 @@ bool ok() { return cudaPeekAtLastError() == cudaSuccess; }
 bool sys_ok(const tmps_adj_sys* s) {
     return s && s->n >= 0 && s->npairs >= 0 && s->x && s->v && s->w && s->f && s->t && s->radius && s->mass &&
            (s->npairs == 0 || (s->shear && s->pi && s->pj)) && s->ibeg && s->jbeg && (s->npairs == 0 || s->jlist);
+}
+
+// Launch with programmatic stream serialization (see enter), counted.
+template <typename... P, typename... A>
+void run(void (*kernel)(P...), int grid, int block, cudaStream_t s, A&&... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+    note_launches(1);
+}
+
+// The tape of the k-th step of a run whose tapes lie atom_stride doubles (atom
+// arrays) and pair_stride pairs apart (0: one tape, overwritten).
+tmps_adj_tape tape_at(const tmps_adj_tape& t, int64_t atom_stride, int64_t pair_stride, int64_t k) {
+    tmps_adj_tape o = t;
+    o.xh += k * atom_stride;
+    o.vh += k * atom_stride;
+    o.wh += k * atom_stride;
+    o.f += k * atom_stride;
+    o.t += k * atom_stride;
+    o.shear += 3 * k * pair_stride;
+    o.mask += k * pair_stride;
+    return o;
+}
+
+// Contacts, second half-kick, pressure and servo of a step.
+int rest_of_step(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_adj_servo* sv, const tmps_adj_tape& t,
+                 tmps_adj_rec* d_rec, int64_t step, const Work& W, Queue* q, cudaStream_t st) {
+    const int nbA = grid_for(s->n, kBlk), nbP = grid_for(s->npairs, kPairTile);
+    const tmps_adj_rec* prev = d_rec + (step - 1);
+    if (s->npairs > 0) {
+        run(k_pairs, nbP, kBlk, st, *s, to_params(*p), 1, (const double*)t.xh, (const double*)t.vh, (const double*)t.wh,
+            prev, t.shear, t.mask, W, (const Queue*)q);
+    } else if (cudaMemsetAsync(W.partw, 0, sizeof(double) * 6 * nbP, st) != cudaSuccess) {
+        return TMPS_ERR_CUDA;
+    }
+    if (s->n > 0) {
+        run(k_gather, nbA, kBlk, st, *s, p->dt, 1, (const double*)t.vh, (const double*)t.wh, t.f, t.t,
+            (const uint8_t*)t.mask, W, (const Queue*)q);
+    } else if (cudaMemsetAsync(W.partk, 0, sizeof(double) * 6 * nbA, st) != cudaSuccess) {
+        return TMPS_ERR_CUDA;
+    }
+    run(k_servo, 1, kOne, st, *sv, p->dt, step, prev, d_rec + step, nbP, nbA, W, q);
+    return TMPS_OK;
 }
 
 }  // namespace
@@ -790,13 +983,11 @@ int tmps_adj_setup(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_a
     if (s->n == 0) return TMPS_OK;
     cudaStream_t st = (cudaStream_t)stream;
     Work W = carve(work, s->n, s->npairs);
-    if (s->npairs > 0) {
-        k_pairs<<<grid_for(s->npairs, kBlk), kBlk, 0, st>>>(*s, to_params(*p), 0, s->x, s->v, s->w, d_box,
-                                                             tape->shear, tape->mask, W);
-        note_launches(1);
-    }
-    k_gather<<<grid_for(s->n, kBlk), kBlk, 0, st>>>(*s, p->dt, 0, nullptr, nullptr, tape->f, tape->t, W);
-    note_launches(1);
+    if (s->npairs > 0)
+        run(k_pairs, grid_for(s->npairs, kPairTile), kBlk, st, *s, to_params(*p), 0, (const double*)s->x, (const double*)s->v,
+            (const double*)s->w, d_box, tape->shear, tape->mask, W, (const Queue*)nullptr);
+    run(k_gather, grid_for(s->n, kBlk), kBlk, st, *s, p->dt, 0, (const double*)nullptr, (const double*)nullptr, tape->f,
+        tape->t, (const uint8_t*)tape->mask, W, (const Queue*)nullptr);
     return ok() ? TMPS_OK : TMPS_ERR_CUDA;
 }
 
@@ -805,9 +996,9 @@ int tmps_adj_initial(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps
     if (!sys_ok(s) || !p || !tape || !tape->xh || !tape->vh || !tape->wh || !d_xbuild || !d_disp)
         return TMPS_ERR_BAD_ARG;
     if (s->n == 0) return TMPS_OK;
-    k_initial<<<grid_for(s->n, kBlk), kBlk, 0, (cudaStream_t)stream>>>(*s, p->dt, *tape, d_xbuild,
-                                                                        (unsigned long long*)d_disp);
-    note_launches(1);
+    run(k_initial, grid_for(s->n, kBlk), kBlk, (cudaStream_t)stream, *s, p->dt, *tape, (const double*)nullptr,
+        (const tmps_adj_rec*)nullptr, (const tmps_adj_rec*)nullptr, d_xbuild, (unsigned long long*)d_disp,
+        (Queue*)nullptr, (int64_t)0, 0.0);
     return ok() ? TMPS_OK : TMPS_ERR_CUDA;
 }
 
@@ -817,28 +1008,85 @@ int tmps_adj_finish(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_
         !tape->f || !tape->t)
         return TMPS_ERR_BAD_ARG;
     cudaStream_t st = (cudaStream_t)stream;
+    const int rc = rest_of_step(s, p, sv, *tape, d_rec, step, carve(work, s->n, s->npairs), nullptr, st);
+    if (rc != TMPS_OK) return rc;
+    if (s->n > 0)
+        run(k_remap, grid_for(s->n, kBlk), kBlk, st, s->n, (const double*)tape->xh, (const tmps_adj_rec*)(d_rec + (step - 1)),
+            (const tmps_adj_rec*)(d_rec + step), s->x, (const Queue*)nullptr);
+    return ok() ? TMPS_OK : TMPS_ERR_CUDA;
+}
+
+int tmps_adj_forward(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_adj_servo* sv,
+                     const tmps_adj_tape* tape, int64_t atom_stride, int64_t pair_stride, tmps_adj_rec* d_rec,
+                     int64_t first, int64_t last, const double* d_xbuild, double trigger_sq, int64_t* d_queue, void* work,
+                     void* stream) {
+    if (!sys_ok(s) || !p || !sv || !tape || !d_rec || first < 1 || last < first || !work || !tape->xh || !tape->vh ||
+        !tape->wh || !tape->shear || !tape->mask || !tape->f || !tape->t || !d_queue || !d_xbuild || atom_stride < 0 ||
+        pair_stride < 0)
+        return TMPS_ERR_BAD_ARG;
+    cudaStream_t st = (cudaStream_t)stream;
     Work W = carve(work, s->n, s->npairs);
-    const int nbA = grid_for(s->n, kBlk), nbP = grid_for(s->npairs, kBlk);
-    tmps_adj_rec* prev = d_rec + (step - 1);
-    tmps_adj_rec* next = d_rec + step;
-    if (s->npairs > 0) {
-        k_pairs<<<nbP, kBlk, 0, st>>>(*s, to_params(*p), 1, tape->xh, tape->vh, tape->wh, prev, tape->shear,
-                                      tape->mask, W);
-        note_launches(1);
-    } else if (cudaMemsetAsync(W.partw, 0, sizeof(double) * 6 * nbP, st) != cudaSuccess) {
-        return TMPS_ERR_CUDA;
+    Queue* q = reinterpret_cast<Queue*>(d_queue);
+    if (cudaMemsetAsync(q, 0, sizeof(Queue), st) != cudaSuccess) return TMPS_ERR_CUDA;
+    const double* xlast = nullptr;
+    tmps_adj_tape t = *tape;
+    for (int64_t step = first; step <= last; ++step) {
+        t = tape_at(*tape, atom_stride, pair_stride, step - first);
+        if (s->n > 0)
+            run(k_initial, grid_for(s->n, kBlk), kBlk, st, *s, p->dt, t, xlast,
+                (const tmps_adj_rec*)(step > first ? d_rec + (step - 2) : nullptr), (const tmps_adj_rec*)(d_rec + (step - 1)),
+                d_xbuild, (unsigned long long*)nullptr, q, step, trigger_sq);
+        const int rc = rest_of_step(s, p, sv, t, d_rec, step, W, q, st);
+        if (rc != TMPS_OK) return rc;
+        xlast = t.xh;
     }
-    if (s->n > 0) {
-        k_gather<<<nbA, kBlk, 0, st>>>(*s, p->dt, 1, tape->vh, tape->wh, tape->f, tape->t, W);
-        note_launches(1);
-    } else if (cudaMemsetAsync(W.partk, 0, sizeof(double) * 6 * nbA, st) != cudaSuccess) {
-        return TMPS_ERR_CUDA;
-    }
-    k_servo<<<1, 256, 0, st>>>(*sv, p->dt, step, prev, next, nbP, nbA, W);
-    note_launches(1);
-    if (s->n > 0) {
-        k_remap<<<nbA, kBlk, 0, st>>>(s->n, tape->xh, prev, next, s->x);
-        note_launches(1);
+    if (s->n > 0)
+        run(k_remap, grid_for(s->n, kBlk), kBlk, st, s->n, (const double*)t.xh, (const tmps_adj_rec*)(d_rec + (last - 1)),
+            (const tmps_adj_rec*)(d_rec + last), s->x, (const Queue*)q);
+    return ok() ? TMPS_OK : TMPS_ERR_CUDA;
+}
+
+int tmps_adj_reverse(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_adj_servo* sv,
+                     const tmps_adj_tape* tape, int64_t atom_stride, int64_t pair_stride, const tmps_adj_rec* d_rec,
+                     int64_t first, int64_t last, const double* d_fprev, const double* d_tprev, const double* d_xprev,
+                     int32_t linked, const double* qbar, const tmps_adj_bar* b, void* work, void* stream) {
+    if (!sys_ok(s) || !p || !sv || !tape || !d_rec || first < 1 || last < first || !d_fprev || !d_tprev || !qbar || !b ||
+        !work || atom_stride < 0 || pair_stride < 0)
+        return TMPS_ERR_BAD_ARG;
+    if (!b->x || !b->v || !b->w || !b->f || !b->t || !b->radius || !b->mass || !b->params || !b->box ||
+        (s->npairs > 0 && !b->shear))
+        return TMPS_ERR_BAD_ARG;
+    cudaStream_t st = (cudaStream_t)stream;
+    Work W = carve(work, s->n, s->npairs);
+    const int nbA = grid_for(s->n, kBlk), nbP = grid_for(s->npairs, kPairTile);
+    if (s->n == 0 && cudaMemsetAsync(W.partk, 0, sizeof(double) * 6 * nbA, st) != cudaSuccess) return TMPS_ERR_CUDA;
+    auto rec = [&](int64_t k) { return d_rec + k; };
+    const double* none = nullptr;
+    for (int64_t step = last; step >= first; --step) {
+        const tmps_adj_tape t = tape_at(*tape, atom_stride, pair_stride, step - first);
+        if (step == last && !linked) {
+            // the remap and the servo of the last step; else the call for the steps after it did them
+            if (s->n > 0)
+                run(k_b_atoms, nbA, kBlk, st, *s, p->dt, 0, 0, (const uint8_t*)nullptr, none, none, (const double*)t.xh,
+                    rec(step - 1), rec(step), *b, W);
+            run(k_b_servo, 1, kOne, st, *sv, p->dt, step, rec(step - 1), rec(step), qbar[step - first + 1], nbA, nbP, 0, 1, 0,
+                *b, W);
+        }
+        const double* xh = step > first ? tape_at(*tape, atom_stride, pair_stride, step - 1 - first).xh : d_xprev;
+        if (s->n > 0) {
+            run(k_b_final, nbA, kBlk, st, *s, p->dt, t, *b, W);
+            if (s->npairs > 0)
+                run(k_b_pairs, nbP, kBlk, st, *s, to_params(*p), 1, (const double*)t.xh, (const double*)t.vh,
+                    (const double*)t.wh, (const double*)t.shear, (const uint8_t*)t.mask, rec(step - 1),
+                    (const double*)W.wbar, *b, W);
+            const tmps_adj_tape tp = step > first ? tape_at(*tape, atom_stride, pair_stride, step - 1 - first) : t;
+            run(k_b_atoms, nbA, kBlk, st, *s, p->dt, 1, 1, (const uint8_t*)t.mask,
+                step > first ? (const double*)tp.f : d_fprev, step > first ? (const double*)tp.t : d_tprev, xh,
+                xh ? rec(step - 2) : rec(step - 1), xh ? rec(step - 1) : rec(step), *b, W);
+        }
+        // (the slot of record step - 1 takes the image terms of this step's contacts)
+        run(k_b_servo, 1, kOne, st, *sv, p->dt, step - 1, rec(step > 1 ? step - 2 : 0), rec(step - 1), qbar[step - first], nbA,
+            nbP, s->npairs > 0 ? 1 : 0, xh ? 1 : 0, (int)((step - 1) & 1), *b, W);
     }
     return ok() ? TMPS_OK : TMPS_ERR_CUDA;
 }
@@ -846,37 +1094,8 @@ int tmps_adj_finish(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_
 int tmps_adj_step_back(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_adj_servo* sv,
                        const tmps_adj_tape* tape, const tmps_adj_rec* d_rec, int64_t step, const double* d_fprev,
                        const double* d_tprev, double qbar, const tmps_adj_bar* b, void* work, void* stream) {
-    if (!sys_ok(s) || !p || !sv || !tape || !d_rec || step < 1 || !d_fprev || !d_tprev || !b || !work)
-        return TMPS_ERR_BAD_ARG;
-    if (!b->x || !b->v || !b->w || !b->f || !b->t || !b->radius || !b->mass || !b->params || !b->box ||
-        (s->npairs > 0 && !b->shear))
-        return TMPS_ERR_BAD_ARG;
-    cudaStream_t st = (cudaStream_t)stream;
-    Work W = carve(work, s->n, s->npairs);
-    const int nbA = grid_for(s->n, kBlk), nbP = grid_for(s->npairs, kBlk);
-    const tmps_adj_rec* prev = d_rec + (step - 1);
-    const tmps_adj_rec* next = d_rec + step;
-    if (s->n > 0) {
-        k_b_remap<<<nbA, kBlk, 0, st>>>(s->n, tape->xh, prev, next, b->x, W);
-        note_launches(1);
-    } else if (cudaMemsetAsync(W.partk, 0, sizeof(double) * 6 * nbA, st) != cudaSuccess) {
-        return TMPS_ERR_CUDA;
-    }
-    k_b_servo<<<1, 256, 0, st>>>(*sv, p->dt, step, prev, next, qbar, nbA, b->box, W);
-    note_launches(1);
-    if (s->n == 0) return ok() ? TMPS_OK : TMPS_ERR_CUDA;
-    k_b_final<<<nbA, kBlk, 0, st>>>(*s, p->dt, *tape, *b, W);
-    note_launches(1);
-    if (s->npairs > 0) {
-        k_b_pairs<<<nbP, kBlk, 0, st>>>(*s, to_params(*p), 1, tape->xh, tape->vh, tape->wh, tape->shear, tape->mask,
-                                        prev, W.wbar, *b, W);
-        k_b_reduce<<<1, 256, 0, st>>>(nbP, (int)((step - 1) & 1), *b, W);
-        k_b_gather<<<nbA, kBlk, 0, st>>>(*s, *b, W);
-        note_launches(3);
-    }
-    k_b_initial<<<nbA, kBlk, 0, st>>>(*s, p->dt, d_fprev, d_tprev, *b);
-    note_launches(1);
-    return ok() ? TMPS_OK : TMPS_ERR_CUDA;
+    const double q[2] = {0.0, qbar};
+    return tmps_adj_reverse(s, p, sv, tape, 0, 0, d_rec, step, step, d_fprev, d_tprev, nullptr, 0, q, b, work, stream);
 }
 
 int tmps_adj_setup_back(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_adj_rec* d_box,
@@ -887,12 +1106,12 @@ int tmps_adj_setup_back(const tmps_adj_sys* s, const tmps_adj_params* p, const t
     if (s->n == 0 || s->npairs == 0) return TMPS_OK;
     cudaStream_t st = (cudaStream_t)stream;
     Work W = carve(work, s->n, s->npairs);
-    const int nbA = grid_for(s->n, kBlk), nbP = grid_for(s->npairs, kBlk);
-    k_b_pairs<<<nbP, kBlk, 0, st>>>(*s, to_params(*p), 0, s->x, s->v, s->w, tape->shear, tape->mask, d_box, nullptr,
-                                    *b, W);
-    k_b_reduce<<<1, 256, 0, st>>>(nbP, 0, *b, W);
-    k_b_gather<<<nbA, kBlk, 0, st>>>(*s, *b, W);
-    note_launches(3);
+    const int nbA = grid_for(s->n, kBlk), nbP = grid_for(s->npairs, kPairTile);
+    const double* none = nullptr;
+    run(k_b_pairs, nbP, kBlk, st, *s, to_params(*p), 0, (const double*)s->x, (const double*)s->v, (const double*)s->w,
+        (const double*)tape->shear, (const uint8_t*)tape->mask, d_box, none, *b, W);
+    run(k_b_atoms, nbA, kBlk, st, *s, p->dt, 1, 0, (const uint8_t*)tape->mask, none, none, none, d_box, d_box, *b, W);
+    run(k_b_servo, 1, kOne, st, tmps_adj_servo{}, p->dt, (int64_t)1, d_box, d_box, 0.0, nbA, nbP, 1, 0, 0, *b, W);
     return ok() ? TMPS_OK : TMPS_ERR_CUDA;
 }
 

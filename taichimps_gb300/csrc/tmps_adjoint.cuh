@@ -25,12 +25,32 @@
 #include <math.h>
 
 #if defined(__CUDACC__)
+#include "tmps_common.cuh"
 #define TMPS_HD __host__ __device__ __forceinline__
 #else
 #define TMPS_HD inline
 #endif
 
 namespace tmps_adj {
+
+// 1 / x, and sqrt(x) with 1 / sqrt(x): on the device the short forms of
+// tmps_common.cuh (a correctly rounded division or root is several times their
+// FP64 instructions), on the host the operations themselves.
+TMPS_HD double rcp(double x) {
+#if defined(__CUDA_ARCH__)
+    return tmps::rcp64(x);
+#else
+    return 1.0 / x;
+#endif
+}
+TMPS_HD void root(double x, double& r, double& inv) {
+#if defined(__CUDA_ARCH__)
+    tmps::sqrt_rsqrt64(x, r, inv);
+#else
+    r = sqrt(x);
+    inv = 1.0 / r;
+#endif
+}
 
 enum { M_CONTACT = 1, M_SLIP = 2, M_SHRMAG = 4, M_CLAMP = 8 };
 
@@ -55,9 +75,10 @@ struct PairOut {
 // Forward intermediates the reverse reads.
 struct PairTape {
     double rsq, r, delta, reff, ph, meff, rsqinv, rinv;
+    double irs, ims, iph, ifsmag;  // 1 / (ra + rb), 1 / (ma + mb), 1 / ph, 1 / fsmag (only where it slips)
     double vrel[3], vnnr, s, g[3], wr[3], vtr[3];
     double ccel0, ccel, geff;
-    double sh1[3], rsht, sh2[3], t[3], fs0[3], fsmag, u, fn, ratio, dc[3];
+    double sh1[3], rsht, sh2[3], t[3], fs0[3], u, fn, ratio, dc[3];
     double fs[3], c[3];
 };
 
@@ -99,13 +120,14 @@ TMPS_HD void pair_forward(const Params& P, int shearupdate, const PairIn& in, in
         return;
     }
     m |= M_CONTACT;
-    t.r = sqrt(t.rsq);
+    root(t.rsq, t.r, t.rinv);
+    t.rsqinv = t.rinv * t.rinv;
     t.delta = radsum - t.r;
-    t.reff = (in.ra * in.rb) / (in.ra + in.rb);
-    t.ph = sqrt(t.reff * t.delta);
-    t.meff = (in.ma * in.mb) / (in.ma + in.mb);
-    t.rsqinv = 1.0 / t.rsq;
-    t.rinv = 1.0 / t.r;
+    t.irs = rcp(radsum);
+    t.reff = (in.ra * in.rb) * t.irs;
+    root(t.reff * t.delta, t.ph, t.iph);
+    t.ims = rcp(in.ma + in.mb);
+    t.meff = (in.ma * in.mb) * t.ims;
     for (int k = 0; k < 3; ++k) t.vrel[k] = in.va[k] - in.vb[k];
     t.vnnr = dot3(t.vrel, d);
     t.s = t.vnnr * t.rsqinv;
@@ -126,8 +148,7 @@ TMPS_HD void pair_forward(const Params& P, int shearupdate, const PairIn& in, in
     }
     t.geff = t.meff * P.gammat;
     for (int k = 0; k < 3; ++k) t.sh1[k] = shearupdate ? in.sh[k] + t.vtr[k] * P.dt : in.sh[k];
-    const double shrmag = sqrt(dot3(t.sh1, t.sh1));
-    const bool shnz = forced >= 0 ? (forced & M_SHRMAG) != 0 : shrmag != 0.0;
+    const bool shnz = forced >= 0 ? (forced & M_SHRMAG) != 0 : dot3(t.sh1, t.sh1) != 0.0;  // |sh1| != 0
     if (shnz) m |= M_SHRMAG;
     if (shearupdate) {
         t.rsht = dot3(t.sh1, d) * t.rsqinv;
@@ -140,18 +161,22 @@ TMPS_HD void pair_forward(const Params& P, int shearupdate, const PairIn& in, in
         t.t[k] = P.kt * t.sh2[k] + t.geff * t.vtr[k];
         t.fs0[k] = (-t.ph) * t.t[k];
     }
-    t.fsmag = sqrt(dot3(t.fs0, t.fs0));
+    const double fs2 = dot3(t.fs0, t.fs0);
     t.u = t.ccel * t.r;
     t.fn = P.xmu * fabs(t.u);
     t.ratio = 1.0;
+    t.ifsmag = 0.0;
     for (int k = 0; k < 3; ++k) t.dc[k] = 0.0;
-    const bool slip = forced >= 0 ? (forced & M_SLIP) != 0 : t.fsmag > t.fn;
+    const bool slip = forced >= 0 ? (forced & M_SLIP) != 0 : fs2 > t.fn * t.fn;  // |fs0| > fn
     if (slip) {
         m |= M_SLIP;
         if (shnz) {
-            t.ratio = t.fn / t.fsmag;
+            double fsmag;
+            root(fs2, fsmag, t.ifsmag);
+            t.ratio = t.fn * t.ifsmag;
+            const double ikt = rcp(P.kt);
             for (int k = 0; k < 3; ++k) {
-                t.dc[k] = (t.geff * t.vtr[k]) / P.kt;
+                t.dc[k] = (t.geff * t.vtr[k]) * ikt;
                 o.sh[k] = t.ratio * (t.sh2[k] + t.dc[k]) - t.dc[k];
                 t.fs[k] = t.ratio * t.fs0[k];
             }
@@ -215,6 +240,7 @@ TMPS_HD void pair_reverse(const Params& P, int shearupdate, int mask, const Pair
         if (mask & M_SHRMAG) {
             double ratiob = dot3(fsb, t.fs0);
             double dcb[3];
+            const double ikt = rcp(P.kt);
             for (int k = 0; k < 3; ++k) {
                 ratiob += b.sh[k] * (t.sh2[k] + t.dc[k]);
                 fs0b[k] = t.ratio * fsb[k];
@@ -223,13 +249,13 @@ TMPS_HD void pair_reverse(const Params& P, int shearupdate, int mask, const Pair
             }
             // dc = geff vtr / kt
             for (int k = 0; k < 3; ++k) {
-                geffb += dcb[k] * t.vtr[k] / P.kt;
-                vtrb[k] += t.geff * dcb[k] / P.kt;
+                geffb += dcb[k] * t.vtr[k] * ikt;
+                vtrb[k] += t.geff * dcb[k] * ikt;
             }
-            g.kt -= dot3(dcb, t.dc) / P.kt;
+            g.kt -= dot3(dcb, t.dc) * ikt;
             // ratio = fn / fsmag
-            fnb += ratiob / t.fsmag;
-            fsmagb -= ratiob * t.ratio / t.fsmag;
+            fnb += ratiob * t.ifsmag;
+            fsmagb -= ratiob * t.ratio * t.ifsmag;
         } else {
             for (int k = 0; k < 3; ++k) {
                 fs0b[k] = 0.0;
@@ -248,8 +274,8 @@ TMPS_HD void pair_reverse(const Params& P, int shearupdate, int mask, const Pair
     ccelb += ub * t.r;
     rbar += ub * t.ccel;
     // fsmag = |fs0|
-    if (t.fsmag > 0.0)
-        for (int k = 0; k < 3; ++k) fs0b[k] += fsmagb * t.fs0[k] / t.fsmag;
+    if (fsmagb != 0.0)
+        for (int k = 0; k < 3; ++k) fs0b[k] += fsmagb * t.fs0[k] * t.ifsmag;
     // fs0 = -ph t, t = kt sh2 + geff vtr
     for (int k = 0; k < 3; ++k) {
         phb -= fs0b[k] * t.t[k];
@@ -321,25 +347,25 @@ TMPS_HD void pair_reverse(const Params& P, int shearupdate, int mask, const Pair
     rbar -= rinvb * t.rinv * t.rinv;
     rsqb -= rsqinvb * t.rsqinv * t.rsqinv;
     // meff = ma mb / (ma + mb)
-    const double ms = in.ma + in.mb;
-    g.ma += meffb * in.mb * in.mb / (ms * ms);
-    g.mb += meffb * in.ma * in.ma / (ms * ms);
+    const double ims2 = meffb * (t.ims * t.ims);
+    g.ma += ims2 * in.mb * in.mb;
+    g.mb += ims2 * in.ma * in.ma;
     // ph = sqrt(reff delta)
     if (t.ph > 0.0) {
-        const double u2 = phb / (2.0 * t.ph);
+        const double u2 = 0.5 * phb * t.iph;
         reffb += u2 * t.delta;
         deltab += u2 * t.reff;
     }
     // reff = ra rb / (ra + rb)
-    const double rs = in.ra + in.rb;
-    g.ra += reffb * in.rb * in.rb / (rs * rs);
-    g.rb += reffb * in.ra * in.ra / (rs * rs);
+    const double irs2 = reffb * (t.irs * t.irs);
+    g.ra += irs2 * in.rb * in.rb;
+    g.rb += irs2 * in.ra * in.ra;
     // delta = ra + rb - r
     g.ra += deltab;
     g.rb += deltab;
     rbar -= deltab;
     // r = sqrt(rsq), rsq = d . d
-    rsqb += rbar / (2.0 * t.r);
+    rsqb += 0.5 * rbar * t.rinv;
     for (int k = 0; k < 3; ++k) g.d[k] = db[k] + 2.0 * rsqb * d[k];
 }
 

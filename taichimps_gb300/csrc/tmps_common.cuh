@@ -185,4 +185,53 @@ TMPS_DEV void block_sum(double (&v)[NV], double* smem /* [NV][BLOCK/32] */) {
     }
 }
 
+// Block sum of six FP64 components by halving exchanges: the FP64 pipe charges an instruction per warp however few lanes
+// use it, so a shuffle tree per component (30 additions per warp) costs as
+// much as several atoms' updates.  Padded to eight components, each exchange
+// keeps half of what a lane holds (4 + 2 + 1 + 1 + 1 = 9 additions per
+// warp), after which lane l holds component 4 b4 + 2 b3 + b2 (its lane bits
+// 4, 3, 2: lane >> 2) of the warp's total.  Lanes 0..5 of warp 0 then add the warp
+// totals of their component in warp order and return the block's total; the
+// other threads return 0.  Fixed order: deterministic for a block size.
+TMPS_DEV double warp_sum6_halving(const double (&v)[6]) {
+    const int lane = threadIdx.x & 31;
+    const double a[8] = {v[0], v[1], v[2], v[3], v[4], v[5], 0.0, 0.0};
+    const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0, b2 = (lane & 4) != 0;
+    double r4[4], r2[2];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const double send = b4 ? a[k] : a[4 + k], keep = b4 ? a[4 + k] : a[k];
+        r4[k] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const double send = b3 ? r4[k] : r4[2 + k], keep = b3 ? r4[2 + k] : r4[k];
+        r2[k] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+    }
+    double r = (b2 ? r2[1] : r2[0]) + __shfl_xor_sync(0xffffffffu, b2 ? r2[0] : r2[1], 4);
+    r += __shfl_xor_sync(0xffffffffu, r, 2);  // both lanes of a pair add the same two values
+    r += __shfl_xor_sync(0xffffffffu, r, 1);
+    return r;
+}
+
+// `kept`: lane c < 6 holds a further value of component c; with `any` false
+// (warp-uniform) every v is zero and the exchanges are left out.
+template <int BLOCK>
+TMPS_DEV double block_sum6_halving(const double (&v)[6], double kept, bool any,
+                                                     double* smem /* [6][BLOCK / 32] */) {
+    constexpr int kW = BLOCK / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double r = 0.0;
+    if (any) r = __shfl_sync(0xffffffffu, warp_sum6_halving(v), (lane << 2) & 31);  // lane c < 6: component c
+    if (lane < 6) smem[lane * kW + warp] = any ? r + kept : kept;
+    __syncthreads();
+    double t = 0.0;
+    if (warp == 0 && lane < 6) {
+        t = smem[lane * kW];
+#pragma unroll
+        for (int w = 1; w < kW; ++w) t += smem[lane * kW + w];
+    }
+    return t;
+}
+
 }  // namespace tmps
