@@ -121,8 +121,13 @@ __device__ void sum_partials(const double* part, int nb, double* out, int first)
     if (lane == 0) out[c] = t;
 }
 
-// Programmatic dependent launch (see tmps_fused.cu): wait for the kernel before
-// to complete, then let the next one be scheduled.
+// Programmatic dependent launch: wait for the kernel before to complete, then
+// let the next one be scheduled.  Every kernel of this file does both in this
+// order, so when a block starts, all but the kernel right before it have
+// completed: what those wrote may be read, and worked on, before enter().  The
+// launches of a step depend on one another in a chain, so for few spheres the
+// time of a step is the sum of their load and FP64 latencies, and each kernel
+// does here what does not need its predecessor.
 __device__ __forceinline__ void enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -249,33 +254,40 @@ __global__ void __launch_bounds__(kBlk) k_initial(tmps_adj_sys S, double dt, tmp
                                                   const tmps_adj_rec* before, const tmps_adj_rec* prev,
                                                   const double* __restrict__ xbuild, unsigned long long* disp, Queue* q,
                                                   int64_t step, double trig) {
-    enter();
-    if (q) {
-        const int64_t h = *(volatile const int64_t*)&q->hit;
-        if (h != 0 && h != step) return;  // (another block of this step may have stamped it)
-    }
     const int n = S.n;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double dd = 0.0;
-    if (i < n) {
+    const bool mine = i < n;
+    // all but the new box is from kernels before the last: the half-kick, and the offset in the old box
+    double v[3] = {0, 0, 0}, w[3] = {0, 0, 0}, x0[3] = {0, 0, 0}, xb[3] = {0, 0, 0};
+    if (mine) {
         const double dtf = 0.5 * dt;
         const double m = S.mass[i], r = S.radius[i], im = rcp64(m), iI = rcp64(inertia(m, r));
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const size_t k = (size_t)c * n + i;
-            const double v = S.v[k] + dtf * (S.f[k] * im);
-            double x0;
-            if (before) {
-                const double lam = over(xlast[k] - before->lo[c], before->prd[c], rcp64(before->prd[c]));
-                x0 = prev->prd[c] * lam + prev->lo[c];
-            } else {
-                x0 = S.x[k];
-            }
-            const double x = x0 + dt * v;
-            T.vh[k] = v;
+            v[c] = S.v[k] + dtf * (S.f[k] * im);
+            w[c] = S.w[k] + dtf * (S.t[k] * iI);
+            if (before) x0[c] = over(xlast[k] - before->lo[c], before->prd[c], rcp64(before->prd[c]));
+            xb[c] = xbuild[k];
+        }
+    }
+    enter();
+    if (q) {
+        const int64_t h = *(volatile const int64_t*)&q->hit;
+        if (h != 0 && h != step) return;  // (another block of this step may have stamped it)
+    }
+    double dd = 0.0;
+    if (mine) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const size_t k = (size_t)c * n + i;
+            // (S.x may be the last kernel's, the remap that ends a queued run)
+            x0[c] = before ? prev->prd[c] * x0[c] + prev->lo[c] : S.x[k];
+            const double x = x0[c] + dt * v[c];
+            T.vh[k] = v[c];
             T.xh[k] = x;
-            T.wh[k] = S.w[k] + dtf * (S.t[k] * iI);
-            const double e = x - xbuild[k];
+            T.wh[k] = w[c];
+            const double e = x - xb[c];
             dd += e * e;
         }
     }
@@ -343,8 +355,6 @@ __global__ void __launch_bounds__(kBlk) k_pairs(tmps_adj_sys S, Params P, int sh
                                                 const Queue* q) {
     __shared__ double smem[6 * (kBlk / 32)];
     __shared__ int list[kPairTile], count[kPairTile / 32];
-    enter();
-    if (halted(q)) return;
     const int n = S.n, np = S.npairs;
     double prd[3], iprd[3], nimg[3];
 #pragma unroll
@@ -352,6 +362,17 @@ __global__ void __launch_bounds__(kBlk) k_pairs(tmps_adj_sys S, Params P, int sh
         prd[c] = box->prd[c];
         iprd[c] = rcp64(prd[c]);
     }
+    int pi[kPairTile / kBlk], pj[kPairTile / kBlk];
+    double radsum_[kPairTile / kBlk];
+#pragma unroll
+    for (int u = 0; u < kPairTile / kBlk; ++u) {
+        const int p = blockIdx.x * kPairTile + u * kBlk + threadIdx.x;
+        pi[u] = p < np ? S.pi[p] : 0;
+        pj[u] = p < np ? S.pj[p] : 0;
+        radsum_[u] = S.radius[pi[u]] + S.radius[pj[u]];
+    }
+    enter();
+    if (halted(q)) return;
     double vir[6] = {0, 0, 0, 0, 0, 0};
     bool in_[kPairTile / kBlk];
 #pragma unroll
@@ -359,13 +380,13 @@ __global__ void __launch_bounds__(kBlk) k_pairs(tmps_adj_sys S, Params P, int sh
         const int p = blockIdx.x * kPairTile + u * kBlk + threadIdx.x;
         in_[u] = false;
         if (p < np) {
-            const int i = S.pi[p], j = S.pj[p];
+            const int i = pi[u], j = pj[u];
             double d[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c) d[c] = xs[(size_t)c * n + i] - xs[(size_t)c * n + j];
             min_image(prd, iprd, d, nimg);
             const double rsq = (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2];
-            const double radsum = S.radius[i] + S.radius[j];
+            const double radsum = radsum_[u];
             in_[u] = rsq < radsum * radsum && rsq > 1e-28;
             if (!in_[u]) {
                 mask_rec[p] = 0;
@@ -416,33 +437,64 @@ __global__ void __launch_bounds__(kBlk) k_gather(tmps_adj_sys S, double dt, int 
                                                  const double* __restrict__ wh, double* __restrict__ ft,
                                                  double* __restrict__ tt, const uint8_t* mask, Work W, const Queue* q) {
     __shared__ double smem[6 * (kBlk / 32)];
-    enter();
-    if (halted(q)) return;
     const int n = S.n, np = S.npairs;
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     double kin[6] = {0, 0, 0, 0, 0, 0};
+    int i0 = 0, ni = 0, j0 = 0, nj = 0;
+    double ra = 0.0, m = 1.0, im = 1.0, iI = 1.0, vh0[3] = {0, 0, 0}, wh0[3] = {0, 0, 0};
+    if (a < n) {
+        i0 = S.ibeg[a];
+        ni = S.ibeg[a + 1] - i0;
+        j0 = S.jbeg[a];
+        nj = S.jbeg[a + 1] - j0;
+        ra = S.radius[a];
+        m = S.mass[a];
+        im = rcp64(m);
+        iI = rcp64(inertia(m, ra));
+        if (final_)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                vh0[c] = vh[(size_t)c * n + a];
+                wh0[c] = wh[(size_t)c * n + a];
+            }
+    }
+    // the pair of entry k: first the atom's pairs as i, then as j
+    auto pair_of = [&](int k) { return k < ni ? i0 + k : S.jlist[j0 + k - ni]; };
+    int p0[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) p0[u] = u < ni + nj ? pair_of(u) : 0;
+    enter();
+    if (halted(q)) return;
     if (a < n) {
         double F[3] = {0, 0, 0}, Tq[3] = {0, 0, 0};
-        const double ra = S.radius[a];
-        const int i0 = S.ibeg[a], i1 = S.ibeg[a + 1], j0 = S.jbeg[a], j1 = S.jbeg[a + 1];
-        for (int p = i0; p < i1; ++p) {
-            if (!mask[p]) continue;
+        // four pairs' masks and terms in flight together (a term is used where the mask says contact)
+        for (int k0 = 0; k0 < ni + nj; k0 += 4) {
+            int p[4];
+            uint8_t on[4];
+            double f[4][6];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                F[c] += W.fp[(size_t)c * np + p];
-                Tq[c] += -ra * W.tp[(size_t)c * np + p];
+            for (int u = 0; u < 4; ++u) p[u] = k0 == 0 ? p0[u] : (k0 + u < ni + nj ? pair_of(k0 + u) : 0);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                on[u] = k0 + u < ni + nj ? mask[p[u]] : 0;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    f[u][c] = W.fp[(size_t)c * np + p[u]];
+                    f[u][3 + c] = W.tp[(size_t)c * np + p[u]];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (!on[u]) continue;
+                const bool first = k0 + u < ni;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    F[c] += first ? f[u][c] : -f[u][c];
+                    Tq[c] += -ra * f[u][3 + c];
+                }
             }
         }
-        for (int k = j0; k < j1; ++k) {
-            const int p = S.jlist[k];
-            if (!mask[p]) continue;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                F[c] -= W.fp[(size_t)c * np + p];
-                Tq[c] += -ra * W.tp[(size_t)c * np + p];
-            }
-        }
-        const double m = S.mass[a], im = rcp64(m), iI = rcp64(inertia(m, ra)), dtf = 0.5 * dt;
+        const double dtf = 0.5 * dt;
         double v[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -454,9 +506,9 @@ __global__ void __launch_bounds__(kBlk) k_gather(tmps_adj_sys S, double dt, int 
                 tt[k] = Tq[c];
             }
             if (final_) {
-                v[c] = vh[k] + dtf * (F[c] * im);
+                v[c] = vh0[c] + dtf * (F[c] * im);
                 S.v[k] = v[c];
-                S.w[k] = wh[k] + dtf * (Tq[c] * iI);
+                S.w[k] = wh0[c] + dtf * (Tq[c] * iI);
             }
         }
         if (final_) {
@@ -519,15 +571,20 @@ __device__ void coupled(int couple, const double* P, double* p) {
 __global__ void __launch_bounds__(kOne) k_servo(tmps_adj_servo sv, double dt, int64_t step, const tmps_adj_rec* prev,
                                                 tmps_adj_rec* next, int nbP, int nbA, Work W, Queue* q) {
     __shared__ double sw[6], sk[6];
+    sum_partials<6>(W.partw, nbP, sw, 0);
+    tmps_adj_rec r;
+    double vol = 1.0, ivol = 1.0;
+    if (threadIdx.x == 0) {
+        r = *prev;
+        vol = (r.prd[0] * r.prd[1]) * r.prd[2];
+        ivol = rcp64(vol);
+    }
     enter();
     if (halted(q)) return;
-    sum_partials<6>(W.partw, nbP, sw, 0);
     sum_partials<6>(W.partk, nbA, sk, 6);
     __syncthreads();
     if (threadIdx.x != 0) return;
     if (q) q->done = step;
-    tmps_adj_rec r = *prev;
-    const double vol = (r.prd[0] * r.prd[1]) * r.prd[2], ivol = rcp64(vol);
     double Pt[6];
     for (int c = 0; c < 6; ++c) {
         r.w[c] = sw[c] + sk[c];
@@ -583,120 +640,153 @@ __global__ void __launch_bounds__(kBlk) k_remap(int n, const double* __restrict_
 __global__ void __launch_bounds__(kOne) k_b_servo(tmps_adj_servo sv, double dt, int64_t step, const tmps_adj_rec* prev,
                                                   const tmps_adj_rec* next, double qbar, int nbA, int nbP, int reduce,
                                                   int servo, int slot, tmps_adj_bar B, Work W) {
-    __shared__ double s[6], g[8];
+    __shared__ double s[6], g[8], box[18], par[5], wbar[6];
+    __shared__ double sPt[6], sratio[3], srate[3];
+    const int tid = threadIdx.x;
+    // what the records alone give, and the accumulated adjoints, before the wait
+    if (tid < 18) box[tid] = B.box[tid];
+    if (tid >= 32 && tid < 37) par[tid - 32] = B.params[tid - 32];
+    if (tid == kOne - 32 && servo) {
+        const double vol = (prev->prd[0] * prev->prd[1]) * prev->prd[2], ivol = rcp64(vol);
+        double Pt[6], p[3];
+        for (int c = 0; c < 6; ++c) sPt[c] = Pt[c] = over(next->w[c], vol, ivol);
+        coupled(sv.couple, Pt, p);
+        for (int d = 0; d < 3; ++d) {
+            bool cl;
+            sratio[d] = next->prd[d] * rcp64(prev->prd[d]);
+            srate[d] = sv.style[d] == 8 ? servo_rate(sv, d, p[d], &cl) : 0.0;
+        }
+    }
+    double prd[3] = {1, 1, 1}, ivol = 1.0;
+    int clamp = 0;
+    if (tid == 0 && servo) {
+        for (int d = 0; d < 3; ++d) prd[d] = prev->prd[d];
+        ivol = rcp64((prd[0] * prd[1]) * prd[2]);
+        clamp = next->clamp;
+    }
     enter();
     if (servo) sum_partials<6>(W.partk, nbA, s, 0);
     if (reduce) sum_partials<8>(W.partg, nbP, g, 6);
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    double* const box_bar = B.box;
-    if (reduce) {
-        for (int c = 0; c < 5; ++c) B.params[c] += g[c];
-        for (int c = 0; c < 3; ++c) box_bar[9 * slot + 3 + c] += g[5 + c];
-    }
-    if (!servo) return;
-    const int n = (int)(step - 1);
-    double* bn = box_bar + 9 * (n & 1);          // record n: lo 0..2, prd 3..5, cum 6..8
-    double* bn1 = box_bar + 9 * ((n + 1) & 1);   // record n + 1
-    double Pt[6], p[3], pb[3] = {0, 0, 0}, Pb[6] = {0, 0, 0, 0, 0, 0};
-    const double vol = (prev->prd[0] * prev->prd[1]) * prev->prd[2], ivol = rcp64(vol);
-    for (int c = 0; c < 6; ++c) Pt[c] = over(next->w[c], vol, ivol);
-    coupled(sv.couple, Pt, p);
-    for (int d = 0; d < 3; ++d) {
-        const double ratio = next->prd[d] * rcp64(prev->prd[d]);
-        // remap
-        bn1[d] += s[d];
-        bn1[3 + d] += s[3 + d];
-        bn[d] -= s[d] * ratio;
-        bn[3 + d] -= s[3 + d] * ratio;
-        if (sv.style[d] != 8) continue;
-        // record n + 1's box from its cumulative shift: lo = lo_s - cum / 2, prd = L + cum
-        const double cumb = bn1[6 + d] + bn1[3 + d] - 0.5 * bn1[d];
-        // cum' = cum + (dt rate) prd
-        bool cl;
-        const double rate = servo_rate(sv, d, p[d], &cl);
-        bn[6 + d] += cumb;
-        bn[3 + d] += cumb * dt * rate;
-        if (!((next->clamp >> d) & 1)) {
-            double rb = cumb * dt * prev->prd[d] * sv.pgain[d];
-            if (sv.normalize == 1) rb = rb / fabs(sv.ptarget[d]);
-            pb[d] += rb;
+    if (tid == 0) {
+        if (reduce) {
+            for (int c = 0; c < 5; ++c) par[c] += g[c];
+            for (int c = 0; c < 3; ++c) box[9 * slot + 3 + c] += g[5 + c];
+        }
+        if (servo) {
+            const int n = (int)((step - 1) & 1);
+            double* const bn = box + 9 * n;          // record step - 1: lo 0..2, prd 3..5, cum 6..8
+            double* const bn1 = box + 9 * (1 - n);   // record step
+            double pb[3] = {0, 0, 0}, Pb[6] = {0, 0, 0, 0, 0, 0};
+            for (int d = 0; d < 3; ++d) {
+                const double ratio = sratio[d];
+                // remap
+                bn1[d] += s[d];
+                bn1[3 + d] += s[3 + d];
+                bn[d] -= s[d] * ratio;
+                bn[3 + d] -= s[3 + d] * ratio;
+                if (sv.style[d] != 8) continue;
+                // record step's box from its cumulative shift: lo = lo_s - cum / 2, prd = L + cum
+                const double cumb = bn1[6 + d] + bn1[3 + d] - 0.5 * bn1[d];
+                // cum' = cum + (dt rate) prd
+                bn[6 + d] += cumb;
+                bn[3 + d] += cumb * dt * srate[d];
+                if (!((clamp >> d) & 1)) {
+                    double rb = cumb * dt * prd[d] * sv.pgain[d];
+                    if (sv.normalize == 1) rb = rb / fabs(sv.ptarget[d]);
+                    pb[d] += rb;
+                }
+            }
+            for (int c = 0; c < 9; ++c) bn1[c] = 0.0;
+            // couple
+            if (sv.couple == 1) {
+                const double m = (pb[0] + pb[1] + pb[2]) / 3.0;
+                Pb[0] = Pb[1] = Pb[2] = m;
+            } else if (sv.couple == 2) {
+                Pb[0] = Pb[1] = 0.5 * (pb[0] + pb[1]);
+                Pb[2] = pb[2];
+            } else if (sv.couple == 3) {
+                Pb[1] = Pb[2] = 0.5 * (pb[1] + pb[2]);
+                Pb[0] = pb[0];
+            } else if (sv.couple == 4) {
+                Pb[0] = Pb[2] = 0.5 * (pb[0] + pb[2]);
+                Pb[1] = pb[1];
+            } else {
+                Pb[0] = pb[0];
+                Pb[1] = pb[1];
+                Pb[2] = pb[2];
+            }
+            // deviatoric stress q = Pzz - (Pxx + Pyy) / 2
+            Pb[2] += qbar;
+            Pb[0] -= 0.5 * qbar;
+            Pb[1] -= 0.5 * qbar;
+            // P = W / vol
+            double volb = 0.0;
+            for (int c = 0; c < 6; ++c) {
+                wbar[c] = Pb[c] * ivol;
+                volb -= Pb[c] * sPt[c] * ivol;
+            }
+            bn[3] += volb * prd[1] * prd[2];
+            bn[4] += volb * prd[0] * prd[2];
+            bn[5] += volb * prd[0] * prd[1];
         }
     }
-    for (int c = 0; c < 9; ++c) bn1[c] = 0.0;
-    // couple
-    if (sv.couple == 1) {
-        const double g = (pb[0] + pb[1] + pb[2]) / 3.0;
-        Pb[0] = Pb[1] = Pb[2] = g;
-    } else if (sv.couple == 2) {
-        Pb[0] = Pb[1] = 0.5 * (pb[0] + pb[1]);
-        Pb[2] = pb[2];
-    } else if (sv.couple == 3) {
-        Pb[1] = Pb[2] = 0.5 * (pb[1] + pb[2]);
-        Pb[0] = pb[0];
-    } else if (sv.couple == 4) {
-        Pb[0] = Pb[2] = 0.5 * (pb[0] + pb[2]);
-        Pb[1] = pb[1];
-    } else {
-        Pb[0] = pb[0];
-        Pb[1] = pb[1];
-        Pb[2] = pb[2];
-    }
-    // deviatoric stress q = Pzz - (Pxx + Pyy) / 2
-    Pb[2] += qbar;
-    Pb[0] -= 0.5 * qbar;
-    Pb[1] -= 0.5 * qbar;
-    // P = W / vol
-    double volb = 0.0;
-    for (int c = 0; c < 6; ++c) {
-        W.wbar[c] = Pb[c] * ivol;
-        volb -= Pb[c] * Pt[c] * ivol;
-    }
-    bn[3] += volb * prev->prd[1] * prev->prd[2];
-    bn[4] += volb * prev->prd[0] * prev->prd[2];
-    bn[5] += volb * prev->prd[0] * prev->prd[1];
+    __syncthreads();
+    if (tid < 18) B.box[tid] = box[tid];
+    if (tid >= 32 && tid < 37) B.params[tid - 32] = par[tid - 32];
+    if (servo && tid >= 64 && tid < 70) W.wbar[tid - 64] = wbar[tid - 64];
 }
 
 // Reverse of the second half-kick and of the kinetic virial term.
 __global__ void __launch_bounds__(kBlk) k_b_final(tmps_adj_sys S, double dt, tmps_adj_tape T, tmps_adj_bar B, Work W) {
-    enter();
     const int n = S.n;
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= n) return;
-    const double m = S.mass[a], r = S.radius[a], im = rcp64(m), iI = rcp64(inertia(m, r)), dtf = 0.5 * dt;
+    const bool mine = a < n;
+    double m = 1.0, r = 1.0, im = 1.0, iI = 1.0, v[3] = {0, 0, 0}, vb[3] = {0, 0, 0}, f[3] = {0, 0, 0}, fb[3] = {0, 0, 0};
+    double mb = 0.0, Ib = 0.0, mass0 = 0.0, rad0 = 0.0;
+    const double dtf = 0.5 * dt;
+    if (mine) {
+        m = S.mass[a];
+        r = S.radius[a];
+        im = rcp64(m);
+        iI = rcp64(inertia(m, r));
+        mass0 = B.mass[a];
+        rad0 = B.radius[a];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const size_t k = (size_t)c * n + a;
+            f[c] = T.f[k];
+            v[c] = T.vh[k] + dtf * (f[c] * im);
+            vb[c] = B.v[k];
+            fb[c] = B.f[k];
+            // w = wh + dtf t / I
+            const double tb = dtf * B.w[k] * iI;
+            B.t[k] += tb;
+            Ib -= tb * T.t[k] * iI;
+        }
+    }
+    enter();
+    if (!mine) return;
     double wb[6];
 #pragma unroll
     for (int c = 0; c < 6; ++c) wb[c] = W.wbar[c];
-    double v[3], vb[3], f[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const size_t k = (size_t)c * n + a;
-        f[c] = T.f[k];
-        v[c] = T.vh[k] + dtf * (f[c] * im);
-        vb[c] = B.v[k];
-    }
     // kinetic m v_a v_b
     vb[0] += m * (2.0 * wb[0] * v[0] + wb[3] * v[1] + wb[4] * v[2]);
     vb[1] += m * (2.0 * wb[1] * v[1] + wb[3] * v[0] + wb[5] * v[2]);
     vb[2] += m * (2.0 * wb[2] * v[2] + wb[4] * v[0] + wb[5] * v[1]);
-    double mb = wb[0] * v[0] * v[0] + wb[1] * v[1] * v[1] + wb[2] * v[2] * v[2] + wb[3] * v[0] * v[1] +
-                wb[4] * v[0] * v[2] + wb[5] * v[1] * v[2];
-    double Ib = 0.0;
+    mb = wb[0] * v[0] * v[0] + wb[1] * v[1] * v[1] + wb[2] * v[2] * v[2] + wb[3] * v[0] * v[1] +
+         wb[4] * v[0] * v[2] + wb[5] * v[1] * v[2];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const size_t k = (size_t)c * n + a;
         // v = vh + dtf f / m
-        B.v[k] = vb[c];
         const double kb = dtf * vb[c] * im;
-        B.f[k] += kb;
+        B.v[k] = vb[c];
+        B.f[k] = fb[c] + kb;
         mb -= kb * f[c] * im;
-        // w = wh + dtf t / I
-        const double tb = dtf * B.w[k] * iI;
-        B.t[k] += tb;
-        Ib -= tb * T.t[k] * iI;
     }
-    B.mass[a] += mb + Ib * 0.4 * r * r;
-    B.radius[a] += Ib * 0.8 * m * r;
+    B.mass[a] = mass0 + (mb + Ib * 0.4 * r * r);
+    B.radius[a] = rad0 + Ib * 0.8 * m * r;
 }
 
 // Reverse of the contact pass: per pair in contact, recompute under the
@@ -709,7 +799,7 @@ __global__ void __launch_bounds__(kBlk) k_b_pairs(tmps_adj_sys S, Params P, int 
                                                   tmps_adj_bar B, Work W) {
     __shared__ double smem[8 * (kBlk / 32)];
     __shared__ int list[kPairTile], count[kPairTile / 32];
-    enter();
+    // (only the adjoints of the forces are the last kernel's: the contacts are recomputed before the wait)
     const int n = S.n, np = S.npairs;
     double prd[3], iprd[3], nimg[3];
 #pragma unroll
@@ -717,6 +807,7 @@ __global__ void __launch_bounds__(kBlk) k_b_pairs(tmps_adj_sys S, Params P, int 
         prd[c] = box->prd[c];
         iprd[c] = rcp64(prd[c]);
     }
+    bool waited = false;
     bool in_[kPairTile / kBlk];
 #pragma unroll
     for (int u = 0; u < kPairTile / kBlk; ++u) {
@@ -742,6 +833,8 @@ __global__ void __launch_bounds__(kBlk) k_b_pairs(tmps_adj_sys S, Params P, int 
         int mask;
         const int rec = mask_rec[p];
         pair_forward(P, shearupdate, in, rec, o, t, &mask);
+        if (!waited) enter();
+        waited = true;
         PairBar b;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -777,6 +870,7 @@ __global__ void __launch_bounds__(kBlk) k_b_pairs(tmps_adj_sys S, Params P, int 
 #pragma unroll
         for (int c = 0; c < 3; ++c) part[5 + c] -= nimg[c] * g.d[c];
     }
+    if (!waited) enter();
     block_sum<8, kBlk>(part, smem);
     if (threadIdx.x == 0) {
         const int nb = gridDim.x;
@@ -797,76 +891,128 @@ __global__ void __launch_bounds__(kBlk) k_b_atoms(tmps_adj_sys S, double dt, int
                                                   const tmps_adj_rec* prev, const tmps_adj_rec* next, tmps_adj_bar B,
                                                   Work W) {
     __shared__ double smem[6 * (kBlk / 32)];
-    enter();
     const int n = S.n, np = S.npairs;
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool mine = a < n;
     double s[6] = {0, 0, 0, 0, 0, 0};
-    if (a < n) {
-        double xb[3] = {0, 0, 0};
+    // everything but the pairs' adjoints before the wait
+    int i0 = 0, ni = 0, j0 = 0, nj = 0;
+    double m = 1.0, r = 1.0, im = 1.0, iI = 1.0, mass0 = 0.0, rad0 = 0.0;
+    double x0[3] = {0, 0, 0}, v0[3] = {0, 0, 0}, w0[3] = {0, 0, 0}, fp[3] = {0, 0, 0}, tp[3] = {0, 0, 0}, lam[3] = {0, 0, 0},
+           scale[3] = {1, 1, 1};
+    if (mine) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const size_t k = (size_t)c * n + a;
+            x0[c] = B.x[k];
+            if (xh) {
+                const double ip = rcp64(prev->prd[c]);
+                lam[c] = (xh[k] - prev->lo[c]) * ip;
+                scale[c] = next->prd[c] * ip;
+            }
+            if (gather) {
+                v0[c] = B.v[k];
+                w0[c] = B.w[k];
+                if (kick) {
+                    fp[c] = fprev[k];
+                    tp[c] = tprev[k];
+                }
+            }
+        }
+        if (gather) {
+            i0 = S.ibeg[a];
+            ni = S.ibeg[a + 1] - i0;
+            j0 = S.jbeg[a];
+            nj = S.jbeg[a + 1] - j0;
+            m = S.mass[a];
+            r = S.radius[a];
+            im = rcp64(m);
+            iI = rcp64(inertia(m, r));
+            mass0 = B.mass[a];
+            rad0 = B.radius[a];
+        }
+    }
+    auto pair_of = [&](int k) { return k < ni ? i0 + k : S.jlist[j0 + k - ni]; };
+    constexpr int kPer = 3;
+    int p0[kPer];
+    uint8_t on0[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        p0[u] = u < ni + nj ? pair_of(u) : 0;
+        on0[u] = u < ni + nj ? mask[p0[u]] : 0;
+    }
+    enter();
+    if (mine) {
         if (gather) {
             const double* G = W.gp;
-            double vb[3] = {0, 0, 0}, wb[3] = {0, 0, 0}, rb = 0.0, mb = 0.0;
-            const int i0 = S.ibeg[a], i1 = S.ibeg[a + 1], j0 = S.jbeg[a], j1 = S.jbeg[a + 1];
-            for (int p = i0; p < i1; ++p) {
-                if (!mask[p]) continue;
+            double xb[3] = {0, 0, 0}, vb[3] = {0, 0, 0}, wb[3] = {0, 0, 0}, rb = 0.0, mb = 0.0;
+            // a few pairs' adjoints in flight together
+            for (int k0 = 0; k0 < ni + nj; k0 += kPer) {
+                int p[kPer];
+                uint8_t on[kPer];
+                double g[kPer][11];
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    xb[c] += G[(size_t)c * np + p];
-                    vb[c] += G[(size_t)(3 + c) * np + p];
-                    wb[c] += G[(size_t)(6 + c) * np + p];
+                for (int u = 0; u < kPer; ++u) {
+                    p[u] = k0 == 0 ? p0[u] : (k0 + u < ni + nj ? pair_of(k0 + u) : 0);
+                    on[u] = k0 == 0 ? on0[u] : (k0 + u < ni + nj ? mask[p[u]] : 0);
                 }
-                rb += G[(size_t)12 * np + p];
-                mb += G[(size_t)14 * np + p];
-            }
-            for (int k = j0; k < j1; ++k) {
-                const int p = S.jlist[k];
-                if (!mask[p]) continue;
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    xb[c] -= G[(size_t)c * np + p];
-                    vb[c] -= G[(size_t)(3 + c) * np + p];
-                    wb[c] += G[(size_t)(9 + c) * np + p];
+                for (int u = 0; u < kPer; ++u) {
+                    const bool first = k0 + u < ni;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        g[u][c] = G[(size_t)c * np + p[u]];
+                        g[u][3 + c] = G[(size_t)(3 + c) * np + p[u]];
+                        g[u][6 + c] = G[(size_t)((first ? 6 : 9) + c) * np + p[u]];
+                    }
+                    g[u][9] = G[(size_t)(first ? 12 : 13) * np + p[u]];
+                    g[u][10] = G[(size_t)(first ? 14 : 15) * np + p[u]];
                 }
-                rb += G[(size_t)13 * np + p];
-                mb += G[(size_t)15 * np + p];
+#pragma unroll
+                for (int u = 0; u < kPer; ++u) {
+                    if (!on[u]) continue;
+                    const bool first = k0 + u < ni;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        xb[c] += first ? g[u][c] : -g[u][c];
+                        vb[c] += first ? g[u][3 + c] : -g[u][3 + c];
+                        wb[c] += g[u][6 + c];
+                    }
+                    rb += g[u][9];
+                    mb += g[u][10];
+                }
             }
-            const double m = S.mass[a], r = S.radius[a], im = rcp64(m), iI = rcp64(inertia(m, r)), dtf = 0.5 * dt;
+            const double dtf = 0.5 * dt;
             double Ib = 0.0;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const size_t k = (size_t)c * n + a;
-                xb[c] = B.x[k] + xb[c];
-                const double v1 = B.v[k] + vb[c], w1 = B.w[k] + wb[c];
+                x0[c] += xb[c];
+                const double v1 = v0[c] + vb[c], w1 = w0[c] + wb[c];
+                B.w[k] = w1;
                 if (kick) {
                     // x = x0 + dt vh; vh = v0 + dtf f / m; wh = w0 + dtf t / I
-                    const double vhb = v1 + dt * xb[c];
+                    const double vhb = v1 + dt * x0[c];
                     const double fb = dtf * vhb * im, tb = dtf * w1 * iI;
                     B.v[k] = vhb;
                     B.f[k] = fb;
-                    mb -= fb * fprev[k] * im;
-                    B.w[k] = w1;
+                    mb -= fb * fp[c] * im;
                     B.t[k] = tb;
-                    Ib -= tb * tprev[k] * iI;
+                    Ib -= tb * tp[c] * iI;
                 } else {
                     B.v[k] = v1;
-                    B.w[k] = w1;
                 }
-                if (!xh) B.x[k] = xb[c];
+                if (!xh) B.x[k] = x0[c];
             }
-            B.mass[a] += mb + Ib * 0.4 * r * r;
-            B.radius[a] += rb + Ib * 0.8 * m * r;
-        } else {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) xb[c] = B.x[(size_t)c * n + a];
+            B.mass[a] = mass0 + (mb + Ib * 0.4 * r * r);
+            B.radius[a] = rad0 + (rb + Ib * 0.8 * m * r);
         }
         if (xh) {
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const size_t k = (size_t)c * n + a;
-                const double ip = rcp64(prev->prd[c]);
-                s[c] = xb[c];
-                s[3 + c] = xb[c] * ((xh[k] - prev->lo[c]) * ip);
-                B.x[k] = xb[c] * (next->prd[c] * ip);
+                s[c] = x0[c];
+                s[3 + c] = x0[c] * lam[c];
+                B.x[(size_t)c * n + a] = x0[c] * scale[c];
             }
         }
     }
@@ -882,12 +1028,13 @@ bool sys_ok(const tmps_adj_sys* s) {
            (s->npairs == 0 || (s->shear && s->pi && s->pj)) && s->ibeg && s->jbeg && (s->npairs == 0 || s->jlist);
 }
 
-// Launch with programmatic stream serialization (see enter), counted.
+// Launch with programmatic stream serialization (see enter), counted; `after`:
+// only once the kernel before has completed.
 template <typename... P, typename... A>
-void run(void (*kernel)(P...), int grid, int block, cudaStream_t s, A&&... args) {
+void run_as(bool after, void (*kernel)(P...), int grid, int block, cudaStream_t s, A&&... args) {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = after ? 0 : 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3((unsigned)block);
@@ -896,6 +1043,10 @@ void run(void (*kernel)(P...), int grid, int block, cudaStream_t s, A&&... args)
     cfg.numAttrs = 1;
     (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
     note_launches(1);
+}
+template <typename... P, typename... A>
+void run(void (*kernel)(P...), int grid, int block, cudaStream_t s, A&&... args) {
+    run_as(false, kernel, grid, block, s, std::forward<A>(args)...);
 }
 
 // The tape of the k-th step of a run whose tapes lie atom_stride doubles (atom
@@ -1080,7 +1231,8 @@ int tmps_adj_reverse(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps
                     (const double*)t.wh, (const double*)t.shear, (const uint8_t*)t.mask, rec(step - 1),
                     (const double*)W.wbar, *b, W);
             const tmps_adj_tape tp = step > first ? tape_at(*tape, atom_stride, pair_stride, step - 1 - first) : t;
-            run(k_b_atoms, nbA, kBlk, st, *s, p->dt, 1, 1, (const uint8_t*)t.mask,
+            // (with no pairs it follows k_b_final, whose velocities it reads before its wait)
+            run_as(s->npairs == 0, k_b_atoms, nbA, kBlk, st, *s, p->dt, 1, 1, (const uint8_t*)t.mask,
                 step > first ? (const double*)tp.f : d_fprev, step > first ? (const double*)tp.t : d_tprev, xh,
                 xh ? rec(step - 2) : rec(step - 1), xh ? rec(step - 1) : rec(step), *b, W);
         }
