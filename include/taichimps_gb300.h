@@ -703,6 +703,15 @@ int64_t tmps_adj_workspace_bytes(int32_t n, int32_t npairs);
 int tmps_adj_pairs(int32_t n, const double* d_x, const double* d_radius, const tmps_adj_rec* d_box, double skin,
                    int32_t* d_count, const int32_t* d_ibeg, int32_t* d_pi, int32_t* d_pj, void* stream);
 
+/* The same list by cells of a gx x gy x gz grid (each at least 3, prd / g at
+ * least the longest ri + rj + skin with some margin); work:
+ * tmps_adj_cells_bytes(n, gx gy gz), kept between the counting and the
+ * filling call. */
+int64_t tmps_adj_cells_bytes(int32_t n, int32_t ncell);
+int tmps_adj_pairs_cells(int32_t n, const double* d_x, const double* d_radius, const tmps_adj_rec* d_box, double skin,
+                         int32_t gx, int32_t gy, int32_t gz, void* work, int32_t* d_count, const int32_t* d_ibeg,
+                         int32_t* d_pi, int32_t* d_pj, void* stream);
+
 /* For each old pair, its index in a new list (-1 if gone); the history
  * carried across a rebuild (contact_history.py:91-139 keyed by the pair). */
 int tmps_adj_pair_map(int32_t nold, const int32_t* d_old_pi, const int32_t* d_old_pj, const int32_t* d_new_ibeg,

@@ -241,6 +241,9 @@ _SIGS = {
                                c_vp]),
     "tmps_adj_workspace_bytes": (ctypes.c_int64, [c_i32, c_i32]),
     "tmps_adj_pairs": (c_i32, [c_i32, c_vp, c_vp, c_vp, c_f64, c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "tmps_adj_cells_bytes": (c_i64, [c_i32, c_i32]),
+    "tmps_adj_pairs_cells": (c_i32, [c_i32, c_vp, c_vp, c_vp, c_f64, c_i32, c_i32, c_i32, c_vp, c_vp, c_vp, c_vp, c_vp,
+                                     c_vp]),
     "tmps_adj_pair_map": (c_i32, [c_i32, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "tmps_adj_carry": (c_i32, [c_i32, c_i32, c_vp, c_vp, c_vp, c_i32, c_vp]),
     "tmps_adj_setup": (c_i32, [ctypes.POINTER(AdjSys), ctypes.POINTER(AdjParams), c_vp, ctypes.POINTER(AdjTape),

@@ -68,22 +68,37 @@ class _Pairs:
         self.jbeg[1:] = torch.cumsum(jc, 0).to(torch.int32)
 
     @staticmethod
-    def build(x: torch.Tensor, radius: torch.Tensor, rec_ptr: int, skin: float) -> "_Pairs":
+    def build(x: torch.Tensor, radius: torch.Tensor, rec_ptr: int, skin: float, prd, rmax: float) -> "_Pairs":
+        """`prd`, `rmax`: the box's lengths and the largest radius on the host, for the cell grid; a box
+        of fewer than three cells along an axis takes the all-pairs build (the same list)."""
         L = _device.lib()
         st = _device.stream()
         n = radius.numel()
         dev = radius.device
         count = torch.zeros(max(n, 1), dtype=torch.int32, device=dev)
-        _lib.check(L.tmps_adj_pairs(n, _p(x), _p(radius), rec_ptr, skin, _p(count), None, None, None, st),
-                   "tmps_adj_pairs")
+        cut = (2.0 * rmax + skin) * 1.000001  # cells wider than the longest cut by far more than rounding
+        # at most four cells per atom: a sparse box needs no finer grid
+        cap = max(3, int(round((4.0 * max(n, 1)) ** (1.0 / 3.0))))
+        g = [min(cap, int(p / cut)) if math.isfinite(p) and cut > 0.0 else 0 for p in prd]
+        cells = None
+        if min(g) >= 3:
+            cells = torch.empty(int(L.tmps_adj_cells_bytes(n, g[0] * g[1] * g[2])), dtype=torch.uint8, device=dev)
+
+        def pairs(*out):
+            if cells is not None:
+                rc = L.tmps_adj_pairs_cells(n, _p(x), _p(radius), rec_ptr, skin, *g, _p(cells), *out, st)
+            else:
+                rc = L.tmps_adj_pairs(n, _p(x), _p(radius), rec_ptr, skin, *out, st)
+            _lib.check(rc, "tmps_adj_pairs")
+
+        pairs(_p(count), None, None, None)
         ibeg = torch.zeros(n + 1, dtype=torch.int32, device=dev)
         ibeg[1:] = torch.cumsum(count[:n], 0).to(torch.int32)
         npairs = int(ibeg[-1].item())
         pi = torch.zeros(max(npairs, 1), dtype=torch.int32, device=dev)
         pj = torch.zeros(max(npairs, 1), dtype=torch.int32, device=dev)
         if npairs:
-            _lib.check(L.tmps_adj_pairs(n, _p(x), _p(radius), rec_ptr, skin, None, _p(ibeg), _p(pi), _p(pj), st),
-                       "tmps_adj_pairs")
+            pairs(None, _p(ibeg), _p(pi), _p(pj))
         return _Pairs(n, pi[:npairs], pj[:npairs], ibeg)
 
 
@@ -217,7 +232,8 @@ class AdjointRun:
         self.rec[:_REC].copy_(torch.from_numpy(np.frombuffer(bytes(r0), dtype=np.uint8).copy()))
         st = dict(x=self.x0.clone(), v=self.v0.clone(), w=self.w0.clone(), f=torch.zeros((3, self.n), **f64),
                   t=torch.zeros((3, self.n), **f64))
-        pairs = _Pairs.build(st["x"], self.r, self._rec_ptr(0), self.skin)
+        rmax = float(self.r.max()) if self.n else 0.0
+        pairs = _Pairs.build(st["x"], self.r, self._rec_ptr(0), self.skin, list(r0.prd), rmax)
         self.lists, self.events = [pairs], {}
         li = 0
         shear = torch.zeros((3, max(pairs.npairs, 1)), **f64)
@@ -244,7 +260,9 @@ class AdjointRun:
             hit = int(queue[0].item())
             if hit:
                 # step `hit` has had its first half: a new pair list, then the rest of it
-                new = _Pairs.build(tape.field(0, "xh"), self.r, self._rec_ptr(hit - 1), self.skin)
+                raw = self.rec[(hit - 1) * _REC:hit * _REC].cpu().numpy().tobytes()
+                new = _Pairs.build(tape.field(0, "xh"), self.r, self._rec_ptr(hit - 1), self.skin,
+                                   list(_lib.AdjRec.from_buffer_copy(raw).prd), rmax)
                 m = torch.zeros(max(pairs.npairs, 1), dtype=torch.int32, device=self.dev)
                 _lib.check(L.tmps_adj_pair_map(pairs.npairs, _p(pairs.pi), _p(pairs.pj), _p(new.ibeg), _p(new.pj),
                                                _p(m), sc), "tmps_adj_pair_map")

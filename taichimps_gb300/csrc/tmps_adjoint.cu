@@ -213,6 +213,112 @@ __global__ void __launch_bounds__(128) k_pairs_build(int n, const double* __rest
     if (act && !pj) count[i] = cnt;
 }
 
+// The same list by cells: atoms binned (positions wrapped) into a grid whose
+// cells are at least the longest cut wide, at least three per axis, each atom
+// tested against the 27 cells around it instead of every atom above it (31,250
+// spheres: 2 x 3.1 ms for all pairs).  The order in which the atomics fill a
+// cell does not show: a row's partners are sorted as they are written.
+__device__ __forceinline__ int cell_axis(double x, double lo, double iprd, int g) {
+    const double l = (x - lo) * iprd, f = l - floor(l);
+    const int c = (int)(f * (double)g);
+    return c < 0 ? 0 : (c < g ? c : g - 1);
+}
+
+struct Cells {
+    int32_t *count, *start, *fill, *cell, *order;  // [m], [m + 1], [m] (the scan's tile totals first), [n], [n]
+    float4* pos;                                   // [n] by cell: FP32 position and radius
+};
+Cells carve_cells(void* work, int n, int m) {
+    char* p = static_cast<char*>(work);
+    Cells c;
+    c.count = reinterpret_cast<int32_t*>(p); p += align256((size_t)m * 4);
+    c.start = reinterpret_cast<int32_t*>(p); p += align256(((size_t)m + 1) * 4);
+    c.fill = reinterpret_cast<int32_t*>(p); p += align256((size_t)m * 4);
+    c.cell = reinterpret_cast<int32_t*>(p); p += align256((size_t)n * 4);
+    c.order = reinterpret_cast<int32_t*>(p); p += align256((size_t)n * 4);
+    c.pos = reinterpret_cast<float4*>(p);
+    return c;
+}
+
+__global__ void __launch_bounds__(128) k_cells_bin(int n, const double* __restrict__ x, const tmps_adj_rec* __restrict__ box,
+                                                   int gx, int gy, int gz, Cells C) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int g[3] = {gx, gy, gz};
+    int lin = 0;
+#pragma unroll
+    for (int c = 2; c >= 0; --c)
+        lin = lin * g[c] + cell_axis(x[(size_t)c * n + i], box->lo[c], rcp64(box->prd[c]), g[c]);
+    C.cell[i] = lin;
+    atomicAdd(&C.count[lin], 1);
+}
+
+__global__ void __launch_bounds__(128) k_cells_fill(int n, const double* __restrict__ x, const double* __restrict__ rad,
+                                                    Cells C) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int c = C.cell[i];
+    const int p = C.start[c] + atomicAdd(&C.fill[c], 1);
+    C.order[p] = i;
+    C.pos[p] = make_float4((float)x[i], (float)x[n + i], (float)x[2 * n + i], (float)rad[i]);
+}
+
+__global__ void __launch_bounds__(64) k_pairs_cells(int n, const double* __restrict__ x, const double* __restrict__ rad,
+                                                    const tmps_adj_rec* __restrict__ box, double skin, int gx, int gy,
+                                                    int gz, Cells C, int32_t* __restrict__ count,
+                                                    const int32_t* __restrict__ ibeg, int32_t* __restrict__ pi,
+                                                    int32_t* __restrict__ pj) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    double prd[3], iprd[3];
+    float prd32[3], iprd32[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        prd[c] = box->prd[c];
+        iprd[c] = rcp64(prd[c]);
+        prd32[c] = (float)prd[c];
+        iprd32[c] = (float)iprd[c];
+    }
+    const int i = C.order[p];
+    const float4 a = C.pos[p];
+    const double xi[3] = {x[i], x[n + i], x[2 * n + i]}, ri = rad[i];
+    const int lin = C.cell[i], cx = lin % gx, cy = (lin / gx) % gy, cz = lin / (gx * gy);
+    const int beg = pj ? ibeg[i] : 0;
+    int cnt = 0;
+    for (int o = 0; o < 27; ++o) {
+        int nx = cx + o % 3 - 1, ny = cy + (o / 3) % 3 - 1, nz = cz + o / 9 - 1;
+        nx += nx < 0 ? gx : (nx >= gx ? -gx : 0);
+        ny += ny < 0 ? gy : (ny >= gy ? -gy : 0);
+        nz += nz < 0 ? gz : (nz >= gz ? -gz : 0);
+        const int c = (nz * gy + ny) * gx + nx;
+        for (int q = C.start[c]; q < C.start[c + 1]; ++q) {
+            const int j = C.order[q];
+            if (j <= i) continue;
+            const float4 b = C.pos[q];
+            float d0 = a.x - b.x, d1 = a.y - b.y, d2 = a.z - b.z;
+            d0 -= prd32[0] * rintf(d0 * iprd32[0]);
+            d1 -= prd32[1] * rintf(d1 * iprd32[1]);
+            d2 -= prd32[2] * rintf(d2 * iprd32[2]);
+            // an FP32 screen with a wide margin, then the exact FP64 test (neighbor.py:348-356)
+            const float cut32 = (a.w + b.w + (float)skin) * 1.0001f + 1e-3f;
+            if (d0 * d0 + d1 * d1 + d2 * d2 >= cut32 * cut32) continue;
+            double d[3] = {xi[0] - x[j], xi[1] - x[n + j], xi[2] - x[2 * n + j]}, nimg[3];
+            min_image(prd, iprd, d, nimg);
+            const double rsq = (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2];
+            const double cut = (ri + rad[j]) + skin;
+            if (!(rsq < cut * cut)) continue;
+            if (pj) {
+                int k = beg + cnt;
+                for (; k > beg && pj[k - 1] > j; --k) pj[k] = pj[k - 1];
+                pj[k] = j;
+                pi[beg + cnt] = i;
+            }
+            ++cnt;
+        }
+    }
+    if (!pj) count[i] = cnt;
+}
+
 __global__ void k_pair_map(int nold, const int32_t* __restrict__ opi, const int32_t* __restrict__ opj,
                            const int32_t* __restrict__ nibeg, const int32_t* __restrict__ npj, int32_t* __restrict__ map) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -792,7 +898,13 @@ __global__ void __launch_bounds__(kBlk) k_b_final(tmps_adj_sys S, double dt, tmp
 // Reverse of the contact pass: per pair in contact, recompute under the
 // recorded mask, then the reverse; per-pair adjoints for the gather, the
 // entering history's adjoint in place, parameter and image partials.
-__global__ void __launch_bounds__(kBlk) k_b_pairs(tmps_adj_sys S, Params P, int shearupdate, const double* xs,
+//
+// kPerSM: resident blocks asked of the compiler.  Four leave it all 255
+// registers and are a wave for up to 608 tiles; beyond that five (168, with
+// spills) were faster: the gradient of 31,250 spheres (806 tiles) 29.5 -> 27.9
+// ms, while that of 2,048 (52 tiles) was 3 % slower with five.
+template <int kPerSM>
+__global__ void __launch_bounds__(kBlk, kPerSM) k_b_pairs(tmps_adj_sys S, Params P, int shearupdate, const double* xs,
                                                   const double* vs, const double* ws, const double* __restrict__ sh_rec,
                                                   const uint8_t* __restrict__ mask_rec,
                                                   const tmps_adj_rec* __restrict__ box, const double* __restrict__ wbar,
@@ -1049,6 +1161,13 @@ void run(void (*kernel)(P...), int grid, int block, cudaStream_t s, A&&... args)
     run_as(false, kernel, grid, block, s, std::forward<A>(args)...);
 }
 
+// The contact pass's reverse at the residency its number of tiles wants.
+template <typename... A>
+void run_b_pairs(int tiles, cudaStream_t s, A&&... args) {
+    if (tiles <= 608) run(k_b_pairs<4>, tiles, kBlk, s, std::forward<A>(args)...);
+    else run(k_b_pairs<5>, tiles, kBlk, s, std::forward<A>(args)...);
+}
+
 // The tape of the k-th step of a run whose tapes lie atom_stride doubles (atom
 // arrays) and pair_stride pairs apart (0: one tape, overwritten).
 tmps_adj_tape tape_at(const tmps_adj_tape& t, int64_t atom_stride, int64_t pair_stride, int64_t k) {
@@ -1101,6 +1220,37 @@ int tmps_adj_pairs(int32_t n, const double* d_x, const double* d_radius, const t
     if (n == 0) return TMPS_OK;
     k_pairs_build<<<grid_for(n, 128), 128, 0, (cudaStream_t)stream>>>(n, d_x, d_radius, d_box, skin, d_count, d_ibeg,
                                                                       d_pi, d_pj);
+    note_launches(1);
+    return ok() ? TMPS_OK : TMPS_ERR_CUDA;
+}
+
+int64_t tmps_adj_cells_bytes(int32_t n, int32_t ncell) {
+    if (n < 0 || ncell < 0) return -1;
+    return (int64_t)(3 * align256(((size_t)ncell + 1) * 4) + 2 * align256((size_t)n * 4) + align256((size_t)n * 16));
+}
+
+int tmps_adj_pairs_cells(int32_t n, const double* d_x, const double* d_radius, const tmps_adj_rec* d_box, double skin,
+                         int32_t gx, int32_t gy, int32_t gz, void* work, int32_t* d_count, const int32_t* d_ibeg,
+                         int32_t* d_pi, int32_t* d_pj, void* stream) {
+    if (n < 0 || !d_x || !d_radius || !d_box || !(skin >= 0.0) || !work) return TMPS_ERR_BAD_ARG;
+    if (gx < 3 || gy < 3 || gz < 3 || (int64_t)gx * gy * gz > (1 << 28)) return TMPS_ERR_BAD_ARG;
+    if (!d_pj && !d_count) return TMPS_ERR_BAD_ARG;
+    if (d_pj && (!d_ibeg || !d_pi)) return TMPS_ERR_BAD_ARG;
+    if (n == 0) return TMPS_OK;
+    cudaStream_t s = (cudaStream_t)stream;
+    const int m = gx * gy * gz;
+    const Cells C = carve_cells(work, n, m);
+    if (!d_pj) {
+        // bins for both calls
+        if (cudaMemsetAsync(C.count, 0, (size_t)m * 4, s) != cudaSuccess) return TMPS_ERR_CUDA;
+        k_cells_bin<<<grid_for(n, 128), 128, 0, s>>>(n, d_x, d_box, gx, gy, gz, C);
+        exclusive_scan(C.count, C.start, C.fill, m, s);
+        if (cudaMemsetAsync(C.fill, 0, (size_t)m * 4, s) != cudaSuccess) return TMPS_ERR_CUDA;
+        k_cells_fill<<<grid_for(n, 128), 128, 0, s>>>(n, d_x, d_radius, C);
+        note_launches(4);
+    }
+    k_pairs_cells<<<grid_for(n, 64), 64, 0, s>>>(n, d_x, d_radius, d_box, skin, gx, gy, gz, C, d_count, d_ibeg, d_pi,
+                                                 d_pj);
     note_launches(1);
     return ok() ? TMPS_OK : TMPS_ERR_CUDA;
 }
@@ -1227,7 +1377,7 @@ int tmps_adj_reverse(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps
         if (s->n > 0) {
             run(k_b_final, nbA, kBlk, st, *s, p->dt, t, *b, W);
             if (s->npairs > 0)
-                run(k_b_pairs, nbP, kBlk, st, *s, to_params(*p), 1, (const double*)t.xh, (const double*)t.vh,
+                run_b_pairs(nbP, st, *s, to_params(*p), 1, (const double*)t.xh, (const double*)t.vh,
                     (const double*)t.wh, (const double*)t.shear, (const uint8_t*)t.mask, rec(step - 1),
                     (const double*)W.wbar, *b, W);
             const tmps_adj_tape tp = step > first ? tape_at(*tape, atom_stride, pair_stride, step - 1 - first) : t;
@@ -1260,7 +1410,7 @@ int tmps_adj_setup_back(const tmps_adj_sys* s, const tmps_adj_params* p, const t
     Work W = carve(work, s->n, s->npairs);
     const int nbA = grid_for(s->n, kBlk), nbP = grid_for(s->npairs, kPairTile);
     const double* none = nullptr;
-    run(k_b_pairs, nbP, kBlk, st, *s, to_params(*p), 0, (const double*)s->x, (const double*)s->v, (const double*)s->w,
+    run_b_pairs(nbP, st, *s, to_params(*p), 0, (const double*)s->x, (const double*)s->v, (const double*)s->w,
         (const double*)tape->shear, (const uint8_t*)tape->mask, d_box, none, *b, W);
     run(k_b_atoms, nbA, kBlk, st, *s, p->dt, 1, 0, (const uint8_t*)tape->mask, none, none, none, d_box, d_box, *b, W);
     run(k_b_servo, 1, kOne, st, tmps_adj_servo{}, p->dt, (int64_t)1, d_box, d_box, 0.0, nbA, nbP, 1, 0, 0, *b, W);
