@@ -233,6 +233,8 @@ typedef struct tmps_engine {
                               * zeros (its C flag clear), which would leave it unchanged */
     int64_t pairs;           /* entries of the last tmps_fused_bounds' rows whose partner has the
                               * higher index: the pairs of tmps_pairs_build */
+    int32_t ablocks;         /* A's blocks among nblocks: their partials come first (0: not told) */
+    int32_t pad4_;
 } tmps_engine;
 
 /* One instance of a batched run (tmps_batch_*): the device state of one
@@ -535,7 +537,8 @@ int tmps_probe_fp64(int32_t blocks, int32_t threads, int32_t iters, double* d_ou
  * 2 the hi + lo split of a (two outputs per operand).  d_mine and d_hw
  * (n doubles, 2n for which 2) must agree bit for bit.  which 3, 4, 5: the
  * FP64 laws' 1/a, 1/sqrt(a) and sqrt(a) beside the correctly rounded ones
- * (within 2, 2 and 1 units in the last place).  No reference counterpart. */
+ * (within 2, 2 and 1 units in the last place).  which 6: a[i] / a[n-1-i] by
+ * the divisor's reciprocal, bit for bit.  No reference counterpart. */
 int tmps_selftest_arith(int32_t which, const double* d_a, int32_t n, double* d_mine, double* d_hw, void* stream);
 
 /* ---- batched runs ----------------------------------------------------------

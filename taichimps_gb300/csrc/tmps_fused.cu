@@ -1085,12 +1085,7 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
     __shared__ int32_t bgrp[kBlockC / 32][kLive];
     __shared__ uint32_t bold[kBlockC / 32][kLive], bnear[kBlockC / 32][kLive];
     __shared__ CfWarp<MIXED> cwarp[kBlockC / 32];
-    pdl_enter();
-    if (E->aborted || E->step >= E->stop_step) return;
-    const int64_t s = E->step + 1;
-    if (rebuild_due(E, s)) return;  // S marks the step aborted; the host rebuilds
-    const int nb = E->nblocks;      // partials are component-major, [6][nb]
-    part += nb - nblk;              // C's blocks follow A's
+    // the box and the engine's constants are the last S's, complete since A passed its wait
     const int n = A.n;
     CfEnv<STYLE, MIXED> V;
     V.load(P, B, E);
@@ -1099,6 +1094,12 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
     __shared__ float4 soff[MIXED ? 27 : 1], sofl[MIXED ? 27 : 1];
     __shared__ PairParams32 sP;
     if constexpr (MIXED) V.tables(P, soff, sofl, sP);
+    pdl_enter();
+    if (E->aborted || E->step >= E->stop_step) return;
+    const int64_t s = E->step + 1;
+    if (rebuild_due(E, s)) return;  // S marks the step aborted; the host rebuilds
+    const int nb = E->nblocks;      // partials are component-major, [6][nb]
+    part += nb - nblk;              // C's blocks follow A's
     double Vd[6] = {0, 0, 0, 0, 0, 0};
     float Vh[6] = {0, 0, 0, 0, 0, 0}, Vl[6] = {0, 0, 0, 0, 0, 0};  // mixed: per-thread double words
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1793,9 +1794,7 @@ __global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
     __shared__ int32_t sfirst[kBlockC / 32][kPairRing], sentry[kBlockC / 32][kPairRing];  // and its words
     __shared__ float4 soff[MIXED ? 27 : 1], sofl[MIXED ? 27 : 1];
     __shared__ PairParams32 sP;
-    pdl_enter();
-    if (E->aborted || E->step >= E->stop_step) return;
-    if (rebuild_due(E, E->step + 1)) return;  // S marks the step aborted; the host rebuilds
+    // the box and the engine's constants are the last S's, complete since A passed its wait
     CfEnv<STYLE, MIXED> V;
     V.load(P, B, E);
     if constexpr (MIXED) V.tables(P, soff, sofl, sP);
@@ -1925,7 +1924,10 @@ __global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
             }
         }
     };
-    fetch(words - 1 - gw);
+    fetch(words - 1 - gw);  // (the touch words are the last step's)
+    pdl_enter();
+    if (E->aborted || E->step >= E->stop_step) return;
+    if (rebuild_due(E, E->step + 1)) return;  // S marks the step aborted; the host rebuilds
     for (int w = words - 1 - gw; w >= 0; w -= nwarps) {
         const int p = (w << 5) + lane;
         bool near = false;
@@ -2184,13 +2186,13 @@ __global__ void __launch_bounds__(kBlockG, MIXED ? 4 : 3)
 
 // ---------------------------------------------------------------------- S
 
-__device__ double limit_rate_f(double rate, double ptarget, int normalize, double max_rate) {
+__device__ double limit_rate_f(double rate, double ptarget, double iptarget, int normalize, double max_rate) {
     double out = rate;
     if (normalize) {
         if (ptarget == 0.0) {
             if (out != 0.0) out = copysign(max_rate, out);
         } else {
-            out = out / fabs(ptarget);
+            out = div_by(out, fabs(ptarget), iptarget);
         }
     }
     if (max_rate != 0.0 && fabs(out) > max_rate) out = copysign(max_rate, out);
@@ -2201,25 +2203,43 @@ constexpr int kBlockS = 768;  // four warps per virial component
 
 // The servo's arithmetic on staged copies of the three structs.  On this
 // part an FP64 instruction costs ~64 cycles of latency and a division ~670,
-// however few lanes are active, so the work is laid out for the SM's four
-// FP64 units: warp 0 runs the serial chain (pressure -> rate -> new box,
+// however few lanes are active, and the next A waits for all of it.  So the
+// reciprocals of what the last step left (ServoInv) are formed before the
+// dependency wait, beside C, and the quotients after it come from them
+// (div_by: the same correctly rounded values).  Warp 0 runs the serial chain (pressure -> rate -> new box,
 // lane k < 6 one pressure component, lane d < 3 one dimension), then the
 // independent derived quantities are spread over the block's warps.  Each
 // value is the same FP64 expression as a one-thread form would compute.
+struct ServoInv {
+    double vol, prd[3], g[3], dt, three, ptarget[3];  // 1 / each
+};
+// lanes 0..11 of one warp, a division each
+__device__ __forceinline__ void servo_inverses(const tmps_box& b, const tmps_servo& sv, double dt, ServoInv& o) {
+    const int lane = threadIdx.x & 31;
+    if (lane >= 12) return;
+    double x = 3.0;
+    if (lane == 0) x = b.prd[0] * b.prd[1] * b.prd[2];
+    else if (lane < 4) x = b.prd[lane - 1];
+    else if (lane < 7) x = (double)b.g[lane - 4];
+    else if (lane == 7) x = dt;
+    else if (lane > 8) x = fabs(sv.ptarget[lane - 9]);
+    reinterpret_cast<double*>(&o)[lane] = 1.0 / x;
+}
+
 struct ServoNew {
     double lo[3], hi[3], prd[3];   // new box
     double olo[3], oprd[3];        // old box
     int bad;
 };
 
-__device__ void servo_chain_warp(const tmps_box& b, tmps_servo& sv, const tmps_engine& e, const double* acc,
-                                 ServoNew& o) {
+__device__ void servo_chain_warp(const tmps_box& b, tmps_servo& sv, const tmps_engine& e, const ServoInv& inv,
+                                 const double* acc, ServoNew& o) {
     const int lane = threadIdx.x & 31;
     const double dt = e.dt;
     const double vol = b.prd[0] * b.prd[1] * b.prd[2];
     double t = 0.0;
     if (lane < 6) {
-        t = vol > 0.0 ? acc[lane] / vol : 0.0;
+        t = vol > 0.0 ? div_by(acc[lane], vol, inv.vol) : 0.0;
         sv.pressure[lane] = t;
     }
     const double t0 = __shfl_sync(0xffffffffu, t, 0), t1 = __shfl_sync(0xffffffffu, t, 1),
@@ -2265,7 +2285,7 @@ __device__ void servo_chain_warp(const tmps_box& b, tmps_servo& sv, const tmps_e
         } else if (st == 8 || st == 9) {
             // coupled axes share their mean pressure; style 9 (pressure/scalar)
             // with no coupling uses the scalar pressure
-            const double scalar = ((t0 + t1) + t2) / 3.0;
+            const double scalar = div_by((t0 + t1) + t2, 3.0, inv.three);
             double pd = d == 0 ? t0 : (d == 1 ? t1 : t2);
             if (sv.couple == 1) pd = scalar;
             else if (sv.couple == 2 && d < 2) pd = (t0 + t1) / 2.0;
@@ -2273,7 +2293,7 @@ __device__ void servo_chain_warp(const tmps_box& b, tmps_servo& sv, const tmps_e
             else if (sv.couple == 4 && d != 1) pd = (t0 + t2) / 2.0;
             if (sv.couple == 0 && st == 9) pd = scalar;
             const double tgt = sv.ptarget[d];
-            const double rate = limit_rate_f(sv.pgain[d] * (pd - tgt), tgt, sv.normalize, sv.max_rate);
+            const double rate = limit_rate_f(sv.pgain[d] * (pd - tgt), tgt, inv.ptarget[d], sv.normalize, sv.max_rate);
             sv.cum[d] += (dt * rate) * prd;
             nlo = ls - 0.5 * sv.cum[d];
             nhi = hs + 0.5 * sv.cum[d];
@@ -2302,37 +2322,42 @@ __device__ void servo_chain_warp(const tmps_box& b, tmps_servo& sv, const tmps_e
 
 // The quantities derived from the new box, one kind per warp (lanes 0..2 =
 // dimensions); nothing is written when the new box is not positive.
-__device__ void servo_derive(tmps_box& b, const tmps_servo& sv, tmps_engine& e, const ServoNew& o) {
+__device__ void servo_derive(tmps_box& b, const tmps_servo& sv, tmps_engine& e, const ServoInv& inv,
+                             const ServoNew& o) {
     if (o.bad) return;
     const int warp = threadIdx.x >> 5, d = threadIdx.x & 31;
     if (d >= 3) return;
     const double nprd = o.prd[d], prd = o.oprd[d];
     switch (warp) {
         case 0:
-            b.inv_prd[d] = 1.0 / nprd;
-            if (e.mixed) e.iprd32[d] = (float)b.inv_prd[d];
+        {
+            // 1 / prd by one more step of rcp64 (correctly rounded but for rare last bits)
+            const double y = rcp64(nprd);
+            b.inv_prd[d] = __fma_rn(__fma_rn(-nprd, y, 1.0), y, y);
+            if (e.mixed) e.iprd32[d] = f32_rn(b.inv_prd[d]);
             break;
+        }
         case 1: {
-            const double hc = nprd / (double)b.g[d];
+            const double hc = div_by(nprd, (double)b.g[d], inv.g[d]);
             b.hcell[d] = hc;
             if (e.mixed) {
                 split(hc, e.h32[d], e.hlo32[d]);
-                e.dh32[d] = (float)(hc - e.h0[d]);
+                e.dh32[d] = f32_rn(hc - e.h0[d]);
             }
             break;
         }
         case 2:
-            b.h_rate[d] = (nprd - prd) / e.dt;
+            b.h_rate[d] = div_by(nprd - prd, e.dt, inv.dt);
             b.h_rate[3 + d] = 0.0;
             break;
         case 3:
-            if (e.mixed) split((nprd - prd) / prd, e.eps_hi[d], e.eps_lo[d]);
-            else e.remap_scale[d] = nprd / prd;
+            if (e.mixed) split(div_by(nprd - prd, prd, inv.prd[d]), e.eps_hi[d], e.eps_lo[d]);
+            else e.remap_scale[d] = div_by(nprd, prd, inv.prd[d]);
             break;
         case 4:
             if (e.mixed) {
                 split(nprd, e.prd32[d], e.prdlo32[d]);
-                e.dlo32[d] = (float)(o.lo[d] - e.lo0[d]);
+                e.dlo32[d] = f32_rn(o.lo[d] - e.lo0[d]);
             }
             break;
         case 5: {
@@ -2367,34 +2392,43 @@ __device__ __forceinline__ void copy_words(S* dst, const S* src) {
 }
 
 // S: finish the step.  Decide the rebuild, sum the virial partials of A and
-// C in a fixed order, run the servo.  The box and servo structs are written
-// by S alone, and the previous step's S has completed before this one can
-// start, so they are staged before the dependency wait; the engine struct
-// (A and C write parts of it) after.  The partials are component-major,
-// [6][nblocks]: four warps per component each take every fourth run of 32
-// blocks (coalesced, all loads of a lane in flight at once), then a shuffle
-// tree and the four warp sums in order.  The mixed form's partials are
-// double words and are summed as such; only the six totals become FP64.
+// C in a fixed order, run the servo.  What bounds it is latency, and the next A
+// waits for it; so all that C does not write is done before the dependency
+// wait, while C runs (when C has passed its own wait, A and the S before it are
+// complete): the three records staged, the decision, A's partials summed, the
+// reciprocals formed.  (C writes the engine's final_pending alone: 1 when the
+// step goes on, set here in the staged copy.)  The partials are
+// component-major, [6][nblocks]: four warps per component each take every
+// fourth run of 32 blocks (coalesced, the loads of a lane in flight together),
+// in block order, then a shuffle tree and the four warp sums in order.  The
+// mixed form's partials are double words and are summed as such; only the six
+// totals become FP64.
 constexpr int kWarpsS = kBlockS / 32;
 static_assert(kWarpsS == 24, "four warps per virial component");
 constexpr int kPartLoads = 10;  // per lane: up to 32 * 4 * 10 = 1280 partial blocks in one round
 
+// acc + row[k] over k = k0, k0 + 128, ... < end, in that order
 template <typename V, typename Add>
-__device__ __forceinline__ V sum_component(const V* row, int nb, int q, int lane, V zero, Add add) {
-    V acc = zero;
-    for (int k0 = q * 32 + lane; k0 < nb; k0 += 128 * kPartLoads) {
+__device__ __forceinline__ V sum_component(V acc, const V* row, int k0, int end, V zero, Add add) {
+    for (; k0 < end; k0 += 128 * kPartLoads) {
         V v[kPartLoads];
 #pragma unroll
         for (int u = 0; u < kPartLoads; ++u) {
             const int k = k0 + 128 * u;
-            v[u] = k < nb ? row[k] : zero;
+            v[u] = k < end ? row[k] : zero;
         }
 #pragma unroll
         for (int u = 0; u < kPartLoads; ++u) acc = add(acc, v[u]);
     }
     return acc;
 }
+// the lane's first block at or past `from`
+__device__ __forceinline__ int first_block(int q, int lane, int from) {
+    const int k = q * 32 + lane;
+    return k >= from ? k : k + (from - k + 127) / 128 * 128;
+}
 
+template <int WARPS>
 __device__ __forceinline__ void s_body(tmps_box* b, tmps_servo* sv, tmps_engine* e, const char* scratch,
                                        int32_t* status) {
     __shared__ double tot[6];
@@ -2403,35 +2437,59 @@ __device__ __forceinline__ void s_body(tmps_box* b, tmps_servo* sv, tmps_engine*
     __shared__ tmps_box sb;
     __shared__ tmps_servo ssv;
     __shared__ tmps_engine se;
+    __shared__ ServoInv sinv;
     __shared__ ServoNew snew;
     copy_words(&sb, b);
     copy_words(&ssv, sv);
-    // run constants of the engine record (only the host changes them, between
-    // launches), so the partial sums can be fetched with this step's words
-    const int nb = e->nblocks;
-    const int64_t part_off = e->part_off;
-    const bool mixed = e->mixed != 0, servo = e->servo != 0;
+    copy_words(&se, e);
     __syncthreads();
-    const bool servo_now = servo && ((ssv.step_count + 1) % ssv.nevery == 0);
-    pdl_enter();
-    // this step's engine words (A and C write some) and the virial partials in
-    // flight together; one word per thread (the batched S has 192 threads)
-    constexpr int kEngineWords = (int)(sizeof(tmps_engine) / 4);
-    static_assert(kEngineWords <= 192, "one engine word per thread of the batched S");
-    const uint32_t ew = (int)threadIdx.x < kEngineWords ? reinterpret_cast<const uint32_t*>(e)[threadIdx.x] : 0u;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t s = se.step + 1;
+    const bool idle = se.aborted || se.step >= se.stop_step, due = !idle && rebuild_due(&se, s);
+    const int nb = se.nblocks, na = se.ablocks;
+    const bool mixed = se.mixed != 0;
+    const bool servo_now = !idle && !due && se.servo != 0 && ((ssv.step_count + 1) % ssv.nevery == 0);
+    const double* part = reinterpret_cast<const double*>(scratch + se.part_off);
+    auto addf = [](float2 x, float2 y) {
+        dw_add2(x.x, x.y, y.x, y.y);
+        return x;
+    };
+    auto addd = [](double x, double y) { return x + y; };
+    // kWarpsS virtual warps, four per component; a block of fewer warps runs several in turn, with the
+    // same arithmetic each
+    constexpr int kTurns = kWarpsS / WARPS;
+    float2 accf[kTurns];
+    double accd[kTurns];
+#pragma unroll
+    for (int t = 0; t < kTurns; ++t) {
+        accf[t] = make_float2(0.0f, 0.0f);
+        accd[t] = 0.0;
+    }
     if (servo_now) {
-        const double* part = reinterpret_cast<const double*>(scratch + part_off);
-        // kWarpsS virtual warps, four per component; a block of fewer warps
-        // runs several in turn, with the same arithmetic each
-        if (mixed) {
-            for (int vw = warp; vw < kWarpsS; vw += (int)(blockDim.x >> 5)) {
-                const int c = vw >> 2, q = vw & 3;
-                const float2* row = reinterpret_cast<const float2*>(part) + (size_t)c * nb;
-                float2 acc = sum_component(row, nb, q, lane, make_float2(0.0f, 0.0f), [](float2 x, float2 y) {
-                    dw_add2(x.x, x.y, y.x, y.y);
-                    return x;
-                });
+#pragma unroll
+        for (int t = 0; t < kTurns; ++t) {
+            const int vw = warp + t * WARPS, c = vw >> 2, q = vw & 3;
+            if (mixed)
+                accf[t] = sum_component(accf[t], reinterpret_cast<const float2*>(part) + (size_t)c * nb, q * 32 + lane, na,
+                                        make_float2(0.0f, 0.0f), addf);
+            else
+                accd[t] = sum_component(accd[t], part + (size_t)c * nb, q * 32 + lane, na, 0.0, addd);
+        }
+        if (warp == WARPS - 1) servo_inverses(sb, ssv, se.dt, sinv);
+    }
+    pdl_enter();
+    if (idle) return;
+    if (due) {
+        if (threadIdx.x == 0) e->aborted = 1;
+        return;
+    }
+    if (servo_now) {
+#pragma unroll
+        for (int t = 0; t < kTurns; ++t) {
+            const int vw = warp + t * WARPS, c = vw >> 2, q = vw & 3;
+            if (mixed) {
+                float2 acc = sum_component(accf[t], reinterpret_cast<const float2*>(part) + (size_t)c * nb,
+                                           first_block(q, lane, na), nb, make_float2(0.0f, 0.0f), addf);
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
                     const float bh = __shfl_down_sync(0xffffffffu, acc.x, o),
@@ -2439,43 +2497,29 @@ __device__ __forceinline__ void s_body(tmps_box* b, tmps_servo* sv, tmps_engine*
                     dw_add2(acc.x, acc.y, bh, bl);
                 }
                 if (lane == 0) wsumf[vw] = acc;
-            }
-        } else {
-            for (int vw = warp; vw < kWarpsS; vw += (int)(blockDim.x >> 5)) {
-                const int c = vw >> 2, q = vw & 3;
-                const double* row = part + (size_t)c * nb;
-                double t = sum_component(row, nb, q, lane, 0.0, [](double x, double y) { return x + y; });
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-                if (lane == 0) wsum[vw] = t;
-            }
-        }
-    }
-    if ((int)threadIdx.x < kEngineWords) reinterpret_cast<uint32_t*>(&se)[threadIdx.x] = ew;
-    __syncthreads();
-    if (se.aborted || se.step >= se.stop_step) return;
-    const int64_t s = se.step + 1;
-    if (rebuild_due(&se, s)) {
-        if (threadIdx.x == 0) e->aborted = 1;
-        return;
-    }
-    if (servo_now) {
-        if (threadIdx.x < 6) {
-            if (mixed) {
-                float h = 0.0f, l = 0.0f;
-#pragma unroll
-                for (int w = 0; w < 4; ++w) dw_add2(h, l, wsumf[4 * threadIdx.x + w].x, wsumf[4 * threadIdx.x + w].y);
-                tot[threadIdx.x] = (double)h + (double)l;
             } else {
-                tot[threadIdx.x] = ((wsum[4 * threadIdx.x] + wsum[4 * threadIdx.x + 1]) + wsum[4 * threadIdx.x + 2]) +
-                                   wsum[4 * threadIdx.x + 3];
+                double t1 = sum_component(accd[t], part + (size_t)c * nb, first_block(q, lane, na), nb, 0.0, addd);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) t1 += __shfl_down_sync(0xffffffffu, t1, o);
+                if (lane == 0) wsum[vw] = t1;
             }
         }
         __syncthreads();
     }
     if (warp == 0) {
+        if (servo_now && lane < 6) {
+            if (mixed) {
+                float h = 0.0f, l = 0.0f;
+#pragma unroll
+                for (int w = 0; w < 4; ++w) dw_add2(h, l, wsumf[4 * lane + w].x, wsumf[4 * lane + w].y);
+                tot[lane] = f64_of(h) + f64_of(l);
+            } else {
+                tot[lane] = ((wsum[4 * lane] + wsum[4 * lane + 1]) + wsum[4 * lane + 2]) + wsum[4 * lane + 3];
+            }
+        }
         if (lane == 0) {
             se.step = s;
+            se.final_pending = 1;
             se.order_ready = se.cull;  // C has had its first pass since the bounds
             sb.remap_pending = 0;
             if (se.servo) {
@@ -2485,7 +2529,7 @@ __device__ __forceinline__ void s_body(tmps_box* b, tmps_servo* sv, tmps_engine*
         }
         __syncwarp();
         if (servo_now) {
-            servo_chain_warp(sb, ssv, se, tot, snew);
+            servo_chain_warp(sb, ssv, se, sinv, tot, snew);
             if (lane == 0 && snew.bad) atomicOr(status, TMPS_STATUS_BOX_NONPOSITIVE);
             if (se.plog != nullptr && se.plog_len > 0 && lane < 6)
                 se.plog[(size_t)(s % se.plog_len) * 6 + lane] = ssv.pressure[lane];
@@ -2493,7 +2537,7 @@ __device__ __forceinline__ void s_body(tmps_box* b, tmps_servo* sv, tmps_engine*
     }
     __syncthreads();
     if (servo_now) {
-        servo_derive(sb, ssv, se, snew);
+        servo_derive(sb, ssv, se, sinv, snew);
         __syncthreads();
     }
     copy_words(e, &se);
@@ -2503,7 +2547,7 @@ __device__ __forceinline__ void s_body(tmps_box* b, tmps_servo* sv, tmps_engine*
 
 __global__ void __launch_bounds__(kBlockS) k_s(tmps_box* b, tmps_servo* sv, tmps_engine* e, const char* scratch,
                                                int32_t* status) {
-    s_body(b, sv, e, scratch, status);
+    s_body<kWarpsS>(b, sv, e, scratch, status);
 }
 
 // ---------------------------------------------------------------- batched
@@ -2561,7 +2605,7 @@ __global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
 constexpr int kBlockSB = 192;
 __global__ void __launch_bounds__(kBlockSB) kb_s(const tmps_instance* __restrict__ inst, int32_t* status) {
     const tmps_instance& I = inst[blockIdx.x];
-    s_body(I.box, I.servo, I.eng, static_cast<const char*>(I.scratch), status);
+    s_body<kBlockSB / 32>(I.box, I.servo, I.eng, static_cast<const char*>(I.scratch), status);
 }
 
 __global__ void kb_state(const tmps_instance* __restrict__ inst, int ninst, int64_t* out) {

@@ -46,6 +46,7 @@ extern "C" int tmps_probe_fp64(int32_t blocks, int32_t threads, int32_t iters, d
 //   which 3: 1 / a[i]                rcp64
 //   which 4: 1 / sqrt(a[i])          rsqrt64   (a[i] >= 0)
 //   which 5: sqrt(a[i])              sqrt64    (a[i] >= 0)
+//   which 6: a[i] / a[n - 1 - i]     div_by    (bit for bit; zero divisors left out)
 namespace {
 
 __global__ void k_selftest(int which, const double* __restrict__ a, int n, double* __restrict__ mine,
@@ -76,6 +77,12 @@ __global__ void k_selftest(int which, const double* __restrict__ a, int n, doubl
             mine[i] = sqrt64(x);
             hw[i] = sqrt(x);
             break;
+        case 6: {
+            const double b = a[n - 1 - i], y = b != 0.0 ? 1.0 / b : 0.0;
+            mine[i] = b != 0.0 ? div_by(x, b, y) : 0.0;
+            hw[i] = b != 0.0 ? x / b : 0.0;
+            break;
+        }
         default: {
             float h, l;
             split_dw(x, h, l);
@@ -94,7 +101,7 @@ __global__ void k_selftest(int which, const double* __restrict__ a, int n, doubl
 
 extern "C" int tmps_selftest_arith(int32_t which, const double* d_a, int32_t n, double* d_mine, double* d_hw,
                                    void* stream) {
-    if (which < 0 || which > 5 || n < 0 || !d_a || !d_mine || !d_hw) return TMPS_ERR_BAD_ARG;
+    if (which < 0 || which > 6 || n < 0 || !d_a || !d_mine || !d_hw) return TMPS_ERR_BAD_ARG;
     if (n == 0) return TMPS_OK;
     k_selftest<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(which, d_a, n, d_mine, d_hw);
     note_launches(1);

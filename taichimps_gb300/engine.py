@@ -168,7 +168,7 @@ class FusedEngine:
             return
         self._shape(self._n)
         e = self._engine_state()
-        e.nblocks = self.nblocks
+        e.nblocks, e.ablocks = self.nblocks, self.a_blocks
         _device.push_struct(self._eng, e)
         self._graph = None
 
@@ -209,7 +209,7 @@ class FusedEngine:
         e.cundall = 1 if self.cundall is not None else 0
         e.servo = 1 if self.deform is not None else 0
         e.mixed = 1 if self.mixed else 0
-        e.nblocks = self.nblocks
+        e.nblocks, e.ablocks = self.nblocks, self.a_blocks
         e.dt = float(sim.dt)
         if self.cundall is not None:
             e.gamma_lin, e.gamma_ang = self.cundall.gamma_lin, self.cundall.gamma_ang

@@ -42,3 +42,18 @@ def test_reciprocals_and_roots(gpu, which, ulps):
     edge = np.array([0.0, np.inf, np.nan, 5e-324, 2.0 ** -1022, 2.0 ** -1005, 2.0 ** 1005, 1.7e308])
     mine, hw = _run(which, edge)
     np.testing.assert_array_equal(mine, hw)
+
+
+def test_quotient_by_reciprocal(gpu):
+    """div_by against the division, bit for bit: random mantissas and exponents, quotients near one,
+    near powers of two, zeros, and operands that must take the division."""
+    rng = np.random.default_rng(6)
+    usual = rng.uniform(-1e4, 1e4, size=400_000)
+    wide = np.ldexp(rng.uniform(1.0, 2.0, size=400_000), rng.integers(-480, 480, size=400_000))
+    near = 1.0 + np.arange(-200_000, 200_000) * 2.0 ** -52
+    p2 = np.ldexp(1.0, np.arange(-520, 520))
+    edge = np.array([0.0, -0.0, 1e300, 5e-324, 1e-300, np.inf, 3.0, 1.0])
+    a = np.concatenate([usual, wide, near, p2, np.nextafter(p2, np.inf), edge])
+    rng.shuffle(a)
+    mine, hw = _run(6, a)
+    np.testing.assert_array_equal(mine.view(np.int64), hw.view(np.int64))
