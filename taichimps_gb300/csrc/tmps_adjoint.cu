@@ -47,20 +47,21 @@ struct Work {
     double* partw;  // [6][nbP] pair virial partials
     double* partk;  // [6][nbA] kinetic / remap partials
     double* partg;  // [8][nbP] parameter and image partials of the reverse
-    double* wbar;   // [6] dL/d(virial total) of the current reverse step
+    double* wbar;   // [6] dL/d(virial total) of the current reverse step: at the base, where the calls of
+                    // a linked run find it whatever their numbers of pairs
 };
 
 Work carve(void* base, int n, int npairs) {
     const int nbA = grid_for(n, kBlk), nbP = grid_for(npairs, kPairTile);
     char* p = static_cast<char*>(base);
     Work w;
+    w.wbar = reinterpret_cast<double*>(p); p += align256(sizeof(double) * 8);
     w.fp = reinterpret_cast<double*>(p); p += align256(sizeof(double) * 3 * (size_t)npairs);
     w.tp = reinterpret_cast<double*>(p); p += align256(sizeof(double) * 3 * (size_t)npairs);
     w.gp = reinterpret_cast<double*>(p); p += align256(sizeof(double) * kNG * (size_t)npairs);
     w.partw = reinterpret_cast<double*>(p); p += align256(sizeof(double) * 6 * (size_t)nbP);
     w.partk = reinterpret_cast<double*>(p); p += align256(sizeof(double) * 6 * (size_t)nbA);
-    w.partg = reinterpret_cast<double*>(p); p += align256(sizeof(double) * 8 * (size_t)nbP);
-    w.wbar = reinterpret_cast<double*>(p);
+    w.partg = reinterpret_cast<double*>(p);
     return w;
 }
 

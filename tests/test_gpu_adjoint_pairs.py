@@ -52,3 +52,28 @@ def test_cells_equal_all_pairs(gpu, n, box, g):
     if n > 1 and max(box) < 20.0:
         assert got[0][1][-1] > 0
     assert ctypes.sizeof(_lib.AdjRec) == len(bytes(rec))
+
+
+def test_reverse_across_lists_of_unequal_length(gpu):
+    """A run whose pair lists differ in length by more than a page of the workspace, against the same
+    run on one wide list: the reverse's running values do not depend on a list's number of pairs."""
+    import torch
+    from taichimps_gb300.adjoint import stress_curve
+    from taichimps_gb300.packing import compress_packing
+    from test_gpu_adjoint import BASE, _run
+    pk = compress_packing(343, seed=11)
+    v = np.random.default_rng(4).normal(0.0, 3.0, size=pk["x"].shape)
+    got = []
+    for skin in (0.01, 0.3):
+        run = _run(pk, 80, 20, 30, skin=skin, v=v)
+        ps = {k: torch.tensor(a, dtype=torch.float64, requires_grad=True) for k, a in BASE.items()}
+        r = torch.tensor(pk["radius"], dtype=torch.float64, device="cuda", requires_grad=True)
+        q = stress_curve(run, ps["kn"], ps["kt"], ps["gamman"], ps["gammat"], ps["xmu"], r)
+        (q ** 2).sum().backward()
+        got.append((run, {k: float(a.grad) for k, a in ps.items()}, r.grad))
+    (few, g, gr), (one, h, hr) = got
+    counts = [p.npairs for p in few.lists]
+    assert one.rebuilds == 0 and max(abs(a - b) for a, b in zip(counts, counts[1:])) >= 32, counts
+    for k in BASE:  # the tolerance of the comparison with autograd
+        assert abs(g[k] - h[k]) <= 1e-8 * abs(h[k]) + 1e-12, (k, g[k], h[k])
+    assert (gr - hr).abs().max() <= 1e-8 * hr.abs().max()
