@@ -234,7 +234,11 @@ typedef struct tmps_engine {
     int64_t pairs;           /* entries of the last tmps_fused_bounds' rows whose partner has the
                               * higher index: the pairs of tmps_pairs_build */
     int32_t ablocks;         /* A's blocks among nblocks: their partials come first (0: not told) */
-    int32_t pad4_;
+    int32_t fold;            /* 1: no servo and at least one atom: the contact kernel ends the step, and
+                              * tmps_fused_servo does nothing */
+    int64_t attempt;         /* the step in hand, 0: none (A; tmps_fused_prepare) */
+    int32_t walk_order;      /* order_ready as A saw it */
+    int32_t pad5_;
 } tmps_engine;
 
 /* One instance of a batched run (tmps_batch_*): the device state of one

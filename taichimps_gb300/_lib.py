@@ -108,7 +108,8 @@ class Engine(ctypes.Structure):
         ("cull_tol", ctypes.c_float),
         ("plog", ctypes.c_void_p), ("plog_len", c_i32), ("order_ready", c_i32),
         ("stop_step", ctypes.c_int64), ("touching", c_i32), ("kick_all", c_i32),
-        ("pairs", ctypes.c_int64), ("ablocks", c_i32), ("pad4_", c_i32),
+        ("pairs", ctypes.c_int64), ("ablocks", c_i32), ("fold", c_i32),
+        ("attempt", ctypes.c_int64), ("walk_order", c_i32), ("pad5_", c_i32),
     ]
 
 

@@ -157,6 +157,17 @@ __device__ __forceinline__ void note_displacement(tmps_engine* __restrict__ e, f
     if ((threadIdx.x & 31) == 0 && m > *(volatile uint32_t*)&e->maxd2_bits) atomicMax(&e->maxd2_bits, m);
 }
 
+// What the rest of the step goes by, written by A's first block: the number of
+// the step in hand (0: none, the launches do nothing) and whether C walks the
+// gap order.  Where no servo runs, C's own first block moves step and aborted
+// on (step_done), so the kernels after A must not read those.
+__device__ __forceinline__ void open_step(tmps_engine* __restrict__ e, int bid, bool idle) {
+    if (bid == 0 && threadIdx.x == 0) {
+        e->attempt = idle ? 0 : e->step + 1;
+        e->walk_order = e->order_ready;
+    }
+}
+
 // Bit of atom i in the flag words: its force and torque may be nonzero (the
 // words of C's first pass; all ones before the first pass after a build).
 __device__ __forceinline__ bool force_live(const uint32_t* __restrict__ flags, int i) {
@@ -214,7 +225,9 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
                                          const int nblk) {
     __shared__ double smem[6 * (kBlockA / 32)];
     pdl_enter();
-    if (e->aborted || e->step >= e->stop_step) return;
+    const bool idle = e->aborted || e->step >= e->stop_step;
+    open_step(e, bid, idle);
+    if (idle) return;
     const int n = a.n;
     const int nb = e->nblocks;  // partials are component-major, [6][nb]
     const int lane = threadIdx.x & 31;
@@ -228,12 +241,15 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
     double K[6] = {0, 0, 0, 0, 0, 0};
     double kept = 0.0;  // lane c < 6: component c of the kept group sums
     bool kicked = false;
+    const bool sums = e->servo != 0;  // nobody reads the kinetic sums otherwise
+    // consecutive groups to consecutive blocks: a small system's warps spread over the SMs, whose FP64
+    // units they would otherwise share
     const int stride = nblk * blockDim.x;
-    for (int b0 = bid * blockDim.x + (threadIdx.x & ~31); b0 < n; b0 += stride) {
+    for (int b0 = (bid + nblk * (int)(threadIdx.x >> 5)) * 32; b0 < n; b0 += stride) {
         const int i = b0 + lane;
         const bool mine = i < n;
         double* const row = kin + 8 * (size_t)(b0 >> 5);
-        const double kr = lane < 8 ? row[lane] : 0.0;
+        const double kr = sums && lane < 8 ? row[lane] : 0.0;
         double4 x = make_double4(0, 0, 0, 0), v = x;
         double x0x = 0.0, x0y = 0.0, x0z = 0.0;
         bool kick = false;
@@ -267,7 +283,8 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
         // the kinetic terms: read back where no velocity of the group changed and they are held
         const bool moved = __any_sync(0xffffffffu, kick);
         const bool held = !moved && __shfl_sync(0xffffffffu, __double2hiint(kr), 6) != 0;
-        if (held) {
+        if (!sums) {
+        } else if (held) {
             kept += kr;  // (lanes 6 and 7 sum nothing that is used)
         } else {
             const double k6[6] = {(v.w * v.x) * v.x, (v.w * v.y) * v.y, (v.w * v.z) * v.z,
@@ -326,6 +343,7 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
     }
     if (__any_sync(0xffffffffu, hit) && lane == 0) e->disp_stamp = s;
     note_displacement(e, dd);
+    if (!sums) return;
     const double tot = block_sum6_halving<kBlockA>(K, kept, kicked, smem);
     if (threadIdx.x < 6) part[(size_t)threadIdx.x * nb + bid] = tot;
 }
@@ -383,7 +401,9 @@ __device__ __forceinline__ void a32_body(const tmps_atoms& a, const tmps_box* __
     // issues no FP64 instruction at all.
     __shared__ float2 smem[6 * (kBlockA / 32)];
     pdl_enter();
-    if (e->aborted || e->step >= e->stop_step) return;
+    const bool idle = e->aborted || e->step >= e->stop_step;
+    open_step(e, bid, idle);
+    if (idle) return;
     const int n = a.n;
     const int nb = e->nblocks;  // partials are component-major, [6][nb]
     const int lane = threadIdx.x & 31;
@@ -450,6 +470,7 @@ __device__ __forceinline__ void a32_body(const tmps_atoms& a, const tmps_box* __
     }
     if (__any_sync(0xffffffffu, hit) && lane == 0) e->disp_stamp = s;
     note_displacement(e, dd);
+    if (!e->servo) return;  // nobody reads the sums
     block_sum_dw<6, kBlockA>(Kh, Kl, smem);
     if (threadIdx.x == 0) {
 #pragma unroll
@@ -466,6 +487,20 @@ __global__ void __launch_bounds__(kBlockA, 3) k_a32(tmps_atoms a, const tmps_box
 }
 
 // ---------------------------------------------------------------------- C
+
+// The end of a step without a servo, by the first block of its last contact
+// kernel in place of S: step and aborted move on (the other blocks go by
+// attempt), or the rebuild is marked.  Measured: a step of 4,000 spheres, FP64,
+// without S and with its blocks spread (a_blocks) 32 -> 25.4 us.
+__device__ __forceinline__ void step_done(tmps_engine* __restrict__ E, int64_t s, bool due) {
+    if (!E->fold) return;
+    if (due) {
+        E->aborted = 1;
+    } else {
+        E->step = s;
+        E->order_ready = E->cull;
+    }
+}
 
 constexpr int kLive = 8;  // live groups a warp screens together (8 measured best: 4 and 12 are slower)
 
@@ -1095,11 +1130,15 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
     __shared__ PairParams32 sP;
     if constexpr (MIXED) V.tables(P, soff, sofl, sP);
     pdl_enter();
-    if (E->aborted || E->step >= E->stop_step) return;
-    const int64_t s = E->step + 1;
-    if (rebuild_due(E, s)) return;  // S marks the step aborted; the host rebuilds
-    const int nb = E->nblocks;      // partials are component-major, [6][nb]
-    part += nb - nblk;              // C's blocks follow A's
+    const int64_t s = E->attempt;
+    if (s == 0) return;
+    if (rebuild_due(E, s)) {  // S (or step_done) marks the step aborted; the host rebuilds
+        if (threadIdx.x == 0 && bid == 0) step_done(E, s, true);
+        return;
+    }
+    const int nb = E->nblocks;  // partials are component-major, [6][nb]
+    part += nb - nblk;          // C's blocks follow A's
+    const bool sums = E->servo != 0;  // nobody reads the virial otherwise
     double Vd[6] = {0, 0, 0, 0, 0, 0};
     float Vh[6] = {0, 0, 0, 0, 0, 0}, Vl[6] = {0, 0, 0, 0, 0, 0};  // mixed: per-thread double words
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1194,12 +1233,14 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
                 // must not depend on the path the contact is inlined into
                 tc[c] = add_rn(mul_rn(arm, out.tor[c]), sg * out.troll[c]);
             }
-            vc[0] = T(0.5) * (in.d[0] * out.f[0]);
-            vc[1] = T(0.5) * (in.d[1] * out.f[1]);
-            vc[2] = T(0.5) * (in.d[2] * out.f[2]);
-            vc[3] = T(0.5) * (in.d[0] * out.f[1]);
-            vc[4] = T(0.5) * (in.d[0] * out.f[2]);
-            vc[5] = T(0.5) * (in.d[1] * out.f[2]);
+            if (MIXED || sums) {
+                vc[0] = T(0.5) * (in.d[0] * out.f[0]);
+                vc[1] = T(0.5) * (in.d[1] * out.f[1]);
+                vc[2] = T(0.5) * (in.d[2] * out.f[2]);
+                vc[3] = T(0.5) * (in.d[0] * out.f[1]);
+                vc[4] = T(0.5) * (in.d[0] * out.f[2]);
+                vc[5] = T(0.5) * (in.d[1] * out.f[2]);
+            }
         }
         return near;
     };
@@ -1464,12 +1505,14 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
                 T im;
                 if constexpr (MIXED) im = __fdividef(1.0f, mi);
                 else im = A.rinv[i];
-                T dk[6];
-                kinetic_change<T>(mi, im, T(0.5) * dt, F, vi, dk);
+                if (MIXED || sums) {
+                    T dk[6];
+                    kinetic_change<T>(mi, im, T(0.5) * dt, F, vi, dk);
 #pragma unroll
-                for (int c = 0; c < 6; ++c) {
-                    if constexpr (MIXED) dw_add(Vh[c], Vl[c], V[c] + dk[c]);
-                    else Vd[c] += V[c] + dk[c];
+                    for (int c = 0; c < 6; ++c) {
+                        if constexpr (MIXED) dw_add(Vh[c], Vl[c], V[c] + dk[c]);
+                        else Vd[c] += V[c] + dk[c];
+                    }
                 }
             }
         }
@@ -1483,7 +1526,7 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
     // out stays out with its flags clear, and the live groups are a prefix of
     // the ascending gap order.  Walking that order instead of the group
     // index gives every warp the same number of live groups (+-1).
-    const bool ordered = cull && E->order_ready != 0;
+    const bool ordered = cull && E->walk_order != 0;
     for (int base = gw; base < ngroups; base += 32 * nwarps) {
         const int k = base + lane * nwarps;
         int mygrp = k;
@@ -1581,6 +1624,11 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
             __syncwarp();
         }
     }
+    if (threadIdx.x == 0 && bid == 0) {
+        E->final_pending = 1;
+        step_done(E, s, false);
+    }
+    if (!sums) return;
     if constexpr (MIXED) {
         block_sum_dw<6, kBlockC>(Vh, Vl, reinterpret_cast<float2*>(smem));
         if (threadIdx.x == 0) {
@@ -1591,7 +1639,6 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
         const double tot = block_sum6_halving<kBlockC>(Vd, 0.0, true, smem);
         if (threadIdx.x < 6) part[(size_t)threadIdx.x * nb + bid] = tot;
     }
-    if (threadIdx.x == 0 && bid == 0) E->final_pending = 1;
 }
 
 template <int STYLE, bool MIXED>
@@ -1909,7 +1956,9 @@ __global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
     // atoms, finds the records written last in L2 (contiguous runs per warp: 6 us slower per step of
     // 1M jammed spheres)
     const int words = (np + 31) >> 5;
-    const int nwarps = (gridDim.x * kBlockC) >> 5, gw = blockIdx.x * (kBlockC / 32) + wib;
+    // (one word a warp or less: spread over the SMs)
+    const int nwarps = (gridDim.x * kBlockC) >> 5;
+    const int gw = words <= nwarps ? blockIdx.x + gridDim.x * wib : blockIdx.x * (kBlockC / 32) + wib;
     int head = 0, tail = 0;
     // the words of the next 32 pairs are on their way while these are tested
     int i_n = 0, e_n = 0;
@@ -1926,8 +1975,7 @@ __global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
     };
     fetch(words - 1 - gw);  // (the touch words are the last step's)
     pdl_enter();
-    if (E->aborted || E->step >= E->stop_step) return;
-    if (rebuild_due(E, E->step + 1)) return;  // S marks the step aborted; the host rebuilds
+    if (E->attempt == 0 || rebuild_due(E, E->attempt)) return;  // (the gather kernel marks it)
     for (int w = words - 1 - gw; w >= 0; w -= nwarps) {
         const int p = (w << 5) + lane;
         bool near = false;
@@ -2008,8 +2056,12 @@ __global__ void __launch_bounds__(kBlockG, MIXED ? 4 : 3)
     __shared__ double smem[6 * (kBlockG / 32)];
     __shared__ float sV[MIXED ? 6 : 1][kBlockG];
     pdl_enter();
-    if (E->aborted || E->step >= E->stop_step) return;
-    if (rebuild_due(E, E->step + 1)) return;
+    const int64_t s = E->attempt;
+    if (s == 0) return;
+    if (rebuild_due(E, s)) {  // S (or step_done) marks the step aborted; the host rebuilds
+        if (threadIdx.x == 0 && blockIdx.x == 0) step_done(E, s, true);
+        return;
+    }
     const int nb = E->nblocks;
     part += nb - gridDim.x;  // C's blocks follow A's
     const int n = A.n, lane = threadIdx.x & 31;
@@ -2181,7 +2233,10 @@ __global__ void __launch_bounds__(kBlockG, MIXED ? 4 : 3)
         if (threadIdx.x < 6)
             part[(size_t)threadIdx.x * nb + blockIdx.x] = tot + Q.part[(size_t)threadIdx.x * gridDim.x + blockIdx.x];
     }
-    if (threadIdx.x == 0 && blockIdx.x == 0) E->final_pending = 1;
+    if (threadIdx.x == 0 && blockIdx.x == 0) {
+        E->final_pending = 1;
+        step_done(E, s, false);
+    }
 }
 
 // ---------------------------------------------------------------------- S
@@ -2445,7 +2500,7 @@ __device__ __forceinline__ void s_body(tmps_box* b, tmps_servo* sv, tmps_engine*
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t s = se.step + 1;
-    const bool idle = se.aborted || se.step >= se.stop_step, due = !idle && rebuild_due(&se, s);
+    const bool idle = se.fold || se.aborted || se.step >= se.stop_step, due = !idle && rebuild_due(&se, s);
     const int nb = se.nblocks, na = se.ablocks;
     const bool mixed = se.mixed != 0;
     const bool servo_now = !idle && !due && se.servo != 0 && ((ssv.step_count + 1) % ssv.nevery == 0);
@@ -2602,7 +2657,7 @@ __global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
 // S of a batch: one block of six warps per instance (the derived quantities
 // take one warp per kind, the virial sum runs the 24 virtual warps of the
 // single-instance S four at a time), so many instances fit in one wave.
-constexpr int kBlockSB = 192;
+constexpr int kBlockSB = 384;
 __global__ void __launch_bounds__(kBlockSB) kb_s(const tmps_instance* __restrict__ inst, int32_t* status) {
     const tmps_instance& I = inst[blockIdx.x];
     s_body<kBlockSB / 32>(I.box, I.servo, I.eng, static_cast<const char*>(I.scratch), status);
@@ -2683,6 +2738,8 @@ __global__ void __launch_bounds__(kBlockA) k_prepare(tmps_atoms a, const tmps_bo
 __global__ void k_prepare_engine(const tmps_box* __restrict__ b, tmps_engine* e, int64_t part_off) {
     if (threadIdx.x || blockIdx.x) return;
     e->part_off = part_off;
+    e->attempt = e->step + 1;  // a rebuild step's contacts run without an A before them
+    e->walk_order = 0;
     e->cull = 0;  // until tmps_fused_bounds sets the bounds
     e->touching = 0;
     e->pairs = 0;
@@ -2872,9 +2929,17 @@ int a_wave(bool mixed) {
     if (!v) v = mixed ? wave_blocks(k_a32, kBlockA) : wave_blocks(k_a64, kBlockA);
     return v;
 }
-int a_blocks(int n, bool mixed) { const int b = grid_for(n, kBlockA); return b < a_wave(mixed) ? b : a_wave(mixed); }
+// The FP64 form takes as many blocks as there are 32-atom groups, up to the
+// wave: an SM's FP64 units are shared by its warps (one FP64 instruction of a
+// warp every ~15 cycles), so a small system runs one warp on each of many SMs
+// (a step of 4,000 spheres without a servo 28 -> 25.4 us).  The mixed form's warps share
+// nothing as narrow and its partial sums keep the fuller blocks.
+int a_blocks(int n, bool mixed) {
+    const int b = grid_for(n, mixed ? kBlockA : 32);
+    return b < a_wave(mixed) ? b : a_wave(mixed);
+}
 int contact_blocks(int n, int style, bool mixed) {
-    const int b = grid_for(n, kBlockC);
+    const int b = grid_for(n, mixed ? kBlockC : 32);
     return b < contact_wave(style, mixed) ? b : contact_wave(style, mixed);
 }
 // Grids under a launch shape of g 32-atom groups per warp: one block per

@@ -158,6 +158,11 @@ class FusedEngine:
         _lib.check(_device.lib().tmps_fused_shape(n, style, mixed, self.launch_shape[0], self.launch_shape[1],
                                                   ctypes.byref(a_b), ctypes.byref(c_b)), "tmps_fused_shape")
         self.a_blocks, self.c_blocks = a_b.value, c_b.value
+        if not self.mixed and self.deform is not None:
+            # the FP64 form's one block of C per 32-atom group spreads a small system over the SMs; where
+            # a servo sums the blocks' partials every step, two groups share one (a step of 1,000, 4,000
+            # and 12,000 spheres: 17.2, 23.5 and 30.2 us against 17.5, 24.2 and 29.3)
+            self.c_blocks = min(self.c_blocks, (n + 63) // 64)
         self.nblocks = self.a_blocks + self.c_blocks
 
     def set_launch_shape(self, shape: tuple[int, int]) -> None:
@@ -208,6 +213,9 @@ class FusedEngine:
         e.delay, e.every, e.check = int(nl.delay), max(1, int(nl.every)), 1 if nl.check else 0
         e.cundall = 1 if self.cundall is not None else 0
         e.servo = 1 if self.deform is not None else 0
+        # without a servo the contact kernel itself ends the step (two launches a step, not three)
+        self.fold = self.deform is None and n > 0
+        e.fold = 1 if self.fold else 0
         e.mixed = 1 if self.mixed else 0
         e.nblocks, e.ablocks = self.nblocks, self.a_blocks
         e.dt = float(sim.dt)
@@ -315,6 +323,8 @@ class FusedEngine:
         _lib.check(rc, "tmps_fused_a")
         with _device.timed("fused_c"):
             self._launch_c(L, st, atoms, nl_struct, params)
+        if self.fold:
+            return
         with _device.timed("fused_s"):
             rc = L.tmps_fused_servo(dbox, self._servo_ptr(), eng, self.part.data_ptr(), self.status.data_ptr(), st)
         _lib.check(rc, "tmps_fused_servo")
@@ -423,7 +433,7 @@ class FusedEngine:
             self._graph, self._graph_key = _device.capture_graph(chunk), key
         self._graph.replay()
         self.graph_replays += 1
-        self.graph_kernel_launches += self.chunk * (self.LAUNCHES_PER_STEP + (1 if self.rows else 0))
+        self.graph_kernel_launches += self.chunk * (self.LAUNCHES_PER_STEP + (1 if self.rows else 0) - (1 if self.fold else 0))
 
     def cull_stats(self) -> tuple[int, int]:
         """(32-atom groups, groups the contact bound rules out right now), from the
@@ -488,8 +498,9 @@ class FusedEngine:
         nl_struct = sim.history.cstruct(nl)
         dbox, eng = sim.domain.dbox, self._eng.data_ptr()
         self._launch_c(L, st, atoms, nl_struct, sim.pair_style.params)
-        _lib.check(L.tmps_fused_servo(dbox, self._servo_ptr(), eng, self.part.data_ptr(), self.status.data_ptr(),
-                                      st), "tmps_fused_servo")
+        if not self.fold:
+            _lib.check(L.tmps_fused_servo(dbox, self._servo_ptr(), eng, self.part.data_ptr(),
+                                          self.status.data_ptr(), st), "tmps_fused_servo")
 
     def finish(self) -> None:
         """Settle pending updates and hand the state back to the per-hook path."""
