@@ -238,7 +238,7 @@ typedef struct tmps_engine {
                               * tmps_fused_servo does nothing */
     int64_t attempt;         /* the step in hand, 0: none (A; tmps_fused_prepare) */
     int32_t walk_order;      /* order_ready as A saw it */
-    int32_t pad5_;
+    int32_t walls;           /* FP64 form: tmps_fused_walls runs after the contacts of every step */
 } tmps_engine;
 
 /* One instance of a batched run (tmps_batch_*): the device state of one
@@ -614,6 +614,21 @@ typedef struct tmps_wall_params {
  * double[3][nslots], d_touch int32[nslots] (nslots > every uid). */
 int tmps_wall_gran(const tmps_atoms* a, const tmps_wall_params* p, double dt, int32_t history_update,
                    double* d_shear, int32_t* d_touch, int32_t nslots, void* stream);
+
+/* The walls of a fused step (FP64 form), after its contacts: the same forces,
+ * added for every wall in order.  Steps whose engine record has walls = 1
+ * need this call between tmps_fused_c (or _c_pairs) and tmps_fused_servo; no
+ * servo reads what the walls add, so walls and a servo do not go together. */
+#define TMPS_MAX_FUSED_WALLS 8
+typedef struct tmps_fused_wall {
+    tmps_wall_params p;
+    double* shear;           /* as tmps_wall_gran's */
+    int32_t* touch;
+    int32_t nslots;
+    int32_t history_update;
+} tmps_fused_wall;
+int tmps_fused_walls(const tmps_atoms* a, const tmps_engine* d_eng, const tmps_fused_wall* walls, int32_t count,
+                     void* scratch, void* stream);
 
 /* ---- differentiable run (hand-written adjoint) --------------------------
  * gran/hertz/history (GRANULAR/hertz_history.py:57-171) + fix nve/sphere

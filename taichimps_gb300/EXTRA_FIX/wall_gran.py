@@ -17,6 +17,7 @@ from __future__ import annotations
 import math
 from typing import Any
 
+import numpy as np
 import torch
 
 from .. import _device, _lib
@@ -36,9 +37,21 @@ class _WallBase(Fix):
         self.touch.zero_()
 
     def _launch(self, atom, dt: float, p: _lib.WallParams) -> None:
-        n = atom.nlocal
-        if n == 0:
+        if atom.nlocal == 0:
             return
+        self.ready(atom)
+        with _device.timed("wall"):
+            rc = _device.lib().tmps_wall_gran(atom.cstruct(), p, float(dt), 1 if self.history_update else 0,
+                                              self.shear.data_ptr(), self.touch.data_ptr(), self.max_atoms,
+                                              _device.stream())
+        _lib.check(rc, "tmps_wall_gran")
+
+    def passed(self, steps: int, dt: float) -> None:
+        """`steps` steps were made by the fused step."""
+
+    def ready(self, atom) -> None:
+        """The checks of a wall before its force: room for the atoms, and their count as last time."""
+        n = atom.nlocal
         if n > self.max_atoms:
             raise ValueError(f"{type(self).__name__} was built for max_atoms={self.max_atoms}, the system has {n}")
         if n != self._n_seen:
@@ -46,11 +59,6 @@ class _WallBase(Fix):
             if self._n_seen >= 0:
                 self.reset_history()
             self._n_seen = n
-        with _device.timed("wall"):
-            rc = _device.lib().tmps_wall_gran(atom.cstruct(), p, float(dt), 1 if self.history_update else 0,
-                                              self.shear.data_ptr(), self.touch.data_ptr(), self.max_atoms,
-                                              _device.stream())
-        _lib.check(rc, "tmps_wall_gran")
 
 
 class FixWallGran(_WallBase):
@@ -115,6 +123,10 @@ class FixWallGran(_WallBase):
             return
         self._launch(atom, dt, self.params())
         self.elapsed += dt
+
+    def passed(self, steps: int, dt: float) -> None:
+        # one addition a step, as post_force makes them
+        self.elapsed = float(np.add.accumulate(np.concatenate(([self.elapsed], np.full(steps, dt))))[-1])
 
     def setup(self, nsteps_total: int = 0, dt: float = 0.0) -> None:
         """Restart the clock the wall motion is referenced to."""

@@ -109,7 +109,7 @@ class Engine(ctypes.Structure):
         ("plog", ctypes.c_void_p), ("plog_len", c_i32), ("order_ready", c_i32),
         ("stop_step", ctypes.c_int64), ("touching", c_i32), ("kick_all", c_i32),
         ("pairs", ctypes.c_int64), ("ablocks", c_i32), ("fold", c_i32),
-        ("attempt", ctypes.c_int64), ("walk_order", c_i32), ("pad5_", c_i32),
+        ("attempt", ctypes.c_int64), ("walk_order", c_i32), ("walls", c_i32),
     ]
 
 
@@ -131,6 +131,13 @@ class WallParams(ctypes.Structure):
                 ("coord", c_f64), ("vwall_n", c_f64), ("vwall_s", c_f64), ("c1", c_f64), ("c2", c_f64),
                 ("radius", c_f64), ("axis_lo", c_f64), ("axis_hi", c_f64), ("kn", c_f64), ("kt", c_f64),
                 ("gamman", c_f64), ("gammat", c_f64), ("xmu", c_f64)]
+
+
+class FusedWall(ctypes.Structure):
+    _fields_ = [("p", WallParams), ("shear", c_vp), ("touch", c_vp), ("nslots", c_i32), ("history_update", c_i32)]
+
+
+MAX_FUSED_WALLS = 8
 
 
 class AdjParams(ctypes.Structure):
@@ -224,6 +231,7 @@ _SIGS = {
     "tmps_pairs_history": (c_i32, [ctypes.POINTER(NList), ctypes.POINTER(PairParams), c_i32, c_i32, c_vp, c_vp]),
     "tmps_fused_c_pairs": (c_i32, [ctypes.POINTER(Atoms), ctypes.POINTER(NList), c_vp, c_vp,
                                    ctypes.POINTER(PairParams), c_i32, c_vp, c_i32, c_vp, c_vp]),
+    "tmps_fused_walls": (c_i32, [ctypes.POINTER(Atoms), c_vp, ctypes.POINTER(FusedWall), c_i32, c_vp, c_vp]),
     "tmps_fused_servo": (c_i32, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "tmps_fused_blocks": (c_i32, [c_i32, c_i32, c_i32]),
     "tmps_probe_fp64": (c_i32, [c_i32, c_i32, c_i32, c_vp, c_vp]),

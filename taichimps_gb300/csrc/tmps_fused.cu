@@ -21,6 +21,7 @@
 //          accumulation; FP64 kept for the velocity and position updates, the
 //          per-contact shear history and the virial reduction.
 #include "tmps_contact.cuh"
+#include "tmps_wall.cuh"
 #include "tmps_servo.cuh"
 
 using namespace tmps;
@@ -122,8 +123,8 @@ __device__ __forceinline__ void pdl_enter() {
 // Scratch layout of one instance: [flag words, one per 32-atom group + 1]
 // [per-group gaps][per-atom gaps][groups in ascending gap order][their gaps]
 // [sort keys, a power of two of them][FP64 form: kept kinetic sums, eight
-// doubles per group][virial partials, component-major [6][blocks of A and C]],
-// each region on a 256-byte boundary.
+// doubles per group][flag words of the walls, one per group][virial partials,
+// component-major [6][blocks of A and C]], each region on a 256-byte boundary.
 __host__ __device__ inline size_t lay_round256(size_t b) { return (b + 255) & ~size_t(255); }
 __host__ __device__ inline int lay_groups(int n) { return (n + 31) / 32; }
 __host__ __device__ inline int lay_npad(int n) {
@@ -137,7 +138,8 @@ __host__ __device__ inline size_t lay_order(int n) { return lay_agap(n) + lay_ro
 __host__ __device__ inline size_t lay_sgap(int n) { return lay_order(n) + lay_round256((size_t)lay_groups(n) * sizeof(int32_t)); }
 __host__ __device__ inline size_t lay_keys(int n) { return lay_sgap(n) + lay_round256((size_t)lay_groups(n) * sizeof(float)); }
 __host__ __device__ inline size_t lay_kin(int n) { return lay_keys(n) + lay_round256((size_t)lay_npad(n) * sizeof(uint64_t)); }
-__host__ __device__ inline size_t lay_part(int n) { return lay_kin(n) + lay_round256((size_t)lay_groups(n) * 8 * sizeof(double)); }
+__host__ __device__ inline size_t lay_wall(int n) { return lay_kin(n) + lay_round256((size_t)lay_groups(n) * 8 * sizeof(double)); }
+__host__ __device__ inline size_t lay_part(int n) { return lay_wall(n) + lay_round256((size_t)lay_groups(n) * sizeof(uint32_t)); }
 
 __device__ __forceinline__ bool rebuild_due(const tmps_engine* __restrict__ e, int64_t s) {
     const int64_t since = s - e->last_build_step;
@@ -221,8 +223,8 @@ __device__ __forceinline__ float bits_diff(double x, double x0, float& err, bool
 // instructions per atom (drift 3, remap 6).
 __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __restrict__ b,
                                          tmps_engine* __restrict__ e, const uint32_t* __restrict__ flags,
-                                         double* __restrict__ kin, double* __restrict__ part, const int bid,
-                                         const int nblk) {
+                                         const uint32_t* __restrict__ wflags, double* __restrict__ kin,
+                                         double* __restrict__ part, const int bid, const int nblk) {
     __shared__ double smem[6 * (kBlockA / 32)];
     pdl_enter();
     const bool idle = e->aborted || e->step >= e->stop_step;
@@ -242,6 +244,7 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
     double kept = 0.0;  // lane c < 6: component c of the kept group sums
     bool kicked = false;
     const bool sums = e->servo != 0;  // nobody reads the kinetic sums otherwise
+    const bool walls = e->walls != 0;
     // consecutive groups to consecutive blocks: a small system's warps spread over the SMs, whose FP64
     // units they would otherwise share
     const int stride = nblk * blockDim.x;
@@ -260,7 +263,7 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
             x0x = __ldcs(a.x0 + i);
             x0y = __ldcs(a.x0 + n + i);
             x0z = __ldcs(a.x0 + 2 * n + i);
-            const bool live = force_live(flags, i);
+            const bool live = force_live(flags, i) || (walls && force_live(wflags, i));
             kick = live || kick_all;
             if (kick) {
                 double4 w = ld4(a.om, i);
@@ -352,8 +355,9 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
 // runs in 19.7 instead of 22.5 us, the dilute 1M one in 33.4 instead of 34.9.
 __global__ void __launch_bounds__(kBlockA, 3) k_a64(tmps_atoms a, const tmps_box* __restrict__ b,
                                                   tmps_engine* __restrict__ e, const uint32_t* __restrict__ flags,
-                                                  double* __restrict__ kin, double* __restrict__ part) {
-    a64_body(a, b, e, flags, kin, part, blockIdx.x, gridDim.x);
+                                                  const uint32_t* __restrict__ wflags, double* __restrict__ kin,
+                                                  double* __restrict__ part) {
+    a64_body(a, b, e, flags, wflags, kin, part, blockIdx.x, gridDim.x);
 }
 
 // ------------------------------------------------------------------ A, mixed
@@ -542,7 +546,8 @@ __device__ __forceinline__ void zero_force(const tmps_atoms& A, int i) {
 // its force may be nonzero.
 __global__ void __launch_bounds__(kBlockA) k_bounds(tmps_atoms A, tmps_nlist L, const tmps_box* __restrict__ B,
                                                      tmps_engine* __restrict__ E, int hist, int cull, uint32_t* flags,
-                                                     float* gap, float* agap, double* __restrict__ kin) {
+                                                     float* gap, float* agap, double* __restrict__ kin,
+                                                     uint32_t* __restrict__ wflags) {
     const int n = A.n;
     const int lane = threadIdx.x & 31;
     const int ngroups = (n + 31) >> 5;
@@ -612,6 +617,7 @@ __global__ void __launch_bounds__(kBlockA) k_bounds(tmps_atoms A, tmps_nlist L, 
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) gmin = fminf(gmin, __shfl_down_sync(0xffffffffu, gmin, o));
         if (lane == 0) {
+            wflags[g] = 0u;                // (flags, below, has every atom's force)
             kin[8 * (size_t)g + 6] = 0.0;  // no kept kinetic sum (a64_body)
             gap[g] = gmin;
             // bits of existing atoms only: a set bit makes C clear that atom's force
@@ -2239,6 +2245,91 @@ __global__ void __launch_bounds__(kBlockG, MIXED ? 4 : 3)
     }
 }
 
+// ------------------------------------------------------------------- walls
+
+struct WallList {
+    int count;
+    tmps_fused_wall w[TMPS_MAX_FUSED_WALLS];
+};
+
+// The walls of a step, after C, FP64.  An atom's flag bit of C says whether C
+// has written its force in this step; the walls add to it or write it, and
+// keep bits of their own (wflags), which A takes together with C's: C's
+// bookkeeping sees pair forces alone.
+//
+// What bounds it is latency (a root of the distance per atom near the wall and
+// the law's chain, ~64 cycles an FP64 instruction): everything but the forces
+// themselves needs A's state alone, which is complete once C has passed its
+// wait, so it runs beside C, before this kernel's own wait; an atom clear of a
+// wall takes no root (wall_clear) and writes nothing.  Small blocks spread the
+// warps over the SMs' FP64 units.  3,001 spheres in a cylinder: 30 us a
+// step with the walls in the fused step, 85 us hook by hook.
+constexpr int kBlockW = 32;
+__global__ void __launch_bounds__(kBlockW) k_walls(tmps_atoms A, const tmps_engine* __restrict__ E,
+                                                   const uint32_t* __restrict__ flags, uint32_t* __restrict__ wflags,
+                                                   const __grid_constant__ WallList L) {
+    const int lane = threadIdx.x & 31, n = A.n;
+    const int i = blockIdx.x * kBlockW + threadIdx.x;
+    const int64_t s = E->attempt;
+    const bool run = s != 0 && !rebuild_due(E, s);
+    const bool mine = run && i < n;
+    const uint32_t old = run ? wflags[i >> 5] : 0u;
+    bool any = false;
+    double F[3] = {0, 0, 0}, T[3] = {0, 0, 0};
+    if (mine) {
+        const double dt = E->dt;
+        const double4 xr = ld4(A.xr, i), vm = ld4(A.vm, i), om = ld4(A.om, i);
+        const int u = A.uid ? A.uid[i] : i;
+        const double x[3] = {xr.x, xr.y, xr.z}, v[3] = {vm.x, vm.y, vm.z}, w[3] = {om.x, om.y, om.z};
+        for (int k = 0; k < L.count; ++k) {
+            const tmps_fused_wall& W = L.w[k];
+            const size_t ns = (size_t)W.nslots;
+            int touch = W.p.history ? W.touch[u] : 0;
+            const int was = touch;
+            bool contact = false;
+            if (!tmps_wall_law::wall_clear(W.p, x, xr.w)) {
+                double sh[3] = {0, 0, 0}, f[3] = {0, 0, 0}, t[3] = {0, 0, 0};
+                if (was) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) sh[c] = W.shear[c * ns + u];
+                }
+                contact = tmps_wall_law::wall_force(W.p, dt, W.history_update, x, xr.w, v, vm.w, w, sh, touch, f, t);
+                if (contact) {
+                    any = true;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        F[c] += f[c];
+                        T[c] += t[c];
+                        if (W.p.history) W.shear[c * ns + u] = sh[c];
+                    }
+                }
+            }
+            if (W.p.history) {
+                if (!contact && was) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) W.shear[c * ns + u] = 0.0;
+                }
+                touch = contact ? touch : 0;
+                if (touch != was) W.touch[u] = touch;
+            }
+        }
+    }
+    pdl_enter();
+    if (!run) return;
+    if (mine) {
+        const bool pair = force_live(flags, i), stale = !any && !pair && ((old >> lane) & 1u);
+        if (any || stale) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                A.f[(size_t)c * n + i] = pair ? A.f[(size_t)c * n + i] + F[c] : F[c];
+                A.torque[(size_t)c * n + i] = pair ? A.torque[(size_t)c * n + i] + T[c] : T[c];
+            }
+        }
+    }
+    const uint32_t now = __ballot_sync(0xffffffffu, any);
+    if (lane == 0 && now != old) wflags[i >> 5] = now;
+}
+
 // ---------------------------------------------------------------------- S
 
 __device__ double limit_rate_f(double rate, double ptarget, double iptarget, int normalize, double max_rate) {
@@ -2626,7 +2717,7 @@ __global__ void __launch_bounds__(kBlockA) kb_a64(const tmps_instance* __restric
     const tmps_instance& I = stage_instance(si, inst, block_inst[blockIdx.x]);
     char* sc = static_cast<char*>(I.scratch);
     a64_body(I.a, I.box, I.eng, reinterpret_cast<const uint32_t*>(sc),
-             reinterpret_cast<double*>(sc + lay_kin(I.a.n)), reinterpret_cast<double*>(sc + lay_part(I.a.n)),
+             reinterpret_cast<const uint32_t*>(sc + lay_wall(I.a.n)), reinterpret_cast<double*>(sc + lay_kin(I.a.n)), reinterpret_cast<double*>(sc + lay_part(I.a.n)),
              (int)blockIdx.x - I.a_first, I.a_blocks);
 }
 
@@ -3075,6 +3166,7 @@ int tmps_fused_a(const tmps_atoms* a, tmps_box* d_box, tmps_engine* d_eng, int32
         launch_pdl(k_a32, g, kBlockA, s, *a, (const tmps_box*)d_box, d_eng, flags, part);
     } else {
         launch_pdl(k_a64, g, kBlockA, s, *a, (const tmps_box*)d_box, d_eng, flags,
+                   (const uint32_t*)((char*)scratch + lay_wall(n)),
                    (double*)((char*)scratch + lay_kin(n)), part);
     }
     note_launches(1);
@@ -3181,6 +3273,27 @@ int tmps_fused_c_pairs(const tmps_atoms* a, const tmps_nlist* nl, const tmps_box
     return launch_ok() ? TMPS_OK : TMPS_ERR_CUDA;
 }
 
+int tmps_fused_walls(const tmps_atoms* a, const tmps_engine* d_eng, const tmps_fused_wall* walls, int32_t count,
+                     void* scratch, void* stream) {
+    if (!a || !d_eng || !walls || !scratch || a->n < 0 || count < 1 || count > TMPS_MAX_FUSED_WALLS || a->pos32)
+        return TMPS_ERR_BAD_ARG;
+    WallList L = {};
+    L.count = count;
+    for (int k = 0; k < count; ++k) {
+        const tmps_wall_params& p = walls[k].p;
+        if (p.kind < 0 || p.kind > 1 || p.axis < 0 || p.axis > 2 || (p.side != -1 && p.side != 1) ||
+            (p.kind == 0 && (p.shear_axis < -1 || p.shear_axis > 2 || p.shear_axis == p.axis)) ||
+            (p.history && (!walls[k].shear || !walls[k].touch || walls[k].nslots < a->n)))
+            return TMPS_ERR_BAD_ARG;
+        L.w[k] = walls[k];
+    }
+    if (a->n == 0) return TMPS_OK;
+    launch_pdl(k_walls, grid_for(a->n, kBlockW), kBlockW, (cudaStream_t)stream, *a, d_eng, (const uint32_t*)scratch,
+               (uint32_t*)((char*)scratch + lay_wall(a->n)), L);
+    note_launches(1);
+    return launch_ok() ? TMPS_OK : TMPS_ERR_CUDA;
+}
+
 int tmps_fused_servo(tmps_box* d_box, tmps_servo* d_servo, tmps_engine* d_eng, const void* scratch,
                      int32_t* d_status, void* stream) {
     if (!d_box || !d_servo || !d_eng || !scratch || !d_status) return TMPS_ERR_BAD_ARG;
@@ -3201,7 +3314,7 @@ int tmps_fused_bounds(const tmps_atoms* a, const tmps_nlist* nl, const tmps_box*
     const int g = n > 0 ? grid_for(n, kBlockA) : 1;
     cudaStream_t st = (cudaStream_t)stream;
     k_bounds<<<g, kBlockA, 0, st>>>(*a, *nl, d_box, d_eng, has_history(p) ? 1 : 0, cull ? 1 : 0, flags, gap, agap,
-                                  (double*)((char*)scratch + lay_kin(n)));
+                                  (double*)((char*)scratch + lay_kin(n)), (uint32_t*)((char*)scratch + lay_wall(n)));
     note_launches(1);
     if (cull && n > 0) {
         // the groups in ascending gap order (C's ordered pass)

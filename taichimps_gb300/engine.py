@@ -3,8 +3,10 @@ The fused step engine behind ``Simulation.run``.
 
 One step of Simulation._sub_step_inner (simulation.py:205-247) with fix
 nve/sphere, optionally damping/cundall and deform/pressure, becomes three
-kernels (tmps_fused_a, tmps_fused_c, tmps_fused_servo) that decide on the
-device whether the step needs a neighbor rebuild.  Steps are queued in
+kernels (tmps_fused_a, tmps_fused_c, tmps_fused_servo; two where no servo runs)
+that decide on the device whether the step needs a neighbor rebuild; in the
+FP64 form without a servo, fixed granular walls add a kernel after the contacts
+(tmps_fused_walls).  Steps are queued in
 chunks (replayed as CUDA graphs) with one host synchronisation per chunk.
 When a step finds it needs a rebuild, every later launch of the chunk does
 nothing; the host then rebuilds exactly as the reference does at that step
@@ -33,13 +35,26 @@ import torch
 from . import _device, _lib
 from .EXTRA_FIX.damping_cundall import FixDampingCundall
 from .EXTRA_FIX.deform_pressure import FixDeformPressure
+from .EXTRA_FIX.wall_gran import FixWallGran
+from .EXTRA_FIX.wall_gran_region import FixWallGranRegion
 
 
-def fusable(sim) -> bool:
-    """The configurations the fused step covers."""
+def fusable(sim, walls: bool = False) -> bool:
+    """The configurations the fused step covers.  `walls`: granular walls too, where they stand still,
+    follow any damping in the list of fixes (their force is not damped) and no servo reads the virial;
+    up to the number one kernel takes."""
     if sim.integrator is None or sim.pair_style is None or sim.neighbor is None or sim.history is None:
         return False
     kinds = [type(f) for f in sim.fixes]
+    on_walls = [i for i, k in enumerate(kinds) if k in (FixWallGran, FixWallGranRegion)] if walls else []
+    if on_walls:
+        if len(on_walls) > _lib.MAX_FUSED_WALLS or FixDeformPressure in kinds:
+            return False
+        if FixDampingCundall in kinds[on_walls[0]:]:
+            return False
+        if any(getattr(sim.fixes[i], "wiggle_amplitude", 0.0) != 0.0 for i in on_walls):
+            return False
+        kinds = [k for i, k in enumerate(kinds) if i not in on_walls]
     if any(k not in (FixDampingCundall, FixDeformPressure) for k in kinds):
         return False
     if kinds.count(FixDampingCundall) > 1 or kinds.count(FixDeformPressure) > 1:
@@ -74,6 +89,7 @@ class FusedEngine:
         self.dev = _device.device()
         self.cundall = next((f for f in sim.fixes if isinstance(f, FixDampingCundall)), None)
         self.deform = next((f for f in sim.fixes if isinstance(f, FixDeformPressure)), None)
+        self.walls = [f for f in sim.fixes if type(f) in (FixWallGran, FixWallGranRegion)]
         self._eng = _device.struct_buffer(_lib.Engine())
         self.status = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self._dummy_servo = _device.struct_buffer(_lib.Servo())
@@ -208,7 +224,7 @@ class FusedEngine:
             if np.any(g > 1023):
                 raise NotImplementedError("the mixed form packs cell coordinates in 10 bits (<= 1023 bins per axis)")
         e = _lib.Engine()
-        e.step = sim.timestep
+        e.step = self._begun = sim.timestep
         e.last_build_step = nl.last_build_step
         e.delay, e.every, e.check = int(nl.delay), max(1, int(nl.every)), 1 if nl.check else 0
         e.cundall = 1 if self.cundall is not None else 0
@@ -216,6 +232,12 @@ class FusedEngine:
         # without a servo the contact kernel itself ends the step (two launches a step, not three)
         self.fold = self.deform is None and n > 0
         e.fold = 1 if self.fold else 0
+        e.walls = 1 if self.walls else 0
+        self._wall_args = (_lib.FusedWall * len(self.walls))() if self.walls else None
+        for k, f in enumerate(self.walls):
+            f.ready(atom)
+            self._wall_args[k] = _lib.FusedWall(f.params(), f.shear.data_ptr(), f.touch.data_ptr(), f.max_atoms,
+                                                1 if f.history_update else 0)
         e.mixed = 1 if self.mixed else 0
         e.nblocks, e.ablocks = self.nblocks, self.a_blocks
         e.dt = float(sim.dt)
@@ -337,6 +359,10 @@ class FusedEngine:
         else:
             _lib.check(L.tmps_fused_c(atoms, nl_struct, dbox, eng, params, self.c_blocks, part, 0, st),
                        "tmps_fused_c")
+        if self.walls:
+            with _device.timed("wall"):
+                rc = L.tmps_fused_walls(atoms, eng, self._wall_args, len(self.walls), part, st)
+            _lib.check(rc, "tmps_fused_walls")
 
     def instance(self, a_first: int, a_blocks: int, c_first: int, c_blocks: int) -> _lib.Instance:
         """This system's descriptor for a batched run (tmps_instance)."""
@@ -433,7 +459,8 @@ class FusedEngine:
             self._graph, self._graph_key = _device.capture_graph(chunk), key
         self._graph.replay()
         self.graph_replays += 1
-        self.graph_kernel_launches += self.chunk * (self.LAUNCHES_PER_STEP + (1 if self.rows else 0) - (1 if self.fold else 0))
+        self.graph_kernel_launches += self.chunk * (self.LAUNCHES_PER_STEP + (1 if self.rows else 0) - (1 if self.fold else 0)
+                                                    + (1 if self.walls else 0))
 
     def cull_stats(self) -> tuple[int, int]:
         """(32-atom groups, groups the contact bound rules out right now), from the
@@ -524,6 +551,9 @@ class FusedEngine:
         got = _device.pull_many(items)
         e, status, box = got[0], int(got[1].view(np.int32)[0]), got[2]
         sim.domain.take_pulled(box)
+        for f in self.walls:
+            f.passed(int(e.step) - self._begun, float(sim.dt))
+        self._begun = int(e.step)
         sim.timestep = int(e.step)
         sim.neighbor.current_step = int(e.step)
         sim.neighbor.last_build_step = int(e.last_build_step)

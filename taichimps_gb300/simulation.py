@@ -199,7 +199,7 @@ class Simulation:
             seg = remaining
             if self.restart_every > 0:
                 seg = min(seg, self.restart_every - self.timestep % self.restart_every)
-            if self.fused and seg > 0 and fusable(self) and self.atom.nlocal > 0:
+            if self.fused and seg > 0 and fusable(self, walls=self.precision == "fp64") and self.atom.nlocal > 0:
                 eng = FusedEngine(self, self.precision)
                 self.last_engine = eng
                 eng.begin()
