@@ -156,21 +156,22 @@ def list_stats(sim):
 def algorithmic_bytes(kernel: str, precision: str, n_nb: float, n_c: float, flagged: float) -> float:
     """Bytes per atom a launch must move through HBM.
 
-    fused_a (A), every atom: the Verlet stream of the step plus the skin check's reference words.
-      mixed: reads and writes the position, velocity and angular velocity (high and low FP32 words,
-             72 + 72), reads m (kinetic term, 4), the offset at the last build (12) and the packed cell
-             (4)                                                                                  = 164
-             plus per flagged atom (`flagged` = fraction) the force and torque and 1/m, 1/I: 32
-      FP64:  reads x, v, omega (72), x at the last build (24); writes x, v, omega (72)      = 168
-             plus per flagged atom the force and torque and 1/m, 1/I: 64
-      A's records also carry per-build constants in their fourth lanes for C's gathers (radius hi and
-      lo, m), which it reads and writes with them (layout_bytes: 184 mixed / 216 FP64 per atom); those
+    fused_a (A), every atom: the position's Verlet stream plus the skin check's reference words.
+      mixed: reads and writes the position (high and low FP32 words, 24 + 24), reads the velocity (24),
+             m (kinetic term, 4), the offset at the last build (12) and the packed cell (4)       =  92
+             plus per flagged atom (`flagged` = fraction) the angular velocity, force, torque, 1/m and
+             1/I read (24 + 24 + 8) and both velocities written (48): 104
+      FP64:  reads x, v (48), x at the last build (24); writes x (24)                       =  96
+             plus per flagged atom omega, force, torque, 1/m and 1/I read (24 + 48 + 16) and v, omega
+             written (48): 136
+      A's records also carry per-build constants and padding in their fourth lanes for C's gathers,
+      which move with them (layout_bytes: 112 + 104 mixed / 122 + 160 FP64 per flagged atom); those
       are not counted here.
     fused_c (C): the contact kernel's per-atom bytes, S + 4 n_nb + 52 n_c (own state read once and
       force written once, S = 84 mixed / 140 FP64; 4 per neighbor index; 4 partner + 48 shear per
       touching slot)."""
     if kernel == "fused_a":
-        return (164.0 + 32.0 * flagged) if precision == "mixed" else (168.0 + 64.0 * flagged)
+        return (92.0 + 104.0 * flagged) if precision == "mixed" else (96.0 + 136.0 * flagged)
     if kernel == "fused_c":
         return (84.0 if precision == "mixed" else 140.0) + 4.0 * n_nb + 52.0 * n_c
     return 0.0
@@ -179,7 +180,7 @@ def algorithmic_bytes(kernel: str, precision: str, n_nb: float, n_c: float, flag
 def layout_bytes(kernel: str, precision: str, flagged: float) -> float:
     """Bytes per atom A's record layout makes it read and write (see algorithmic_bytes)."""
     if kernel == "fused_a":
-        return (184.0 + 32.0 * flagged) if precision == "mixed" else (216.0 + 64.0 * flagged)
+        return (112.0 + 104.0 * flagged) if precision == "mixed" else (122.0 + 160.0 * flagged)
     return 0.0
 
 
