@@ -66,7 +66,7 @@ def fusable(sim, walls: bool = False) -> bool:
 
 
 class FusedEngine:
-    # kernels per step: A, C, S (C is two launches on the rows path)
+    # kernels per step: A, C, S (C is two launches on the pair path; walls add one, no servo takes S off)
     LAUNCHES_PER_STEP = 3
     MAX_PAIRS = 2**31 - 64  # pair indices carry one more bit
 
