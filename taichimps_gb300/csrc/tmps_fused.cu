@@ -2762,7 +2762,7 @@ __global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
 // S of a batch: one block of six warps per instance (the derived quantities
 // take one warp per kind, the virial sum runs the 24 virtual warps of the
 // single-instance S four at a time), so many instances fit in one wave.
-constexpr int kBlockSB = 384;
+constexpr int kBlockSB = 192;
 __global__ void __launch_bounds__(kBlockSB) kb_s(const tmps_instance* __restrict__ inst, int32_t* status) {
     const tmps_instance& I = inst[blockIdx.x];
     s_body<kBlockSB / 32>(I.box, I.servo, I.eng, static_cast<const char*>(I.scratch), status);
