@@ -95,6 +95,7 @@ class FusedEngine:
         self._dummy_servo = _device.struct_buffer(_lib.Servo())
         self._n = -1
         self.rebuilds = 0
+        self._interval = self.chunk  # steps between the last two builds
         # A chunk of `chunk` steps is captured once as a CUDA graph and replayed;
         # a rebuild swaps buffers, so the graph is captured again after one.
         self.graphs = bool(graphs)
@@ -419,6 +420,11 @@ class FusedEngine:
                 self._known = (e, status)
                 break
             count = min(self.chunk, target - done)
+            if self._interval < self.chunk:
+                # rebuilds come sooner than a chunk ends, and every launch queued past one is idle work: as
+                # many steps as the last interval held and an eighth more, then half of what has passed
+                since, held = done - int(e.last_build_step), self._interval + self._interval // 8 + 1
+                count = min(count, held - since if since < held else max(4, since // 2))
             if self.graphs and count == self.chunk and _device.TIMED is None:
                 self._replay_chunk(L)
             else:
@@ -516,6 +522,7 @@ class FusedEngine:
         e = self._engine_state()
         e.aborted = 0
         e.disp_stamp = 0
+        self._interval = s - int(e.last_build_step)
         e.last_build_step = s
         _device.push_struct(self._eng, e)
         if atom.nlocal != self._n:

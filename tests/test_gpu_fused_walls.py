@@ -44,12 +44,15 @@ def _sim(n, kind, fused, cundall=False, first=True, precision="fp64", extra=()):
     return sim, walls
 
 
-@pytest.mark.parametrize("n,kind,cundall", [(1, "planes", False), (31, "tube", False), (32, "planes", True), (33, "post", False),
-                                            (129, "hertz", True), (512, "planes", True), (511, "tube", False)])
-def test_fused_walls_match_hooks(gpu, n, kind, cundall):
+@pytest.mark.parametrize("n,kind,cundall,path", [
+    (1, "planes", False, "auto"), (31, "tube", False, "auto"), (32, "planes", True, "auto"), (33, "post", False, "auto"),
+    (129, "hertz", True, "auto"), (512, "planes", True, "auto"), (511, "tube", False, "auto"), (511, "planes", True, "rows"),
+    (257, "tube", False, "screened")])
+def test_fused_walls_match_hooks(gpu, n, kind, cundall, path):
     out = []
     for fused in (True, False):
         sim, walls = _sim(n, kind, fused, cundall)
+        sim.contact_path = path
         sim.run(90)
         sim.run_pre = False
         sim.run(70)
