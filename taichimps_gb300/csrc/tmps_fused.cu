@@ -482,8 +482,9 @@ __device__ __forceinline__ void a32_body(const tmps_atoms& a, const tmps_box* __
     }
 }
 
-// Three resident blocks per SM (80 registers, no spill): measured 2-3 % faster
-// in the step than four at 64 registers, which spilled.
+// Three resident blocks per SM (80 registers): at four (64 registers, no spill)
+// the step of 1M spheres is 1.5 % faster contact-free and 0.3 % slower jammed, at
+// five (spills) 15 % slower.
 __global__ void __launch_bounds__(kBlockA, 3) k_a32(tmps_atoms a, const tmps_box* __restrict__ b,
                                                      tmps_engine* __restrict__ e, const uint32_t* __restrict__ flags,
                                                      double* __restrict__ part) {
@@ -2562,7 +2563,9 @@ __device__ __forceinline__ void copy_words(S* dst, const S* src) {
 // fourth run of 32 blocks (coalesced, the loads of a lane in flight together),
 // in block order, then a shuffle tree and the four warp sums in order.  The
 // mixed form's partials are double words and are summed as such; only the six
-// totals become FP64.
+// totals become FP64.  Staging and reciprocals beside C: a mixed step of 1M
+// spheres 34.2 -> 31.6 us.  A smaller block, so that it fits beside C's wave,
+// sums in more turns after the wait: 33.1 us with 8 warps, 32.5 with 12.
 constexpr int kWarpsS = kBlockS / 32;
 static_assert(kWarpsS == 24, "four warps per virial component");
 constexpr int kPartLoads = 10;  // per lane: up to 32 * 4 * 10 = 1280 partial blocks in one round

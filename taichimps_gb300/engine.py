@@ -107,7 +107,7 @@ class FusedEngine:
         # contact once and sums every atom's row from the pairs' records.  "auto" picks rows at a build
         # where more than half of the atoms touch or overlap at the build positions (their gap bound is
         # <= 0): there the screen rules out little and half of the contact arithmetic is saved (jammed
-        # packings, C per step: 1M spheres mixed 278 -> 193 us, 109k FP64 363 -> 177 us); on dilute
+        # packings, C per step: 1M spheres mixed 278 -> 191 us, 109k FP64 363 -> 150 us); on dilute
         # states the screen reads a few bytes per group where rows would read every list entry.  Both
         # paths sum each atom's contacts in slot order with the same per-contact code; only the order of
         # the virial sums differs.
