@@ -20,8 +20,8 @@
 // What bounds these kernels: the FP64 pipe (one instruction of a warp every 16
 // cycles per SM, 64 cycles to its result) and, below a few ten thousand
 // spheres, the chain of such results.  Hence small blocks (two warps), so that
-// a few thousand atoms already reach every SM; reciprocals by rcp64 instead of
-// divisions; pairs out of contact dropped before the law, so that its warps run
+// a few thousand atoms already reach every SM; quotients and roots by the short
+// forms of tmps_common.cuh; pairs out of contact dropped before the law, so that its warps run
 // full; and few launches, queued by one call for a run of steps with no host
 // synchronisation in between: a step whose displacement check fires marks the
 // run and every later launch of it does nothing.
@@ -35,6 +35,7 @@ namespace {
 
 constexpr int kBlk = 64;       // threads of the per-atom and per-pair kernels
 constexpr int kPairTile = 128;  // pairs a block of the contact passes takes
+constexpr int kSum = 256;       // atoms or pairs the forward's sums join first (see sum_groups)
 constexpr int kOne = 512;      // threads of the one-block kernels
 constexpr int kNG = 16;        // doubles per pair in the reverse's per-pair record
 
@@ -44,15 +45,19 @@ struct Work {
     double* fp;     // [3][P] pair force on a
     double* tp;     // [3][P] pair torque term (d x fs) / r
     double* gp;     // [16][P] per-pair adjoints for the gather
-    double* partw;  // [6][nbP] pair virial partials
-    double* partk;  // [6][nbA] kinetic / remap partials
+    double* partw;  // [6][2 groups of kSum pairs] pair virial partials
+    double* partk;  // [6][4 groups of kSum atoms] kinetic partials; [6][nbA] remap partials
     double* partg;  // [8][nbP] parameter and image partials of the reverse
     double* wbar;   // [6] dL/d(virial total) of the current reverse step: at the base, where the calls of
                     // a linked run find it whatever their numbers of pairs
 };
 
+// Blocks of the forward's per-atom and per-pair passes: whole groups of kSum.
+int blocks_a(int n) { return kSum / kBlk * grid_for(n, kSum); }
+int blocks_p(int npairs) { return kSum / kPairTile * grid_for(npairs, kSum); }
+
 Work carve(void* base, int n, int npairs) {
-    const int nbA = grid_for(n, kBlk), nbP = grid_for(npairs, kPairTile);
+    const int nbA = blocks_a(n), nbP = blocks_p(npairs);
     char* p = static_cast<char*>(base);
     Work w;
     w.wbar = reinterpret_cast<double*>(p); p += align256(sizeof(double) * 8);
@@ -66,7 +71,7 @@ Work carve(void* base, int n, int npairs) {
 }
 
 size_t work_bytes(int n, int npairs) {
-    const int nbA = grid_for(n, kBlk), nbP = grid_for(npairs, kPairTile);
+    const int nbA = blocks_a(n), nbP = blocks_p(npairs);
     return align256(sizeof(double) * 3 * (size_t)npairs) * 2 + align256(sizeof(double) * kNG * (size_t)npairs) +
            align256(sizeof(double) * 6 * (size_t)nbP) + align256(sizeof(double) * 6 * (size_t)nbA) +
            align256(sizeof(double) * 8 * (size_t)nbP) + align256(sizeof(double) * 8);
@@ -81,6 +86,7 @@ Params to_params(const tmps_adj_params& p) {
     q.xmu = p.xmu;
     q.dt = p.dt;
     q.limit_damping = p.limit_damping;
+    q.ikt = 1.0 / p.kt;
     return q;
 }
 
@@ -122,6 +128,39 @@ __device__ void sum_partials(const double* part, int nb, double* out, int first)
     if (lane == 0) out[c] = t;
 }
 
+// The forward's virial: the servo feeds a pressure's last bits back into every
+// position, and the radius adjoints of barely touching pairs show those, so the
+// sums keep one order whatever the kernels' blocks are: a tree over each 32
+// consecutive atoms or pairs, a tree over the eight of a group of kSum, the
+// groups a lane stride apart one after another, a tree over the lanes.  A block
+// of the passes takes those warps of a group that its tree joins first and
+// writes their sum; PER consecutive sums here make a group (PER - 1 additions).
+// One warp per component (warps first, first + 1, ...).
+template <int PER>
+__device__ void sum_groups(const double* part, int ng, double* out, int first) {
+    const int c = (threadIdx.x >> 5) - first, lane = threadIdx.x & 31;
+    if (c < 0 || c >= 6) return;
+    const double2* row = reinterpret_cast<const double2*>(part + (size_t)c * PER * ng);
+    double t = 0.0;
+    for (int k0 = lane; k0 < ng; k0 += 128) {
+        double2 v[4][PER / 2];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int h = 0; h < PER / 2; ++h)
+                v[u][h] = k0 + 32 * u < ng ? row[(size_t)(k0 + 32 * u) * (PER / 2) + h] : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            double g = v[u][0].x + v[u][0].y;
+            if constexpr (PER == 4) g += v[u][1].x + v[u][1].y;
+            t += g;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (lane == 0) out[c] = t;
+}
+
 // Programmatic dependent launch: wait for the kernel before to complete, then
 // let the next one be scheduled.  Every kernel of this file does both in this
 // order, so when a block starts, all but the kernel right before it have
@@ -140,14 +179,6 @@ struct Queue {
     int64_t hit, done;
 };
 __device__ __forceinline__ bool halted(const Queue* q) { return q && *(volatile const int64_t*)&q->hit != 0; }
-
-// x / prd with the box's reciprocal at hand: the product corrected by its
-// residual, correctly rounded but for rare last bits (a position must not
-// move by one: the overlaps cancel its leading digits).
-__device__ __forceinline__ double over(double x, double prd, double iprd) {
-    const double q = __dmul_rn(x, iprd);
-    return __fma_rn(__fma_rn(-q, prd, x), iprd, q);
-}
 
 // ------------------------------------------------------------------ pairs
 
@@ -368,13 +399,13 @@ __global__ void __launch_bounds__(kBlk) k_initial(tmps_adj_sys S, double dt, tmp
     double v[3] = {0, 0, 0}, w[3] = {0, 0, 0}, x0[3] = {0, 0, 0}, xb[3] = {0, 0, 0};
     if (mine) {
         const double dtf = 0.5 * dt;
-        const double m = S.mass[i], r = S.radius[i], im = rcp64(m), iI = rcp64(inertia(m, r));
+        const double m = S.mass[i], r = S.radius[i], I = inertia(m, r);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const size_t k = (size_t)c * n + i;
-            v[c] = S.v[k] + dtf * (S.f[k] * im);
-            w[c] = S.w[k] + dtf * (S.t[k] * iI);
-            if (before) x0[c] = over(xlast[k] - before->lo[c], before->prd[c], rcp64(before->prd[c]));
+            v[c] = S.v[k] + dtf * quot64(S.f[k], m);
+            w[c] = S.w[k] + dtf * quot64(S.t[k], I);
+            if (before) x0[c] = quot64(xlast[k] - before->lo[c], before->prd[c]);
             xb[c] = xbuild[k];
         }
     }
@@ -455,12 +486,14 @@ __device__ __forceinline__ int pack_tile(const bool (&in)[kPairTile / kBlk], int
 // Contacts of one pass: pair forces and torque terms into the workspace,
 // history updated in place (the entering history recorded), virial partials.
 // The tile's distances first; pairs out of contact are finished with zeros,
-// the law runs over the rest with full warps.
+// the law runs over the rest with full warps.  The tile of block 2 g + h is
+// warps h, h + 2, h + 4, h + 6 of group g (sum_groups): its threads' first
+// round h and h + 4, their second h + 2 and h + 6.
 __global__ void __launch_bounds__(kBlk) k_pairs(tmps_adj_sys S, Params P, int shearupdate, const double* xs,
                                                 const double* vs, const double* ws, const tmps_adj_rec* __restrict__ box,
                                                 double* __restrict__ sh_rec, uint8_t* __restrict__ mask_rec, Work W,
                                                 const Queue* q) {
-    __shared__ double smem[6 * (kBlk / 32)];
+    __shared__ double svir[6][kPairTile], smem[6][kPairTile / 32];
     __shared__ int list[kPairTile], count[kPairTile / 32];
     const int n = S.n, np = S.npairs;
     double prd[3], iprd[3], nimg[3];
@@ -469,23 +502,27 @@ __global__ void __launch_bounds__(kBlk) k_pairs(tmps_adj_sys S, Params P, int sh
         prd[c] = box->prd[c];
         iprd[c] = rcp64(prd[c]);
     }
+    // the pair of the tile's entry e = 64 round + thread
+    const int group = (int)(blockIdx.x >> 1) * kSum, h = blockIdx.x & 1;
+    auto pair_at = [&](int e) { return group + 32 * (h + 2 * (e >> 6) + 4 * ((e >> 5) & 1)) + (e & 31); };
     int pi[kPairTile / kBlk], pj[kPairTile / kBlk];
     double radsum_[kPairTile / kBlk];
 #pragma unroll
     for (int u = 0; u < kPairTile / kBlk; ++u) {
-        const int p = blockIdx.x * kPairTile + u * kBlk + threadIdx.x;
+        const int p = pair_at(u * kBlk + threadIdx.x);
         pi[u] = p < np ? S.pi[p] : 0;
         pj[u] = p < np ? S.pj[p] : 0;
         radsum_[u] = S.radius[pi[u]] + S.radius[pj[u]];
     }
     enter();
     if (halted(q)) return;
-    double vir[6] = {0, 0, 0, 0, 0, 0};
     bool in_[kPairTile / kBlk];
 #pragma unroll
     for (int u = 0; u < kPairTile / kBlk; ++u) {
-        const int p = blockIdx.x * kPairTile + u * kBlk + threadIdx.x;
+        const int p = pair_at(u * kBlk + threadIdx.x);
         in_[u] = false;
+#pragma unroll
+        for (int c = 0; c < 6; ++c) svir[c][u * kBlk + threadIdx.x] = 0.0;
         if (p < np) {
             const int i = pi[u], j = pj[u];
             double d[3];
@@ -507,7 +544,7 @@ __global__ void __launch_bounds__(kBlk) k_pairs(tmps_adj_sys S, Params P, int sh
     }
     const int total = pack_tile(in_, list, count);
     for (int k = threadIdx.x; k < total; k += kBlk) {
-        const int p = blockIdx.x * kPairTile + list[k];
+        const int p = pair_at(list[k]);
         PairIn in;
         load_pair(S, xs, vs, ws, prd, iprd, p, S.pi[p], S.pj[p], in, nimg);
 #pragma unroll
@@ -526,29 +563,45 @@ __global__ void __launch_bounds__(kBlk) k_pairs(tmps_adj_sys S, Params P, int sh
             W.fp[(size_t)c * np + p] = o.F[c];
             W.tp[(size_t)c * np + p] = o.tor[c];
         }
-        vir[0] += in.d[0] * o.F[0];
-        vir[1] += in.d[1] * o.F[1];
-        vir[2] += in.d[2] * o.F[2];
-        vir[3] += in.d[0] * o.F[1];
-        vir[4] += in.d[0] * o.F[2];
-        vir[5] += in.d[1] * o.F[2];
+        const int e = list[k];
+        svir[0][e] = in.d[0] * o.F[0];
+        svir[1][e] = in.d[1] * o.F[1];
+        svir[2][e] = in.d[2] * o.F[2];
+        svir[3][e] = in.d[0] * o.F[1];
+        svir[4][e] = in.d[0] * o.F[2];
+        svir[5][e] = in.d[1] * o.F[2];
     }
-    const double tot = block_sum6_halving<kBlk>(vir, 0.0, true, smem);
-    if (threadIdx.x < 6) W.partw[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = tot;
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kPairTile / kBlk; ++u) {
+        const int e = u * kBlk + threadIdx.x;
+        const double v[6] = {svir[0][e], svir[1][e], svir[2][e], svir[3][e], svir[4][e], svir[5][e]};
+        const double t = warp_sum6_halving(v);  // lane >> 2 is the component
+        const int c = (threadIdx.x & 31) >> 2;
+        if ((threadIdx.x & 3) == 0 && c < 6) smem[c][e >> 5] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        const double* w = smem[threadIdx.x];
+        W.partw[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = (w[0] + w[1]) + (w[2] + w[3]);
+    }
 }
 
 // Per-atom force and torque from the pairs in contact (as i: +F, then as j:
 // -F; the torque term times -r either way), then the second half-kick (final =
-// 1) and the kinetic partials m v v.
+// 1) and the kinetic partials m v v.  Blocks 4 g .. 4 g + 3 take warps 0 and 4,
+// 2 and 6, 1 and 5, 3 and 7 of group g (sum_groups).
 __global__ void __launch_bounds__(kBlk) k_gather(tmps_adj_sys S, double dt, int final_, const double* __restrict__ vh,
                                                  const double* __restrict__ wh, double* __restrict__ ft,
                                                  double* __restrict__ tt, const uint8_t* mask, Work W, const Queue* q) {
-    __shared__ double smem[6 * (kBlk / 32)];
+    __shared__ double smem[6][kBlk / 32];
     const int n = S.n, np = S.npairs;
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+    const int quarter = blockIdx.x & 3;
+    const int a = (int)(blockIdx.x >> 2) * kSum +
+                  32 * (((quarter & 1) << 1 | quarter >> 1) + 4 * (int)(threadIdx.x >> 5)) + (threadIdx.x & 31);
     double kin[6] = {0, 0, 0, 0, 0, 0};
     int i0 = 0, ni = 0, j0 = 0, nj = 0;
-    double ra = 0.0, m = 1.0, im = 1.0, iI = 1.0, vh0[3] = {0, 0, 0}, wh0[3] = {0, 0, 0};
+    double ra = 0.0, m = 1.0, I = 1.0, im = 1.0, iI = 1.0, vh0[3] = {0, 0, 0}, wh0[3] = {0, 0, 0};
     if (a < n) {
         i0 = S.ibeg[a];
         ni = S.ibeg[a + 1] - i0;
@@ -556,8 +609,9 @@ __global__ void __launch_bounds__(kBlk) k_gather(tmps_adj_sys S, double dt, int 
         nj = S.jbeg[a + 1] - j0;
         ra = S.radius[a];
         m = S.mass[a];
-        im = rcp64(m);
-        iI = rcp64(inertia(m, ra));
+        I = inertia(m, ra);
+        im = near_rcp64(m);  // for div_by
+        iI = near_rcp64(I);
         if (final_)
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
@@ -613,9 +667,9 @@ __global__ void __launch_bounds__(kBlk) k_gather(tmps_adj_sys S, double dt, int 
                 tt[k] = Tq[c];
             }
             if (final_) {
-                v[c] = vh0[c] + dtf * (F[c] * im);
+                v[c] = vh0[c] + dtf * div_by(F[c], m, im);
                 S.v[k] = v[c];
-                S.w[k] = wh0[c] + dtf * (Tq[c] * iI);
+                S.w[k] = wh0[c] + dtf * div_by(Tq[c], I, iI);
             }
         }
         if (final_) {
@@ -628,8 +682,12 @@ __global__ void __launch_bounds__(kBlk) k_gather(tmps_adj_sys S, double dt, int 
         }
     }
     if (!final_) return;
-    const double tot = block_sum6_halving<kBlk>(kin, 0.0, true, smem);
-    if (threadIdx.x < 6) W.partk[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = tot;
+    const double t = warp_sum6_halving(kin);  // lane >> 2 is the component
+    const int c = (threadIdx.x & 31) >> 2;
+    if ((threadIdx.x & 3) == 0 && c < 6) smem[c][threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x < 6)
+        W.partk[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = smem[threadIdx.x][0] + smem[threadIdx.x][1];
 }
 
 // The servo rate of a pressure axis: gain, normalize/pressure, max/rate
@@ -676,26 +734,26 @@ __device__ void coupled(int couple, const double* P, double* p) {
 
 // Virial total, pressure tensor, deviatoric stress, the servo's new box.
 __global__ void __launch_bounds__(kOne) k_servo(tmps_adj_servo sv, double dt, int64_t step, const tmps_adj_rec* prev,
-                                                tmps_adj_rec* next, int nbP, int nbA, Work W, Queue* q) {
+                                                tmps_adj_rec* next, int ngP, int ngA, Work W, Queue* q) {
     __shared__ double sw[6], sk[6];
-    sum_partials<6>(W.partw, nbP, sw, 0);
+    sum_groups<2>(W.partw, ngP, sw, 0);
     tmps_adj_rec r;
     double vol = 1.0, ivol = 1.0;
     if (threadIdx.x == 0) {
         r = *prev;
         vol = (r.prd[0] * r.prd[1]) * r.prd[2];
-        ivol = rcp64(vol);
+        ivol = near_rcp64(vol);  // for div_by
     }
     enter();
     if (halted(q)) return;
-    sum_partials<6>(W.partk, nbA, sk, 6);
+    sum_groups<4>(W.partk, ngA, sk, 6);
     __syncthreads();
     if (threadIdx.x != 0) return;
     if (q) q->done = step;
     double Pt[6];
     for (int c = 0; c < 6; ++c) {
         r.w[c] = sw[c] + sk[c];
-        Pt[c] = over(r.w[c], vol, ivol);
+        Pt[c] = div_by(r.w[c], vol, ivol);
     }
     r.q = Pt[2] - 0.5 * (Pt[0] + Pt[1]);
     r.elapsed = (double)step * dt;
@@ -734,7 +792,7 @@ __global__ void __launch_bounds__(kBlk) k_remap(int n, const double* __restrict_
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const size_t k = (size_t)c * n + i;
-        const double lam = over(xh[k] - prev->lo[c], prev->prd[c], rcp64(prev->prd[c]));
+        const double lam = quot64(xh[k] - prev->lo[c], prev->prd[c]);
         x[k] = next->prd[c] * lam + next->lo[c];
     }
 }
@@ -754,21 +812,22 @@ __global__ void __launch_bounds__(kOne) k_b_servo(tmps_adj_servo sv, double dt, 
     if (tid < 18) box[tid] = B.box[tid];
     if (tid >= 32 && tid < 37) par[tid - 32] = B.params[tid - 32];
     if (tid == kOne - 32 && servo) {
-        const double vol = (prev->prd[0] * prev->prd[1]) * prev->prd[2], ivol = rcp64(vol);
+        const double vol = (prev->prd[0] * prev->prd[1]) * prev->prd[2];
         double Pt[6], p[3];
-        for (int c = 0; c < 6; ++c) sPt[c] = Pt[c] = over(next->w[c], vol, ivol);
+        for (int c = 0; c < 6; ++c) sPt[c] = Pt[c] = quot64(next->w[c], vol);
         coupled(sv.couple, Pt, p);
         for (int d = 0; d < 3; ++d) {
             bool cl;
-            sratio[d] = next->prd[d] * rcp64(prev->prd[d]);
+            sratio[d] = quot64(next->prd[d], prev->prd[d]);
             srate[d] = sv.style[d] == 8 ? servo_rate(sv, d, p[d], &cl) : 0.0;
         }
     }
-    double prd[3] = {1, 1, 1}, ivol = 1.0;
+    double prd[3] = {1, 1, 1}, vol = 1.0, ivol = 1.0;
     int clamp = 0;
     if (tid == 0 && servo) {
         for (int d = 0; d < 3; ++d) prd[d] = prev->prd[d];
-        ivol = rcp64((prd[0] * prd[1]) * prd[2]);
+        vol = (prd[0] * prd[1]) * prd[2];
+        ivol = near_rcp64(vol);  // for div_by
         clamp = next->clamp;
     }
     enter();
@@ -830,8 +889,8 @@ __global__ void __launch_bounds__(kOne) k_b_servo(tmps_adj_servo sv, double dt, 
             // P = W / vol
             double volb = 0.0;
             for (int c = 0; c < 6; ++c) {
-                wbar[c] = Pb[c] * ivol;
-                volb -= Pb[c] * sPt[c] * ivol;
+                wbar[c] = div_by(Pb[c], vol, ivol);
+                volb -= div_by(Pb[c] * sPt[c], vol, ivol);
             }
             bn[3] += volb * prd[1] * prd[2];
             bn[4] += volb * prd[0] * prd[2];
@@ -849,27 +908,28 @@ __global__ void __launch_bounds__(kBlk) k_b_final(tmps_adj_sys S, double dt, tmp
     const int n = S.n;
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     const bool mine = a < n;
-    double m = 1.0, r = 1.0, im = 1.0, iI = 1.0, v[3] = {0, 0, 0}, vb[3] = {0, 0, 0}, f[3] = {0, 0, 0}, fb[3] = {0, 0, 0};
+    double m = 1.0, r = 1.0, I = 1.0, im = 1.0, iI = 1.0, v[3] = {0, 0, 0}, vb[3] = {0, 0, 0}, f[3] = {0, 0, 0}, fb[3] = {0, 0, 0};
     double mb = 0.0, Ib = 0.0, mass0 = 0.0, rad0 = 0.0;
     const double dtf = 0.5 * dt;
     if (mine) {
         m = S.mass[a];
         r = S.radius[a];
-        im = rcp64(m);
-        iI = rcp64(inertia(m, r));
+        I = inertia(m, r);
+        im = near_rcp64(m);  // for div_by
+        iI = near_rcp64(I);
         mass0 = B.mass[a];
         rad0 = B.radius[a];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const size_t k = (size_t)c * n + a;
             f[c] = T.f[k];
-            v[c] = T.vh[k] + dtf * (f[c] * im);
+            v[c] = T.vh[k] + dtf * div_by(f[c], m, im);
             vb[c] = B.v[k];
             fb[c] = B.f[k];
             // w = wh + dtf t / I
-            const double tb = dtf * B.w[k] * iI;
-            B.t[k] += tb;
-            Ib -= tb * T.t[k] * iI;
+            const double wb = dtf * B.w[k];
+            B.t[k] += div_by(wb, I, iI);
+            Ib -= div_by(wb * T.t[k], I * I, iI * iI);
         }
     }
     enter();
@@ -887,10 +947,10 @@ __global__ void __launch_bounds__(kBlk) k_b_final(tmps_adj_sys S, double dt, tmp
     for (int c = 0; c < 3; ++c) {
         const size_t k = (size_t)c * n + a;
         // v = vh + dtf f / m
-        const double kb = dtf * vb[c] * im;
+        const double kb = dtf * vb[c];
         B.v[k] = vb[c];
-        B.f[k] = fb[c] + kb;
-        mb -= kb * f[c] * im;
+        B.f[k] = fb[c] + div_by(kb, m, im);
+        mb -= div_by(kb * f[c], m * m, im * im);
     }
     B.mass[a] = mass0 + (mb + Ib * 0.4 * r * r);
     B.radius[a] = rad0 + Ib * 0.8 * m * r;
@@ -1010,7 +1070,7 @@ __global__ void __launch_bounds__(kBlk) k_b_atoms(tmps_adj_sys S, double dt, int
     double s[6] = {0, 0, 0, 0, 0, 0};
     // everything but the pairs' adjoints before the wait
     int i0 = 0, ni = 0, j0 = 0, nj = 0;
-    double m = 1.0, r = 1.0, im = 1.0, iI = 1.0, mass0 = 0.0, rad0 = 0.0;
+    double m = 1.0, r = 1.0, I = 1.0, im = 1.0, iI = 1.0, mass0 = 0.0, rad0 = 0.0;
     double x0[3] = {0, 0, 0}, v0[3] = {0, 0, 0}, w0[3] = {0, 0, 0}, fp[3] = {0, 0, 0}, tp[3] = {0, 0, 0}, lam[3] = {0, 0, 0},
            scale[3] = {1, 1, 1};
     if (mine) {
@@ -1019,9 +1079,8 @@ __global__ void __launch_bounds__(kBlk) k_b_atoms(tmps_adj_sys S, double dt, int
             const size_t k = (size_t)c * n + a;
             x0[c] = B.x[k];
             if (xh) {
-                const double ip = rcp64(prev->prd[c]);
-                lam[c] = (xh[k] - prev->lo[c]) * ip;
-                scale[c] = next->prd[c] * ip;
+                lam[c] = quot64(xh[k] - prev->lo[c], prev->prd[c]);
+                scale[c] = quot64(next->prd[c], prev->prd[c]);
             }
             if (gather) {
                 v0[c] = B.v[k];
@@ -1039,8 +1098,9 @@ __global__ void __launch_bounds__(kBlk) k_b_atoms(tmps_adj_sys S, double dt, int
             nj = S.jbeg[a + 1] - j0;
             m = S.mass[a];
             r = S.radius[a];
-            im = rcp64(m);
-            iI = rcp64(inertia(m, r));
+            I = inertia(m, r);
+            im = near_rcp64(m);  // for div_by
+            iI = near_rcp64(I);
             mass0 = B.mass[a];
             rad0 = B.radius[a];
         }
@@ -1106,12 +1166,12 @@ __global__ void __launch_bounds__(kBlk) k_b_atoms(tmps_adj_sys S, double dt, int
                 if (kick) {
                     // x = x0 + dt vh; vh = v0 + dtf f / m; wh = w0 + dtf t / I
                     const double vhb = v1 + dt * x0[c];
-                    const double fb = dtf * vhb * im, tb = dtf * w1 * iI;
+                    const double fb = dtf * vhb, tb = dtf * w1;
                     B.v[k] = vhb;
-                    B.f[k] = fb;
-                    mb -= fb * fp[c] * im;
-                    B.t[k] = tb;
-                    Ib -= tb * tp[c] * iI;
+                    B.f[k] = div_by(fb, m, im);
+                    mb -= div_by(fb * fp[c], m * m, im * im);
+                    B.t[k] = div_by(tb, I, iI);
+                    Ib -= div_by(tb * tp[c], I * I, iI * iI);
                 } else {
                     B.v[k] = v1;
                 }
@@ -1186,7 +1246,7 @@ tmps_adj_tape tape_at(const tmps_adj_tape& t, int64_t atom_stride, int64_t pair_
 // Contacts, second half-kick, pressure and servo of a step.
 int rest_of_step(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_adj_servo* sv, const tmps_adj_tape& t,
                  tmps_adj_rec* d_rec, int64_t step, const Work& W, Queue* q, cudaStream_t st) {
-    const int nbA = grid_for(s->n, kBlk), nbP = grid_for(s->npairs, kPairTile);
+    const int nbA = blocks_a(s->n), nbP = blocks_p(s->npairs);
     const tmps_adj_rec* prev = d_rec + (step - 1);
     if (s->npairs > 0) {
         run(k_pairs, nbP, kBlk, st, *s, to_params(*p), 1, (const double*)t.xh, (const double*)t.vh, (const double*)t.wh,
@@ -1200,7 +1260,7 @@ int rest_of_step(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_adj
     } else if (cudaMemsetAsync(W.partk, 0, sizeof(double) * 6 * nbA, st) != cudaSuccess) {
         return TMPS_ERR_CUDA;
     }
-    run(k_servo, 1, kOne, st, *sv, p->dt, step, prev, d_rec + step, nbP, nbA, W, q);
+    run(k_servo, 1, kOne, st, *sv, p->dt, step, prev, d_rec + step, grid_for(s->npairs, kSum), grid_for(s->n, kSum), W, q);
     return TMPS_OK;
 }
 
@@ -1286,9 +1346,9 @@ int tmps_adj_setup(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_a
     cudaStream_t st = (cudaStream_t)stream;
     Work W = carve(work, s->n, s->npairs);
     if (s->npairs > 0)
-        run(k_pairs, grid_for(s->npairs, kPairTile), kBlk, st, *s, to_params(*p), 0, (const double*)s->x, (const double*)s->v,
+        run(k_pairs, blocks_p(s->npairs), kBlk, st, *s, to_params(*p), 0, (const double*)s->x, (const double*)s->v,
             (const double*)s->w, d_box, tape->shear, tape->mask, W, (const Queue*)nullptr);
-    run(k_gather, grid_for(s->n, kBlk), kBlk, st, *s, p->dt, 0, (const double*)nullptr, (const double*)nullptr, tape->f,
+    run(k_gather, blocks_a(s->n), kBlk, st, *s, p->dt, 0, (const double*)nullptr, (const double*)nullptr, tape->f,
         tape->t, (const uint8_t*)tape->mask, W, (const Queue*)nullptr);
     return ok() ? TMPS_OK : TMPS_ERR_CUDA;
 }

@@ -33,22 +33,57 @@
 
 namespace tmps_adj {
 
-// 1 / x, and sqrt(x) with 1 / sqrt(x): on the device the short forms of
-// tmps_common.cuh (a correctly rounded division or root is several times their
-// FP64 instructions), on the host the operations themselves.
-TMPS_HD double rcp(double x) {
+// a / b (y: 1 / b within two units in the last place), 1 / x, square roots,
+// sqrt(x) > m: on the device the short forms of tmps_common.cuh, on the host
+// the operations themselves (the same values; a y is not looked at).  The
+// overlap ra + rb - |d| cancels the leading digits of a barely touching pair,
+// so one unit in the last place of a position or a distance shows in that
+// pair's radius adjoints at 1e-9 to 1e-7: every operation here is rounded as
+// written.
+TMPS_HD double quot(double a, double b, double y) {
 #if defined(__CUDA_ARCH__)
-    return tmps::rcp64(x);
+    return tmps::div_by(a, b, y);
+#else
+    (void)y;
+    return a / b;
+#endif
+}
+TMPS_HD double near_rcp(double x) {  // within two units in the last place
+#if defined(__CUDA_ARCH__)
+    return tmps::near_rcp64(x);
 #else
     return 1.0 / x;
 #endif
 }
-TMPS_HD void root(double x, double& r, double& inv) {
+TMPS_HD void root(double x, double& r, double& inv) {  // inv = 1 / r
+#if defined(__CUDA_ARCH__)
+    tmps::sqrt_rcp64(x, r, inv);
+#else
+    r = sqrt(x);
+    inv = 1.0 / r;
+#endif
+}
+TMPS_HD void root_near(double x, double& r, double& inv) {  // inv within two units in the last place of 1 / r
 #if defined(__CUDA_ARCH__)
     tmps::sqrt_rsqrt64(x, r, inv);
 #else
     r = sqrt(x);
     inv = 1.0 / r;
+#endif
+}
+TMPS_HD double rcp_of_square(double x, double y) {  // 1 / x, y = 1 / sqrt(x)
+#if defined(__CUDA_ARCH__)
+    return tmps::rcp_of_square64(x, y);
+#else
+    (void)y;
+    return 1.0 / x;
+#endif
+}
+TMPS_HD bool root_exceeds(double s, double m) {
+#if defined(__CUDA_ARCH__)
+    return tmps::root_exceeds64(s, m);
+#else
+    return sqrt(s) > m;
 #endif
 }
 
@@ -57,6 +92,7 @@ enum { M_CONTACT = 1, M_SLIP = 2, M_SHRMAG = 4, M_CLAMP = 8 };
 struct Params {
     double kn, kt, gamman, gammat, xmu, dt;
     int limit_damping;
+    double ikt = 0.0;  // 1 / kt (for quot)
 };
 
 struct PairIn {
@@ -75,10 +111,10 @@ struct PairOut {
 // Forward intermediates the reverse reads.
 struct PairTape {
     double rsq, r, delta, reff, ph, meff, rsqinv, rinv;
-    double irs, ims, iph, ifsmag;  // 1 / (ra + rb), 1 / (ma + mb), 1 / ph, 1 / fsmag (only where it slips)
+    double irs, ims, iph, ifsmag;  // near 1 / (ra + rb), 1 / (ma + mb), 1 / ph, 1 / fsmag (only where it slips), for quot
     double vrel[3], vnnr, s, g[3], wr[3], vtr[3];
     double ccel0, ccel, geff;
-    double sh1[3], rsht, sh2[3], t[3], fs0[3], u, fn, ratio, dc[3];
+    double sh1[3], rsht, sh2[3], t[3], fs0[3], fsmag, u, fn, ratio, dc[3];  // (fsmag: only where it slips)
     double fs[3], c[3];
 };
 
@@ -121,13 +157,13 @@ TMPS_HD void pair_forward(const Params& P, int shearupdate, const PairIn& in, in
     }
     m |= M_CONTACT;
     root(t.rsq, t.r, t.rinv);
-    t.rsqinv = t.rinv * t.rinv;
+    t.rsqinv = rcp_of_square(t.rsq, t.rinv);
     t.delta = radsum - t.r;
-    t.irs = rcp(radsum);
-    t.reff = (in.ra * in.rb) * t.irs;
-    root(t.reff * t.delta, t.ph, t.iph);
-    t.ims = rcp(in.ma + in.mb);
-    t.meff = (in.ma * in.mb) * t.ims;
+    t.irs = near_rcp(radsum);
+    t.reff = quot(in.ra * in.rb, radsum, t.irs);
+    root_near(t.reff * t.delta, t.ph, t.iph);
+    t.ims = near_rcp(in.ma + in.mb);
+    t.meff = quot(in.ma * in.mb, in.ma + in.mb, t.ims);
     for (int k = 0; k < 3; ++k) t.vrel[k] = in.va[k] - in.vb[k];
     t.vnnr = dot3(t.vrel, d);
     t.s = t.vnnr * t.rsqinv;
@@ -165,18 +201,16 @@ TMPS_HD void pair_forward(const Params& P, int shearupdate, const PairIn& in, in
     t.u = t.ccel * t.r;
     t.fn = P.xmu * fabs(t.u);
     t.ratio = 1.0;
-    t.ifsmag = 0.0;
+    t.fsmag = t.ifsmag = 0.0;
     for (int k = 0; k < 3; ++k) t.dc[k] = 0.0;
-    const bool slip = forced >= 0 ? (forced & M_SLIP) != 0 : fs2 > t.fn * t.fn;  // |fs0| > fn
+    const bool slip = forced >= 0 ? (forced & M_SLIP) != 0 : root_exceeds(fs2, t.fn);  // |fs0| > fn
     if (slip) {
         m |= M_SLIP;
         if (shnz) {
-            double fsmag;
-            root(fs2, fsmag, t.ifsmag);
-            t.ratio = t.fn * t.ifsmag;
-            const double ikt = rcp(P.kt);
+            root_near(fs2, t.fsmag, t.ifsmag);
+            t.ratio = quot(t.fn, t.fsmag, t.ifsmag);
             for (int k = 0; k < 3; ++k) {
-                t.dc[k] = (t.geff * t.vtr[k]) * ikt;
+                t.dc[k] = quot(t.geff * t.vtr[k], P.kt, P.ikt);
                 o.sh[k] = t.ratio * (t.sh2[k] + t.dc[k]) - t.dc[k];
                 t.fs[k] = t.ratio * t.fs0[k];
             }
@@ -240,7 +274,6 @@ TMPS_HD void pair_reverse(const Params& P, int shearupdate, int mask, const Pair
         if (mask & M_SHRMAG) {
             double ratiob = dot3(fsb, t.fs0);
             double dcb[3];
-            const double ikt = rcp(P.kt);
             for (int k = 0; k < 3; ++k) {
                 ratiob += b.sh[k] * (t.sh2[k] + t.dc[k]);
                 fs0b[k] = t.ratio * fsb[k];
@@ -249,13 +282,13 @@ TMPS_HD void pair_reverse(const Params& P, int shearupdate, int mask, const Pair
             }
             // dc = geff vtr / kt
             for (int k = 0; k < 3; ++k) {
-                geffb += dcb[k] * t.vtr[k] * ikt;
-                vtrb[k] += t.geff * dcb[k] * ikt;
+                geffb += quot(dcb[k] * t.vtr[k], P.kt, P.ikt);
+                vtrb[k] += quot(t.geff * dcb[k], P.kt, P.ikt);
             }
-            g.kt -= dot3(dcb, t.dc) * ikt;
+            g.kt -= quot(dot3(dcb, t.dc), P.kt, P.ikt);
             // ratio = fn / fsmag
-            fnb += ratiob * t.ifsmag;
-            fsmagb -= ratiob * t.ratio * t.ifsmag;
+            fnb += quot(ratiob, t.fsmag, t.ifsmag);
+            fsmagb -= quot(ratiob * t.ratio, t.fsmag, t.ifsmag);
         } else {
             for (int k = 0; k < 3; ++k) {
                 fs0b[k] = 0.0;
@@ -274,8 +307,8 @@ TMPS_HD void pair_reverse(const Params& P, int shearupdate, int mask, const Pair
     ccelb += ub * t.r;
     rbar += ub * t.ccel;
     // fsmag = |fs0|
-    if (fsmagb != 0.0)
-        for (int k = 0; k < 3; ++k) fs0b[k] += fsmagb * t.fs0[k] * t.ifsmag;
+    if (t.fsmag > 0.0)
+        for (int k = 0; k < 3; ++k) fs0b[k] += quot(fsmagb * t.fs0[k], t.fsmag, t.ifsmag);
     // fs0 = -ph t, t = kt sh2 + geff vtr
     for (int k = 0; k < 3; ++k) {
         phb -= fs0b[k] * t.t[k];
@@ -347,25 +380,27 @@ TMPS_HD void pair_reverse(const Params& P, int shearupdate, int mask, const Pair
     rbar -= rinvb * t.rinv * t.rinv;
     rsqb -= rsqinvb * t.rsqinv * t.rsqinv;
     // meff = ma mb / (ma + mb)
-    const double ims2 = meffb * (t.ims * t.ims);
-    g.ma += ims2 * in.mb * in.mb;
-    g.mb += ims2 * in.ma * in.ma;
+    const double ms = in.ma + in.mb;
+    const double ims2 = t.ims * t.ims;
+    g.ma += quot(meffb * in.mb * in.mb, ms * ms, ims2);
+    g.mb += quot(meffb * in.ma * in.ma, ms * ms, ims2);
     // ph = sqrt(reff delta)
     if (t.ph > 0.0) {
-        const double u2 = 0.5 * phb * t.iph;
+        const double u2 = quot(phb, 2.0 * t.ph, 0.5 * t.iph);
         reffb += u2 * t.delta;
         deltab += u2 * t.reff;
     }
     // reff = ra rb / (ra + rb)
-    const double irs2 = reffb * (t.irs * t.irs);
-    g.ra += irs2 * in.rb * in.rb;
-    g.rb += irs2 * in.ra * in.ra;
+    const double rs = in.ra + in.rb;
+    const double irs2 = t.irs * t.irs;
+    g.ra += quot(reffb * in.rb * in.rb, rs * rs, irs2);
+    g.rb += quot(reffb * in.ra * in.ra, rs * rs, irs2);
     // delta = ra + rb - r
     g.ra += deltab;
     g.rb += deltab;
     rbar -= deltab;
     // r = sqrt(rsq), rsq = d . d
-    rsqb += 0.5 * rbar * t.rinv;
+    rsqb += quot(rbar, 2.0 * t.r, 0.5 * t.rinv);
     for (int k = 0; k < 3; ++k) g.d[k] = db[k] + 2.0 * rsqb * d[k];
 }
 

@@ -96,29 +96,55 @@ TMPS_DEV void split_dw(double v, float& hi, float& lo) {
     lo = f32_rn(__dsub_rn(v, f64_of(hi)));
 }
 
-// FP64 reciprocals and square roots.  This part issues an FP64 instruction for
-// a warp every 16 cycles per SM, and the compiler's correctly rounded division
-// and square root are some ten to twenty of them each.  These start from the
-// hardware's 20-bit approximations (rcp.approx, rsqrt.approx: not on the FP64
-// pipe) and take one third-order step -- Halley's iteration, whose error is
-// the cube of the seed's -- in three to five instructions; results are within
-// two units in the last place (sqrt64's root within one).  Arguments outside
-// 2^+-1000, zeros, infinities and NaNs take the correctly rounded operation.
+// FP64 quotients, reciprocals and square roots, rounded as the operations
+// themselves.  This part issues an FP64 instruction for a warp every 16 cycles
+// per SM, and the compiler's division and square root are some ten to twenty
+// of them each.  These start from the hardware's 20-bit approximations
+// (rcp.approx, rsqrt.approx: not on the FP64 pipe) and take one third-order
+// step -- Halley's iteration, whose error is the cube of the seed's -- and one
+// correction by the exact residual (Markstein 1990): six FP64 instructions a
+// quotient (three for each further one by the same divisor), five a
+// reciprocal, nine a root.  Before its last rounding a result is within 2^-48
+// units in the last place of the exact one, so it is the correctly rounded one
+// unless the exact one lies that close to the middle of two neighbours.
+// Arguments outside 2^+-1000 (quotients: 2^+-500), zeros, infinities and NaNs
+// take the operation itself.
 TMPS_DEV bool plain64(double x) {
     const int e = (__double2hiint(x) >> 20) & 0x7ff;
     return e >= 23 && e <= 2023;
 }
 
-// 1 / x
-TMPS_DEV double rcp64(double x) {
-    if (!plain64(x)) return 1.0 / x;
+// 1 / x within 0.51 units in the last place (x plain)
+TMPS_DEV double near_rcp64(double x) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double e = __fma_rn(-x, y, 1.0);
     return __fma_rn(y, __fma_rn(e, e, e), y);
 }
+// 1 / x from y, a few units in the last place off (x plain)
+TMPS_DEV double refine_rcp64(double x, double y) { return __fma_rn(__fma_rn(-x, y, 1.0), y, y); }
 
-// 1 / sqrt(x) for x > 0
+// 1 / x
+TMPS_DEV double rcp64(double x) {
+    if (!plain64(x)) return 1.0 / x;
+    return refine_rcp64(x, near_rcp64(x));
+}
+
+// a / b with y = 1 / b within two units in the last place at hand: the product
+// corrected by its residual, at three dependent FP64 instructions instead of a
+// division's latency.  Operands outside 2^+-500 take the division.
+TMPS_DEV double div_by(double a, double b, double y) {
+    const int ha = __double2hiint(a), ea = (ha >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
+    const bool zero = ((ha & 0x7fffffff) | __double2loint(a)) == 0;
+    if (((ea < 523 || ea > 1523) && !zero) || eb < 523 || eb > 1523) return a / b;
+    const double q = __dmul_rn(a, y);
+    if (zero) return q;  // with its sign, as the quotient's
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+// a / b
+TMPS_DEV double quot64(double a, double b) { return div_by(a, b, near_rcp64(b)); }
+
+// 1 / sqrt(x) for x > 0, within two units in the last place
 TMPS_DEV double rsqrt64(double x) {
     if (!plain64(x) || !(__double2hiint(x) > 0)) return 1.0 / sqrt(x);
     double y;
@@ -127,8 +153,8 @@ TMPS_DEV double rsqrt64(double x) {
     return __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
 }
 
-// root = sqrt(x) and inv = 1 / sqrt(x): the product x * inv corrected by its
-// own residual, which rounds it correctly (Markstein) but for rare last bits.
+// root = sqrt(x): the product x / sqrt(x) corrected by its own residual; inv =
+// 1 / root within two units in the last place.
 TMPS_DEV void sqrt_rsqrt64(double x, double& root, double& inv) {
     if (!plain64(x) || !(__double2hiint(x) > 0)) {
         root = sqrt(x);
@@ -139,22 +165,31 @@ TMPS_DEV void sqrt_rsqrt64(double x, double& root, double& inv) {
     const double g = __dmul_rn(x, inv);
     root = __fma_rn(__fma_rn(-g, g, x), __dmul_rn(0.5, inv), g);
 }
-// a / b with y = 1 / b correctly rounded at hand: the product corrected by its
-// residual is the correctly rounded quotient (Markstein 1990), at three
-// dependent FP64 instructions instead of a division's latency.  Operands
-// outside 2^+-500 take the division.
-TMPS_DEV double div_by(double a, double b, double y) {
-    const int ha = __double2hiint(a), ea = (ha >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
-    const bool zero = ((ha & 0x7fffffff) | __double2loint(a)) == 0;
-    if (((ea < 523 || ea > 1523) && !zero) || eb < 523 || eb > 1523) return a / b;
-    const double q = __dmul_rn(a, y);
-    if (zero) return q;  // with its sign, as the quotient's
-    return __fma_rn(__fma_rn(-q, b, a), y, q);
+// The same with inv = 1 / root.
+TMPS_DEV void sqrt_rcp64(double x, double& root, double& inv) {
+    sqrt_rsqrt64(x, root, inv);
+    if (plain64(x)) inv = refine_rcp64(root, inv);
 }
 TMPS_DEV double sqrt64(double x) {
     double root, inv;
     sqrt_rsqrt64(x, root, inv);
     return root;
+}
+// 1 / x where y = 1 / sqrt64(x) is at hand
+TMPS_DEV double rcp_of_square64(double x, double y) {
+    return plain64(x) ? refine_rcp64(x, __dmul_rn(y, y)) : 1.0 / x;
+}
+
+// sqrt(s) > m, as the rounded root compares (s a sum of squares): by the high
+// words of s and m * m where they differ by more than the roundings of either
+// can move them, without a root.
+TMPS_DEV bool root_exceeds64(double s, double m) {
+    const uint32_t hs = (uint32_t)__double2hiint(s), hm = (uint32_t)__double2hiint(__dmul_rn(m, m));
+    if (hs < 0x7ff00000u && hm < 0x7ff00000u && __double2hiint(m) >= 0) {
+        if (hs > hm + 1u) return true;
+        if (hs + 1u < hm) return false;
+    }
+    return sqrt64(s) > m;
 }
 
 // a * b >= 0.0, as the FP64 product compares: from the sign bits where the

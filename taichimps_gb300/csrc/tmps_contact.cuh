@@ -28,7 +28,7 @@ struct StyleTraits {
 };
 
 // Division and square root of the law.  The FP64 form forms quotients from
-// rcp64 and roots from rsqrt64 (within two units in the last place: the
+// near_rcp64 and roots from rsqrt64 (within two units in the last place: the
 // results follow the reference to 1e-12; the contact distance |d|, whose
 // difference from the radii cancels three digits, keeps the rounded root of
 // the caller).  The mixed form's
@@ -39,7 +39,7 @@ struct StyleTraits {
 template <typename T>
 TMPS_DEV T ldiv(T a, T b);
 template <>
-TMPS_DEV double ldiv<double>(double a, double b) { return a * rcp64(b); }
+TMPS_DEV double ldiv<double>(double a, double b) { return a * (plain64(b) ? near_rcp64(b) : 1.0 / b); }
 template <>
 TMPS_DEV float ldiv<float>(float a, float b) { return __fdividef(a, b); }
 template <typename T>

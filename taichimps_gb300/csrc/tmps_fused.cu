@@ -2492,9 +2492,7 @@ __device__ void servo_derive(tmps_box& b, const tmps_servo& sv, tmps_engine& e, 
     switch (warp) {
         case 0:
         {
-            // 1 / prd by one more step of rcp64 (correctly rounded but for rare last bits)
-            const double y = rcp64(nprd);
-            b.inv_prd[d] = __fma_rn(__fma_rn(-nprd, y, 1.0), y, y);
+            b.inv_prd[d] = rcp64(nprd);
             if (e.mixed) e.iprd32[d] = f32_rn(b.inv_prd[d]);
             break;
         }

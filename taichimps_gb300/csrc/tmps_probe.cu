@@ -47,6 +47,10 @@ extern "C" int tmps_probe_fp64(int32_t blocks, int32_t threads, int32_t iters, d
 //   which 4: 1 / sqrt(a[i])          rsqrt64   (a[i] >= 0)
 //   which 5: sqrt(a[i])              sqrt64    (a[i] >= 0)
 //   which 6: a[i] / a[n - 1 - i]     div_by    (bit for bit; zero divisors left out)
+//   which 7: a[i] / a[n - 1 - i]     quot64    (bit for bit; zero divisors left out)
+//   which 8: sqrt(a[i]) > a[n - 1 - i] as 1 or 0   root_exceeds64
+//   which 9: 1 / sqrt(a[i]) of the rounded root    sqrt_rcp64, bit for bit
+//   which 10: 1 / a[i] from 1 / sqrt(a[i])         rcp_of_square64, bit for bit
 namespace {
 
 __global__ void k_selftest(int which, const double* __restrict__ a, int n, double* __restrict__ mine,
@@ -83,6 +87,24 @@ __global__ void k_selftest(int which, const double* __restrict__ a, int n, doubl
             hw[i] = b != 0.0 ? x / b : 0.0;
             break;
         }
+        case 7: {
+            const double b = a[n - 1 - i];
+            mine[i] = b != 0.0 ? quot64(x, b) : 0.0;
+            hw[i] = b != 0.0 ? x / b : 0.0;
+            break;
+        }
+        case 8:
+            mine[i] = root_exceeds64(x, a[n - 1 - i]) ? 1.0 : 0.0;
+            hw[i] = sqrt(x) > a[n - 1 - i] ? 1.0 : 0.0;
+            break;
+        case 9:
+        case 10: {
+            double r, inv;
+            sqrt_rcp64(x, r, inv);
+            mine[i] = which == 9 ? inv : rcp_of_square64(x, inv);
+            hw[i] = which == 9 ? 1.0 / sqrt(x) : 1.0 / x;
+            break;
+        }
         default: {
             float h, l;
             split_dw(x, h, l);
@@ -101,7 +123,7 @@ __global__ void k_selftest(int which, const double* __restrict__ a, int n, doubl
 
 extern "C" int tmps_selftest_arith(int32_t which, const double* d_a, int32_t n, double* d_mine, double* d_hw,
                                    void* stream) {
-    if (which < 0 || which > 6 || n < 0 || !d_a || !d_mine || !d_hw) return TMPS_ERR_BAD_ARG;
+    if (which < 0 || which > 10 || n < 0 || !d_a || !d_mine || !d_hw) return TMPS_ERR_BAD_ARG;
     if (n == 0) return TMPS_OK;
     k_selftest<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(which, d_a, n, d_mine, d_hw);
     note_launches(1);

@@ -57,3 +57,26 @@ def test_quotient_by_reciprocal(gpu):
     rng.shuffle(a)
     mine, hw = _run(6, a)
     np.testing.assert_array_equal(mine.view(np.int64), hw.view(np.int64))
+
+
+# which: 3 rcp64, 5 sqrt64, 7 quot64, 8 root_exceeds64, 9 and 10 the reciprocals of sqrt_rcp64 and rcp_of_square64
+@pytest.mark.parametrize("which", [3, 5, 7, 8, 9, 10])
+def test_rounded_as_the_operations(gpu, which):
+    """Bit for bit the compiler's division and square root.  (A result within 2^-50 units of the middle of two
+    neighbours may round the other way; of the divisors here only those one unit below a power of two have such
+    reciprocals, and they are left out.)"""
+    rng = np.random.default_rng(40 + which)
+    usual = rng.uniform(1e-6, 1e6, size=1_500_000)
+    wide = np.ldexp(rng.uniform(1.0, 2.0, size=500_000), rng.integers(-240, 240, size=500_000))
+    p2 = np.ldexp(1.0, np.arange(-240, 240))
+    near = 1.0 + np.arange(0, 200_000) * 2.0 ** -52
+    a = np.concatenate([usual, wide, p2, np.nextafter(p2, np.inf), near, [0.0, 5e-324, 1e-300, 1e300, np.inf, np.nan]])
+    if which == 8:  # a bound near the root, on either side of it and on it
+        root = np.sqrt(a) * (1.0 + rng.integers(-3, 4, size=len(a)) * rng.choice([2.0 ** -52, 2.0 ** -30, 2.0 ** -20], size=len(a)))
+        a = np.concatenate([a, [0.0, 1.0, 1.0, -1.0], root[::-1]])
+    elif which in (3, 7):
+        a = a * rng.choice([1.0, -1.0], size=len(a))
+        rng.shuffle(a)
+    mine, hw = _run(which, a)
+    same = (mine.view(np.int64) == hw.view(np.int64)) | (np.isnan(mine) & np.isnan(hw))
+    assert same.all(), (int((~same).sum()), a[~same][:4], mine[~same][:4], hw[~same][:4])
