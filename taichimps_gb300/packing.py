@@ -19,6 +19,7 @@ The result has no overlapping pair, so it starts with no contacts.
 from __future__ import annotations
 
 import math
+from pathlib import Path
 
 import numpy as np
 
@@ -164,10 +165,23 @@ def config2(seed: int = 2, n: int = 1_000_000):
     return p
 
 
+def _stored_packing(n: int, seed: int, args: dict) -> dict | None:
+    """The packing kept for these arguments of compress_packing, if there is one."""
+    f = Path(__file__).resolve().parent / "data" / f"compressed_{n}_{seed}.npz"
+    if not f.exists():
+        return None
+    z = np.load(f)
+    if any(z["arg_" + k].item() != v for k, v in args.items()):
+        return None
+    return {"x": z["x"], "radius": z["radius"], "lo": z["lo"], "L": z["L"], "pressure": z["pressure"],
+            "phi": float(z["phi"]), "density": float(z["density"])}
+
+
 def compress_packing(n: int, seed: int, dmin: float = 0.8, dmax: float = 1.2, density: float = 2.5,
                      kn: float = 1.0e5, xmu: float = 0.5, ptarget: float = 1.0, pgain: float = 1.0,
                      max_rate: float = 0.005, cycles: int = 100, relax_cycles: int = 10, cycle_steps: int = 2000,
-                     dt: float = 5e-4, precision: str = "fp64", phi0: float = 0.3, jitter: float = 0.3):
+                     dt: float = 5e-4, precision: str = "fp64", phi0: float = 0.3, jitter: float = 0.3,
+                     regenerate: bool = False):
     """An isotropically compressed packing: `make_packing_box` at solid
     fraction `phi0` with the sites jittered by `jitter` lattice constants (a
     disordered gas; sites on an unjittered lattice would jam as a crystal of
@@ -182,7 +196,17 @@ def compress_packing(n: int, seed: int, dmin: float = 0.8, dmax: float = 1.2, de
     about 0.01 at kn 1e5 and p 1 -- or the contacts overshoot and the servo
     stops on dynamic pressure.  Returns
     positions wrapped into the final box, radii, box edges and lower corner,
-    the last pressure tensor and the solid fraction.  Runs on the GPU path."""
+    the last pressure tensor and the solid fraction.  Runs on the GPU path.
+
+    The last bits of a run of 220,000 steps decide which packing it ends in, so packings that results are judged
+    on are kept as data (data/compressed_<n>_<seed>.npz, with the arguments they were made with) and read from
+    there for those arguments; regenerate=True makes the run all the same."""
+    stored = None if regenerate else _stored_packing(n, seed, dict(
+        dmin=dmin, dmax=dmax, density=density, kn=kn, xmu=xmu, ptarget=ptarget, pgain=pgain, max_rate=max_rate,
+        cycles=cycles, relax_cycles=relax_cycles, cycle_steps=cycle_steps, dt=dt, precision=precision, phi0=phi0,
+        jitter=jitter))
+    if stored is not None:
+        return stored
     from . import (AtomSystem, ContactHistory, Domain, FixDampingCundall, FixDeformPressure, FixNVESphere,
                    GranHertzHistory, NeighborList, Simulation)
 
@@ -257,7 +281,6 @@ def dense_cell(path=None, regenerate: bool = False) -> dict:
     50, gammat 25, xmu 0.5), d ~ U[0.8, 1.2], density 2.5, 15,625 spheres compressed by compress_packing
     with DENSE_CELL_ARGS.  Read from the package's data file (written by this function on a GPU run with
     regenerate=True, so every run of the workload starts from the same bits)."""
-    from pathlib import Path
     f = Path(path) if path is not None else Path(__file__).resolve().parent / "data" / DENSE_CELL_FILE
     if f.exists() and not regenerate:
         z = np.load(f)
