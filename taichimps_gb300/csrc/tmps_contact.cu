@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kBlock)
         double nimg[3];
         if (!geom(j, ld4(A.xr, j), in, nimg)) continue;
         const double radsum = in.ra + in.rb;
-        sqrt_rsqrt64(in.rsq, in.r, in.rinv);
+        sqrt_rcp64(in.rsq, in.r, in.rinv);
         in.delta = radsum - in.r;
         const double4 vj = ld4(A.vm, j), wj = ld4(A.om, j);
         const double4 va = lo ? vi : vj, vb = lo ? vj : vi, wa = lo ? wi : wj, wb = lo ? wj : wi;

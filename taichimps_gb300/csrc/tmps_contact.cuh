@@ -27,11 +27,10 @@ struct StyleTraits {
     static constexpr bool legacy_history = STYLE == STYLE_HOOKE_HISTORY || STYLE == STYLE_HERTZ_HISTORY;
 };
 
-// Division and square root of the law.  The FP64 form forms quotients from
-// near_rcp64 and roots from rsqrt64 (within two units in the last place: the
-// results follow the reference to 1e-12; the contact distance |d|, whose
-// difference from the radii cancels three digits, keeps the rounded root of
-// the caller).  The mixed form's
+// Division and square root of the law.  The FP64 form's are rounded as the
+// operations themselves (quot64, sqrt64: its results follow the reference to
+// 1e-12, and the contact distance |d| loses three digits to its difference
+// from the radii).  The mixed form's
 // law is FP32 arithmetic whose every operation already rounds at 2^-24, so
 // it uses the hardware's approximate reciprocal and reciprocal square root
 // (errors of a few ulp, the same order): a tenth of the instructions of the
@@ -39,7 +38,7 @@ struct StyleTraits {
 template <typename T>
 TMPS_DEV T ldiv(T a, T b);
 template <>
-TMPS_DEV double ldiv<double>(double a, double b) { return a * (plain64(b) ? near_rcp64(b) : 1.0 / b); }
+TMPS_DEV double ldiv<double>(double a, double b) { return quot64(a, b); }
 template <>
 TMPS_DEV float ldiv<float>(float a, float b) { return __fdividef(a, b); }
 template <typename T>
@@ -219,7 +218,7 @@ TMPS_DEV void contact_law(const PP& P, T dt, int shearupdate, const PairIn<T>& i
         T rsqinv, rinv;
         if constexpr (sizeof(T) == sizeof(double)) {
             rinv = in.rinv;
-            rsqinv = rinv * rinv;
+            rsqinv = rcp_of_square64(in.rsq, rinv);
         } else {
             rsqinv = ldiv(T(1), in.rsq);
             rinv = ldiv(T(1), r);
@@ -276,20 +275,19 @@ TMPS_DEV void contact_law(const PP& P, T dt, int shearupdate, const PairIn<T>& i
                 else fs[k] = -t;
             }
             const T fn = T(P.xmu) * fabs(ccel * r);
-            T fsmag, fs2 = T(0);
+            T fsmag = T(0);
             bool slip;
-            if constexpr (sizeof(T) == sizeof(double)) {  // the squares decide: a root only where it slips
-                fs2 = dot3(fs, fs);
-                slip = fs2 > fn * fn;
+            if constexpr (sizeof(T) == sizeof(double)) {  // a root only where it slips
+                const T fs2 = dot3(fs, fs);
+                slip = root_exceeds64(fs2, fn);
+                if (slip) fsmag = sqrt64(fs2);
             } else {
                 fsmag = norm3(fs);
                 slip = fsmag > fn;
             }
             if (slip) {
                 if (moved) {
-                    T ratio;
-                    if constexpr (sizeof(T) == sizeof(double)) ratio = fn * rsqrt64(fs2);
-                    else ratio = ldiv(fn, fsmag);
+                    const T ratio = ldiv(fn, fsmag);
 #pragma unroll
                     for (int k = 0; k < 3; ++k) {
                         const T dc = ldiv(geff * vtr[k], T(P.kt));
@@ -350,14 +348,14 @@ TMPS_DEV void contact_law(const PP& P, T dt, int shearupdate, const PairIn<T>& i
             }
             default: break;
         }
-        // the mixed form's multiply-add is written out: which of the two products is fused into the
-        // difference must not depend on the kernel the law is inlined into
+        // the multiply-add is written out: which of the two products is fused into the difference must not
+        // depend on the kernel the law is inlined into
         T fntot;
         if constexpr (sizeof(T) == sizeof(float)) {
             const T kna = P.normal_id != 0 ? T(P.kn) * a : T(P.kn);
             fntot = __fmaf_rn(kna, delta, -__fmul_rn(dpf, vnnr));
         } else {
-            fntot = fne - dpf * vnnr;
+            fntot = __fma_rn(-dpf, vnnr, fne);
         }
         if (P.limit_damping == 1 && fntot < T(0)) fntot = T(0);
         const T fscrit = T(P.mu) * fabs(fntot);

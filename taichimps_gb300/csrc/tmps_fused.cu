@@ -1014,7 +1014,7 @@ __device__ __forceinline__ bool contact_core(
         const T radsum = in.ra + in.rb;
         near = in.rsq < __dmul_rn(radsum, radsum) && apart64(in.rsq);
         if (near) {
-            sqrt_rsqrt64(in.rsq, in.r, in.rinv);
+            sqrt_rcp64(in.rsq, in.r, in.rinv);
             in.delta = radsum - in.r;
         }
     }
