@@ -3037,8 +3037,12 @@ int a_wave(bool mixed) {
 }
 // The FP64 form takes as many blocks as there are 32-atom groups, up to the
 // wave: an SM's FP64 units are shared by its warps (one FP64 instruction of a
-// warp every ~15 cycles), so a small system runs one warp on each of many SMs
-// (a step of 4,000 spheres without a servo 28 -> 25.4 us).  The mixed form's warps share
+// warp every ~15 cycles), so a small system runs one warp on each of many SMs.
+// A step with a servo, one group a block of C against two and four: jammed
+// packings 34, 43, 48 us (1,000 spheres), 37, 57, 64 (4,000), 61, 78, 104
+// (15,600), 85, 85, 107 (31,200), 127 each at 62,500, where the wave is full;
+// loose ones (500 to 64,000 spheres) the same within the spread of repeats, 0.4
+// us.  Without a servo 28 -> 25.4 us at 4,000.  The mixed form's warps share
 // nothing as narrow and its partial sums keep the fuller blocks.
 int a_blocks(int n, bool mixed) {
     const int b = grid_for(n, mixed ? kBlockA : 32);

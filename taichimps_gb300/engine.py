@@ -175,11 +175,6 @@ class FusedEngine:
         _lib.check(_device.lib().tmps_fused_shape(n, style, mixed, self.launch_shape[0], self.launch_shape[1],
                                                   ctypes.byref(a_b), ctypes.byref(c_b)), "tmps_fused_shape")
         self.a_blocks, self.c_blocks = a_b.value, c_b.value
-        if not self.mixed and self.deform is not None:
-            # the FP64 form's one block of C per 32-atom group spreads a small system over the SMs; where
-            # a servo sums the blocks' partials every step, two groups share one (a step of 1,000, 4,000
-            # and 12,000 spheres: 17.2, 23.5 and 30.2 us against 17.5, 24.2 and 29.3)
-            self.c_blocks = min(self.c_blocks, (n + 63) // 64)
         self.nblocks = self.a_blocks + self.c_blocks
 
     def set_launch_shape(self, shape: tuple[int, int]) -> None:
