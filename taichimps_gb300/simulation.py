@@ -199,17 +199,24 @@ class Simulation:
             seg = remaining
             if self.restart_every > 0:
                 seg = min(seg, self.restart_every - self.timestep % self.restart_every)
-            if self.fused and seg > 0 and fusable(self, walls=self.precision == "fp64") and self.atom.nlocal > 0:
+            fused = 0
+            if self.fused and seg > 0 and self.atom.nlocal > 0:
+                if fusable(self):
+                    fused = seg
+                elif self.precision == "fp64" and fusable(self, walls=True):
+                    # the last step hook by hook: it leaves the per-atom virial of its contacts, which the
+                    # pressure of a run without a servo is taken from
+                    fused = seg - 1
+            if fused > 0:
                 eng = FusedEngine(self, self.precision)
                 self.last_engine = eng
                 eng.begin()
                 try:
-                    eng.run(seg)
+                    eng.run(fused)
                 finally:
                     eng.finish()
-            else:
-                for _ in range(seg):
-                    self._sub_step_inner()
+            for _ in range(seg - fused):
+                self._sub_step_inner()
             remaining -= seg
             if self.restart_every > 0 and seg > 0 and self.timestep % self.restart_every == 0:
                 self.check_device_status()

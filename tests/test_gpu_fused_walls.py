@@ -89,3 +89,23 @@ def test_what_stays_hook_by_hook(gpu):
     assert not fusable(_sim(33, "planes", True)[0])                                # batches and the mixed form
     with pytest.raises(NotImplementedError):
         _sim(33, "planes", True, precision="mixed")[0].run(1)
+
+
+@pytest.mark.parametrize("steps", [1, 2, 60])
+def test_pressure_after_a_run_with_walls(gpu, steps):
+    """The pressure tensor after a run is the last step's, through the fused step as hook by hook."""
+    import taichimps_gb300 as G
+    got = []
+    for fused in (True, False):
+        sim, _ = _sim(512, "planes", fused)
+        sim.run(40)
+        early = sim.atom.virial.to_numpy().copy()
+        sim.run_pre = False
+        sim.run(steps)
+        got.append((G.Computes().compute_pressure_tensor(sim.atom, sim.domain), sim.atom.virial.to_numpy()[:512].copy()))
+        assert np.abs(sim.atom.virial.to_numpy() - early).max() > 0.0
+    (p, v), (q, w) = got
+    assert np.abs(w).max() > 0.0
+    # two orders of FP64 sums over the run, as the states
+    assert np.abs(p - q).max() <= 1e-10 * np.abs(q).max()
+    assert np.abs(v - w).max() <= 1e-10 * np.abs(w).max()
