@@ -126,7 +126,10 @@ class FixWallGran(_WallBase):
 
     def passed(self, steps: int, dt: float) -> None:
         # one addition a step, as post_force makes them
-        self.elapsed = float(np.add.accumulate(np.concatenate(([self.elapsed], np.full(steps, dt))))[-1])
+        for first in range(0, steps, 65536):
+            terms = np.full(min(steps - first, 65536) + 1, dt)
+            terms[0] = self.elapsed
+            self.elapsed = float(np.add.accumulate(terms)[-1])
 
     def setup(self, nsteps_total: int = 0, dt: float = 0.0) -> None:
         """Restart the clock the wall motion is referenced to."""
