@@ -164,7 +164,9 @@ __device__ void sum_groups(const double* part, int ng, double* out, int first) {
 // Programmatic dependent launch: wait for the kernel before to complete, then
 // let the next one be scheduled.  Every kernel of this file does both in this
 // order, so when a block starts, all but the kernel right before it have
-// completed: what those wrote may be read, and worked on, before enter().  The
+// completed: what those wrote may be read, and worked on, before enter().  That
+// holds within one call of the interface; the first launch of every call is
+// made without the attribute (Chain), whatever the caller queued before it.  The
 // launches of a step depend on one another in a chain, so for few spheres the
 // time of a step is the sum of their load and FP64 latencies, and each kernel
 // does here what does not need its predecessor.
@@ -1201,33 +1203,37 @@ bool sys_ok(const tmps_adj_sys* s) {
            (s->npairs == 0 || (s->shear && s->pi && s->pj)) && s->ibeg && s->jbeg && (s->npairs == 0 || s->jlist);
 }
 
-// Launch with programmatic stream serialization (see enter), counted; `after`:
-// only once the kernel before has completed.
-template <typename... P, typename... A>
-void run_as(bool after, void (*kernel)(P...), int grid, int block, cudaStream_t s, A&&... args) {
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = after ? 0 : 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.stream = s;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
-    note_launches(1);
-}
-template <typename... P, typename... A>
-void run(void (*kernel)(P...), int grid, int block, cudaStream_t s, A&&... args) {
-    run_as(false, kernel, grid, block, s, std::forward<A>(args)...);
-}
+// The launches of one call: with programmatic stream serialization (see enter),
+// but for the first, which starts once all that was queued before the call has
+// completed; counted.
+struct Chain {
+    cudaStream_t stream;
+    bool first = true;
 
-// The contact pass's reverse at the residency its number of tiles wants.
-template <typename... A>
-void run_b_pairs(int tiles, cudaStream_t s, A&&... args) {
-    if (tiles <= 608) run(k_b_pairs<4>, tiles, kBlk, s, std::forward<A>(args)...);
-    else run(k_b_pairs<5>, tiles, kBlk, s, std::forward<A>(args)...);
-}
+    template <typename... P, typename... A>
+    void run(void (*kernel)(P...), int grid, int block, A&&... args) {
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = first ? 0 : 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3((unsigned)block);
+        cfg.stream = stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+        first = false;
+        note_launches(1);
+    }
+    // the next launch reads before its wait what the one before it writes
+    void join() { first = true; }
+    // The contact pass's reverse at the residency its number of tiles wants.
+    template <typename... A>
+    void run_b_pairs(int tiles, A&&... args) {
+        if (tiles <= 608) run(k_b_pairs<4>, tiles, kBlk, std::forward<A>(args)...);
+        else run(k_b_pairs<5>, tiles, kBlk, std::forward<A>(args)...);
+    }
+};
 
 // The tape of the k-th step of a run whose tapes lie atom_stride doubles (atom
 // arrays) and pair_stride pairs apart (0: one tape, overwritten).
@@ -1245,22 +1251,22 @@ tmps_adj_tape tape_at(const tmps_adj_tape& t, int64_t atom_stride, int64_t pair_
 
 // Contacts, second half-kick, pressure and servo of a step.
 int rest_of_step(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_adj_servo* sv, const tmps_adj_tape& t,
-                 tmps_adj_rec* d_rec, int64_t step, const Work& W, Queue* q, cudaStream_t st) {
+                 tmps_adj_rec* d_rec, int64_t step, const Work& W, Queue* q, Chain& ch) {
     const int nbA = blocks_a(s->n), nbP = blocks_p(s->npairs);
     const tmps_adj_rec* prev = d_rec + (step - 1);
     if (s->npairs > 0) {
-        run(k_pairs, nbP, kBlk, st, *s, to_params(*p), 1, (const double*)t.xh, (const double*)t.vh, (const double*)t.wh,
+        ch.run(k_pairs, nbP, kBlk, *s, to_params(*p), 1, (const double*)t.xh, (const double*)t.vh, (const double*)t.wh,
             prev, t.shear, t.mask, W, (const Queue*)q);
-    } else if (cudaMemsetAsync(W.partw, 0, sizeof(double) * 6 * nbP, st) != cudaSuccess) {
+    } else if (cudaMemsetAsync(W.partw, 0, sizeof(double) * 6 * nbP, ch.stream) != cudaSuccess) {
         return TMPS_ERR_CUDA;
     }
     if (s->n > 0) {
-        run(k_gather, nbA, kBlk, st, *s, p->dt, 1, (const double*)t.vh, (const double*)t.wh, t.f, t.t,
+        ch.run(k_gather, nbA, kBlk, *s, p->dt, 1, (const double*)t.vh, (const double*)t.wh, t.f, t.t,
             (const uint8_t*)t.mask, W, (const Queue*)q);
-    } else if (cudaMemsetAsync(W.partk, 0, sizeof(double) * 6 * nbA, st) != cudaSuccess) {
+    } else if (cudaMemsetAsync(W.partk, 0, sizeof(double) * 6 * nbA, ch.stream) != cudaSuccess) {
         return TMPS_ERR_CUDA;
     }
-    run(k_servo, 1, kOne, st, *sv, p->dt, step, prev, d_rec + step, grid_for(s->npairs, kSum), grid_for(s->n, kSum), W, q);
+    ch.run(k_servo, 1, kOne, *sv, p->dt, step, prev, d_rec + step, grid_for(s->npairs, kSum), grid_for(s->n, kSum), W, q);
     return TMPS_OK;
 }
 
@@ -1343,12 +1349,12 @@ int tmps_adj_setup(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_a
                    const tmps_adj_tape* tape, void* work, void* stream) {
     if (!sys_ok(s) || !p || !d_box || !tape || !work || !tape->shear || !tape->mask) return TMPS_ERR_BAD_ARG;
     if (s->n == 0) return TMPS_OK;
-    cudaStream_t st = (cudaStream_t)stream;
+    Chain ch{(cudaStream_t)stream};
     Work W = carve(work, s->n, s->npairs);
     if (s->npairs > 0)
-        run(k_pairs, blocks_p(s->npairs), kBlk, st, *s, to_params(*p), 0, (const double*)s->x, (const double*)s->v,
+        ch.run(k_pairs, blocks_p(s->npairs), kBlk, *s, to_params(*p), 0, (const double*)s->x, (const double*)s->v,
             (const double*)s->w, d_box, tape->shear, tape->mask, W, (const Queue*)nullptr);
-    run(k_gather, blocks_a(s->n), kBlk, st, *s, p->dt, 0, (const double*)nullptr, (const double*)nullptr, tape->f,
+    ch.run(k_gather, blocks_a(s->n), kBlk, *s, p->dt, 0, (const double*)nullptr, (const double*)nullptr, tape->f,
         tape->t, (const uint8_t*)tape->mask, W, (const Queue*)nullptr);
     return ok() ? TMPS_OK : TMPS_ERR_CUDA;
 }
@@ -1358,7 +1364,8 @@ int tmps_adj_initial(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps
     if (!sys_ok(s) || !p || !tape || !tape->xh || !tape->vh || !tape->wh || !d_xbuild || !d_disp)
         return TMPS_ERR_BAD_ARG;
     if (s->n == 0) return TMPS_OK;
-    run(k_initial, grid_for(s->n, kBlk), kBlk, (cudaStream_t)stream, *s, p->dt, *tape, (const double*)nullptr,
+    Chain ch{(cudaStream_t)stream};
+    ch.run(k_initial, grid_for(s->n, kBlk), kBlk, *s, p->dt, *tape, (const double*)nullptr,
         (const tmps_adj_rec*)nullptr, (const tmps_adj_rec*)nullptr, d_xbuild, (unsigned long long*)d_disp,
         (Queue*)nullptr, (int64_t)0, 0.0);
     return ok() ? TMPS_OK : TMPS_ERR_CUDA;
@@ -1369,11 +1376,11 @@ int tmps_adj_finish(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps_
     if (!sys_ok(s) || !p || !sv || !tape || !d_rec || step < 1 || !work || !tape->xh || !tape->shear || !tape->mask ||
         !tape->f || !tape->t)
         return TMPS_ERR_BAD_ARG;
-    cudaStream_t st = (cudaStream_t)stream;
-    const int rc = rest_of_step(s, p, sv, *tape, d_rec, step, carve(work, s->n, s->npairs), nullptr, st);
+    Chain ch{(cudaStream_t)stream};
+    const int rc = rest_of_step(s, p, sv, *tape, d_rec, step, carve(work, s->n, s->npairs), nullptr, ch);
     if (rc != TMPS_OK) return rc;
     if (s->n > 0)
-        run(k_remap, grid_for(s->n, kBlk), kBlk, st, s->n, (const double*)tape->xh, (const tmps_adj_rec*)(d_rec + (step - 1)),
+        ch.run(k_remap, grid_for(s->n, kBlk), kBlk, s->n, (const double*)tape->xh, (const tmps_adj_rec*)(d_rec + (step - 1)),
             (const tmps_adj_rec*)(d_rec + step), s->x, (const Queue*)nullptr);
     return ok() ? TMPS_OK : TMPS_ERR_CUDA;
 }
@@ -1387,6 +1394,7 @@ int tmps_adj_forward(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps
         pair_stride < 0)
         return TMPS_ERR_BAD_ARG;
     cudaStream_t st = (cudaStream_t)stream;
+    Chain ch{st};
     Work W = carve(work, s->n, s->npairs);
     Queue* q = reinterpret_cast<Queue*>(d_queue);
     if (cudaMemsetAsync(q, 0, sizeof(Queue), st) != cudaSuccess) return TMPS_ERR_CUDA;
@@ -1395,15 +1403,15 @@ int tmps_adj_forward(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps
     for (int64_t step = first; step <= last; ++step) {
         t = tape_at(*tape, atom_stride, pair_stride, step - first);
         if (s->n > 0)
-            run(k_initial, grid_for(s->n, kBlk), kBlk, st, *s, p->dt, t, xlast,
+            ch.run(k_initial, grid_for(s->n, kBlk), kBlk, *s, p->dt, t, xlast,
                 (const tmps_adj_rec*)(step > first ? d_rec + (step - 2) : nullptr), (const tmps_adj_rec*)(d_rec + (step - 1)),
                 d_xbuild, (unsigned long long*)nullptr, q, step, trigger_sq);
-        const int rc = rest_of_step(s, p, sv, t, d_rec, step, W, q, st);
+        const int rc = rest_of_step(s, p, sv, t, d_rec, step, W, q, ch);
         if (rc != TMPS_OK) return rc;
         xlast = t.xh;
     }
     if (s->n > 0)
-        run(k_remap, grid_for(s->n, kBlk), kBlk, st, s->n, (const double*)t.xh, (const tmps_adj_rec*)(d_rec + (last - 1)),
+        ch.run(k_remap, grid_for(s->n, kBlk), kBlk, s->n, (const double*)t.xh, (const tmps_adj_rec*)(d_rec + (last - 1)),
             (const tmps_adj_rec*)(d_rec + last), s->x, (const Queue*)q);
     return ok() ? TMPS_OK : TMPS_ERR_CUDA;
 }
@@ -1419,6 +1427,7 @@ int tmps_adj_reverse(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps
         (s->npairs > 0 && !b->shear))
         return TMPS_ERR_BAD_ARG;
     cudaStream_t st = (cudaStream_t)stream;
+    Chain ch{st};
     Work W = carve(work, s->n, s->npairs);
     const int nbA = grid_for(s->n, kBlk), nbP = grid_for(s->npairs, kPairTile);
     if (s->n == 0 && cudaMemsetAsync(W.partk, 0, sizeof(double) * 6 * nbA, st) != cudaSuccess) return TMPS_ERR_CUDA;
@@ -1429,26 +1438,29 @@ int tmps_adj_reverse(const tmps_adj_sys* s, const tmps_adj_params* p, const tmps
         if (step == last && !linked) {
             // the remap and the servo of the last step; else the call for the steps after it did them
             if (s->n > 0)
-                run(k_b_atoms, nbA, kBlk, st, *s, p->dt, 0, 0, (const uint8_t*)nullptr, none, none, (const double*)t.xh,
+                ch.run(k_b_atoms, nbA, kBlk, *s, p->dt, 0, 0, (const uint8_t*)nullptr, none, none, (const double*)t.xh,
                     rec(step - 1), rec(step), *b, W);
-            run(k_b_servo, 1, kOne, st, *sv, p->dt, step, rec(step - 1), rec(step), qbar[step - first + 1], nbA, nbP, 0, 1, 0,
+            ch.run(k_b_servo, 1, kOne, *sv, p->dt, step, rec(step - 1), rec(step), qbar[step - first + 1], nbA, nbP, 0, 1, 0,
                 *b, W);
         }
         const double* xh = step > first ? tape_at(*tape, atom_stride, pair_stride, step - 1 - first).xh : d_xprev;
         if (s->n > 0) {
-            run(k_b_final, nbA, kBlk, st, *s, p->dt, t, *b, W);
+            ch.run(k_b_final, nbA, kBlk, *s, p->dt, t, *b, W);
             if (s->npairs > 0)
-                run_b_pairs(nbP, st, *s, to_params(*p), 1, (const double*)t.xh, (const double*)t.vh,
+                ch.run_b_pairs(nbP, *s, to_params(*p), 1, (const double*)t.xh, (const double*)t.vh,
                     (const double*)t.wh, (const double*)t.shear, (const uint8_t*)t.mask, rec(step - 1),
                     (const double*)W.wbar, *b, W);
             const tmps_adj_tape tp = step > first ? tape_at(*tape, atom_stride, pair_stride, step - 1 - first) : t;
             // (with no pairs it follows k_b_final, whose velocities it reads before its wait)
-            run_as(s->npairs == 0, k_b_atoms, nbA, kBlk, st, *s, p->dt, 1, 1, (const uint8_t*)t.mask,
+            if (s->npairs == 0) ch.join();
+            ch.run(k_b_atoms, nbA, kBlk, *s, p->dt, 1, 1, (const uint8_t*)t.mask,
                 step > first ? (const double*)tp.f : d_fprev, step > first ? (const double*)tp.t : d_tprev, xh,
                 xh ? rec(step - 2) : rec(step - 1), xh ? rec(step - 1) : rec(step), *b, W);
         }
-        // (the slot of record step - 1 takes the image terms of this step's contacts)
-        run(k_b_servo, 1, kOne, st, *sv, p->dt, step - 1, rec(step > 1 ? step - 2 : 0), rec(step - 1), qbar[step - first], nbA,
+        // (the slot of record step - 1 takes the image terms of this step's contacts; with no atoms the
+        // launch before is another of itself, whose sums it reads before its wait)
+        if (s->n == 0) ch.join();
+        ch.run(k_b_servo, 1, kOne, *sv, p->dt, step - 1, rec(step > 1 ? step - 2 : 0), rec(step - 1), qbar[step - first], nbA,
             nbP, s->npairs > 0 ? 1 : 0, xh ? 1 : 0, (int)((step - 1) & 1), *b, W);
     }
     return ok() ? TMPS_OK : TMPS_ERR_CUDA;
@@ -1467,14 +1479,14 @@ int tmps_adj_setup_back(const tmps_adj_sys* s, const tmps_adj_params* p, const t
         !b->radius || !b->mass || !b->params || !b->box || (s->npairs > 0 && (!b->shear || !tape->shear || !tape->mask)))
         return TMPS_ERR_BAD_ARG;
     if (s->n == 0 || s->npairs == 0) return TMPS_OK;
-    cudaStream_t st = (cudaStream_t)stream;
+    Chain ch{(cudaStream_t)stream};
     Work W = carve(work, s->n, s->npairs);
     const int nbA = grid_for(s->n, kBlk), nbP = grid_for(s->npairs, kPairTile);
     const double* none = nullptr;
-    run_b_pairs(nbP, st, *s, to_params(*p), 0, (const double*)s->x, (const double*)s->v, (const double*)s->w,
+    ch.run_b_pairs(nbP, *s, to_params(*p), 0, (const double*)s->x, (const double*)s->v, (const double*)s->w,
         (const double*)tape->shear, (const uint8_t*)tape->mask, d_box, none, *b, W);
-    run(k_b_atoms, nbA, kBlk, st, *s, p->dt, 1, 0, (const uint8_t*)tape->mask, none, none, none, d_box, d_box, *b, W);
-    run(k_b_servo, 1, kOne, st, tmps_adj_servo{}, p->dt, (int64_t)1, d_box, d_box, 0.0, nbA, nbP, 1, 0, 0, *b, W);
+    ch.run(k_b_atoms, nbA, kBlk, *s, p->dt, 1, 0, (const uint8_t*)tape->mask, none, none, none, d_box, d_box, *b, W);
+    ch.run(k_b_servo, 1, kOne, tmps_adj_servo{}, p->dt, (int64_t)1, d_box, d_box, 0.0, nbA, nbP, 1, 0, 0, *b, W);
     return ok() ? TMPS_OK : TMPS_ERR_CUDA;
 }
 
