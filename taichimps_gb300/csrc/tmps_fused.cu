@@ -104,12 +104,32 @@ __device__ __forceinline__ void block_sum_dw(float (&h)[NV], float (&l)[NV], flo
     }
 }
 
-// Programmatic dependent launch.  The four kernels of a step are launched
-// with programmatic stream serialization, so each may be scheduled while its
-// predecessor drains.  Each one first waits for its predecessor grid to
-// complete and its writes to be visible (griddepcontrol.wait: a hardware
-// wait, no spin), and only then touches memory and lets its own successor be
-// scheduled.  Waits chain, so every earlier kernel has completed too.
+// Programmatic dependent launch.  The kernels of a step are launched with
+// programmatic stream serialization.  Each waits for its predecessor grid to
+// complete and its writes to be visible (griddepcontrol.wait: a hardware wait,
+// no spin) before it lets its own successor be scheduled, so when a block
+// starts, every launch but the one right before it has completed.  Before its
+// wait a kernel touches only what that one launch does not write:
+//
+//   A                 nothing
+//   C (k_cf)          the box and the engine's step constants (S or
+//                     tmps_fused_prepare), the gap order (used only in a pass
+//                     after the one behind tmps_fused_bounds); the launch before
+//                     is A, the bounds or a change of the histories' form
+//   k_pair_contacts   the same constants, the pairs and their touch bits; the
+//                     launch before is A or k_pair_back (which writes the rows'
+//                     pair indices alone)
+//   k_pair_gather     nothing
+//   k_walls           the state, the engine record, the walls' flag words and
+//                     histories (these it also writes); the launch before is C
+//                     or the gather
+//   S                 the box, servo and engine records (C and the gather write
+//                     of these only final_pending, which S sets itself) and A's
+//                     partial sums; the launch before is C or the gather
+//
+// A batch's kernels read their instance's descriptor too, which no kernel
+// writes.  A pointer to words that the launch before writes and that are read
+// after the wait carries no __restrict__, which would let a load cross it.
 // A history component in the row atom's own sense: the two copies of a
 // contact are exact negatives (for a double word, both words negated).
 __device__ __forceinline__ double hsign(double h, bool keep) { return keep ? h : -h; }
@@ -141,7 +161,7 @@ __host__ __device__ inline size_t lay_kin(int n) { return lay_keys(n) + lay_roun
 __host__ __device__ inline size_t lay_wall(int n) { return lay_kin(n) + lay_round256((size_t)lay_groups(n) * 8 * sizeof(double)); }
 __host__ __device__ inline size_t lay_part(int n) { return lay_wall(n) + lay_round256((size_t)lay_groups(n) * sizeof(uint32_t)); }
 
-__device__ __forceinline__ bool rebuild_due(const tmps_engine* __restrict__ e, int64_t s) {
+__device__ __forceinline__ bool rebuild_due(const tmps_engine* e, int64_t s) {
     const int64_t since = s - e->last_build_step;
     if (since <= 0) return false;  // built in this very step already
     if (since < e->delay) return false;
@@ -154,7 +174,7 @@ __device__ __forceinline__ bool rebuild_due(const tmps_engine* __restrict__ e, i
 
 // Running maximum of |x - x0|^2 since the reference of the contact bounds
 // (non-negative FP32 values order as their bit patterns; NaN above all).
-__device__ __forceinline__ void note_displacement(tmps_engine* __restrict__ e, float dd) {
+__device__ __forceinline__ void note_displacement(tmps_engine* e, float dd) {
     const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(dd));
     if ((threadIdx.x & 31) == 0 && m > *(volatile uint32_t*)&e->maxd2_bits) atomicMax(&e->maxd2_bits, m);
 }
@@ -163,7 +183,7 @@ __device__ __forceinline__ void note_displacement(tmps_engine* __restrict__ e, f
 // the step in hand (0: none, the launches do nothing) and whether C walks the
 // gap order.  Where no servo runs, C's own first block moves step and aborted
 // on (step_done), so the kernels after A must not read those.
-__device__ __forceinline__ void open_step(tmps_engine* __restrict__ e, int bid, bool idle) {
+__device__ __forceinline__ void open_step(tmps_engine* e, int bid, bool idle) {
     if (bid == 0 && threadIdx.x == 0) {
         e->attempt = idle ? 0 : e->step + 1;
         e->walk_order = e->order_ready;
@@ -172,7 +192,7 @@ __device__ __forceinline__ void open_step(tmps_engine* __restrict__ e, int bid, 
 
 // Bit of atom i in the flag words: its force and torque may be nonzero (the
 // words of C's first pass; all ones before the first pass after a build).
-__device__ __forceinline__ bool force_live(const uint32_t* __restrict__ flags, int i) {
+__device__ __forceinline__ bool force_live(const uint32_t* flags, int i) {
     return flags == nullptr || ((flags[i >> 5] >> (i & 31)) & 1u);
 }
 
@@ -221,9 +241,8 @@ __device__ __forceinline__ float bits_diff(double x, double x0, float& err, bool
 // What bounds it: on a nearly contact-free state the 88 bytes read and 32
 // written per atom (state x, v and the build position; x) against 9 FP64
 // instructions per atom (drift 3, remap 6).
-__device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __restrict__ b,
-                                         tmps_engine* __restrict__ e, const uint32_t* __restrict__ flags,
-                                         const uint32_t* __restrict__ wflags, double* __restrict__ kin,
+__device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* b, tmps_engine* e,
+                                         const uint32_t* flags, const uint32_t* wflags, double* __restrict__ kin,
                                          double* __restrict__ part, const int bid, const int nblk) {
     __shared__ double smem[6 * (kBlockA / 32)];
     pdl_enter();
@@ -237,7 +256,8 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
     const double dt = e->dt, dtf = 0.5 * dt;
     const bool fin = e->final_pending != 0, remap = b->remap_pending != 0;
     const bool kick_all = e->kick_all != 0 || !(dtf > 0.0);
-    const float trig32 = approx_f32(e->trigger_sq), trigd = sqrtf(trig32);
+    const double trig64 = e->trigger_sq;
+    const float trig32 = approx_f32(trig64), trigd = sqrtf(trig32);
     bool hit = false;
     float dd = 0.0f;
     double K[6] = {0, 0, 0, 0, 0, 0};
@@ -337,7 +357,7 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
             const double d0 = __dsub_rn(x.x, x0x), d1 = __dsub_rn(x.y, x0y), d2 = __dsub_rn(x.z, x0z);
             const double q = __dadd_rn(__dadd_rn(__dmul_rn(d0, d0), __dmul_rn(d1, d1)), __dmul_rn(d2, d2));
             // a non-finite displacement forces the rebuild, whose binning reports the position
-            far = !(q <= e->trigger_sq);
+            far = !(q <= trig64);
         }
         hit = hit || far;
         // the running maximum only has to bound |d|^2 from above (C's cull threshold)
@@ -353,9 +373,9 @@ __device__ __forceinline__ void a64_body(const tmps_atoms& a, const tmps_box* __
 
 // Three resident blocks per SM (80 registers): the contact-dense 110k update
 // runs in 19.7 instead of 22.5 us, the dilute 1M one in 33.4 instead of 34.9.
-__global__ void __launch_bounds__(kBlockA, 3) k_a64(tmps_atoms a, const tmps_box* __restrict__ b,
-                                                  tmps_engine* __restrict__ e, const uint32_t* __restrict__ flags,
-                                                  const uint32_t* __restrict__ wflags, double* __restrict__ kin,
+__global__ void __launch_bounds__(kBlockA, 3) k_a64(tmps_atoms a, const tmps_box* b, tmps_engine* e,
+                                                  const uint32_t* flags, const uint32_t* wflags,
+                                                  double* __restrict__ kin,
                                                   double* __restrict__ part) {
     a64_body(a, b, e, flags, wflags, kin, part, blockIdx.x, gridDim.x);
 }
@@ -396,8 +416,8 @@ __device__ __forceinline__ void store_vw(const tmps_atoms& a, int i, float4 v, f
 __device__ __forceinline__ float4 ld4f_cs(const float* p, int i) { return __ldcs(reinterpret_cast<const float4*>(p) + i); }
 __device__ __forceinline__ void st4f_cs(float* p, int i, float4 v) { __stcs(reinterpret_cast<float4*>(p) + i, v); }
 
-__device__ __forceinline__ void a32_body(const tmps_atoms& a, const tmps_box* __restrict__ b,
-                                         tmps_engine* __restrict__ e, const uint32_t* __restrict__ flags,
+__device__ __forceinline__ void a32_body(const tmps_atoms& a, const tmps_box* b, tmps_engine* e,
+                                         const uint32_t* flags,
                                          double* __restrict__ part, const int bid, const int nblk) {
     // Double-word state (hi + lo, both FP32) updated with error-free FP32
     // transforms: the FP64 pipe of this part is ~70x narrower than FP32, and
@@ -416,6 +436,7 @@ __device__ __forceinline__ void a32_body(const tmps_atoms& a, const tmps_box* __
     // merged half-kicks: the previous step's second and this step's first
     const float kick = e->final_pending ? dth : 0.5f * dth;
     const bool remap = b->remap_pending != 0;
+    const float trig32 = e->trigger32;
     bool hit = false;
     float dd = 0.0f;
     float Kh[6] = {0, 0, 0, 0, 0, 0}, Kl[6] = {0, 0, 0, 0, 0, 0};
@@ -464,7 +485,7 @@ __device__ __forceinline__ void a32_body(const tmps_atoms& a, const tmps_box* __
         const float d1 = ((p.y - o0y) + pl.y) + (float)cell_y(c) * e->dh32[1] + e->dlo32[1];
         const float d2 = ((p.z - o0z) + pl.z) + (float)cell_z(c) * e->dh32[2] + e->dlo32[2];
         const float q = (d0 * d0 + d1 * d1) + d2 * d2;
-        hit = hit || !(q <= e->trigger32);  // NaN included (see a64_body)
+        hit = hit || !(q <= trig32);  // NaN included (see a64_body)
         dd = q == q ? fmaxf(dd, q) : __int_as_float(0x7fffffff);
         // kinetic term from the high words (vel32.w = m)
         const float kin[6] = {(v.w * v.x) * v.x, (v.w * v.y) * v.y, (v.w * v.z) * v.z,
@@ -485,8 +506,8 @@ __device__ __forceinline__ void a32_body(const tmps_atoms& a, const tmps_box* __
 // Three resident blocks per SM (80 registers): at four (64 registers, no spill)
 // the step of 1M spheres is 1.5 % faster contact-free and 0.3 % slower jammed, at
 // five (spills) 15 % slower.
-__global__ void __launch_bounds__(kBlockA, 3) k_a32(tmps_atoms a, const tmps_box* __restrict__ b,
-                                                     tmps_engine* __restrict__ e, const uint32_t* __restrict__ flags,
+__global__ void __launch_bounds__(kBlockA, 3) k_a32(tmps_atoms a, const tmps_box* b, tmps_engine* e,
+                                                     const uint32_t* flags,
                                                      double* __restrict__ part) {
     a32_body(a, b, e, flags, part, blockIdx.x, gridDim.x);
 }
@@ -497,7 +518,7 @@ __global__ void __launch_bounds__(kBlockA, 3) k_a32(tmps_atoms a, const tmps_box
 // kernel in place of S: step and aborted move on (the other blocks go by
 // attempt), or the rebuild is marked.  Measured: a step of 4,000 spheres, FP64,
 // without S and with its blocks spread (a_blocks) 32 -> 25.4 us.
-__device__ __forceinline__ void step_done(tmps_engine* __restrict__ E, int64_t s, bool due) {
+__device__ __forceinline__ void step_done(tmps_engine* E, int64_t s, bool due) {
     if (!E->fold) return;
     if (due) {
         E->aborted = 1;
@@ -806,7 +827,7 @@ struct CfEnv {
     bool vremap, hist, roll;
 
     __device__ __forceinline__ void load(const tmps_pair_params& P, const tmps_box* __restrict__ B,
-                                         const tmps_engine* __restrict__ E) {
+                                         const tmps_engine* E) {
         hist = kHist && (STYLE != STYLE_GRANULAR || P.tangential_id >= 2 || P.rolling_id != 0);
         roll = STYLE == STYLE_GRANULAR && P.rolling_id != 0;
         if constexpr (MIXED) dt = E->dt_hi;
@@ -1112,8 +1133,8 @@ __device__ __forceinline__ void kinetic_change(T mi, T im, T hdt, const T (&F)[3
 
 template <int STYLE, bool MIXED>
 __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L, const tmps_pair_params& P,
-                                        const tmps_box* __restrict__ B, tmps_engine* __restrict__ E,
-                                        uint32_t* __restrict__ flags, const float* __restrict__ gap,
+                                        const tmps_box* __restrict__ B, tmps_engine* E,
+                                        uint32_t* flags, const float* __restrict__ gap,
                                         const float* __restrict__ agap, const int32_t* __restrict__ order,
                                         const float* __restrict__ sgap, double* __restrict__ part, const int bid,
                                         const int nblk) {
@@ -1140,18 +1161,17 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
     const int nwarps = (nblk * blockDim.x) >> 5;
     // consecutive groups (neighbours in space) go to consecutive blocks
     const int gw = bid + nblk * (threadIdx.x >> 5);
-    // the warp's first groups' words, the last C's and the bounds' (before the wait: one round trip
-    // off the chain, an FP64 step of 1M spheres 72.7 -> 71.4 us, a mixed one 36.7 -> 36.2)
+    // the warp's first groups in the gap order (before the wait: one round trip off the chain, an FP64
+    // step of 1M spheres 72.7 -> 71.4 us, a mixed one 36.7 -> 36.2).  The ordered pass alone uses them,
+    // and a pass over the bounds has gone before it; the pass right behind the bounds reads their words
+    // after its wait.
     int grp0 = 0;
-    float sgap0 = 0.0f, gap0 = 0.0f;
-    uint32_t flag0 = 0u;
+    float sgap0 = 0.0f;
     {
         const int k = gw + (threadIdx.x & 31) * nwarps;
         if (k < ngroups) {
             grp0 = order[k];
             sgap0 = sgap[k];
-            gap0 = gap[k];
-            flag0 = flags[k];
         }
     }
     pdl_enter();
@@ -1558,8 +1578,8 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
                 mygrp = base == gw ? grp0 : order[k];
                 live = !((base == gw ? sgap0 : sgap[k]) > thr);
             } else {
-                myold = base == gw ? flag0 : flags[mygrp];
-                live = !(cull && (base == gw ? gap0 : gap[mygrp]) > thr);
+                myold = flags[mygrp];
+                live = !(cull && gap[mygrp] > thr);
                 if (!live && myold != 0u) {
                     // ruled out now, flagged last step: clear the stale forces
                     for (uint32_t w = myold; w; w &= w - 1) zero_force<MIXED>(A, (mygrp << 5) + __ffs(w) - 1);
@@ -1665,7 +1685,7 @@ __device__ __forceinline__ void cf_body(const tmps_atoms& A, const tmps_nlist& L
 template <int STYLE, bool MIXED>
 __global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
     k_cf(tmps_atoms A, tmps_nlist L, tmps_pair_params P, const tmps_box* __restrict__ B,
-         tmps_engine* __restrict__ E, uint32_t* __restrict__ flags, const float* __restrict__ gap,
+         tmps_engine* E, uint32_t* flags, const float* __restrict__ gap,
          const float* __restrict__ agap, double* __restrict__ part) {
     const char* sc = reinterpret_cast<const char*>(flags);  // the scratch base
     cf_body<STYLE, MIXED>(A, L, P, B, E, flags, gap, agap, reinterpret_cast<const int32_t*>(sc + lay_order(A.n)),
@@ -1852,7 +1872,7 @@ constexpr int kPairRing = 64;  // queued pairs per warp: < 32 waiting + 32 from 
 
 template <int STYLE, bool MIXED>
 __global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
-    k_pair_contacts(tmps_atoms A, tmps_pair_params P, const tmps_box* __restrict__ B, const tmps_engine* __restrict__ E,
+    k_pair_contacts(tmps_atoms A, tmps_pair_params P, const tmps_box* __restrict__ B, const tmps_engine* E,
                     PairLay Q, int np) {
     using T = typename CfEnv<STYLE, MIXED>::T;
     using HT = typename CfLoad<MIXED>::HT;
@@ -2069,8 +2089,8 @@ constexpr int kCompG = 6 / kSubG;         // virial components a sub-block adds
 // warps and the additions spread over all of them.
 template <int STYLE, bool MIXED>
 __global__ void __launch_bounds__(kBlockG, MIXED ? 4 : 3)
-    k_pair_gather(tmps_atoms A, tmps_nlist L, const tmps_box* __restrict__ B, tmps_engine* __restrict__ E,
-                  uint32_t* __restrict__ flags, double* __restrict__ part, PairLay Q) {
+    k_pair_gather(tmps_atoms A, tmps_nlist L, const tmps_box* __restrict__ B, tmps_engine* E,
+                  uint32_t* flags, double* __restrict__ part, PairLay Q) {
     using T = typename std::conditional<MIXED, float, double>::type;
     using W4 = typename std::conditional<MIXED, float4, double2>::type;
     constexpr int kW = MIXED ? kRecWords<STYLE> / 4 : kRecDoubles<STYLE> / 2;  // 16-byte words of a record
@@ -2280,8 +2300,8 @@ struct WallList {
 // warps over the SMs' FP64 units.  3,001 spheres in a cylinder: 30 us a
 // step with the walls in the fused step, 85 us hook by hook.
 constexpr int kBlockW = 32;
-__global__ void __launch_bounds__(kBlockW) k_walls(tmps_atoms A, const tmps_engine* __restrict__ E,
-                                                   const uint32_t* __restrict__ flags, uint32_t* __restrict__ wflags,
+__global__ void __launch_bounds__(kBlockW) k_walls(tmps_atoms A, const tmps_engine* E,
+                                                   const uint32_t* flags, uint32_t* __restrict__ wflags,
                                                    const __grid_constant__ WallList L) {
     const int lane = threadIdx.x & 31, n = A.n;
     const int i = blockIdx.x * kBlockW + threadIdx.x;
