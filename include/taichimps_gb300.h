@@ -472,12 +472,11 @@ int tmps_fused_a(const tmps_atoms* a, tmps_box* d_box, tmps_engine* d_eng, int32
  * caller memory: flag words, per-group and per-atom gaps, then the
  * d_eng->nblocks virial partial sums, A's blocks then C's).  c_blocks: C's
  * grid from tmps_fused_shape, or <= 0 for the default; d_eng->nblocks must be
- * A's blocks + C's blocks of the same shape.  `rows` is taken and ignored: the
- * path for contact-dense states is tmps_fused_c_pairs, and both sum each atom's
- * contacts in slot order and keep the flag words' meaning, so they may
- * alternate between builds. */
+ * A's blocks + C's blocks of the same shape.  The path for contact-dense states
+ * is tmps_fused_c_pairs; both sum each atom's contacts in slot order and keep
+ * the flag words' meaning, so they may alternate between builds. */
 int tmps_fused_c(const tmps_atoms* a, const tmps_nlist* nl, const tmps_box* d_box, tmps_engine* d_eng,
-                 const tmps_pair_params* p, int32_t c_blocks, void* scratch, int32_t rows, void* stream);
+                 const tmps_pair_params* p, int32_t c_blocks, void* scratch, void* stream);
 
 /* C for contact-dense states: every contact evaluated once, over the half list
  * of pairs (i < j in internal order) of the rows, then each atom's row summed

@@ -225,7 +225,7 @@ _SIGS = {
                                   ctypes.POINTER(PairParams), c_i32, c_vp, c_vp]),
     "tmps_fused_a": (c_i32, [ctypes.POINTER(Atoms), c_vp, c_vp, c_i32, c_vp, c_vp]),
     "tmps_fused_c": (c_i32, [ctypes.POINTER(Atoms), ctypes.POINTER(NList), c_vp, c_vp,
-                             ctypes.POINTER(PairParams), c_i32, c_vp, c_i32, c_vp]),
+                             ctypes.POINTER(PairParams), c_i32, c_vp, c_vp]),
     "tmps_pairs_bytes": (ctypes.c_int64, [c_i32, c_i32, c_i32, c_i32, c_i32, c_i32]),
     "tmps_pairs_build": (c_i32, [ctypes.POINTER(NList), ctypes.POINTER(PairParams), c_i32, c_i32, c_vp, c_vp]),
     "tmps_pairs_history": (c_i32, [ctypes.POINTER(NList), ctypes.POINTER(PairParams), c_i32, c_i32, c_vp, c_vp]),

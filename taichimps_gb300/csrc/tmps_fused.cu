@@ -3213,12 +3213,11 @@ int tmps_fused_a(const tmps_atoms* a, tmps_box* d_box, tmps_engine* d_eng, int32
 }
 
 int tmps_fused_c(const tmps_atoms* a, const tmps_nlist* nl, const tmps_box* d_box, tmps_engine* d_eng,
-                 const tmps_pair_params* p, int32_t c_blocks, void* scratch, int32_t rows, void* stream) {
+                 const tmps_pair_params* p, int32_t c_blocks, void* scratch, void* stream) {
     if (!a || !nl || !d_box || !d_eng || !p || !scratch || a->n < 0 || nl->n != a->n) return TMPS_ERR_BAD_ARG;
     if (!a->pos32 && !a->rinv) return TMPS_ERR_BAD_ARG;
     if (p->style < 0 || p->style > 4 || nl->slots < 1 || nl->slots > kMaxSlots) return TMPS_ERR_BAD_ARG;
     if (p->style == 4 && p->rolling_id != 0 && !nl->rolling) return TMPS_ERR_BAD_ARG;
-    (void)rows;  // once chose a path for contact-dense states, which tmps_fused_c_pairs is now
     const int n = a->n;
     const bool mixed = a->pos32 != nullptr;
     const int g2def = contact_blocks(n, p->style, mixed);

@@ -353,8 +353,7 @@ class FusedEngine:
             _lib.check(L.tmps_fused_c_pairs(atoms, nl_struct, dbox, eng, params, self.c_blocks, part, self.npairs,
                                             self.pairs.data_ptr(), st), "tmps_fused_c_pairs")
         else:
-            _lib.check(L.tmps_fused_c(atoms, nl_struct, dbox, eng, params, self.c_blocks, part, 0, st),
-                       "tmps_fused_c")
+            _lib.check(L.tmps_fused_c(atoms, nl_struct, dbox, eng, params, self.c_blocks, part, st), "tmps_fused_c")
         if self.walls:
             with _device.timed("wall"):
                 rc = L.tmps_fused_walls(atoms, eng, self._wall_args, len(self.walls), part, st)

@@ -42,7 +42,7 @@ def test_contacts_behind_the_bounds(gpu, precision, cull):
         if sync:
             torch.cuda.synchronize()
         _lib.check(L.tmps_fused_c(atoms, nl, sim.domain.dbox, eng._eng.data_ptr(), par, eng.c_blocks, eng.part.data_ptr(),
-                                  *ROWS, st), "tmps_fused_c")
+                                  st), "tmps_fused_c")
         return force.clone()
 
     want = once(True)
@@ -50,6 +50,3 @@ def test_contacts_behind_the_bounds(gpu, precision, cull):
     assert 0 < touching < n and float(want.abs().max()) != 7.0
     for _ in range(40):
         assert torch.equal(once(False), want)
-
-
-ROWS = (0,)
