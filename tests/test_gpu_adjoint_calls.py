@@ -96,3 +96,22 @@ def test_reverse_one_step_a_call(gpu, monkeypatch):
     for k, w in want.items():
         w, g = torch.as_tensor(w).cpu(), torch.as_tensor(got[k]).cpu()
         assert float((w - g).abs().max()) <= 1e-12 * float(w.abs().max()), k
+
+
+def test_queue_follows_the_rebuilds(gpu):
+    """Frequent rebuilds under one long checkpoint: the launches stay near five a step, and the run is that of
+    short checkpoints bit for bit."""
+    from taichimps_gb300 import _device
+    got = []
+    for ckpt in (300, 7):
+        job = _job(steps=300, every=50, ckpt=ckpt, skin=0.005, v=3.0)
+        n0 = _device.lib().tmps_launch_count()
+        q = job.forward(**PRM)
+        got.append((q.cpu().numpy(), job.q_all(), job.rebuilds, _device.lib().tmps_launch_count() - n0))
+    (qa, ra, na, la), (qb, rb, nb, _) = got
+    assert na == nb >= 10
+    np.testing.assert_array_equal(qa, qb)
+    np.testing.assert_array_equal(ra, rb)
+    # five launches a step, a remap per queue, a pair list (some 20 launches) per rebuild, and as much again
+    # for what is queued past a rebuild
+    assert la < 2 * (6 * 300 + 20 * na), la
