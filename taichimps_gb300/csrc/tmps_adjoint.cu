@@ -963,9 +963,11 @@ __global__ void __launch_bounds__(kBlk) k_b_final(tmps_adj_sys S, double dt, tmp
 // entering history's adjoint in place, parameter and image partials.
 //
 // kPerSM: resident blocks asked of the compiler.  Four leave it all 255
-// registers and are a wave for up to 608 tiles; beyond that five (168, with
-// spills) were faster: the gradient of 31,250 spheres (806 tiles) 29.5 -> 27.9
-// ms, while that of 2,048 (52 tiles) was 3 % slower with five.
+// registers; five have 168 and spill.  Five pay where they take up most of a
+// second wave of four and no more (run_b_pairs).  Gradient of 60 steps, four
+// against five, by the tiles (608 and 760 a wave): 46 6.26 and 6.56 ms, 180
+// 7.56 and 7.87, 401 10.46 and 10.20, 602 11.08 and 12.16, 803 14.10 and 13.24,
+// 1,201 15.18 and 17.30, 1,606 21.28 and 21.62, 3,212 38.5 and 39.4.
 template <int kPerSM>
 __global__ void __launch_bounds__(kBlk, kPerSM) k_b_pairs(tmps_adj_sys S, Params P, int shearupdate, const double* xs,
                                                   const double* vs, const double* ws, const double* __restrict__ sh_rec,
@@ -1227,10 +1229,12 @@ struct Chain {
     }
     // the next launch reads before its wait what the one before it writes
     void join() { first = true; }
-    // The contact pass's reverse at the residency its number of tiles wants.
+    // The contact pass's reverse at the residency its number of tiles wants: with five blocks an SM
+    // between one wave of four and one and a half.
     template <typename... A>
     void run_b_pairs(int tiles, A&&... args) {
-        if (tiles <= 608) run(k_b_pairs<4>, tiles, kBlk, std::forward<A>(args)...);
+        static const int wave = wave_blocks(k_b_pairs<4>, kBlk);
+        if (tiles <= wave || tiles > wave + wave / 2) run(k_b_pairs<4>, tiles, kBlk, std::forward<A>(args)...);
         else run(k_b_pairs<5>, tiles, kBlk, std::forward<A>(args)...);
     }
 };

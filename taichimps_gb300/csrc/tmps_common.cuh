@@ -25,6 +25,24 @@ void note_launches(int k);
 // one word per 4,096 of them (two launches, tmps_nlist.cu).
 void exclusive_scan(const int32_t* count, int32_t* start, int32_t* tile_sum, int m, cudaStream_t s);
 
+inline int sm_count() {
+    static const int sms = [] {
+        int dev = 0, v = 0;
+        return cudaGetDevice(&dev) == cudaSuccess &&
+                       cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0
+                   ? v
+                   : 152;
+    }();
+    return sms;
+}
+// One wave of resident blocks: the occupancy of a kernel times the SMs.
+template <typename K>
+int wave_blocks(K kernel, int block) {
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, block, 0) != cudaSuccess || occ < 1) occ = 1;
+    return occ * sm_count();
+}
+
 inline int grid_for(int64_t n, int block) {
     int64_t g = (n + block - 1) / block;
     return (int)(g < 1 ? 1 : g);

@@ -3013,27 +3013,8 @@ bool mixed_ok(const tmps_atoms* a) {
            a->torque32 && a->o0_32;
 }
 
-int sm_count() {
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0, v = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess &&
-            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0)
-            sms = v;
-        else
-            sms = 152;
-    }
-    return sms;
-}
-// Grids of the two passes of C: exactly one wave of resident blocks each
-// (occupancy of the kernel instance x SMs), so the static grid-stride split
-// leaves no partial second wave.
-template <typename K>
-int wave_blocks(K kernel, int block) {
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, block, 0) != cudaSuccess || occ < 1) occ = 1;
-    return occ * sm_count();
-}
+// Grids of the two passes of C: exactly one wave of resident blocks each, so
+// the static grid-stride split leaves no partial second wave.
 int contact_wave(int style, bool mixed) {
     static int w[5][2] = {};
     if (style < 0 || style > 4) style = 4;
