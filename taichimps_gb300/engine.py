@@ -295,23 +295,28 @@ class FusedEngine:
             self.npairs = int(got[0][at:at + 8].view(np.int64)[0])
             self.rows = self.contact_path == "rows" or touching * 2 > self._n
             self.rows = self.rows and self._n > 0 and self.npairs <= self.MAX_PAIRS
-        if self.rows:
-            self._build_pairs()
-        else:
+        self.rows = self.rows and self._build_pairs()
+        if not self.rows:
             self._history_form(True)
 
-    def _build_pairs(self) -> None:
-        """The rows path's pair buffer for the current list, with the contact histories."""
+    def _build_pairs(self) -> bool:
+        """The rows path's pair buffer for the current list, with the contact histories; False (and nothing
+        changed) where the device has no room for it: the screened path, which keeps no records, has the
+        same results."""
         sim = self.sim
         nl, par, L = sim.neighbor, sim.pair_style.params, _device.lib()
         mixed = 1 if self.mixed else 0
         need = int(L.tmps_pairs_bytes(self._n, nl.slots, self.npairs, int(par.style), mixed, int(par.rolling_id)))
         if self.pairs is None or self.pairs.numel() < need:
             self.pairs = None
-            self.pairs = torch.empty(need, dtype=torch.uint8, device=self.dev)
+            try:
+                self.pairs = torch.empty(need, dtype=torch.uint8, device=self.dev)
+            except torch.OutOfMemoryError:
+                return False
         _lib.check(L.tmps_pairs_build(sim.history.cstruct(nl), par, self.npairs, mixed, self.pairs.data_ptr(),
                                       _device.stream()), "tmps_pairs_build")
         self._in_pairs = True
+        return True
 
     def _history_back(self) -> None:
         """The contact histories back in the list's rows as doubles, both copies of each."""
