@@ -95,6 +95,7 @@ class FusedEngine:
         self._dummy_servo = _device.struct_buffer(_lib.Servo())
         self._n = -1
         self.rebuilds = 0
+        self._stepped = False  # whether run() was called since begin()
         self._interval = self.chunk  # steps between the last two builds
         # A chunk of `chunk` steps is captured once as a CUDA graph and replayed;
         # a rebuild swaps buffers, so the graph is captured again after one.
@@ -213,6 +214,7 @@ class FusedEngine:
         atom, nl = sim.atom, sim.neighbor
         n = atom.nlocal
         self._alloc(n)
+        self._stepped = False
         if sim.pair_style.params.rolling_id:
             sim.history.enable_rolling()
         if self.mixed:
@@ -276,10 +278,12 @@ class FusedEngine:
         _lib.check(rc, "tmps_fused_bounds")
         # one synchronisation for what the host needs before the steps: the counts of touching atoms
         # and of pairs (the contact path) and the status of a neighbor build that did not wait for the
-        # device
-        counts = self.contact_path != "screened"
+        # device.  The FP64 form asks for the counts once a list, with that status: a run of a few steps
+        # on the same list would wait longer for them (90 us a call) than for its steps.  The mixed form
+        # asks again, as contacts that formed since the build change its path.
+        ask = self.contact_path != "screened" and (self.mixed or nl.counts is None)
         items = []
-        if counts:
+        if ask:
             off = _lib.Engine.touching.offset
             items.append((self._eng[off:], None))
         if nl.status_pending:
@@ -287,12 +291,13 @@ class FusedEngine:
         got = _device.pull_many(items) if items else []
         if nl.status_pending:
             nl.check_status(int(got[-1].view(np.int32)[0]))
-        if counts:
+        if ask:
             # the bounds kernel counted the atoms whose gap bound is <= 0, and the pairs, into the
             # engine record
-            touching = int(got[0][:4].view(np.int32)[0])
             at = _lib.Engine.pairs.offset - off
-            self.npairs = int(got[0][at:at + 8].view(np.int64)[0])
+            nl.counts = int(got[0][:4].view(np.int32)[0]), int(got[0][at:at + 8].view(np.int64)[0])
+        if self.contact_path != "screened":
+            touching, self.npairs = nl.counts
             self.rows = self.contact_path == "rows" or touching * 2 > self._n
             self.rows = self.rows and self._n > 0 and self.npairs <= self.MAX_PAIRS
         self.rows = self.rows and self._build_pairs()
@@ -399,9 +404,11 @@ class FusedEngine:
         sim = self.sim
         L = _device.lib()
         st = _device.stream()
-        if not self.mixed and self._n > 0:
-            # the FP64 update's kept kinetic sums hold while only its own steps change a velocity
+        if self._stepped and not self.mixed and self._n > 0:
+            # the FP64 update's kept kinetic sums (none since the last bounds, if no step has been made)
+            # hold while only its own steps change a velocity
             _lib.check(L.tmps_fused_forget_kinetic(self._n, self.part.data_ptr(), st), "tmps_fused_forget_kinetic")
+        self._stepped = True
         start = sim.timestep
         target = start + int(nsteps)
         while True:

@@ -135,6 +135,8 @@ class NeighborList:
         self._atom = None
         self.status = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self._status_pending = False
+        # (touching atoms, pairs) of the list as the fused step counted them, None until it has
+        self.counts: tuple[int, int] | None = None
         self.flag = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self._ws = torch.zeros(0, dtype=torch.uint8, device=self.dev)
         self.nbr = self.nnb = self.prev_nbr = self.prev_nnb = None
@@ -204,6 +206,7 @@ class NeighborList:
         if atom.nlocal == 0:
             return
         self.check_status()  # an earlier deferred build's status first (this one clears the word)
+        self.counts = None
         L = _device.lib()
         self.domain.pull()
         self.setup_grid(2.0 * atom.max_radius)

@@ -1,0 +1,52 @@
+"""
+Runs of a few steps on a list that stands: what the host waits for, and that the contact path follows the list.
+"""
+
+import numpy as np
+import pytest
+
+from _twin import dense_packing, gpu_state, make_twin
+
+pytestmark = pytest.mark.gpu
+
+
+def _sim(oracle, lo=0.50, hi=0.56):
+    rng = np.random.default_rng(6)
+    x, r = dense_packing(rng, 343, 7.0, lo, hi)
+    sim, _ = make_twin(oracle, x, r, 2.5, [0.0] * 3, [7.0] * 3, v=rng.normal(scale=0.1, size=x.shape),
+                       pair="hertz/history", dt=5e-5, skin=0.1, cundall=(0.7, 0.7))
+    return sim
+
+
+def test_one_wait_a_run(gpu, oracle, monkeypatch):
+    """FP64 runs on the list of the run before: one read-back each, at the end (the counts were read with the
+    list).  A build drops them."""
+    from taichimps_gb300 import _device
+    sim = _sim(oracle)
+    sim.run(2)
+    kept = sim.neighbor.counts
+    assert kept is not None and sim.last_engine.rows
+    sim.run_pre = False
+    calls = []
+    pull = _device.pull_many
+    monkeypatch.setattr(_device, "pull_many", lambda items: (calls.append(len(items)), pull(items))[1])
+    for k in range(1, 4):
+        sim.run(1)
+        assert len(calls) == k and sim.last_engine.rows and sim.neighbor.counts == kept
+    sim.reneighbor_if_needed(force=True)
+    assert sim.neighbor.counts is None
+    sim.run(1)
+    nnb = sim.neighbor.nnb.cpu().numpy()
+    assert sim.neighbor.counts[1] * 2 == int(nnb.sum())
+
+
+@pytest.mark.parametrize("loose_first", [True, False])
+def test_path_follows_the_list(gpu, oracle, loose_first):
+    """Radii changed between runs with a build: the next list is counted anew."""
+    sim = _sim(oracle)
+    r = sim.atom.radius.to_numpy()[:343].copy()
+    for loose in (loose_first, not loose_first):
+        sim.atom.radius.from_numpy(r * (0.8 if loose else 1.0))
+        sim.run(3)
+        assert sim.last_engine.rows == (not loose)
+    assert np.isfinite(gpu_state(sim)["f"]).all()
