@@ -210,7 +210,7 @@ class Simulation:
             if fused > 0:
                 eng = FusedEngine(self, self.precision)
                 self.last_engine = eng
-                eng.begin()
+                eng.begin(steps=fused)
                 try:
                     eng.run(fused)
                 finally:

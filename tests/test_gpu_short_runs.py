@@ -50,3 +50,23 @@ def test_path_follows_the_list(gpu, oracle, loose_first):
         sim.run(3)
         assert sim.last_engine.rows == (not loose)
     assert np.isfinite(gpu_state(sim)["f"]).all()
+
+
+def test_few_mixed_steps_stay_screened(gpu, oracle):
+    """The shortest runs do not number the pairs; the two paths agree within the mixed form's rounding."""
+    runs = []
+    for steps in (4, 5):
+        sim = _sim(oracle)
+        sim.precision = "mixed"
+        sim.run(steps)
+        assert sim.last_engine.rows == (steps == 5)
+        assert (sim.neighbor.counts is not None) == (steps == 5)
+        runs.append(sim)
+    whole, parts = _sim(oracle), runs[0]
+    whole.precision = "mixed"
+    whole.run(5)
+    parts.run_pre = False
+    parts.run(1)
+    a, b = gpu_state(whole), gpu_state(parts)
+    for k in ("x", "v", "f"):
+        assert np.abs(a[k] - b[k]).max() <= 1e-4 * np.abs(a[k]).max(), k
