@@ -70,3 +70,34 @@ def test_few_mixed_steps_stay_screened(gpu, oracle):
     a, b = gpu_state(whole), gpu_state(parts)
     for k in ("x", "v", "f"):
         assert np.abs(a[k] - b[k]).max() <= 1e-4 * np.abs(a[k]).max(), k
+
+
+@pytest.mark.parametrize("steps,fused", [(2, False), (11, False), (12, True)])
+def test_few_steps_with_walls_go_hook_by_hook(gpu, steps, fused):
+    """Setting the fused step up costs what a dozen steps with walls save; the results are the hooks' either way."""
+    import taichimps_gb300 as G
+
+    def run(on):
+        rng = np.random.default_rng(2)
+        g = np.stack(np.meshgrid(*[np.arange(4)] * 3, indexing="ij"), -1).reshape(-1, 3) + 0.5
+        dom = G.Domain(boxlo=[0.0] * 3, boxhi=[4.0] * 3, boundary=("f", "f", "f"))
+        atom = G.AtomSystem(max_atoms=64)
+        atom.add_particles(x=g + rng.uniform(-0.04, 0.04, size=g.shape), radius=rng.uniform(0.48, 0.52, size=64),
+                           density=np.full(64, 2.5), v=rng.normal(0.0, 1.0, size=g.shape))
+        law = dict(kn=2e5, kt=2e5 * 2 / 7, gamman=50.0, gammat=25.0, xmu=0.5)
+        sim = G.Simulation(domain=dom, atom=atom, neighbor=G.NeighborList(domain=dom, skin=0.02, max_atoms=64),
+                           history=G.ContactHistory(max_atoms=64), pair=G.GranHookeHistory(domain=dom, dampflag=1, **law),
+                           dt=1e-4)
+        sim.add_fix(G.FixNVESphere(domain=dom))
+        sim.add_fix(G.FixWallGran(domain=dom, wall_axis=2, wall_side=-1, wall_coord=0.0, max_atoms=64, **law))
+        sim.fused = on
+        for _ in range(3):
+            sim.run(steps)
+            sim.run_pre = False
+        assert (getattr(sim, "last_engine", None) is not None) == (on and fused)
+        return gpu_state(sim)
+
+    a, b = run(True), run(False)
+    for k in ("x", "v", "omega", "f", "torque", "virial"):
+        # two orders of FP64 sums over at most 36 steps
+        assert np.abs(a[k] - b[k]).max() <= 1e-11 * max(np.abs(b[k]).max(), 1e-300), k
