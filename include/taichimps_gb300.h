@@ -556,9 +556,11 @@ int tmps_selftest_arith(int32_t which, const double* d_a, int32_t n, double* d_m
  * instance.  All instances share the arithmetic form (mixed) and the pair
  * style. */
 
-/* Blocks one instance of n atoms owns in the A and C grids under the default
- * launch shape (tmps_fused_shape with both counts 0).  An instance may
- * own any grid tmps_fused_shape gives; its engine's nblocks must match. */
+/* Blocks one instance of n atoms owns in the A and C grids of a batch by
+ * default: one 32-atom group per warp (tmps_fused_shape with both counts 1;
+ * with 0 it gives a single system's grids, which in the FP64 form spread a
+ * small one over the SMs).  An instance may own any grid tmps_fused_shape
+ * gives; its engine's nblocks must match. */
 int tmps_batch_blocks(int32_t n, int32_t style, int32_t mixed, int32_t* a_blocks, int32_t* c_blocks);
 
 int tmps_batch_a(const tmps_instance* d_inst, const int32_t* d_block_inst, int32_t nblocks, int32_t mixed,

@@ -3378,7 +3378,7 @@ int tmps_fused_pressure_log(tmps_engine* d_eng, double* h_log, int32_t len, void
 }
 
 int tmps_batch_blocks(int32_t n, int32_t style, int32_t mixed, int32_t* a_b, int32_t* c_b) {
-    return tmps_fused_shape(n, style, mixed, 0, 0, a_b, c_b);
+    return tmps_fused_shape(n, style, mixed, 1, 1, a_b, c_b);
 }
 
 int tmps_fused_shape(int32_t n, int32_t style, int32_t mixed, int32_t a_groups_per_warp, int32_t c_groups_per_warp,

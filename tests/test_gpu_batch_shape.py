@@ -39,3 +39,18 @@ def test_default_grids_of_a_batch(gpu, oracle, precision):
         for k in ("x", "v", "f"):
             np.testing.assert_array_equal(p[k], q[k], err_msg=k)
         np.testing.assert_array_equal(b.domain.prd, s.domain.prd)
+
+
+@pytest.mark.parametrize("mixed", [0, 1])
+def test_default_blocks_of_the_c_interface(gpu, mixed):
+    """tmps_batch_blocks: the grids of one group per warp, up to the wave."""
+    import ctypes
+    from taichimps_gb300 import _device, _lib
+    L = _device.lib()
+    for n in (1, 33, 500, 16000, 1_000_000):
+        got, want = [(ctypes.c_int32(), ctypes.c_int32()) for _ in range(2)]
+        assert L.tmps_batch_blocks(n, 3, mixed, *map(ctypes.byref, got)) == _lib.TMPS_OK
+        assert L.tmps_fused_shape(n, 3, mixed, 1, 1, *map(ctypes.byref, want)) == _lib.TMPS_OK
+        assert [v.value for v in got] == [v.value for v in want]
+        if n <= 16000:
+            assert [v.value for v in got] == [(n + 255) // 256, (n + 127) // 128]
