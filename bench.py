@@ -316,7 +316,7 @@ def run_gpu_arm(args, p, precision, rank, world):
     kern = {k: (sum(v) / len(v) if v else None) for k, v in timed.items()}
     return dict(sim=sim, n=n, ms=ms, launches=launches, clocks=clk, kern_ms=kern, n_nb=n_nb, n_c=n_c,
                 pressure=pressure, builds=sim.neighbor.build_count, rebuilds_timed=eng.rebuilds,
-                steps_run=sim.timestep, cull=cull, flagged=flagged)
+                steps_run=sim.timestep, cull=cull, flagged=flagged, rows=eng.rows)
 
 
 def run_e2e(args, p, precision):
@@ -542,6 +542,11 @@ def contact_bytes(precision: str, n_nb: float, n_c: float) -> float:
     return (84.0 if precision == "mixed" else 140.0) + 4.0 * n_nb + 52.0 * n_c
 
 
+# the contact-dense state's two contact kernels, timed together, and what holds them
+PAIR_KERNELS = "k_pair_contacts + k_pair_gather"
+DENSE_BOUND = {"mixed": "instruction issue", "fp64": "fp64 pipe"}
+
+
 def dense_traffic(kernel: str, precision: str):
     if not DENSE_TRAFFIC_FILE.exists():
         return None
@@ -578,14 +583,15 @@ def run_dense(args, rank, world, forms):
         kb = contact_bytes(prec, r["n_nb"], r["n_c"])
         c_ms = r["kern_ms"].get("fused_c")
         ach = kb * n / (c_ms * 1e-3) / 1e9 if c_ms else None
-        tr = dense_traffic(KERNEL_NAMES[("fused_c", prec)], prec)
+        name = PAIR_KERNELS if r["rows"] else KERNEL_NAMES[("fused_c", prec)]
+        tr = dense_traffic(name, prec)
         out["forms"][prec] = {
             "value": world * n * args.steps / (r["ms"] * 1e-3), "ms_per_step": r["ms"] / args.steps,
             "kernel_ms": r["kern_ms"], "neighbors_per_atom": r["n_nb"], "contacts_per_atom": r["n_c"],
             "flagged_atoms_frac": r["flagged"], "rebuilds_in_timed_steps": r["rebuilds_timed"],
             "mean_pressure": scal(r["pressure"]), "pressure": list(map(float, r["pressure"])),
             "gpu_launches": r["launches"], "clocks": r["clocks"],
-            "contact_kernel": {"kernel": KERNEL_NAMES[("fused_c", prec)], "bound": "hbm", "achieved": ach,
+            "contact_kernel": {"kernel": name, "bound": DENSE_BOUND[prec], "achieved": ach,
                                "peak": peak, "unit": "GB/s", "frac": (ach / peak) if ach else None,
                                "bytes_per_atom": kb, "algorithmic_bytes_per_launch": kb * n,
                                "bytes_formula": "S + 4 n_nb + 52 n_c, S = 84 mixed / 140 FP64",

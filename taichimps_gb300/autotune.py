@@ -145,8 +145,11 @@ def tune_launch_shape(batched, candidates=CANDIDATES, reps: int = 8) -> dict:
     best_a = min(a_us, key=lambda k: (a_us[k], k))
     # C's times on a quiet state hardly differ where the launch's own latency is all there is, and fewer,
     # fuller warps lose once contacts form: the smallest count within 5% of the best (24 systems of
-    # 500-16,000 spheres: 10.5, 10.3, 10.4, 10.1 us for 4, 8, 16, 32 groups per warp at the start, the
-    # run at 41.6, 41.4, 42.3, 45.5 ms)
+    # 500-16,000 spheres, mixed: 10.5, 10.3, 10.4, 10.1 us for 4, 8, 16, 32 groups per warp at the start,
+    # the run of 1,024 steps at 41.6, 41.4, 42.3, 45.5 ms when this was chosen; one batch.  Where C fills
+    # several waves, as with 512 systems, its times part by far more than 5% and the margin decides
+    # nothing).  The FP64 form's default grid, one group per block, is not among the candidates: a batch
+    # fills the SMs by its number of systems.
     fair = 1.05 * min(c_us.values())
     best_c = min(k for k in c_us if c_us[k] <= fair)
     return {"launch_shape": (best_a, best_c), "a_us": a_us, "c_us": c_us}

@@ -1,7 +1,8 @@
 // The fused step: Simulation._sub_step_inner (simulation.py:205-247) for
 // fix nve/sphere + optional damping/cundall + optional deform/pressure, as
-// three launches per step with no host round trip (see tmps_engine in the
-// header).
+// three launches per step (A, C, S; two where no servo runs, one more where
+// the contacts go by pairs or walls follow) with no host round trip (see
+// tmps_engine in the header).
 //
 //   A  final half-kick of the previous step, pending remap x, first
 //      half-kick, drift, skin check          (nve_sphere.py:44-96,
@@ -16,10 +17,10 @@
 // Two arithmetic forms share the launch structure:
 //   FP64:  absolute FP64 positions, every operation FP64 (divisions by m and
 //          I become products with 1/m, 1/I computed at each rebuild).
-//   mixed: split positions (FP64 offset from the atom's cell origin at the
-//          last build), FP32 contact arithmetic and FP32 per-atom force
-//          accumulation; FP64 kept for the velocity and position updates, the
-//          per-contact shear history and the virial reduction.
+//   mixed: positions (as offsets from the atom's cell origin at the last
+//          build), velocities, contact histories and virial sums are FP32
+//          double words; contact arithmetic and per-atom force accumulation
+//          FP32; the six virial totals and the servo FP64.
 #include "tmps_contact.cuh"
 #include "tmps_wall.cuh"
 #include "tmps_servo.cuh"
@@ -2782,7 +2783,7 @@ __global__ void __launch_bounds__(kBlockC, MIXED ? 4 : 3)
 
 // S of a batch: one block of six warps per instance (the derived quantities
 // take one warp per kind, the virial sum runs the 24 virtual warps of the
-// single-instance S four at a time), so many instances fit in one wave.
+// single-instance S six at a time), so many instances fit in one wave.
 constexpr int kBlockSB = 192;
 __global__ void __launch_bounds__(kBlockSB) kb_s(const tmps_instance* __restrict__ inst, int32_t* status) {
     const tmps_instance& I = inst[blockIdx.x];
