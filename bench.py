@@ -544,7 +544,8 @@ def contact_bytes(precision: str, n_nb: float, n_c: float) -> float:
 
 # the contact-dense state's two contact kernels, timed together, and what holds them
 PAIR_KERNELS = "k_pair_contacts + k_pair_gather"
-DENSE_BOUND = {"mixed": "instruction issue", "fp64": "fp64 pipe"}
+# (profiles/pair_kernels_dense_ncu.md)
+DENSE_BOUND = {"mixed": "latency of the gathers", "fp64": "fp64 pipe"}
 
 
 def dense_traffic(kernel: str, precision: str):
